@@ -178,6 +178,35 @@ def test_gemm_f32_is_exact_and_batch_invariant(M, N, K):
     assert torch.equal(one[0], out[M - 1])          # a row's bits do not depend on the other rows
 
 
+@pytest.mark.parametrize("M,N,K,pad", [
+    # a warp's rows of W: 8, 16 and 32 features, every share of rows a lane takes, K below and past a stage of 128
+    (1, 8, 4, 0), (4, 4736, 132, 0), (8, 4737, 128, 0), (16, 40, 516, 4), (2, 4800, 100, 0), (3, 4800, 260, 0), (7, 4744, 24, 0), (16, 4800, 392, 0),
+    # tiles of 32 x 32, 32 x 64, 64 x 64 and 64 x 128: one row too many, one column too few, K no multiple of 16
+    (17, 33, 20, 0), (33, 4801, 36, 0), (9, 19000, 16, 0), (100, 11000, 60, 4), (450, 3000, 44, 0), (600, 5001, 28, 0),
+    # rows that do not start on 16 bytes
+    (5, 70, 129, 1), (16, 5000, 63, 0), (17, 65, 33, 0), (129, 3001, 18, 1), (600, 700, 31, 0),
+])
+def test_gemm_f32_same_bits_from_every_kernel(M, N, K, pad):
+    """Every output is the sum over k = 0, 1, 2, ..., so a row has the same bits alone and among others, whatever kernel
+    either takes; and no sum of K float32 FMAs is further than K 2^-24 sum |a w| from the exact one."""
+    from lgml_b200 import ops
+
+    torch.manual_seed(M + N + K)
+    a = torch.randn(M, K + pad)[:, :K].to(DEV) if pad == 0 else torch.randn(M, K + pad).to(DEV)[:, :K]
+    w = torch.randn(N, K + pad).to(DEV)[:, :K]
+    b = torch.randn(N).to(DEV) if M % 2 else None
+    out = torch.full((M, N + 3), 7.0, device=DEV)
+    ops.gemm_f32(a, w, out[:, :N], b)
+    exact = a.double() @ w.double().t() + (b.double() if b is not None else 0.0)
+    bound = (K + 1) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t() + (b.double().abs() if b is not None else 0.0))
+    assert bool(((out[:, :N].double() - exact).abs() <= bound).all())
+    assert bool((out[:, N:] == 7.0).all())
+    for m in {0, M // 2, M - 1}:
+        one = torch.empty(1, N, device=DEV)
+        ops.gemm_f32(a[m:m + 1], w, one, b)
+        assert torch.equal(one[0], out[m, :N])
+
+
 @pytest.mark.parametrize("M,N,K,bias,f32,splits", [
     (1, 128, 64, False, False, None), (8, 331 * 8, 120, True, True, None), (5, 200, 192, True, False, 3),
     (64, 1000, 1096, True, True, 4), (100, 320, 96, False, False, None), (129, 520, 264, True, False, None),
