@@ -37,6 +37,7 @@ LIBRARIES: Dict[str, tuple] = {
     "gemm_f32": ("gemm_f32.cu", []),
     "rope_cache": ("rope_cache.cu", []),
     "attention_ref": ("attention_ref.cu", []),
+    "attention_f32": ("attention_f32.cu", []),
     "sampling": ("sampling.cu", []),
     "attention_decode": ("attention_decode.cu", []),
     "gemm_tcgen05": ("gemm_tcgen05.cu", []),

@@ -106,7 +106,9 @@ class Runtime:
     # ---- attention ---------------------------------------------------------------------
     def attention(self, q, batch, cache, out, n_heads: int, scale: float, window: int, softcap: float = 0.0) -> torch.Tensor:
         """Attention of the step's queries over the cache.  A cap on the scores (``softcap`` > 0)
-        is known to the general kernel only, so it takes that kernel in both compute types."""
+        is known to the 32-bit kernels and the general one only."""
+        if self.dtype == torch.float32 and self.attention_backend != "ref" and ops.attention_f32_supports(q, out, cache.k, n_heads):
+            return ops.paged_attention_f32(q, batch, cache, out, n_heads, scale, window, self.status, softcap=softcap)
         if self.dtype == torch.float32 or self.attention_backend == "ref" or softcap:
             return ops.paged_attention_ref(q, batch.positions, batch.seq_of_token, cache.block_table, cache.k, cache.v,
                                            out, n_heads, scale, window, self.status, softcap=softcap)

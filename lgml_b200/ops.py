@@ -2621,6 +2621,51 @@ def prefill_tc_supports(q: torch.Tensor, out: torch.Tensor) -> bool:
     return q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
 
 
+def attention_f32_supports(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor, n_heads: int) -> bool:
+    """The 32-bit kernels that share keys between rows: float32, head sizes that are multiples of 4 up to 128, rows on 16 bytes.
+    (Nothing here depends on a step's batch: a layer's results all come from one of the two arithmetics.)"""
+    return (q.dtype == torch.float32 and k_pages.dtype == torch.float32 and k_pages.shape[3] % 4 == 0 and k_pages.shape[3] <= 128
+            and n_heads // k_pages.shape[1] <= 64 and q.stride(0) % 4 == 0 and out.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0
+            and out.data_ptr() % 16 == 0)
+
+
+def paged_attention_f32(q: torch.Tensor, batch, cache, out: torch.Tensor, n_heads: int, scale: float, window: int, status: torch.Tensor,
+                        softcap: float = 0.0) -> torch.Tensor:
+    """``paged_attention_ref`` for steps described by ``batch``, where ``attention_f32_supports``: prompts and portions in tiles of 64
+    rows, few tokens with their keys in chunks side by side.  A token's result has the same bits either way.  The line between
+    the two is the bfloat16 path's: at up to eight tokens a request a tile's rows would mostly be padding."""
+    _need(q, "queries", torch.float32, 2)
+    _need(out, "attention output", torch.float32, 2)
+    ldq, ldo = _rows_contiguous(q, "queries"), _rows_contiguous(out, "attention output")
+    k_pages, v_pages, block_table = cache.k, cache.v, cache.block_table
+    n, (n_pages, hkv, page, d) = q.shape[0], k_pages.shape
+    _need(k_pages, "key pages", torch.float32, 4)
+    _need(v_pages, "value pages", torch.float32, 4)
+    _need(batch.positions, "positions", torch.int32, 1)
+    _need(batch.seq_of_token, "request index of tokens", torch.int32, 1)
+    _need(block_table, "block table", torch.int32, 2)
+    if q.shape[1] != n_heads * d or out.shape != (n, n_heads * d) or v_pages.shape != k_pages.shape:
+        raise KernelError(f"paged_attention: q {tuple(q.shape)} / out {tuple(out.shape)} do not fit {n_heads} heads of {d}")
+    if not k_pages.is_contiguous() or not v_pages.is_contiguous() or not block_table.is_contiguous():
+        raise KernelError("paged_attention: pages and block table must be contiguous")
+    tiles, n_chunks, part_o, part_ml = None, 1, None, None
+    if batch.max_q_len > DECODE_MAX_Q:
+        tiles = batch.attention_tiles(64 // (n_heads // hkv))
+    else:
+        n_chunks = -(-batch.max_kv_len // 128)
+        if n_chunks > 1:
+            part_o = torch.empty(n * n_heads * n_chunks * d, dtype=torch.float32, device=q.device)
+            part_ml = torch.empty(n * n_heads * n_chunks * 2, dtype=torch.float32, device=q.device)
+    fn = _fn("attention_f32", "lgml_attention_f32", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,
+                                                     c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_float, c_int, c_void_p,
+                                                     c_void_p, c_void_p, c_void_p])
+    _check("attention_f32", fn(_ptr(q), ldq, _ptr(batch.positions), _ptr(batch.seq_of_token), _ptr(tiles), 0 if tiles is None else tiles.shape[0],
+                               _ptr(block_table), block_table.shape[1], _ptr(k_pages), _ptr(v_pages), n_pages, page, _ptr(out), ldo, n, n_heads, hkv, d,
+                               float(scale), int(window or 0), float(softcap or 0.0), n_chunks, _ptr(part_o), _ptr(part_ml), _ptr(status), _stream()),
+           "paged_attention_f32")
+    return out
+
+
 # which kernel runs prompts and portions: "tcgen05" (default: two tiles per CTA for head sizes 64
 # and 128, one tile otherwise), "single" (one tile per CTA for every head size) or "mma" (the
 # mma.sync kernel)

@@ -523,6 +523,37 @@ def test_attention_ref_kernel(H, G, D, dtype, window):
     assert torch.isfinite(got).all() and torch.allclose(got, want, **tol)
 
 
+@pytest.mark.parametrize("H,G,D", ATT_SHAPES + [(3, 1, 40), (40, 40, 128), (12, 1, 128), (64, 1, 20)])
+@pytest.mark.parametrize("window,softcap", [(0, 0.0), (37, 0.0), (130, 0.0), (0, 5.0)])
+def test_attention_f32_kernels(H, G, D, window, softcap):
+    """The 32-bit kernels against float64 at contexts around a block of 64 and a chunk of 128 keys, and the same bits from both: every
+    request's last token through the chunks' kernel (each context with as many chunks as the longest) and in its portion's tiles."""
+    from types import SimpleNamespace
+
+    from lgml_b200 import ops
+
+    kv, ql = [300, 1, 64, 65, 128, 129, 257], [290, 1, 9, 65, 2, 1, 12]
+    case = make_attention_case(7, H, G, D, kv_lens=kv, q_lens=ql, dtype=torch.float32)
+    scale, st = D ** -0.5, status()
+    q, kp, vp, tab = (case[n].to(DEV) for n in ("q", "k_pages", "v_pages", "table"))
+    cache, b = SimpleNamespace(k=kp, v=vp, block_table=tab), FakeBatch(case)
+    out = torch.full_like(q, float("nan"))
+    assert ops.attention_f32_supports(q, out, kp, H)
+    ops.paged_attention_f32(q, b, cache, out, H, scale, window, st, softcap=softcap)
+    if softcap:
+        ref = torch.empty_like(q)
+        ops.paged_attention_ref(q, b.positions, b.seq_of_token, tab, kp, vp, ref, H, scale, window, st, softcap=softcap)
+        want = ref.double().cpu()
+    else:
+        want = ref_attention(case, scale, window)
+    assert torch.isfinite(out).all() and torch.allclose(out.double().cpu(), want, atol=2e-5, rtol=1e-4)
+    ends = torch.tensor(ql).cumsum(0) - 1
+    few = SimpleNamespace(positions=b.positions[ends].contiguous(), seq_of_token=b.seq_of_token[ends].contiguous(), max_q_len=1, max_kv_len=max(kv))
+    one = torch.full_like(q[ends], float("nan"))
+    ops.paged_attention_f32(q[ends].contiguous(), few, cache, one, H, scale, window, st, softcap=softcap)
+    assert int(st.item()) == 0 and torch.equal(one, out[ends])
+
+
 @pytest.mark.parametrize("H,G,D", ATT_SHAPES + [(16, 1, 32), (4, 2, 256)])
 @pytest.mark.parametrize("window,n_splits", [(0, 1), (0, 5), (100, 3), (0, 8), (0, 11), (100, 9)])
 def test_attention_decode_kernel(H, G, D, window, n_splits):
