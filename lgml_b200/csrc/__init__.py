@@ -47,6 +47,7 @@ LIBRARIES: Dict[str, tuple] = {
     "attention_decode_noalloc": ("attention_decode_noalloc.cu", []),
     "attention_sink": ("attention_sink.cu", []),
     "delta_rule": ("delta_rule.cu", []),
+    "delta_block": ("delta_block.cu", []),
     "attention_heads": ("attention_heads.cu", []),
     "moe": ("moe.cu", []),
     "token_mix": ("token_mix.cu", []),

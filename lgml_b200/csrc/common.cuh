@@ -93,7 +93,21 @@ static inline cudaError_t lgml_launch(void (*kernel)(KArgs...), dim3 grid, dim3 
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
-// The same with a thread-block cluster of `cluster` CTAs along x (1: no cluster).
+// A launch without that attribute: the kernel's blocks start when the kernel ahead is done.  For kernels of about one block an
+// SM whose time is an SM's own work (a recurrence, products on CUDA cores): blocks that start while the kernel ahead still
+// holds a part of the SMs are placed two and three on the others and stay there.  (The scan of delta_block.cu over 512 tokens,
+// 128 blocks: 145 us behind its preparation with the attribute, 74 without; 208 tiles of 64 x 64 of gemm_f32.cu: 518 and 355.)
+template <typename... KArgs, typename... Args>
+static inline cudaError_t lgml_launch_alone(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+// lgml_launch with a thread-block cluster of `cluster` CTAs along x (1: no cluster).
 template <typename... KArgs, typename... Args>
 static inline cudaError_t lgml_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
                                               Args &&...args) {

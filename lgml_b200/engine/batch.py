@@ -238,16 +238,18 @@ class StepBatch:
         key = ("chunks", chunk_tokens, longer_than)
         cached = self._tiles.get(key)
         if cached is None:
-            rows, first, reqs, start = [], [0], [], 0
-            for s, n in enumerate(self.seq_lens):
-                if n > longer_than:
-                    rows += [(start + t0, start + min(t0 + chunk_tokens, n)) for t0 in range(0, n, chunk_tokens)]
-                    first.append(len(rows))
-                    reqs.append(s)
-                start += n
-            flat = self._to_device(np.concatenate([np.asarray(rows, dtype=np.int32).reshape(-1), np.asarray(first, dtype=np.int32), np.asarray(reqs, dtype=np.int32)]))
-            a, b = 2 * len(rows), 2 * len(rows) + len(first)
-            cached = self._tiles[key] = ScanChunks(flat[:a].view(-1, 2), flat[a:b], flat[b:], longer_than, len(reqs) < len(self.seq_lens))
+            lens = np.asarray(self.seq_lens, dtype=np.int64)
+            reqs = np.nonzero(lens > longer_than)[0]
+            start = (np.cumsum(lens) - lens)[reqs]
+            end = start + lens[reqs]
+            counts = -(-lens[reqs] // chunk_tokens)
+            first = np.concatenate([[0], np.cumsum(counts)])
+            of = np.repeat(np.arange(len(reqs)), counts)                             # the long request of every chunk
+            lo = start[of] + (np.arange(first[-1]) - first[of]) * chunk_tokens
+            rows = np.stack([lo, np.minimum(lo + chunk_tokens, end[of])], axis=1)
+            flat = self._to_device(np.concatenate([rows.reshape(-1), first, reqs]).astype(np.int32))
+            a, b = rows.size, rows.size + first.size
+            cached = self._tiles[key] = ScanChunks(flat[:a].view(-1, 2), flat[a:b], flat[b:], longer_than, len(reqs) < len(lens))
         return cached
 
     @staticmethod

@@ -2153,14 +2153,19 @@ def delta_prepare(proj: torch.Tensor, a_pre: torch.Tensor, conv_w: torch.Tensor,
     return out_c, gb
 
 
+# tokens of a block of the delta rule with a decay per channel, and the portion length from which its blocks are worth their preparation
+DELTA_BLOCK, DELTA_BLOCK_FROM = 8, 16
+
+
 def delta_scan(qkv_c: torch.Tensor, gb: torch.Tensor, state: torch.Tensor, seq_start: torch.Tensor, slots: torch.Tensor,
-               n_heads: int, n_kv_heads: int, dim: int, vdim: int, chunks=None) -> torch.Tensor:
+               n_heads: int, n_kv_heads: int, dim: int, vdim: int, chunks=None, blocks=None) -> torch.Tensor:
     """The recurrence S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q over each request's
     tokens in order, from and into its slot of ``state`` (S of head h at floats [h D Dv, (h + 1) D Dv)).
     ``qkv_c`` [tokens, q | k | v] and ``gb`` [tokens, H, D + 4] (per head the decays, then beta) as
     ``delta_prepare`` returns them, or [tokens, H, 4] (one decay per head, beta, its logarithm, zero) as ``delta_head_prepare`` does.
     Returns o float32 [tokens, H Dv].  ``chunks`` (one decay per head) as for ``chunk_scan``: the requests with many tokens take
-    that form (where the sizes allow), the others the sequential one."""
+    that form (where the sizes allow), the others the sequential one.  ``blocks`` (a decay per channel; chunks of ``DELTA_BLOCK`` tokens):
+    the same for eight tokens at a time, whose sums come in another order than the sequential form's."""
     n = qkv_c.shape[0]
     head_decay = gb.dim() == 3 and gb.shape[2] == 4
     _need(qkv_c, "prepared q, k, v", torch.float32, 2)
@@ -2181,6 +2186,18 @@ def delta_scan(qkv_c: torch.Tensor, gb: torch.Tensor, state: torch.Tensor, seq_s
             if not chunks.short:
                 return o
             max_tokens = chunks.longer_than
+    elif blocks is not None and not head_decay and n and dim % 4 == 0 and dim <= 128 and n_heads * vdim % 4 == 0 \
+            and qkv_c.data_ptr() % 16 == 0 and gb.data_ptr() % 16 == 0:
+        n_blocks = blocks.rows.shape[0]
+        records = torch.empty(n_blocks * n_heads * (25 * dim + 136), dtype=torch.float32, device=qkv_c.device)
+        block_fn = _fn("delta_block", "lgml_delta_block_scan", [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p,
+                                                                c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
+        _check("delta_block", block_fn(_ptr(qkv_c), _ptr(gb), _ptr(state), state.stride(0), _ptr(blocks.rows), n_blocks, _ptr(blocks.first),
+                                       _ptr(blocks.requests), blocks.requests.numel(), _ptr(slots), _ptr(records), _ptr(o), n_heads, n_kv_heads, dim, vdim,
+                                       _stream()), "delta_scan")
+        if not blocks.short:
+            return o
+        max_tokens = blocks.longer_than
     _check("delta_rule", fn(_ptr(qkv_c), _ptr(gb), _ptr(state), state.stride(0), _ptr(seq_start), _ptr(slots), _ptr(o),
                             slots.numel(), n_heads, n_kv_heads, dim, vdim, 1 if head_decay else 0, max_tokens, _stream()), "delta_scan")
     return o

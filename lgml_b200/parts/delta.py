@@ -77,7 +77,11 @@ class ChannelDelta(Part):
         g_pre = rt.linear(low[:, self.rank_a:], self.w_g2, out_dtype=torch.float32)
         qkv_c, gb = ops.delta_prepare(proj, a_pre, self.conv_w, cache.state, self.state_floats, batch.seq_of_token,
                                       batch.seq_start, batch.slots, self.a_log, self.dt_bias, H, G, D, Dv)
-        o = ops.delta_scan(qkv_c, gb, cache.state, batch.seq_start, batch.slots, H, G, D, Dv)
+        # (the 32-bit path keeps the token-by-token form: there a portion's results have the same bits however it is cut)
+        blocks = None
+        if rt.dtype == torch.bfloat16 and batch.max_q_len >= ops.DELTA_BLOCK_FROM:
+            blocks = batch.scan_chunks(ops.DELTA_BLOCK, ops.DELTA_BLOCK_FROM - 1)
+        o = ops.delta_scan(qkv_c, gb, cache.state, batch.seq_start, batch.slots, H, G, D, Dv, blocks=blocks)
         y = ops.delta_output(o, self.norm_w, g_pre, self.eps, rt.dtype, H)
         return rt.linear(y, self.wo, partials_ok=True)
 

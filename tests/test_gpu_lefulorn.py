@@ -197,6 +197,60 @@ def test_sink_share_temperature_mixing_and_gate():
     assert float((got_split - want).abs().max()) < 3e-2
 
 
+@pytest.mark.parametrize("D,Dv,Hh,G", [(12, 20, 3, 1), (64, 16, 2, 2), (68, 17, 4, 2), (128, 64, 2, 1)])
+@pytest.mark.parametrize("spread", [0.2, 8.0])
+def test_delta_scan_in_blocks_is_as_exact_as_token_by_token(D, Dv, Hh, G, spread):
+    """Requests of 16, 41, 5 and 64 tokens, those over 15 in blocks of eight, with decays from about one (rand^0.2) or of all sizes with
+    exact zeros among them (rand^8) and keys that resemble each other: the read-outs and the states are as near the float64 recurrence as
+    the sequential form's are (both are float32 sums, whose order differs: at most three times as far, and that within 1e-5)."""
+    from types import SimpleNamespace
+
+    from lgml_b200 import ops
+
+    torch.manual_seed(int(D + 10 * spread))
+    lens, slot_of = [16, 41, 5, 64], [3, 0, 4, 1]
+    n, C = sum(lens), 2 * G * D + Hh * Dv
+    unit = lambda t: torch.nn.functional.normalize(t, dim=-1)
+    q, k = unit(torch.randn(n, G, D)) * D ** -0.5, unit(torch.randn(n, G, D) + 2.0 * torch.randn(G, D))
+    v, beta, decay = torch.randn(n, Hh, Dv), torch.rand(n, Hh), torch.rand(n, Hh, D) ** spread
+    decay[7:9], decay[20:30, :, ::3] = 0.0, 1.0
+    qkv = torch.cat([q.reshape(n, -1), k.reshape(n, -1), v.reshape(n, -1)], 1)
+    gb = torch.cat([decay, beta[:, :, None], torch.zeros(n, Hh, 3)], 2)
+    start = torch.randn(6, Hh * D * Dv + 4)
+    ends = torch.tensor(lens).cumsum(0)
+    seq_start = torch.cat([torch.zeros(1, dtype=torch.int64), ends]).int().to(DEV)
+    slots = torch.tensor(slot_of, dtype=torch.int32, device=DEV)
+    rows, first, long = [], [0], [s for s, m in enumerate(lens) if m > 15]
+    for s in long:
+        t0, t1 = int(ends[s]) - lens[s], int(ends[s])
+        rows += [(t, min(t + 8, t1)) for t in range(t0, t1, 8)]
+        first.append(len(rows))
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    blocks = SimpleNamespace(rows=i32(rows), first=i32(first), requests=i32(long), longer_than=15, short=True)
+
+    def run(blocks):
+        state = start.to(DEV)
+        o = ops.delta_scan(qkv.to(DEV), gb.to(DEV), state, seq_start, slots, Hh, G, D, Dv, blocks=blocks)
+        return o.cpu().double(), state.cpu().double()
+
+    exact_o, exact_s = torch.zeros(n, Hh, Dv, dtype=F64), start.double()
+    for s, m in enumerate(lens):
+        for h in range(Hh):
+            S = start[slot_of[s], h * D * Dv:(h + 1) * D * Dv].double().view(D, Dv)
+            for t in range(int(ends[s]) - m, int(ends[s])):
+                S = decay[t, h].double()[:, None] * S
+                u = beta[t, h].double() * (v[t, h].double() - S.T @ k[t, h // (Hh // G)].double())
+                S = S + torch.outer(k[t, h // (Hh // G)].double(), u)
+                exact_o[t, h] = S.T @ q[t, h // (Hh // G)].double()
+            exact_s[slot_of[s], h * D * Dv:(h + 1) * D * Dv] = S.reshape(-1)
+    (o_b, s_b), (o_t, s_t) = run(blocks), run(None)
+    off = lambda x, y: float((x - y).norm() / y.norm())
+    for got, plain, exact in ((o_b, o_t, exact_o.view(n, -1)), (s_b, s_t, exact_s)):
+        assert off(got, exact) < min(1e-5, 3.0 * off(plain, exact) + 1e-7), (off(got, exact), off(plain, exact))
+        print("off", off(got, exact), off(plain, exact))
+    assert torch.equal(o_b[int(ends[1]):int(ends[2])], o_t[int(ends[1]):int(ends[2])])      # the short one takes the sequential form
+
+
 @pytest.mark.parametrize("D,Dv,Hh,G", [(12, 20, 3, 1), (40, 12, 2, 2), (128, 64, 2, 1), (200, 130, 1, 1)])
 def test_delta_scan_in_pieces_matches_the_plain_recurrence(D, Dv, Hh, G):
     """Two requests of unequal length in one launch, then the same tokens in pieces of 1, 2, 9, ...
