@@ -206,28 +206,44 @@ class CacheManager:
                 t[slot].zero_()
         self.live[rid] = req
         if self.prefix_cache and tokens:
-            for pages in self._cached_prefix(tokens):
-                for gi, page in enumerate(pages):
-                    self.groups[gi].pool.share(page)
-                    req.tables[gi].append(page)
-                req.n_tokens += self.page_size
+            found = self._cached_prefix(tokens)
+            for gi, grp in enumerate(self.groups):
+                pages = [p[gi] for p in found]
+                for page in pages:
+                    grp.pool.share(page)
+                req.tables[gi] += pages
+            req.n_tokens += len(found) * self.page_size
         return req
 
     # ---- prefix cache ------------------------------------------------------------------
     def _keys(self, tokens: Sequence[int], n_blocks: int):
         """The keys of the first ``n_blocks`` full pages of ``tokens``: each hashes the key
         before it and its own tokens, so a key stands for the whole prefix."""
+        # (eight pages' tokens are packed at a time: a prompt of thousands of tokens costs more in packing than in hashing)
         key = b"lgml_b200 page %d" % self.page_size
-        for b in range(n_blocks):
-            block = tokens[b * self.page_size:(b + 1) * self.page_size]
-            key = hashlib.sha256(key + struct.pack(f"<{self.page_size}q", *block)).digest()
-            yield key
+        page, sha256 = self.page_size, hashlib.sha256
+        size = struct.calcsize("<q") * page
+        for b in range(0, n_blocks, 8):
+            part = tokens[b * page:min(b + 8, n_blocks) * page]
+            raw = struct.pack(f"<{len(part)}q", *part)
+            for at in range(0, len(raw), size):
+                key = sha256(key + raw[at:at + size]).digest()
+                yield key
 
     def _cached_prefix(self, tokens: Sequence[int]) -> List[List[int]]:
         """Per leading full page of ``tokens`` that every group still holds under its key: the
         group's pages.  The last token is never part of it."""
         out: List[List[int]] = []
-        for key in self._keys(tokens, (len(tokens) - 1) // self.page_size):
+        keys = self._keys(tokens, (len(tokens) - 1) // self.page_size)
+        if len(self.groups) == 1:
+            lookup = self.groups[0].pool.lookup
+            for key in keys:
+                page = lookup(key)
+                if page is None:
+                    break
+                out.append([page])
+            return out
+        for key in keys:
             pages = [g.pool.lookup(key) for g in self.groups]
             if any(p is None for p in pages):
                 break

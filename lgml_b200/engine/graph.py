@@ -140,9 +140,7 @@ class DecodeGraph:
             self.events[i].synchronize()          # the copy that last used this staging buffer has run
         self.pinned_np[i][:] = b.host
         b.dev.copy_(self.pinned[i], non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record()
-        self.events[i] = ev
+        self.events[i] = ops.record_event(self.events[i])
         if device_tokens is not None:
             b.token_ids[:n].copy_(device_tokens)
             if spare:

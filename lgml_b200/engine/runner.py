@@ -15,6 +15,7 @@ from typing import Hashable, List, Optional, Sequence, Tuple
 import numpy as np
 import torch
 
+from .. import ops
 from ..cache import CacheManager, PoolFull, Request
 from ..models import build_model
 from ..weights import load_tensors, random_tensors
@@ -88,7 +89,6 @@ class ModelRunner:
                     **kw) -> "ModelRunner":
         """Random weights without a folder: drawn on the device, or on the host; either way
         the values of ``write_random_model(folder, cfg, seed)``, bit for bit (one generator)."""
-        from .. import ops
         from ..weights.loader import INT_TABLE, target_dtype
         from ..weights.random_init import random_table, tensor_key
 
@@ -113,8 +113,7 @@ class ModelRunner:
     @staticmethod
     def _mark_busy(stage) -> None:
         """The copies out of this staging buffer queued so far must run before it is written again."""
-        stage[1] = torch.cuda.Event()
-        stage[1].record()
+        stage[1] = ops.record_event(stage[1])
 
     # ---- requests ----------------------------------------------------------------------
     def open(self, rid: Hashable, tokens: Optional[Sequence[int]] = None) -> Request:
@@ -194,7 +193,6 @@ class ModelRunner:
 
     def _graphs_now(self) -> bool:
         """Captured graphs, unless the kernels are being timed one by one (a replay would hide them)."""
-        from .. import ops
         return self.use_graphs and ops.KernelTimes.active is None
 
     def graph_kernels(self, batch_size: int) -> int:
@@ -258,8 +256,7 @@ class ModelRunner:
             if device_tokens is not None:
                 toks = [[int(t)] for t in device_tokens.cpu().tolist()]
             batch = StepBatch(self.cache, reqs, toks, [e[2] for e in entries], self.rt.device, stage[0])
-            stage[1] = torch.cuda.Event()
-            stage[1].record()
+            self._mark_busy(stage)
             self.last_batch = batch
             return self.model.forward(self.rt, batch)
         g = self._graphs.get(key)
@@ -294,8 +291,7 @@ class ModelRunner:
         else:
             toks = [[int(t)] for t in device_tokens.cpu().tolist()]
             batch = StepBatch(self.cache, list(requests), toks, [[0]] * len(requests), self.rt.device, stage[0])
-            stage[1] = torch.cuda.Event()
-            stage[1].record()
+            self._mark_busy(stage)
             self.last_batch = batch
             logits = self.model.forward(self.rt, batch)
         for r in requests:

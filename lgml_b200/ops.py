@@ -50,6 +50,18 @@ def _stream() -> int:
     return _raw_stream(_raw_device())
 
 
+def record_event(event: Optional[torch.cuda.Event]) -> torch.cuda.Event:
+    """Record ``event`` (a new one if None) on the current stream.  (``Event.record()`` without a stream spends several times the
+    call itself on finding the device's index; a step records one after every copy from its staging buffer.)"""
+    event = torch.cuda.Event() if event is None else event
+    if _raw_device is None:
+        event.record()
+        return event
+    stream_id, device, kind = torch._C._cuda_getCurrentStream(_raw_device())
+    event.record(torch.cuda.Stream(stream_id=stream_id, device_index=device, device_type=kind))
+    return event
+
+
 def _need(t: torch.Tensor, what: str, dtype=None, ndim=None) -> None:
     if not t.is_cuda:
         raise KernelError(f"{what} must be on the CUDA device (it is on {t.device}); there is no CPU path")
@@ -2363,6 +2375,13 @@ def _tcgen05_splits(M: int, N: int, K: int) -> int:
     return -(-k_blocks // -(-k_blocks // splits))
 
 
+_GEMM_TCGEN05_ARGS = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p]
+
+
+def _gemm_tcgen05_fn():
+    return _fn("gemm_tcgen05", "lgml_gemm_tcgen05", _GEMM_TCGEN05_ARGS)
+
+
 def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], bias: Optional[torch.Tensor], status: torch.Tensor,
                  n_splits: Optional[int] = None, scratch: Optional[torch.Tensor] = None, swiglu: bool = False,
                  partials_ok: bool = False, checked: bool = False, relu_sq: bool = False):
@@ -2412,9 +2431,7 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], 
         if out.shape != (M, n_out) or out.dtype not in (torch.bfloat16, torch.float32):
             raise KernelError(f"gemm_tcgen05: output {tuple(out.shape)} {out.dtype} does not fit [{M}, {n_out}]")
         y_f32 = 1 if out.dtype == torch.float32 else 0
-    fn = _fn("gemm_tcgen05", "lgml_gemm_tcgen05", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                                                   c_int, c_void_p, c_int, c_int, c_void_p, c_void_p])
-    _check("gemm_tcgen05", fn(_ptr(x), _ptr(w), _ptr(bias), _ptr(None if raw else out), y_f32, M, N, K, ldx, ldw, ldy,
+    _check("gemm_tcgen05", _gemm_tcgen05_fn()(_ptr(x), _ptr(w), _ptr(bias), _ptr(None if raw else out), y_f32, M, N, K, ldx, ldw, ldy,
                               n_splits, _ptr(scratch if n_splits > 1 else None), 1 if swiglu else (2 if relu_sq else 0), 0 if raw else 1, _ptr(status),
                               _stream()), "gemm_tcgen05")
     if raw:
@@ -2438,6 +2455,22 @@ def gemm_bf16(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, bias: Op
     y is bfloat16 or float32.  ``backend``: "tcgen05" is the hand-written tensor-core kernel,
     "cublas" the library product; "auto" takes tcgen05 whenever its operands fit TMA's
     alignment rules.  With ``partials_ok`` the result may be ``Partials``."""
+    if x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and bias is None and status is not None and backend in ("auto", "tcgen05") \
+            and x.dim() == 2 and w.dim() == 2 and x.is_cuda and w.is_cuda:
+        # What nearly every product of a step is.  The same checks and the same launch as below, without their calls: a step of a
+        # few hundred tokens is bound by its launches, and a product's checks in three functions cost more than its launch.
+        (M, K), (N, kw), (ldx, sx), (ldw, sw) = x.shape, w.shape, x.stride(), w.stride()
+        px, pw = x.data_ptr(), w.data_ptr()
+        if K == kw and M and sx == 1 and sw == 1 and ldx >= K and ldw >= K and not (ldx | ldw) & 7 and not (px | pw) & 15 \
+                and (out_dtype is torch.bfloat16 or out_dtype is torch.float32):
+            n_splits = max(1, min(tcgen05_splits(M, N, K), -(-K // 64)))
+            raw = partials_ok and n_splits > 1
+            scratch = torch.empty((n_splits, M, N), dtype=torch.float32, device=x.device) if n_splits > 1 else None
+            out = None if raw else torch.empty((M, N), dtype=out_dtype, device=x.device)
+            _check("gemm_tcgen05", _gemm_tcgen05_fn()(px, pw, 0, 0 if raw else out.data_ptr(), 0 if raw or out_dtype is torch.bfloat16 else 1, M, N, K, ldx, ldw,
+                                                      N, n_splits, 0 if scratch is None else scratch.data_ptr(), 0, 0 if raw else 1, status.data_ptr(),
+                                                      _stream()), "gemm_tcgen05")
+            return Partials(scratch, None) if raw else out
     _need(x, "gemm input", torch.bfloat16, 2)
     _need(w, "gemm weight", torch.bfloat16, 2)
     if x.shape[1] != w.shape[1]:
