@@ -305,12 +305,18 @@ struct Call {
     cudaStream_t stream;
 };
 
+// Products of this many multiply-adds a row and more are launched alone: their blocks are few an SM and as long as K, so where
+// they lie decides (four requests at width 2,048: 24 us a product of N or K 2,048 with the attribute, 19 without).  Smaller ones
+// end within a few microseconds, of which an early start is a part.
+bool balanced(const Call &c) { return (long long)c.N * c.K >= 1 << 21; }
+
 template <int F, int MT, bool VEC, typename TO> int launch_rows(const Call &c) {
     static bool done = false;
     auto kernel = gemm_f32_rows_kernel<F, MT, VEC, TO>;
     if (allow_smem(kernel, RowsShape<F, MT>::SMEM, &done)) return -1;
-    lgml_launch(kernel, dim3((unsigned)((c.N + F - 1) / F)), 32, RowsShape<F, MT>::SMEM, c.stream, c.A, c.W, c.bias, (TO *)c.C, c.M, c.N, c.K, c.lda, c.ldw,
-                c.ldc);
+    const dim3 grid((unsigned)((c.N + F - 1) / F));
+    if (balanced(c)) lgml_launch_alone(kernel, grid, 32, RowsShape<F, MT>::SMEM, c.stream, c.A, c.W, c.bias, (TO *)c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc);
+    else lgml_launch(kernel, grid, 32, RowsShape<F, MT>::SMEM, c.stream, c.A, c.W, c.bias, (TO *)c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc);
     return lgml_launch_status("gemm_f32");
 }
 
@@ -322,7 +328,9 @@ template <int BM, int BN, int TM, int TN, typename TO> int launch_tiles(const Ca
     const int tiles_m = (c.M + BM - 1) / BM;
     const long long tiles = (long long)tiles_m * ((c.N + BN - 1) / BN);
     if (tiles > 0x7fffffffLL) LGML_FAIL("gemm_f32: M=%d N=%d make too many tiles", c.M, c.N);
-    lgml_launch(kernel, dim3((unsigned)tiles), S::THREADS, S::SMEM, c.stream, c.A, c.W, c.bias, (TO *)c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc, tiles_m);
+    const dim3 grid((unsigned)tiles);
+    if (balanced(c)) lgml_launch_alone(kernel, grid, S::THREADS, S::SMEM, c.stream, c.A, c.W, c.bias, (TO *)c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc, tiles_m);
+    else lgml_launch(kernel, grid, S::THREADS, S::SMEM, c.stream, c.A, c.W, c.bias, (TO *)c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc, tiles_m);
     return lgml_launch_status("gemm_f32");
 }
 template <typename TO> int launch_ragged(const Call &c) {
