@@ -166,9 +166,8 @@ struct Args {
 // d += parts 1 .. n_parts - 1 of one quad, in order.  The loads of up to eight parts are issued
 // before the first is used: one after the other they would cost a round trip to L2 each, which
 // is most of this kernel's time when a product leaves nine partial sums.
-template <typename TD>
+template <typename TD, int AHEAD = 8>
 __device__ __forceinline__ void add_parts(const TD *dr, int n_parts, long long part_stride, int i, int c1, int vec, float (&d)[PER]) {
-    constexpr int AHEAD = 8;
     for (int p0 = 1; p0 < n_parts; p0 += AHEAD) {
         float e[AHEAD][PER];
 #pragma unroll
@@ -302,6 +301,78 @@ __global__ void __launch_bounds__(MODE == 2 ? GROUP * MAX_CS : GROUP) rmsnorm_ke
     if (CLUSTERED) cg::this_cluster().sync();     // no CTA leaves while another may still read its slice's sum
 }
 
+// Many rows whose slices are one round each: TPS threads (whole warps, as many as a slice of at most 4 TPS elements needs) a
+// slice, SIDE slices side by side, KS of them a thread; FULL: every slice is 4 TPS elements and 16-byte accesses are allowed.  The sums are those of rmsnorm_kernel in the same order (a thread's
+// quad, its warp's tree, the warps of a slice, the slices), so a row has the same bits here and there.
+// Bound by the traffic of x, the delta and the output.  (A block of 128 threads that takes all slices leaves a half of its
+// threads without an element at width 2,048, a quarter at 3,072, and has one quad of each slice in flight a thread.)
+template <typename TD, typename TO, int TPS, int SIDE, int KS, bool FULL>
+__global__ void __launch_bounds__(TPS * SIDE, 65536 / ((FULL ? 48 : 64) * TPS * SIDE)) rmsnorm_slices_kernel(const Args a) {
+    pdl_trigger();
+    pdl_wait();
+    constexpr int W = TPS / 32;
+    __shared__ float red[SIDE * KS][W];
+    const int g = threadIdx.x / TPS, gt = threadIdx.x % TPS, width = a.width;
+    const int r = blockIdx.x, per = FULL ? TPS * PER : (((width + a.cs - 1) / a.cs + 3) & ~3);
+    const size_t src = a.rows ? (size_t)a.rows[r] : (size_t)r;
+    float *xr = a.x + src * width;
+    const TD *dr = a.delta ? reinterpret_cast<const TD *>(a.delta) + src * width : nullptr;
+    const bool vec = FULL || a.vec != 0;
+    auto first = [&](int j) { return (g + j * SIDE) * per + PER * gt; };
+    auto end = [&](int j) { return FULL ? (1 << 30) : min(width, (g + j * SIDE + 1) * per); };
+    float v[KS][PER];
+#pragma unroll
+    for (int j = 0; j < KS; ++j) load_quad(xr, first(j), end(j), vec, v[j]);
+    if (dr) {
+        RawQuad<TD> d0[KS];
+#pragma unroll
+        for (int j = 0; j < KS; ++j) d0[j].load(dr, first(j), end(j), vec);
+#pragma unroll
+        for (int j = 0; j < KS; ++j) {
+            float d[PER];
+            d0[j].get(d);
+            add_parts<TD, 3>(dr, a.n_parts, a.part_stride, first(j), end(j), vec, d);      // (many rows hide what more loads ahead would)
+            if (a.delta_bias) {
+                float bq[PER];
+                load_quad_const(a.delta_bias, first(j), end(j), vec, bq);
+#pragma unroll
+                for (int q = 0; q < PER; ++q) d[q] += bq[q];
+            }
+#pragma unroll
+            for (int q = 0; q < PER; ++q) v[j][q] = fmaf(a.delta_scale, d[q], v[j][q]);
+            if (!a.rows) store_quad(xr, first(j), end(j), vec, v[j]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < KS; ++j) {
+        float ss = 0.f;
+#pragma unroll
+        for (int q = 0; q < PER; ++q) ss = fmaf(v[j][q], v[j][q], ss);
+        ss = warp_sum(ss);
+        if ((gt & 31) == 0) red[g + j * SIDE][gt >> 5] = ss;
+    }
+    __syncthreads();
+    float total = 0.f;
+#pragma unroll
+    for (int k = 0; k < SIDE * KS; ++k) {
+        float slice = 0.f;
+#pragma unroll
+        for (int u = 0; u < W; ++u) slice += red[k][u];
+        total += slice;
+    }
+    const float inv = 1.0f / sqrtf(total / (float)width + a.eps);
+    TO *orow = reinterpret_cast<TO *>(a.out) + (size_t)r * width;
+#pragma unroll
+    for (int j = 0; j < KS; ++j)
+        if (first(j) < end(j)) {
+            float w[PER], y[PER];
+            load_quad_const(a.weight, first(j), end(j), vec, w);
+#pragma unroll
+            for (int q = 0; q < PER; ++q) y[q] = v[j][q] * inv * w[q];
+            store_quad(orow, first(j), end(j), vec, y);
+        }
+}
+
 // Any width: one block per row walks the slices and their rounds, then the row again.
 template <typename TD, typename TO>
 __global__ void __launch_bounds__(GROUP) rmsnorm_any_kernel(const Args a) {
@@ -418,11 +489,29 @@ static int rmsnorm_launch(const rms::Args &a, int n_rows, cudaStream_t stream) {
     } else if (cs == 1 && rounds <= 2) {
         if (rounds == 1) e = lgml_launch(rmsnorm_kernel<TD, TO, 1, 1, 0, false>, n_rows, GROUP, 0, stream, a);
         else e = lgml_launch(rmsnorm_kernel<TD, TO, 2, 1, 0, false>, n_rows, GROUP, 0, stream, a);
-    } else if (cs == MAX_CS && full && rounds == 1) {
+    } else if (cs == MAX_CS && full && rounds == 1 && a.n_parts < 2) {
+        // (width 4,096 with at most one delta: 2,048 rows 17.9 us, 22.2 on slices side by side; with four partial sums 128 rows 6.7 and 3.6)
         e = lgml_launch(rmsnorm_kernel<TD, TO, 1, MAX_CS, 0, true>, n_rows, GROUP, 0, stream, a);
-    } else if (cs > 1 && rounds <= 2) {
-        if (rounds == 1) e = lgml_launch(rmsnorm_kernel<TD, TO, 1, MAX_CS, 0, false>, n_rows, GROUP, 0, stream, a);
-        else e = lgml_launch(rmsnorm_kernel<TD, TO, 2, MAX_CS, 0, false>, n_rows, GROUP, 0, stream, a);
+    } else if (cs > 1 && rounds == 1) {
+        // (bfloat16 delta, 2,048 rows, before and now: width 1,536 21.0 and 8.1 us, 2,048 23.0 and 10.2, 2,784 28.3 and 19, 3,072 24.5 and
+        // 13.2; 512 rows with four partial sums of 2,048: 19.0 and 4.9)
+        const int tps = (per_cta / PER + 31) & ~31;
+#define LGML_SLICES(T, SIDE, KS) \
+    e = full_slices ? lgml_launch(rmsnorm_slices_kernel<TD, TO, T, SIDE, KS, true>, n_rows, T * SIDE, 0, stream, a) \
+                    : lgml_launch(rmsnorm_slices_kernel<TD, TO, T, SIDE, KS, false>, n_rows, T * SIDE, 0, stream, a)
+        const bool full_slices = a.vec && per_cta * cs == a.width && per_cta == tps * PER;
+        if (cs == 4) {
+            if (tps <= 64) LGML_SLICES(64, 2, 2);
+            else if (tps == 96) LGML_SLICES(96, 2, 2);
+            else LGML_SLICES(128, 2, 2);
+        } else {
+            if (tps <= 64) LGML_SLICES(64, 4, 2);
+            else if (tps == 96) LGML_SLICES(96, 4, 2);
+            else LGML_SLICES(128, 4, 2);
+        }
+#undef LGML_SLICES
+    } else if (cs > 1 && rounds == 2) {
+        e = lgml_launch(rmsnorm_kernel<TD, TO, 2, MAX_CS, 0, false>, n_rows, GROUP, 0, stream, a);
     } else {
         e = lgml_launch(rmsnorm_any_kernel<TD, TO>, n_rows, GROUP, 0, stream, a);
     }

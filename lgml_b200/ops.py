@@ -9,6 +9,7 @@ another device is an error.
 from __future__ import annotations
 
 import ctypes
+import math
 import os
 from ctypes import c_double, c_float, c_int, c_longlong, c_ulonglong, c_void_p
 from typing import Optional
@@ -2552,9 +2553,19 @@ def decode_splits(n_tokens: int, n_kv_heads: int, group: int, max_kv_len: int, p
     9.6 with 18; at 8,192 tokens 13.8 us with 16, 15.7 with 37; at 32,768 tokens 38.3 us with 16,
     31.7 with 37; two requests at 2,176 tokens 9.7 us with 9, 11.1 with 16, at 8,192 tokens 18.6 us
     with 16, 21.1 with 9 or 18; eight requests 18.4 us
-    with 4 ranges, 21.8 with 3, 23.4 with 5."""
+    with 4 ranges, 21.8 with 3, 23.4 with 5.
+
+    With more CTAs than the chip holds at once (two an SM) whole ranges leave its last round partly empty: the number of
+    ranges, up to four, whose rounds are fullest, where a range costs about 1.5 % for its CTAs and as much again for every two
+    query heads that share a KV head (the merge).  16 requests at 3,592 tokens, 40 heads on 40: 220 us with 1 range, 204 with 2,
+    199 with 3, 196 with 4, 197 with 5; 64 requests at 1,548, 32 on 8: 73, 85, 88, 88."""
     ctas = max(n_tokens * n_kv_heads * ((group + 7) // 8), 1)
     pages = max(1, -(-max_kv_len // page))
+    if ctas > 2 * sm_count():
+        rounds = ctas / (2.0 * sm_count())
+        empty = lambda s: (math.ceil(rounds * s) - rounds * s) / (rounds * s)       # share of the time's last round that has no CTA
+        cost = lambda s: 0.5 * empty(s) + (0.015 * (s - 1) * (1 + group // 2) + 0.02 if s > 1 else 0.0)
+        return min(range(1, max(1, min(4, pages // 8)) + 1), key=cost)
     per_sm = 1 if ctas <= 16 and pages <= 64 else 2
     return max(1, min(-(-pages // 4), (per_sm * sm_count()) // ctas, max(16, pages // 16), 512))
 

@@ -163,6 +163,33 @@ def test_fill_normal_draws_the_host_generator_bit_for_bit(dtype):
 # matrix products
 # ---------------------------------------------------------------------------------------------
 
+@pytest.mark.parametrize("width", [1024, 1280, 1540, 2048, 2052, 2560, 2789, 3072, 3844, 4096])
+@pytest.mark.parametrize("parts,dtype", [(0, torch.float32), (1, torch.bfloat16), (5, torch.float32)])
+def test_rmsnorm_many_rows_have_the_bits_of_few(width, parts, dtype):
+    """70 rows (slices side by side in a block) against the same rows 7 at a time (groups or a cluster for a row) and against float64; a
+    row list with repeats too."""
+    from lgml_b200 import ops
+
+    torch.manual_seed(width + parts)
+    x, w = torch.randn(70, width, device=DEV), (torch.rand(width) + 0.5).to(DEV)
+    d = None if parts == 0 else torch.randn(parts, 70, width, device=DEV).to(dtype)
+    delta = lambda lo, hi: None if parts == 0 else (d[0, lo:hi].contiguous() if parts == 1 else ops.Partials(d[:, lo:hi].contiguous()))
+    many, xm = torch.empty(70, width, dtype=torch.bfloat16, device=DEV), x.clone()
+    ops.rmsnorm(xm, w, 1e-5, many, delta=delta(0, 70))
+    for lo in range(0, 70, 7):
+        few, xf = torch.empty(7, width, dtype=torch.bfloat16, device=DEV), x[lo:lo + 7].clone()
+        ops.rmsnorm(xf, w, 1e-5, few, delta=delta(lo, lo + 7))
+        assert torch.equal(few, many[lo:lo + 7]) and torch.equal(xf, xm[lo:lo + 7])
+    want = x.double() + (0.0 if parts == 0 else d.double().sum(0))
+    assert torch.allclose(xm.double(), want, rtol=1e-5, atol=1e-5)
+    want = want / torch.sqrt((want * want).mean(-1, keepdim=True) + 1e-5) * w.double()
+    assert torch.allclose(many.double(), want, rtol=2.0 ** -8, atol=1e-5)
+    rows = torch.randint(0, 70, (80,), dtype=torch.int32, device=DEV)
+    picked, xr = torch.empty(80, width, dtype=torch.bfloat16, device=DEV), x.clone()
+    ops.rmsnorm(xr, w, 1e-5, picked, delta=delta(0, 70), rows=rows)
+    assert torch.equal(picked, many[rows.long()]) and torch.equal(xr, x)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 64, 64), (5, 200, 120), (70, 331, 257), (3, 1000, 96)])
 def test_gemm_f32_is_exact_and_batch_invariant(M, N, K):
     from lgml_b200 import ops
