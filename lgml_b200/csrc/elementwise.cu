@@ -304,10 +304,11 @@ __global__ void __launch_bounds__(MODE == 2 ? GROUP * MAX_CS : GROUP) rmsnorm_ke
 // Many rows whose slices are one round each: TPS threads (whole warps, as many as a slice of at most 4 TPS elements needs) a
 // slice, SIDE slices side by side, KS of them a thread; FULL: every slice is 4 TPS elements and 16-byte accesses are allowed.  The sums are those of rmsnorm_kernel in the same order (a thread's
 // quad, its warp's tree, the warps of a slice, the slices), so a row has the same bits here and there.
-// Bound by the traffic of x, the delta and the output.  (A block of 128 threads that takes all slices leaves a half of its
+// Bound by the traffic of x, the delta and the output; 48 registers a thread, since more rows an SM in flight are worth more than
+// what odd widths spill (2,048 rows of 2,784: 20.1 us, 25.4 with 64).  (A block of 128 threads that takes all slices leaves a half of its
 // threads without an element at width 2,048, a quarter at 3,072, and has one quad of each slice in flight a thread.)
 template <typename TD, typename TO, int TPS, int SIDE, int KS, bool FULL>
-__global__ void __launch_bounds__(TPS * SIDE, 65536 / ((FULL ? 48 : 64) * TPS * SIDE)) rmsnorm_slices_kernel(const Args a) {
+__global__ void __launch_bounds__(TPS * SIDE, 65536 / (48 * TPS * SIDE)) rmsnorm_slices_kernel(const Args a) {
     pdl_trigger();
     pdl_wait();
     constexpr int W = TPS / 32;
@@ -493,7 +494,7 @@ static int rmsnorm_launch(const rms::Args &a, int n_rows, cudaStream_t stream) {
         // (width 4,096 with at most one delta: 2,048 rows 17.9 us, 22.2 on slices side by side; with four partial sums 128 rows 6.7 and 3.6)
         e = lgml_launch(rmsnorm_kernel<TD, TO, 1, MAX_CS, 0, true>, n_rows, GROUP, 0, stream, a);
     } else if (cs > 1 && rounds == 1) {
-        // (bfloat16 delta, 2,048 rows, before and now: width 1,536 21.0 and 8.1 us, 2,048 23.0 and 10.2, 2,784 28.3 and 19, 3,072 24.5 and
+        // (bfloat16 delta, 2,048 rows, before and now: width 1,536 21.0 and 8.1 us, 2,048 23.0 and 10.2, 2,784 28.3 and 20.1, 3,072 24.5 and
         // 13.2; 512 rows with four partial sums of 2,048: 19.0 and 4.9)
         const int tps = (per_cta / PER + 31) & ~31;
 #define LGML_SLICES(T, SIDE, KS) \
