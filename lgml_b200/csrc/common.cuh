@@ -69,6 +69,26 @@ __device__ __forceinline__ float2 act_load(const float2 *p) { return __ldcg(p); 
 __device__ __forceinline__ float4 act_load(const float4 *p) { return __ldcg(p); }
 __device__ __forceinline__ uint4 act_load(const uint4 *p) { return __ldcg(p); }
 
+// Loads for before pdl_wait(): of weights, and of what the host sent with the step (positions, block tables).  They stay where they
+// are written; the compiler may move an ordinary load of constant data behind the wait, and with it a trip to HBM onto the chain
+// of a decode step.  The host's data is complete by then: its copy ends before the step's first kernel starts, and no kernel of the
+// step starts before that one has.
+__device__ __forceinline__ float4 early_weights(const float *p) {
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float early_weight(const float *p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ int early_int(const int *p) {
+    int v;
+    asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 static inline bool lgml_pdl_enabled() {
     static int enabled = -1;
     if (enabled < 0) {

@@ -26,14 +26,13 @@ __global__ void __launch_bounds__(ITEMS) rope_kv_write_kernel(
     T *__restrict__ k_pages, T *__restrict__ v_pages, int n_pages, int page_size, int H, int Hkv, int D, int write_kv,
     int *__restrict__ status) {
     pdl_trigger();
-    pdl_wait();
     const int t = blockIdx.x;
     const int half_d = D / 2;
     const int n_heads = write_kv ? H + 2 * Hkv : H;
     const int item = blockIdx.y * ITEMS + threadIdx.x;
     if (item >= n_heads * half_d) return;
     const int head = item / half_d, j = item - head * half_d;
-    const int pos = positions[t];
+    const int pos = early_int(positions + t);
     const int half_rot = n_rot / 2;
 
     // which two dimensions, and whether they turn
@@ -51,18 +50,21 @@ __global__ void __launch_bounds__(ITEMS) rope_kv_write_kernel(
     }
     const size_t col = (size_t)head * D;
     const TS *row = src + (size_t)t * lds + col;
-    // Every load goes out before anything waits for one: the elements and their other parts, the
-    // bias, the frequency, and the chain position -> block -> page for the cell of the cache (two
-    // trips to L2 one after the other, which used to begin only when the rotation was done).
-    float a = to_f32(act_load(row + d0)), b = to_f32(act_load(row + d1));
-    const float bias0 = bias ? bias[col + d0] : 0.f, bias1 = bias ? bias[col + d1] : 0.f;
-    const float f = fi >= 0 ? inv_freq[fi] : 0.f, f_lo = (fi >= 0 && inv_freq_lo) ? inv_freq_lo[fi] : 0.f;
+    // What no kernel of the step writes comes before the wait, with the angle's sine and cosine: the bias, the frequency, and
+    // the chain position -> block -> page for the cell of the cache (two trips to L2 one after the other).
+    const float bias0 = bias ? early_weight(bias + col + d0) : 0.f, bias1 = bias ? early_weight(bias + col + d1) : 0.f;
+    const float f = fi >= 0 ? early_weight(inv_freq + fi) : 0.f, f_lo = (fi >= 0 && inv_freq_lo) ? early_weight(inv_freq_lo + fi) : 0.f;
     int page = -1;      // where this token's k and v go
     if (head >= H) {
-        const int seq = seq_of_token[t];
+        const int seq = early_int(seq_of_token + t);
         const int blk = pos / page_size;
-        if (pos >= 0 && blk < max_blocks) page = block_table[(size_t)seq * max_blocks + blk];
+        if (pos >= 0 && blk < max_blocks) page = early_int(block_table + (size_t)seq * max_blocks + blk);
     }
+    float s = 0.f, c = 1.f;
+    if (fi >= 0) rope_sincos(pos, f, f_lo, &s, &c);
+    pdl_wait();
+    // then every load of the elements and their other parts before anything waits for one
+    float a = to_f32(act_load(row + d0)), b = to_f32(act_load(row + d1));
     // the other parts in order; the loads of up to eight of them are issued before the first is used
     // (one after the other they would cost a round trip to L2 each)
     for (int p0 = 1; p0 < n_parts; p0 += 8) {
@@ -83,8 +85,6 @@ __global__ void __launch_bounds__(ITEMS) rope_kv_write_kernel(
     a += bias0;
     b += bias1;
     if (fi >= 0) {
-        float s, c;
-        rope_sincos(pos, f, f_lo, &s, &c);
         const float r0 = a * c - b * s, r1 = a * s + b * c;
         a = r0;
         b = r1;
