@@ -26,6 +26,7 @@ _STATUS_TEXT = {
 
 
 AHEAD_BYTES = 24 << 20      # weights asked of L2 ahead, per layer (measured best at 24 to 32 MiB)
+AHEAD_MIN_BYTES = 1 << 20   # ... and none for less (a model that small lies in L2 from step to step; asking costs a launch a layer)
 AHEAD_MAX_BATCH = 4         # ... in captured steps of at most this many requests (at 8 the step gets slower)
 MOE_GROUPED_ROWS = 8        # (token, expert) rows of a step from which the experts run as grouped tiles
 MAX_RESULT = 4096     # most sampled rows of a step whose ids travel with the status word
@@ -79,7 +80,7 @@ class Runtime:
         layer's attention runs HBM is mostly idle at small batches, and a product that finds the
         head of its weights in L2 ends that much earlier.  Outside a capture that set ``side``
         this does nothing."""
-        if self.side is None or not self.ahead_bytes:
+        if self.side is None or not self.ahead_bytes or sum(t.numel() * t.element_size() for t in tensors) < AHEAD_MIN_BYTES:
             return
         ev = torch.cuda.Event()
         ev.record(torch.cuda.current_stream())
