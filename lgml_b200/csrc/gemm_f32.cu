@@ -104,12 +104,14 @@ __global__ void __launch_bounds__(32) gemm_f32_rows_kernel(const float *__restri
         cp_async_commit();
         const float *ws = stage(t) + f * ROWS_LD;
         const float *as = stage(t) + (F + m_first) * ROWS_LD;
-#pragma unroll 8
-        for (int k = 0; k < ROWS_BK; k += 4) {
-            const float4 w = *reinterpret_cast<const float4 *>(ws + k);
-            float4 a[MT];
+        // `ahead` times four k at a time, the next ones' reads under way while these ones' chain of FMAs runs (2,048 x 5,632, one to four
+        // rows: 26 to 29 us, 29 to 33 with the reads where they are used; with eight rows a lane the chains alone fill the time)
+        auto read = [&](int k, float4 &w, float4 (&a)[MT]) {
+            w = *reinterpret_cast<const float4 *>(ws + k);
 #pragma unroll
             for (int j = 0; j < MT; ++j) a[j] = *reinterpret_cast<const float4 *>(as + j * ROWS_LD + k);
+        };
+        auto add = [&](const float4 &w, const float4 (&a)[MT]) {
 #pragma unroll
             for (int j = 0; j < MT; ++j) acc[j] = fmaf(a[j].x, w.x, acc[j]);
 #pragma unroll
@@ -118,6 +120,28 @@ __global__ void __launch_bounds__(32) gemm_f32_rows_kernel(const float *__restri
             for (int j = 0; j < MT; ++j) acc[j] = fmaf(a[j].z, w.z, acc[j]);
 #pragma unroll
             for (int j = 0; j < MT; ++j) acc[j] = fmaf(a[j].w, w.w, acc[j]);
+        };
+        if constexpr (MT <= 4) {
+            constexpr int AHEAD = MT <= 2 ? 4 : 2, GROUPS = ROWS_BK / 4 / AHEAD;
+            float4 w[2][AHEAD], a[2][AHEAD][MT];
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) read(u * 4, w[0][u], a[0][u]);
+#pragma unroll
+            for (int g = 0; g < GROUPS; ++g) {
+                if (g + 1 < GROUPS) {
+#pragma unroll
+                    for (int u = 0; u < AHEAD; ++u) read(((g + 1) * AHEAD + u) * 4, w[(g + 1) & 1][u], a[(g + 1) & 1][u]);
+                }
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) add(w[g & 1][u], a[g & 1][u]);
+            }
+        } else {
+#pragma unroll 8
+            for (int k = 0; k < ROWS_BK; k += 4) {
+                float4 w, a[MT];
+                read(k, w, a);
+                add(w, a);
+            }
         }
         __syncwarp();
     }
@@ -340,7 +364,7 @@ template <typename TO> int launch_ragged(const Call &c) {
 }
 
 // Features a warp for M <= 16 rows.  Eight where that is one warp for each of the chip's 592 schedulers or
-// fewer (N 2048, K 2048: 13 us at 4 rows, 15 with sixteen, 21 with thirty-two); more features beside a
+// fewer (N 2048, K 2048: 12.5 us at 4 rows; 15 with sixteen, 21 with thirty-two); more features beside a
 // reading of A as soon as there are warps enough (N 11264, 4 rows: 38, 26 and 29 us; 8 rows: 45, 49 and 36).
 template <bool VEC, typename TO> int run_rows(const Call &c) {
     if (c.N <= 592 * 8) return c.M <= 4 ? launch_rows<8, 1, VEC, TO>(c) : (c.M <= 8 ? launch_rows<8, 2, VEC, TO>(c) : launch_rows<8, 4, VEC, TO>(c));
