@@ -145,6 +145,152 @@ __global__ void __launch_bounds__(NT) sandwich_norm_kernel(const SandwichArgs a)
     }
 }
 
+// The same for rows of whole quads up to 4,096 wide (16-byte aligned): a thread holds the quads tid, tid + 256, ... of its row in
+// registers from the first load to the last store, and every row has 256 threads, so its sums come in one order however many
+// rows the step holds.  Bound by latency for few rows (a chain of up to five reductions over the row; eight warps make each one
+// short) and by traffic for many: x, both deltas and the state are all asked for at once, the weights before the wait.
+// (Before, element by element through shared memory with 1,024 threads for few rows: 13 us a launch in a decode step of width 2,048; two
+// prompts and four steps of two layers 2.89 ms in all, now 2.68.)
+constexpr int QUAD_THREADS = 256, QUAD_TAPS = 4;
+
+__device__ __forceinline__ void take4(float4 q, float (&v)[4]) { v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w; }
+__device__ __forceinline__ void store_quad(float *p, const float (&v)[4]) { *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void store_quad(__nv_bfloat16 *p, const float (&v)[4]) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+    *reinterpret_cast<uint2 *>(p) = make_uint2(*reinterpret_cast<const unsigned *>(&lo), *reinterpret_cast<const unsigned *>(&hi));
+}
+
+// FEW: the weights come before the wait, and a step of one token a request may have its convolution here; many rows do without
+// both and need half the registers.
+template <typename TO, int NQ, bool FEW>
+__global__ void __launch_bounds__(QUAD_THREADS) sandwich_quads_kernel(const SandwichArgs a) {
+    pdl_trigger();
+    __shared__ float2 red[32];
+    const int E = a.E, tid = threadIdx.x, r = blockIdx.x;
+    auto at = [&](int q) { return 4 * (q * QUAD_THREADS + tid); };
+    const bool two = a.d2 != nullptr, has_delta = a.d1 != nullptr;
+    constexpr int NE = FEW ? NQ : 1;
+    float4 wp[NE], wo[NE], u1[NE], u2[NE];
+#pragma unroll
+    for (int q = 0; q < NE; ++q) {
+        if (!FEW || at(q) >= E) continue;
+        if (has_delta && a.w_post) wo[q] = early_weights(a.w_post + at(q));
+        if (a.w_pre) wp[q] = early_weights(a.w_pre + at(q));
+        if (two) u1[q] = early_weights(a.u1 + at(q)), u2[q] = early_weights(a.u2 + at(q));
+    }
+    auto weights = [&](const float4 (&early)[NE], const float *p, int q, float (&c)[4]) {
+        take4(FEW ? early[q % NE] : __ldg(reinterpret_cast<const float4 *>(p + at(q))), c);
+    };
+    pdl_wait();
+    const size_t src = a.rows ? (size_t)a.rows[r] : (size_t)r;
+    float *xr = a.x + src * E;
+    const float invE = 1.0f / (float)E;
+    const int back = FEW && a.conv_w ? a.taps - 1 : 0;
+    float *st = back > 0 ? a.conv_state + (size_t)a.slots[r] * a.conv_state_ld : nullptr;
+    float v[NQ][4], m[NQ][4], p2[NQ][4];
+    float4 old[NE][QUAD_TAPS - 1];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int i = at(q);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[q][e] = m[q][e] = p2[q][e] = 0.f;
+        if (i >= E) continue;
+        take4(act_load(reinterpret_cast<const float4 *>(xr + i)), v[q]);
+        if (has_delta) take4(act_load(reinterpret_cast<const float4 *>(a.d1 + src * E + i)), m[q]);
+        if (two) take4(act_load(reinterpret_cast<const float4 *>(a.d2 + src * E + i)), p2[q]);
+#pragma unroll
+        for (int j = 0; j < QUAD_TAPS - 1; ++j)
+            if (FEW && j < back) old[q % NE][j] = act_load(reinterpret_cast<const float4 *>(st + (size_t)j * E + i));
+    }
+    // mean and 1 / sqrt(var + eps) of the quads y (zeros behind E), the deviations summed in a second walk
+    auto moments = [&](const float (&y)[NQ][4], float &mean, float &inv) {
+        float s = 0.f, d = 0.f;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) s += (y[q][0] + y[q][1]) + (y[q][2] + y[q][3]);
+        mean = block_sum2(s, 0.f, red).x * invE;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+            if (at(q) < E) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) d = fmaf(y[q][e] - mean, y[q][e] - mean, d);
+            }
+        inv = 1.0f / sqrtf(block_sum2(d, 0.f, red).x * invE + a.eps);
+    };
+    if (has_delta) {
+        if (two) {
+            float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s1 = fmaf(m[q][e], m[q][e], s1), s2 = fmaf(p2[q][e], p2[q][e], s2);
+            const float2 ss = block_sum2(s1, s2, red);
+            const float i1 = 0.5f / sqrtf(ss.x * invE + a.eps), i2 = 0.5f / sqrtf(ss.y * invE + a.eps);
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                if (at(q) >= E) continue;
+                float c1[4], c2[4];
+                weights(u1, a.u1, q, c1), weights(u2, a.u2, q, c2);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) m[q][e] = m[q][e] * i1 * c1[e] + p2[q][e] * i2 * c2[e];
+            }
+        }
+        float mean = 0.f, inv = 1.f;
+        if (a.w_post != nullptr) moments(m, mean, inv);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            if (at(q) >= E) continue;
+            float c[4];
+            if (a.w_post != nullptr) weights(wo, a.w_post, q, c);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[q][e] += a.w_post != nullptr ? (m[q][e] - mean) * inv * c[e] : m[q][e];
+        }
+    }
+    const bool changed = has_delta || a.row_add != nullptr;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int i = at(q);
+        if (i >= E) continue;
+        if (a.row_add != nullptr) {
+            float c[4];
+            take4(__ldg(reinterpret_cast<const float4 *>(a.row_add + i)), c);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[q][e] += c[e];
+        }
+        if (changed && a.rows == nullptr) store_quad(xr + i, v[q]);
+    }
+    if (a.w_pre == nullptr) return;
+    float mean, inv;
+    moments(v, mean, inv);
+    TO *orow = reinterpret_cast<TO *>(a.out) + (size_t)r * E;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int i = at(q);
+        if (i >= E) continue;
+        float w[4], h[4];
+        weights(wp, a.w_pre, q, w);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) h[e] = (v[q][e] - mean) * inv * w[e];
+        if (FEW && a.conv_w != nullptr) {
+            // row r is the one token of request r: the same sums in the same order as short_conv's
+            float acc[4] = {0.f, 0.f, 0.f, 0.f}, o[4], c[4];
+#pragma unroll
+            for (int j = 0; j < QUAD_TAPS - 1; ++j) {
+                if (j >= back) continue;
+                take4(old[q % NE][j], o);
+                take4(__ldg(reinterpret_cast<const float4 *>(a.conv_w + (size_t)j * E + i)), c);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[e] = fmaf(c[e], o[e], acc[e]);
+                if (j > 0) store_quad(st + (size_t)(j - 1) * E + i, o);
+            }
+            if (back > 0) store_quad(st + (size_t)(back - 1) * E + i, h);
+            take4(__ldg(reinterpret_cast<const float4 *>(a.conv_w + (size_t)back * E + i)), c);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) h[e] = fmaf(c[e], h[e], acc[e]) + h[e];
+        }
+        store_quad(orow + i, h);
+    }
+}
+
 __device__ __forceinline__ float silu_(float v) { return v / (1.0f + expf(-v)); }
 
 // u float32 [n, ld_in] (C columns used); w float32 [taps, C] (row j weighs the input taps - 1 - j tokens back);
@@ -361,6 +507,19 @@ LGML_API int lgml_sandwich_norm(float *x, const float *d1, const float *d2, cons
                  "sandwich_norm: the convolution in the same kernel needs a norm, all rows, the slots and a state of taps - 1 rows");
     if (n_out == 0) return 0;
     SandwichArgs a{x, d1, d2, u1, u2, w_post, row_add, w_pre, rows, out, E, eps, conv_w, conv_state, conv_state_ld, slots, taps};
+    const uintptr_t ptrs = (uintptr_t)x | (uintptr_t)d1 | (uintptr_t)d2 | (uintptr_t)u1 | (uintptr_t)u2 | (uintptr_t)w_post | (uintptr_t)row_add |
+                           (uintptr_t)w_pre | (uintptr_t)out | (uintptr_t)conv_w | (uintptr_t)conv_state;
+    if (E % 4 == 0 && E <= 16 * QUAD_THREADS && (ptrs & 15) == 0 && (conv_w == nullptr || (taps <= QUAD_TAPS && conv_state_ld % 4 == 0)) &&
+        (out_dtype == LGML_F32 || out_dtype == LGML_BF16)) {
+        const int nq = (E / 4 + QUAD_THREADS - 1) / QUAD_THREADS;
+        const bool few = n_out <= 296 || conv_w != nullptr;
+#define LGML_SQ(TO, NQ) \
+    (few ? lgml_launch(sandwich_quads_kernel<TO, NQ, true>, n_out, QUAD_THREADS, 0, stream, a) : lgml_launch(sandwich_quads_kernel<TO, NQ, false>, n_out, QUAD_THREADS, 0, stream, a))
+        if (out_dtype == LGML_F32) (void)(nq == 1 ? LGML_SQ(float, 1) : nq == 2 ? LGML_SQ(float, 2) : LGML_SQ(float, 4));
+        else (void)(nq == 1 ? LGML_SQ(__nv_bfloat16, 1) : nq == 2 ? LGML_SQ(__nv_bfloat16, 2) : LGML_SQ(__nv_bfloat16, 4));
+#undef LGML_SQ
+        return lgml_launch_status("sandwich_norm");
+    }
     const size_t smem = (size_t)E * sizeof(float);
     // few rows (a decode step): a row's passes are latency, so more threads share it; many rows: blocks of 256 fill the SMs
     const int threads = (n_out <= 296 && E >= 1024) ? 1024 : ROW_THREADS;

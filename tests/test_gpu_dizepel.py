@@ -88,6 +88,38 @@ def test_norm_of_what_is_read_and_of_what_is_added(out_dtype, E):
     assert np.abs(xd.cpu().numpy() - (x + a)).max() < 1e-6
 
 
+@pytest.mark.parametrize("E", [64, 1028, 2048, 4096])
+def test_sandwich_norm_rows_and_its_convolution(E):
+    """300 rows (many) against float64 (numbers up to 16 and about eight roundings of half a millionth each: 1e-5) and, with the same bits,
+    the same rows by threes (few); and the convolution inside the few rows' kernel is short_conv's,
+    bit for bit, with the state it leaves, for one to four taps."""
+    from lgml_b200 import ops
+
+    rng = np.random.default_rng(E)
+    n, eps = 300, 1e-5
+    x, a, b = (f32(rng.normal(size=(n, E))) for _ in range(3))
+    ua, ub, wpost, wpre = (f32(rng.normal(size=E) * 0.3 + 1) for _ in range(4))
+    many, xm = torch.empty((n, E), dtype=torch.float32, device=DEV), x.clone()
+    ops.sandwich_norm(xm, wpre, eps, many, delta=(a, b), units=(ua, ub), w_post=wpost)
+    d = lambda t: t.double().cpu().numpy()
+    want = d(x) + P.layer_norm(0.5 * (P.rms_unit(d(a), eps) * d(ua) + P.rms_unit(d(b), eps) * d(ub)), d(wpost), eps)
+    assert np.abs(d(xm) - want).max() < 1e-5 and np.abs(d(many) - P.layer_norm(want, d(wpre), eps)).max() < 2e-5
+    for lo in (0, 150, 297):
+        few, xf = torch.empty((3, E), dtype=torch.float32, device=DEV), x[lo:lo + 3].clone()
+        ops.sandwich_norm(xf, wpre, eps, few, delta=(a[lo:lo + 3].contiguous(), b[lo:lo + 3].contiguous()), units=(ua, ub), w_post=wpost)
+        assert torch.equal(few, many[lo:lo + 3]) and torch.equal(xf, xm[lo:lo + 3])
+    for taps in (1, 2, 4):
+        w, slots = f32(rng.normal(size=(taps, E))), i32([2, 0, 3])
+        state = f32(rng.normal(size=(4, max(taps - 1, 1) * E)))
+        s1, s2, x1 = state.clone(), state.clone(), x[:3].clone()
+        got, h = torch.empty((3, E), dtype=torch.float32, device=DEV), torch.empty((3, E), dtype=torch.float32, device=DEV)
+        ops.sandwich_norm(x1, wpre, eps, got, delta=a[:3].contiguous(), w_post=wpost, conv=(w, s1 if taps > 1 else None, slots))
+        ops.sandwich_norm(x[:3].clone(), wpre, eps, h, delta=a[:3].contiguous(), w_post=wpost)
+        want = torch.empty((3, E), dtype=torch.float32, device=DEV)
+        ops.short_conv(h, w, None, s2 if taps > 1 else None, i32([0, 1, 2]), i32([0, 1, 2, 3]), slots, want, residual=True)
+        assert torch.equal(got, want) and torch.equal(s1, s2)
+
+
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("taps,C,act,residual", [(1, 20, "none", True), (2, 33, "silu", False), (3, 64, "none", True), (4, 130, "silu", False),
                                                  (5, 8, "none", False), (8, 12, "silu", True)])
