@@ -501,8 +501,9 @@ LGML_API int lgml_rglru_step(const float *proj, int ldp, const float *conv_w, co
     LGML_REQUIRE((n_tokens + NT - 1) / NT <= 65535, "rglru_step: too many tokens");
     if (n_tokens == 0) return 0;
     dim3 grid((P + CH - 1) / CH, C / P, (n_tokens + NT - 1) / NT);
+    // (alone: behind the product ahead its blocks come to lie two an SM, 18.8 us instead of 13.4 for eight requests of 2,048 channels)
 #define RGLRU_STEP(T, TAPS)                                                                                                                        \
-    lgml_launch(rglru_step_kernel<T, T, TAPS>, grid, 256, smem, stream, proj, ldp, conv_w, conv_b, state, state_ld, slots, positions, (const T *)ra, \
+    lgml_launch_alone(rglru_step_kernel<T, T, TAPS>, grid, 256, smem, stream, proj, ldp, conv_w, conv_b, state, state_ld, slots, positions, (const T *)ra, \
                 ra_b, (const T *)ri, ri_b, sp8, (T *)out, n_tokens, C, P, taps, few_rows_lanes<T>(P), few_rows_vec<T>(ra, P) && few_rows_vec<T>(ri, P) ? 1 : 0)
 #define RGLRU_STEP_TAPS(T)                 \
     switch (taps) {                        \
