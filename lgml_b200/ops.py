@@ -2553,21 +2553,29 @@ def decode_splits(n_tokens: int, n_kv_heads: int, group: int, max_kv_len: int, p
     9.6 with 18; at 8,192 tokens 13.8 us with 16, 15.7 with 37; at 32,768 tokens 38.3 us with 16,
     31.7 with 37; two requests at 2,176 tokens 9.7 us with 9, 11.1 with 16, at 8,192 tokens 18.6 us
     with 16, 21.1 with 9 or 18; eight requests 18.4 us
-    with 4 ranges, 21.8 with 3, 23.4 with 5.
-
-    With more CTAs than the chip holds at once (two an SM) whole ranges leave its last round partly empty: the number of
-    ranges, up to four, whose rounds are fullest, where a range costs about 1.5 % for its CTAs and as much again for every two
-    query heads that share a KV head (the merge).  16 requests at 3,592 tokens, 40 heads on 40: 220 us with 1 range, 204 with 2,
-    199 with 3, 196 with 4, 197 with 5; 64 requests at 1,548, 32 on 8: 73, 85, 88, 88."""
+    with 4 ranges, 21.8 with 3, 23.4 with 5."""
     ctas = max(n_tokens * n_kv_heads * ((group + 7) // 8), 1)
     pages = max(1, -(-max_kv_len // page))
-    if ctas > 2 * sm_count():
-        rounds = ctas / (2.0 * sm_count())
-        empty = lambda s: (math.ceil(rounds * s) - rounds * s) / (rounds * s)       # share of the time's last round that has no CTA
-        cost = lambda s: 0.5 * empty(s) + (0.015 * (s - 1) * (1 + group // 2) + 0.02 if s > 1 else 0.0)
-        return min(range(1, max(1, min(4, pages // 8)) + 1), key=cost)
     per_sm = 1 if ctas <= 16 and pages <= 64 else 2
     return max(1, min(-(-pages // 4), (per_sm * sm_count()) // ctas, max(16, pages // 16), 512))
+
+
+def decode_ranges(n_tokens: int, n_kv_heads: int, group: int, max_kv_len: int, page: int = 64) -> int:
+    """``decode_splits``, and more than its one range where many CTAs of whole contexts fill their rounds badly.
+
+    With more CTAs than the chip holds at once (two an SM) whole ranges leave its last round partly empty: where every query head
+    has keys of its own, the number of ranges, up to four, whose rounds are fullest, the merge taken as 2 % and a
+    further range as 1.5 %.  16 requests at 3,592 tokens, 40 heads on 40: 220 us with 1 range, 204 with 2, 199 with 3, 196 with 4, 197 with
+    5.  Heads that share keys keep whole ranges (a CTA's end and the merge cost several times that: 64 requests at 1,548, 32 on 8: 73 us
+    with 1 range, 85 with 2, 88 with 4; 128 at 1,000: 102, 115, 133)."""
+    ctas = n_tokens * n_kv_heads
+    pages = max(1, -(-max_kv_len // page))
+    if ctas > 2 * sm_count() and group == 1:
+        rounds = ctas / (2.0 * sm_count())
+        empty = lambda s: (math.ceil(rounds * s) - rounds * s) / (rounds * s)       # share of the time's last round that has no CTA
+        cost = lambda s: 0.5 * empty(s) + (0.015 * (s - 1) + 0.02 if s > 1 else 0.0)
+        return min(range(1, max(1, min(4, pages // 8)) + 1), key=cost)
+    return decode_splits(n_tokens, n_kv_heads, group, max_kv_len, page)
 
 
 def decode_attention(q: torch.Tensor, positions: torch.Tensor, seq_of_token: torch.Tensor, block_table: torch.Tensor,
@@ -2744,7 +2752,7 @@ def paged_attention(q, batch, cache, out, n_heads: int, scale: float, window: in
     hkv = cache.k.shape[1]
     if cache.k.shape[2] == 64 and d % 16 == 0:
         if batch.max_q_len <= DECODE_MAX_Q:
-            n_splits = batch.decode_splits if getattr(batch, "decode_splits", None) else decode_splits(q.shape[0], hkv, n_heads // hkv, batch.max_kv_len)
+            n_splits = batch.decode_splits if getattr(batch, "decode_splits", None) else decode_ranges(q.shape[0], hkv, n_heads // hkv, batch.max_kv_len)
             return decode_attention(q, batch.positions, batch.seq_of_token, cache.block_table, cache.k, cache.v, out, n_heads, scale,
                                     window, status, n_splits, max_new_tokens=batch.max_q_len)
         if d in (64, 128) and PREFILL_ATTENTION == "tcgen05" and prefill_tc_supports(q, out):
