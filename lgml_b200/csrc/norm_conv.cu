@@ -40,6 +40,7 @@ struct SandwichArgs {
     long long conv_state_ld;
     const int *slots;
     int taps;
+    bool conv_quads = false;        // at most QUAD_TAPS taps, and the state's rows start on 16 bytes
 };
 
 // sum over the block of two numbers at once, fixed order
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(QUAD_THREADS) sandwich_quads_kernel(const Sand
     const size_t src = a.rows ? (size_t)a.rows[r] : (size_t)r;
     float *xr = a.x + src * E;
     const float invE = 1.0f / (float)E;
-    const int back = FEW && a.conv_w ? a.taps - 1 : 0;
+    const int back = FEW && a.conv_w ? a.taps - 1 : 0, back_early = a.conv_quads ? back : 0;
     float *st = back > 0 ? a.conv_state + (size_t)a.slots[r] * a.conv_state_ld : nullptr;
     float v[NQ][4], m[NQ][4], p2[NQ][4];
     float4 old[NE][QUAD_TAPS - 1];
@@ -200,7 +201,7 @@ __global__ void __launch_bounds__(QUAD_THREADS) sandwich_quads_kernel(const Sand
         if (two) take4(act_load(reinterpret_cast<const float4 *>(a.d2 + src * E + i)), p2[q]);
 #pragma unroll
         for (int j = 0; j < QUAD_TAPS - 1; ++j)
-            if (FEW && j < back) old[q % NE][j] = act_load(reinterpret_cast<const float4 *>(st + (size_t)j * E + i));
+            if (FEW && j < back_early) old[q % NE][j] = act_load(reinterpret_cast<const float4 *>(st + (size_t)j * E + i));
     }
     // mean and 1 / sqrt(var + eps) of the quads y (zeros behind E), the deviations summed in a second walk
     auto moments = [&](const float (&y)[NQ][4], float &mean, float &inv) {
@@ -270,7 +271,20 @@ __global__ void __launch_bounds__(QUAD_THREADS) sandwich_quads_kernel(const Sand
         weights(wp, a.w_pre, q, w);
 #pragma unroll
         for (int e = 0; e < 4; ++e) h[e] = (v[q][e] - mean) * inv * w[e];
-        if (FEW && a.conv_w != nullptr) {
+        if (FEW && a.conv_w != nullptr && !a.conv_quads) {
+            // (element by element: which kernel norms a row must not depend on whether its convolution runs here)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float acc = 0.f, o[MAX_TAPS];
+                for (int j = 0; j < back; ++j) o[j] = act_load(st + (size_t)j * E + i + e);
+                for (int j = 0; j < back; ++j) {
+                    acc = fmaf(__ldg(a.conv_w + (size_t)j * E + i + e), o[j], acc);
+                    if (j > 0) st[(size_t)(j - 1) * E + i + e] = o[j];
+                }
+                if (back > 0) st[(size_t)(back - 1) * E + i + e] = h[e];
+                h[e] = fmaf(__ldg(a.conv_w + (size_t)back * E + i + e), h[e], acc) + h[e];
+            }
+        } else if (FEW && a.conv_w != nullptr) {
             // row r is the one token of request r: the same sums in the same order as short_conv's
             float acc[4] = {0.f, 0.f, 0.f, 0.f}, o[4], c[4];
 #pragma unroll
@@ -507,10 +521,10 @@ LGML_API int lgml_sandwich_norm(float *x, const float *d1, const float *d2, cons
                  "sandwich_norm: the convolution in the same kernel needs a norm, all rows, the slots and a state of taps - 1 rows");
     if (n_out == 0) return 0;
     SandwichArgs a{x, d1, d2, u1, u2, w_post, row_add, w_pre, rows, out, E, eps, conv_w, conv_state, conv_state_ld, slots, taps};
+    a.conv_quads = taps <= QUAD_TAPS && conv_state_ld % 4 == 0 && (((uintptr_t)conv_w | (uintptr_t)conv_state) & 15) == 0;
     const uintptr_t ptrs = (uintptr_t)x | (uintptr_t)d1 | (uintptr_t)d2 | (uintptr_t)u1 | (uintptr_t)u2 | (uintptr_t)w_post | (uintptr_t)row_add |
-                           (uintptr_t)w_pre | (uintptr_t)out | (uintptr_t)conv_w | (uintptr_t)conv_state;
-    if (E % 4 == 0 && E <= 16 * QUAD_THREADS && (ptrs & 15) == 0 && (conv_w == nullptr || (taps <= QUAD_TAPS && conv_state_ld % 4 == 0)) &&
-        (out_dtype == LGML_F32 || out_dtype == LGML_BF16)) {
+                           (uintptr_t)w_pre | (uintptr_t)out;
+    if (E % 4 == 0 && E <= 16 * QUAD_THREADS && (ptrs & 15) == 0 && (out_dtype == LGML_F32 || out_dtype == LGML_BF16)) {
         const int nq = (E / 4 + QUAD_THREADS - 1) / QUAD_THREADS;
         const bool few = n_out <= 296 || conv_w != nullptr;
 #define LGML_SQ(TO, NQ) \

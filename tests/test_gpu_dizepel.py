@@ -92,7 +92,7 @@ def test_norm_of_what_is_read_and_of_what_is_added(out_dtype, E):
 def test_sandwich_norm_rows_and_its_convolution(E):
     """300 rows (many) against float64 (numbers up to 16 and about eight roundings of half a millionth each: 1e-5) and, with the same bits,
     the same rows by threes (few); and the convolution inside the few rows' kernel is short_conv's,
-    bit for bit, with the state it leaves, for one to four taps."""
+    bit for bit, with the state it leaves, for one to eight taps and states whose rows start on 16 bytes and elsewhere."""
     from lgml_b200 import ops
 
     rng = np.random.default_rng(E)
@@ -108,10 +108,10 @@ def test_sandwich_norm_rows_and_its_convolution(E):
         few, xf = torch.empty((3, E), dtype=torch.float32, device=DEV), x[lo:lo + 3].clone()
         ops.sandwich_norm(xf, wpre, eps, few, delta=(a[lo:lo + 3].contiguous(), b[lo:lo + 3].contiguous()), units=(ua, ub), w_post=wpost)
         assert torch.equal(few, many[lo:lo + 3]) and torch.equal(xf, xm[lo:lo + 3])
-    for taps in (1, 2, 4):
+    for taps, pad in ((1, 0), (2, 0), (3, 4), (4, 0), (3, 2), (4, 3), (8, 0), (6, 1)):
         w, slots = f32(rng.normal(size=(taps, E))), i32([2, 0, 3])
-        state = f32(rng.normal(size=(4, max(taps - 1, 1) * E)))
-        s1, s2, x1 = state.clone(), state.clone(), x[:3].clone()
+        state = f32(rng.normal(size=(4, max(taps - 1, 1) * E + pad)))
+        s1, s2, x1 = state.clone()[:, pad:], state.clone()[:, pad:], x[:3].clone()
         got, h = torch.empty((3, E), dtype=torch.float32, device=DEV), torch.empty((3, E), dtype=torch.float32, device=DEV)
         ops.sandwich_norm(x1, wpre, eps, got, delta=a[:3].contiguous(), w_post=wpost, conv=(w, s1 if taps > 1 else None, slots))
         ops.sandwich_norm(x[:3].clone(), wpre, eps, h, delta=a[:3].contiguous(), w_post=wpost)
