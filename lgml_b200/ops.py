@@ -2564,16 +2564,16 @@ def decode_ranges(n_tokens: int, n_kv_heads: int, group: int, max_kv_len: int, p
     """``decode_splits``, and more than its one range where many CTAs of whole contexts fill their rounds badly.
 
     With more CTAs than the chip holds at once (two an SM) whole ranges leave its last round partly empty: where every query head
-    has keys of its own, the number of ranges, up to four, whose rounds are fullest, the merge taken as 2 % and a
-    further range as 1.5 %.  16 requests at 3,592 tokens, 40 heads on 40: 220 us with 1 range, 204 with 2, 199 with 3, 196 with 4, 197 with
-    5.  Heads that share keys keep whole ranges (a CTA's end and the merge cost several times that: 64 requests at 1,548, 32 on 8: 73 us
+    has keys of its own, the number of ranges, up to four, whose rounds are fullest: half of what a last round leaves
+    empty is lost, the merge and a second range cost 2.5 % and the time of a page, a further range two thirds of a page's.  16 requests at 3,592 tokens, 40 heads on 40: 220 us with 1 range, 204 with 2, 199 with 3, 196 with 4, 197 with
+    5; 10 at 3,000, 32 on 32: 122, 98, 92, 89; 32 at 1,030, 32 on 32: 98 with 1, 101 with 2, 106 with 3.  Heads that share keys keep whole ranges (a CTA's end and the merge cost several times that: 64 requests at 1,548, 32 on 8: 73 us
     with 1 range, 85 with 2, 88 with 4; 128 at 1,000: 102, 115, 133)."""
     ctas = n_tokens * n_kv_heads
     pages = max(1, -(-max_kv_len // page))
     if ctas > 2 * sm_count() and group == 1:
         rounds = ctas / (2.0 * sm_count())
         empty = lambda s: (math.ceil(rounds * s) - rounds * s) / (rounds * s)       # share of the time's last round that has no CTA
-        cost = lambda s: 0.5 * empty(s) + (0.015 * (s - 1) + 0.02 if s > 1 else 0.0)
+        cost = lambda s: 0.5 * empty(s) + (0.025 + (0.45 + 0.65 * (s - 1)) / pages if s > 1 else 0.0)
         return min(range(1, max(1, min(4, pages // 8)) + 1), key=cost)
     return decode_splits(n_tokens, n_kv_heads, group, max_kv_len, page)
 
