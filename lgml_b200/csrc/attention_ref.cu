@@ -4,7 +4,7 @@
 // One block per (token, head); the result of a (token, head) depends only on that token's
 // position and its request's cells, in a fixed order, so it is the same however the tokens
 // were cut into steps and whatever else is in the batch.  It is the kernel of the 32-bit
-// path and the plain device twin of the faster bfloat16 kernels.
+// path for the head sizes that attention_f32.cu does not take, and the plain device twin of the faster kernels.
 //
 // softmax over keys of (q . k) * scale with keys at positions <= the query's
 // (lua/lgml/transformer.lua:1805-1816, src/lgml.c:2083-2118, mask :2863-2865); head h
