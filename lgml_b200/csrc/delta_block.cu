@@ -208,12 +208,16 @@ __global__ void __launch_bounds__(THREADS) delta_block_scan_kernel(const float *
         const float4 gl = *reinterpret_cast<const float4 *>(vec + 24 * VEC);
 #pragma unroll
         for (int c = 0; c < NC; ++c) S[c][0] = mul2(S[c][0], make_float2(gl.x, gl.y)), S[c][1] = mul2(S[c][1], make_float2(gl.z, gl.w));
-        // forward substitution; each u goes into S as soon as it is known
+        // Forward substitution; each u goes into S as soon as it is known.  A token adds only the u up to its own: those behind
+        // it have factors of zero, but zero times an infinite value is not zero, and a token's result must not depend on later
+        // ones.  Tokens that are not there have u = 0, whatever S holds, for the same reason.
+        const int t = t0 + b * L + i_own;
+        const bool there = t < t_end;
         float w = v - p[0], out = o[0];
 #pragma unroll
         for (int j = 0; j < L; ++j) {
             const float4 ku = *reinterpret_cast<const float4 *>(vec + (2 * L + j) * VEC);
-            const float mine = beta * w;
+            const float mine = there ? beta * w : 0.f;
             float own = 0.f;
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
@@ -223,10 +227,9 @@ __global__ void __launch_bounds__(THREADS) delta_block_scan_kernel(const float *
                 S[c][0] = fma2(make_float2(ku.x, ku.y), uu, S[c][0]), S[c][1] = fma2(make_float2(ku.z, ku.w), uu, S[c][1]);
             }
             w = fmaf(-cc[j], own, w);
-            out = fmaf(dd[j], own, out);
+            out = j <= i_own ? fmaf(dd[j], own, out) : out;
         }
-        const int t = t0 + b * L + i_own;
-        if (has_own && t < t_end) o_out[(size_t)t * H * Dv + (size_t)h * Dv + col0 + c_own] = out;
+        if (has_own && there) o_out[(size_t)t * H * Dv + (size_t)h * Dv + col0 + c_own] = out;
     }
     cp_async_wait<0>();
 #pragma unroll

@@ -251,6 +251,37 @@ def test_delta_scan_in_blocks_is_as_exact_as_token_by_token(D, Dv, Hh, G, spread
     assert torch.equal(o_b[int(ends[1]):int(ends[2])], o_t[int(ends[1]):int(ends[2])])      # the short one takes the sequential form
 
 
+@pytest.mark.parametrize("D,Dv", [(12, 20), (128, 17)])
+def test_delta_scan_in_blocks_keeps_earlier_tokens_clear_of_later_infinities(D, Dv):
+    """An infinite value and a key that is no number inside blocks of eight: finite results and states are those of the token-by-token form,
+    in their places and within the rounding of float32 sums; what comes before such a token in its block stays finite."""
+    from types import SimpleNamespace
+
+    from lgml_b200 import ops
+
+    torch.manual_seed(D)
+    n, Hh, G = 27, 2, 2
+    unit = lambda t: torch.nn.functional.normalize(t, dim=-1)
+    q, k, v = unit(torch.randn(n, G, D)), unit(torch.randn(n, G, D)), torch.randn(n, Hh, Dv)
+    v[5, 0, 3], v[26, 1, 1], k[19, 1, 2] = math.inf, -math.inf, math.nan
+    qkv = torch.cat([q.reshape(n, -1), k.reshape(n, -1), v.reshape(n, -1)], 1).to(DEV)
+    gb = torch.cat([torch.rand(n, Hh, D) * 0.5 + 0.5, torch.rand(n, Hh, 1) * 0.5 + 0.5, torch.zeros(n, Hh, 3)], 2).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    blocks = SimpleNamespace(rows=i32([(t, min(t + 8, n)) for t in range(0, n, 8)]), first=i32([0, 4]), requests=i32([0]), longer_than=15, short=False)
+
+    def run(blocks):
+        state = torch.zeros(1, Hh * D * Dv, device=DEV)
+        o = ops.delta_scan(qkv, gb, state, i32([0, n]), i32([0]), Hh, G, D, Dv, blocks=blocks)
+        return o.cpu().double(), state.cpu().double()
+
+    for got, plain in zip(run(blocks), run(None)):
+        there = torch.isfinite(plain)
+        assert torch.equal(torch.isfinite(got), there)
+        assert torch.allclose(got[there], plain[there], rtol=1e-4, atol=1e-5)
+    o = run(blocks)[0]
+    assert torch.isfinite(o[:5]).all() and not torch.isfinite(o[5]).all() and torch.isfinite(o[5:19, Dv:]).all() and torch.isfinite(o[:26, Dv - 1]).all()
+
+
 @pytest.mark.parametrize("D,Dv,Hh,G", [(12, 20, 3, 1), (40, 12, 2, 2), (128, 64, 2, 1), (200, 130, 1, 1)])
 def test_delta_scan_in_pieces_matches_the_plain_recurrence(D, Dv, Hh, G):
     """Two requests of unequal length in one launch, then the same tokens in pieces of 1, 2, 9, ...
