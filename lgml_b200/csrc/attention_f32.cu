@@ -62,8 +62,10 @@ __device__ __forceinline__ float finish_score(const float (&s)[4], const Args &a
 __device__ __forceinline__ void add_score(float (&s)[4], float4 q, float4 k) {
     s[0] = fmaf(q.x, k.x, s[0]), s[1] = fmaf(q.y, k.y, s[1]), s[2] = fmaf(q.z, k.z, s[2]), s[3] = fmaf(q.w, k.w, s[3]);
 }
-// a key's probability; hidden keys are marked -1 (their values are not touched, whatever they hold)
-__device__ __forceinline__ float prob_of(float s, bool seen, float m) { return seen ? expf(__fsub_rn(s, m)) : -1.f; }
+// A key's probability; hidden keys are marked -1 (their values are not touched, whatever they hold).  While every score of the
+// chunk so far is -inf so is the maximum, and -inf less -inf is no number: such a key's probability is 0, and the chunk is merged
+// as one without visible keys.
+__device__ __forceinline__ float prob_of(float s, bool seen, float m) { return seen ? expf(__fsub_rn(s, m == -INFINITY ? 0.f : m)) : -1.f; }
 __device__ __forceinline__ float shrink(float m_old, float m_new) { return m_old == m_new ? 1.f : expf(__fsub_rn(m_old, m_new)); }
 // merge a chunk's (m, l) into the running (M, L): the factors of what was there and of what comes
 __device__ __forceinline__ bool merge_ml(float &M, float &L, float m, float l, float &f_old, float &f_new) {

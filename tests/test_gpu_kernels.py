@@ -581,6 +581,37 @@ def test_attention_f32_kernels(H, G, D, window, softcap):
     assert int(st.item()) == 0 and torch.equal(one, out[ends])
 
 
+@pytest.mark.parametrize("hidden", [[130], list(range(64, 128)), list(range(128, 200)), list(range(0, 200))])
+def test_attention_f32_of_keys_with_a_score_of_minus_infinity(hidden):
+    """Keys whose score is -inf have no weight, be they all that a block, a chunk or the last chunk shows; without any other key the result
+    is zero.  Both kernels, against a softmax in float64."""
+    from types import SimpleNamespace
+
+    from lgml_b200 import ops
+
+    D, H, n = 64, 2, 200
+    case = make_attention_case(3, H, 1, D, kv_lens=[n], q_lens=[12], dtype=torch.float32)
+    q, kp, tab = case["q"].abs().to(DEV), case["k_pages"].to(DEV), case["table"].to(DEV)
+    k, v = case["ks"][0][:, 0].clone(), case["vs"][0][:, 0]
+    for j in hidden:
+        kp[int(case["table"][0, j // 64]), 0, j % 64, 5] = -math.inf
+        k[j, 5] = -math.inf
+    cache, b, st = SimpleNamespace(k=kp, v=case["v_pages"].to(DEV), block_table=tab), FakeBatch(case), status()
+    out = torch.full_like(q, float("nan"))
+    ops.paged_attention_f32(q, b, cache, out, H, D ** -0.5, 0, st)
+    few = SimpleNamespace(positions=b.positions, seq_of_token=b.seq_of_token, max_q_len=1, max_kv_len=n)
+    one = torch.full_like(q, float("nan"))
+    ops.paged_attention_f32(q, few, cache, one, H, D ** -0.5, 0, st)
+    want = torch.zeros(12, H, D, dtype=torch.float64)
+    for i in range(12):
+        p = n - 12 + i
+        for h in range(H):
+            s = (k[:p + 1] @ q[i, h * D:(h + 1) * D].double().cpu()) * D ** -0.5
+            want[i, h] = torch.softmax(s, 0).nan_to_num() @ v[:p + 1]
+    assert int(st.item()) == 0 and torch.equal(one, out)
+    assert torch.allclose(out.double().cpu(), want.view(12, H * D), atol=2e-5, rtol=1e-4)
+
+
 @pytest.mark.parametrize("H,G,D", ATT_SHAPES + [(16, 1, 32), (4, 2, 256)])
 @pytest.mark.parametrize("window,n_splits", [(0, 1), (0, 5), (100, 3), (0, 8), (0, 11), (100, 9)])
 def test_attention_decode_kernel(H, G, D, window, n_splits):
