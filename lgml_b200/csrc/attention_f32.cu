@@ -18,7 +18,6 @@
 // ran on 64 CTAs whatever their context.  Measured on one B200 in two layers of 16 heads of 128 on 4: a decode step of
 // 4 requests at 1,030 keys 1.0 -> 0.38 ms (attention 0.33 -> 0.02 ms a layer), prompts of 300 and 600 tokens 9.5 -> 7.2 ms.
 #include <math.h>
-#include <mutex>
 
 #include "common.cuh"
 
@@ -436,26 +435,22 @@ __global__ void __launch_bounds__(128) attention_f32_merge_kernel(const Args a, 
         *reinterpret_cast<float4 *>(a.out + (size_t)t * a.ldo + (size_t)h * a.D + d) = make_float4(finish_out(O[0], L), finish_out(O[1], L), finish_out(O[2], L), finish_out(O[3], L));
 }
 
-template <typename Kernel> int allow_smem(Kernel kernel, size_t smem, bool *done) {
-    static std::mutex lock;
-    std::lock_guard<std::mutex> hold(lock);
-    if (*done || smem <= 48 * 1024) return 0;
+// (At every launch: the attribute belongs to the kernel on the current device, and a process may use several.)
+template <typename Kernel> int allow_smem(Kernel kernel, size_t smem) {
+    if (smem <= 48 * 1024) return 0;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) LGML_FAIL("attention_f32: cannot have %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    *done = true;
     return 0;
 }
 
 template <int DP> int run_prompt(const Args &a, int n_tiles, cudaStream_t stream) {
-    static bool done = false;
-    if (allow_smem(attention_f32_prompt_kernel<DP>, Prompt<DP>::SMEM, &done)) return -1;
+    if (allow_smem(attention_f32_prompt_kernel<DP>, Prompt<DP>::SMEM)) return -1;
     lgml_launch_alone(attention_f32_prompt_kernel<DP>, dim3(n_tiles, a.Hkv), PT, Prompt<DP>::SMEM, stream, a);
     return lgml_launch_status("attention_f32 prompt");
 }
 
 template <int DP> int run_decode(const Args &a, int n_tokens, cudaStream_t stream) {
-    static bool done = false;
-    if (allow_smem(attention_f32_decode_kernel<DP>, Decode<DP>::SMEM, &done)) return -1;
+    if (allow_smem(attention_f32_decode_kernel<DP>, Decode<DP>::SMEM)) return -1;
     const int runs = (a.H / a.Hkv + HEADS - 1) / HEADS;
     // (alone: behind the kernel that writes the cells its CTAs came to lie two and three an SM, 28.5 us instead of 22.8)
     lgml_launch_alone(attention_f32_decode_kernel<DP>, dim3(n_tokens, a.Hkv * runs, a.n_chunks), DT, Decode<DP>::SMEM, stream, a, runs);

@@ -15,7 +15,6 @@
 //   M, N, K:  4, 2048, 2048: 156 -> 13;  4, 11264, 2048: 225 -> 26;  4, 32000, 2048: 435 -> 59;
 //   89, 2048, 5632: 423 -> 158;  512, 11264, 2048: 998 -> 554 (43 TFLOP/s);  1500, 32000, 2048: 7927 -> 4388.
 // From registers alone the FMA units give 65 TFLOP/s, plain or packed (fma.rn.f32x2).
-#include <mutex>
 
 #include "common.cuh"
 
@@ -311,14 +310,11 @@ __global__ void __launch_bounds__(256) gemm_f32_ragged_kernel(const float *__res
 }
 
 // ---- host side -----------------------------------------------------------------------------------
-template <typename Kernel> int allow_smem(Kernel kernel, size_t smem, bool *done) {
-    static std::mutex lock;
+// (At every launch: the attribute belongs to the kernel on the current device, and a process may use several.)
+template <typename Kernel> int allow_smem(Kernel kernel, size_t smem) {
     if (smem <= 48 * 1024) return 0;
-    std::lock_guard<std::mutex> hold(lock);
-    if (*done) return 0;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) LGML_FAIL("gemm_f32: cannot have %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    *done = true;
     return 0;
 }
 
@@ -335,9 +331,8 @@ struct Call {
 bool balanced(const Call &c) { return (long long)c.N * c.K >= 1 << 21; }
 
 template <int F, int MT, bool VEC, typename TO> int launch_rows(const Call &c) {
-    static bool done = false;
     auto kernel = gemm_f32_rows_kernel<F, MT, VEC, TO>;
-    if (allow_smem(kernel, RowsShape<F, MT>::SMEM, &done)) return -1;
+    if (allow_smem(kernel, RowsShape<F, MT>::SMEM)) return -1;
     const dim3 grid((unsigned)((c.N + F - 1) / F));
     if (balanced(c)) lgml_launch_alone(kernel, grid, 32, RowsShape<F, MT>::SMEM, c.stream, c.A, c.W, c.bias, (TO *)c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc);
     else lgml_launch(kernel, grid, 32, RowsShape<F, MT>::SMEM, c.stream, c.A, c.W, c.bias, (TO *)c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc);
@@ -346,9 +341,8 @@ template <int F, int MT, bool VEC, typename TO> int launch_rows(const Call &c) {
 
 template <int BM, int BN, int TM, int TN, typename TO> int launch_tiles(const Call &c) {
     using S = TileShape<BM, BN, TM, TN>;
-    static bool done = false;
     auto kernel = gemm_f32_tile_kernel<BM, BN, TM, TN, TO>;
-    if (allow_smem(kernel, S::SMEM, &done)) return -1;
+    if (allow_smem(kernel, S::SMEM)) return -1;
     const int tiles_m = (c.M + BM - 1) / BM;
     const long long tiles = (long long)tiles_m * ((c.N + BN - 1) / BN);
     if (tiles > 0x7fffffffLL) LGML_FAIL("gemm_f32: M=%d N=%d make too many tiles", c.M, c.N);
