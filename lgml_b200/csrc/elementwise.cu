@@ -840,7 +840,7 @@ __device__ __forceinline__ float seeded_normal(uint64_t seed, uint64_t i) {
 
 template <typename T>
 __global__ void fill_normal_kernel(T *__restrict__ out, size_t n, float mean, float sd, uint64_t seed) {
-    pdl_trigger();
+    // (no trigger: what this writes are weights, which the kernels behind may read before their wait)
     pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         out[i] = from_f32<T>(FA(mean, FM(sd, seeded_normal(seed, i))));

@@ -159,6 +159,26 @@ def test_fill_normal_draws_the_host_generator_bit_for_bit(dtype):
                            host.view(torch.int16 if dtype == torch.bfloat16 else torch.int32)), (key, n)
 
 
+def test_weights_filled_just_before_their_product_are_its_operand():
+    """The kernels that read weights before they wait for the kernel ahead, right behind the one that fills them."""
+    from lgml_b200 import ops
+
+    x = torch.randn(3, 320, device=DEV)
+    w, g = torch.empty(4096, 320, device=DEV), torch.empty(4096, device=DEV)
+    for seed in range(20):
+        out, y, rows = torch.empty(3, 4096, device=DEV), torch.empty(3, 4096, device=DEV), torch.randn(3, 4096, device=DEV)
+        torch.cuda.synchronize()
+        ops.fill_normal(w, 0.0, 1.0, seed)
+        ops.gemm_f32(x, w, out)
+        ops.fill_normal(g, 1.0, 0.5, seed)
+        ops.rmsnorm(rows.clone(), g, 1e-5, y)
+        torch.cuda.synchronize()
+        again, z = torch.empty_like(out), torch.empty_like(y)
+        ops.gemm_f32(x, w, again)
+        ops.rmsnorm(rows.clone(), g, 1e-5, z)
+        assert torch.equal(out, again) and torch.equal(y, z)
+
+
 # ---------------------------------------------------------------------------------------------
 # matrix products
 # ---------------------------------------------------------------------------------------------
