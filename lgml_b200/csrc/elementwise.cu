@@ -224,12 +224,16 @@ __global__ void __launch_bounds__(MODE == 2 ? GROUP * MAX_CS : GROUP) rmsnorm_ke
     auto end = [&](int k) { return FULL ? (1 << 30) : (k < n_slices ? min(width, (rank0 + k + 1) * per_cta) : 0); };
     // One slice a thread, which is how few rows run: the weights come while the kernel ahead ends (in a decode step they come
     // from HBM, a trip on the step's chain: with the position chain of rope_cache.cu 12.58 -> 12.07 ms for 17 steps of 16 requests, width 5,120)
-    constexpr bool EARLY = SLICES == 1;
+    // (two rounds in a block of 1,024 threads have no registers to keep them in: there they are only brought into L2)
+    constexpr bool AHEAD = GROUPED && ROUNDS > 1, EARLY = SLICES == 1 && !AHEAD;
     float4 we[EARLY ? ROUNDS : 1];
-    if (EARLY) {
+    if (EARLY || AHEAD) {
 #pragma unroll
-        for (int rd = 0; rd < ROUNDS; ++rd)
-            if (vec && first(0, rd) + PER <= (FULL ? width : end(0))) we[rd] = early_weights(a.weight + first(0, rd));
+        for (int rd = 0; rd < ROUNDS; ++rd) {
+            if (!vec || first(0, rd) + PER > (FULL ? width : end(0))) continue;
+            if (EARLY) we[EARLY ? rd : 0] = early_weights(a.weight + first(0, rd));
+            else if (gt % 8 == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.weight + first(0, rd)));
+        }
     }
     pdl_wait();
     const size_t src = a.rows ? (size_t)a.rows[r] : (size_t)r;
