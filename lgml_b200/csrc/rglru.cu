@@ -501,9 +501,17 @@ LGML_API int lgml_rglru_step(const float *proj, int ldp, const float *conv_w, co
     LGML_REQUIRE((n_tokens + NT - 1) / NT <= 65535, "rglru_step: too many tokens");
     if (n_tokens == 0) return 0;
     dim3 grid((P + CH - 1) / CH, C / P, (n_tokens + NT - 1) / NT);
-    // (alone: behind the product ahead its blocks come to lie two an SM, 18.8 us instead of 13.4 for eight requests of 2,048 channels)
+    // Alone where there is about one block an SM: behind the product ahead the blocks come to lie two and three on some (parts of 256:
+    // 2,048 channels, eight requests, 64 blocks: 13.8 us, alone 11.6; 4,096 channels, 128 blocks: 16.5 and 11.6).  Fewer blocks leave SMs
+    // free whatever is ahead, and more fill all of them anyway; both gain from the early start (1,024 channels in parts of 128, 32
+    // blocks: 6.9 us, alone 7.4; 64 requests of those, 256 blocks: 9.9 and 10.6).
+    const long long blocks = (long long)grid.x * grid.y * grid.z;
+    auto launch = [&](auto kernel, auto... args) {
+        if (blocks > 48 && blocks <= 148) lgml_launch_alone(kernel, grid, 256, smem, stream, args...);
+        else lgml_launch(kernel, grid, 256, smem, stream, args...);
+    };
 #define RGLRU_STEP(T, TAPS)                                                                                                                        \
-    lgml_launch_alone(rglru_step_kernel<T, T, TAPS>, grid, 256, smem, stream, proj, ldp, conv_w, conv_b, state, state_ld, slots, positions, (const T *)ra, \
+    launch(rglru_step_kernel<T, T, TAPS>, proj, ldp, conv_w, conv_b, state, state_ld, slots, positions, (const T *)ra, \
                 ra_b, (const T *)ri, ri_b, sp8, (T *)out, n_tokens, C, P, taps, few_rows_lanes<T>(P), few_rows_vec<T>(ra, P) && few_rows_vec<T>(ri, P) ? 1 : 0)
 #define RGLRU_STEP_TAPS(T)                 \
     switch (taps) {                        \
