@@ -83,6 +83,7 @@ class StepBatch:
         self.kv_lens = [p + n for p, n in zip(self.pos0, lens)]
         self.max_q_len = max(lens) if lens else 0
         self.max_kv_len = max(self.kv_lens) if lens else 0
+        self.min_kv_len = min(self.kv_lens) if lens else 0
         self.decode_splits = None       # a fixed split count (set by a captured graph)
         self.shared = {}                # what one layer of this step keeps for later layers (by name)
         self._tiles = {}

@@ -27,7 +27,7 @@ class DecodeBatch:
     """The batch description of a captured decode step: the same attributes as ``StepBatch``,
     as views of a device buffer that stays put."""
 
-    def __init__(self, cache_manager, S: int, widths: Sequence[int], device, reach: Optional[int] = None):
+    def __init__(self, cache_manager, S: int, widths: Sequence[int], device, reach: Optional[int] = None, even: bool = False):
         cm = self.cache_manager = cache_manager
         self.n_tokens = self.n_seqs = self.n_rows = S
         self.widths = list(widths)
@@ -38,6 +38,7 @@ class DecodeBatch:
         self.max_kv_len = max(self.widths, default=1) * cm.page_size
         if reach:
             self.max_kv_len = min(self.max_kv_len, reach)       # the longest context of the steps this graph replays
+        self.min_kv_len = reach // 2 + 1 if reach and even else 1       # ... and the shortest
         self.decode_splits = None
         self.shared = {}                # what one layer of the step keeps for later layers (by name)
         total = 3 * S + (S + 1) + 4 * S + S * sum(self.widths)
@@ -109,10 +110,10 @@ class DecodeGraph:
 
     RING = 4
 
-    def __init__(self, runner, S: int, reach: Optional[int] = None):
+    def __init__(self, runner, S: int, reach: Optional[int] = None, even: bool = False):
         self.runner = runner
         self.S = S
-        self.batch = DecodeBatch(runner.cache, S, runner._graph_widths, runner.rt.device, reach=reach)
+        self.batch = DecodeBatch(runner.cache, S, runner._graph_widths, runner.rt.device, reach=reach, even=even)
         self.pinned = [torch.empty(self.batch.total, dtype=torch.int32).pin_memory() for _ in range(self.RING)]
         self.pinned_np = [p.numpy() for p in self.pinned]
         self.events: List[Optional[torch.cuda.Event]] = [None] * self.RING

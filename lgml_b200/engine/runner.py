@@ -48,6 +48,14 @@ def prompt_graph_length(n: int, page: int) -> int:
     return -(-n // page) * page
 
 
+def context_reach(lengths: Sequence[int]) -> Tuple[int, bool]:
+    """(The power of two from 1,024 up that covers the longest of a step's contexts, whether all of them are over half of that.)"""
+    reach = 1024
+    while reach < max(lengths):
+        reach *= 2
+    return reach, 2 * min(lengths) > reach
+
+
 class StepError(ValueError):
     """A step the runner refuses before anything is launched."""
 
@@ -198,7 +206,7 @@ class ModelRunner:
     def graph_kernels(self, batch_size: int) -> int:
         """Launches of this package's kernels that one replay of the graph for ``batch_size`` requests holds."""
         size = graph_size(batch_size)
-        return max((g.kernels for (s, _), g in self._graphs.items() if s == size), default=0)
+        return max((g.kernels for (s, *_), g in self._graphs.items() if s == size), default=0)
 
     def _prompt_graph_fits(self, entries) -> bool:
         """A short portion of one request that starts on a page's edge and wants no logits or
@@ -245,11 +253,9 @@ class ModelRunner:
         # A graph fixes into how many key ranges attention cuts a request's context, and that number is
         # chosen for a context length: so a graph per power of two of the longest context in the step
         # (from 1,024 tokens up), or a pool of 128k tokens would cut a 2k context into ranges of a page.
-        longest = max(r.n_tokens for r in reqs) + 1
-        reach = 1024
-        while reach < longest:
-            reach *= 2
-        key = (size, reach)
+        # Heads with keys of their own are also cut by how even the contexts are (ops.decode_ranges): a graph for each of the two.
+        reach, even = context_reach([r.n_tokens + 1 for r in reqs])
+        key = (size, reach, even and self.rt.own_keys and self.rt.dtype == torch.bfloat16)
         if key not in self._graph_seen:
             self._graph_seen.add(key)
             toks = [e[1] for e in entries]
@@ -261,7 +267,7 @@ class ModelRunner:
             return self.model.forward(self.rt, batch)
         g = self._graphs.get(key)
         if g is None:
-            g = self._graphs[key] = DecodeGraph(self, size, reach=reach)
+            g = self._graphs[key] = DecodeGraph(self, *key)
         logits = g.run(reqs, None if device_tokens is not None else [e[1][0] for e in entries], device_tokens)[:n]
         self.last_batch = g.batch
         self.graph_replays += 1

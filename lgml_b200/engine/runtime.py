@@ -56,6 +56,7 @@ class Runtime:
         # None: the compute type.  A model whose sums into the stream read float32 deltas only sets float32.
         self.delta_dtype: Optional[torch.dtype] = None
         self.attention_backend = "auto"
+        self.own_keys = False         # does a layer's every query head have keys of its own?  (the layer says so when it is bound)
         # Asking L2 for weights ahead of their reader: only inside a captured decode step of few
         # requests, which sets ``side`` (a stream beside the step's chain) for the capture.
         self.ahead_bytes = 0 if os.environ.get("LGML_L2_AHEAD") == "0" else AHEAD_BYTES

@@ -105,7 +105,7 @@ def case_decode_attention(a) -> None:
     positions = torch.full((B,), ctx - 1, dtype=torch.int32, device=DEV)
     seq_of = torch.arange(B, dtype=torch.int32, device=DEV)
     tables = [(torch.randperm(per_set) + i * per_set).to(torch.int32).reshape(B, pages_per_seq).to(DEV) for i in range(nb)]
-    n_splits = a.splits if a.splits > 0 else ops.decode_ranges(B, G, H // G, ctx)
+    n_splits = a.splits if a.splits > 0 else ops.decode_ranges(B, G, H // G, D, ctx, ctx)
     scratch = torch.empty(max(B * H * n_splits * (D + 2), 1), dtype=torch.float32, device=DEV)
     us = timed(lambda i: ops.decode_attention(q, positions, seq_of, tables[i], k, v, out, H, D ** -0.5, 0, status, n_splits, scratch),
                nb, a.warmup, a.iters)

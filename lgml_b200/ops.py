@@ -9,7 +9,6 @@ another device is an error.
 from __future__ import annotations
 
 import ctypes
-import math
 import os
 from ctypes import c_double, c_float, c_int, c_longlong, c_ulonglong, c_void_p
 from typing import Optional
@@ -2560,22 +2559,27 @@ def decode_splits(n_tokens: int, n_kv_heads: int, group: int, max_kv_len: int, p
     return max(1, min(-(-pages // 4), (per_sm * sm_count()) // ctas, max(16, pages // 16), 512))
 
 
-def decode_ranges(n_tokens: int, n_kv_heads: int, group: int, max_kv_len: int, page: int = 64) -> int:
-    """``decode_splits``, and more than its one range where many CTAs of whole contexts fill their rounds badly.
+# CTAs of the decode attention kernel that an SM holds (three stages of keys and values, 57 and 106 KB of shared memory)
+DECODE_CTAS_PER_SM = {64: 4, 128: 2}
 
-    With more CTAs than the chip holds at once (two an SM) whole ranges leave its last round partly empty: where every query head
-    has keys of its own, the number of ranges, up to four, whose rounds are fullest: half of what a last round leaves
-    empty is lost, the merge and a second range cost 2.5 % and the time of a page, a further range two thirds of a page's.  16 requests at 3,592 tokens, 40 heads on 40: 220 us with 1 range, 204 with 2, 199 with 3, 196 with 4, 197 with
-    5; 10 at 3,000, 32 on 32: 122, 98, 92, 89; 32 at 1,030, 32 on 32: 98 with 1, 101 with 2, 106 with 3.  Heads that share keys keep whole ranges (a CTA's end and the merge cost several times that: 64 requests at 1,548, 32 on 8: 73 us
-    with 1 range, 85 with 2, 88 with 4; 128 at 1,000: 102, 115, 133)."""
-    ctas = n_tokens * n_kv_heads
-    pages = max(1, -(-max_kv_len // page))
-    if ctas > 2 * sm_count() and group == 1:
-        rounds = ctas / (2.0 * sm_count())
-        empty = lambda s: (math.ceil(rounds * s) - rounds * s) / (rounds * s)       # share of the time's last round that has no CTA
-        cost = lambda s: 0.5 * empty(s) + (0.025 + (0.45 + 0.65 * (s - 1)) / pages if s > 1 else 0.0)
-        return min(range(1, max(1, min(4, pages // 8)) + 1), key=cost)
-    return decode_splits(n_tokens, n_kv_heads, group, max_kv_len, page)
+
+def decode_ranges(n_tokens: int, n_kv_heads: int, group: int, dim: int, shortest: int, longest: int) -> int:
+    """``decode_splits``, and more than its one range where CTAs of whole contexts fill their last round badly.
+
+    ``shortest`` and ``longest`` bound the contexts (or what a window leaves of them).  With a little more CTAs than the chip holds once
+    or twice, whole ranges leave their last round nearly empty; three ranges (two behind a second round) fill it.  Only where every query head
+    has keys of its own, the contexts are of one size and over 1,024 tokens: there it is never slower.  32 heads of 128 on 32, in microseconds at
+    1,025, 2,049 and 4,097 tokens with 1 range and with 3: 10 requests (1.08 rounds) 46, 86, 163 and 40, 67, 121; 12 (1.30) 48, 89, 172 and
+    45, 73, 133; with 1 and 2: 20 (2.16) 71, 130, 251 and 69, 118, 220.  Further on it is not (1.51 rounds: 51, 90, 176 and 52, 86,
+    156; 1.73: 50, 92, 175 and 58, 99, 178; 2.59 with 2: 75, 136, 275 and 80, 141, 278), nor for short contexts (600 tokens, 1.30 rounds:
+    32.5 and 32.4; 70 tokens: 8.5 and 11.7), nor for uneven ones, whose short requests fill the last round by themselves (12 of up
+    to 600: 20 and 22).  Heads that share keys keep whole ranges (64 requests at 1,548, 32 on 8: 73 with 1, 85 with 2)."""
+    full = DECODE_CTAS_PER_SM.get(dim, 0) * sm_count()
+    if group == 1 and full and shortest > 1024 and longest <= 2 * shortest:
+        rounds, rest = divmod(n_tokens * n_kv_heads, full)
+        if (rounds == 1 and 0 < rest <= 0.31 * full) or (rounds == 2 and 0 < rest <= 0.2 * full):
+            return 3 if rounds == 1 else 2
+    return decode_splits(n_tokens, n_kv_heads, group, longest)
 
 
 def decode_attention(q: torch.Tensor, positions: torch.Tensor, seq_of_token: torch.Tensor, block_table: torch.Tensor,
@@ -2752,7 +2756,12 @@ def paged_attention(q, batch, cache, out, n_heads: int, scale: float, window: in
     hkv = cache.k.shape[1]
     if cache.k.shape[2] == 64 and d % 16 == 0:
         if batch.max_q_len <= DECODE_MAX_Q:
-            n_splits = batch.decode_splits if getattr(batch, "decode_splits", None) else decode_ranges(q.shape[0], hkv, n_heads // hkv, batch.max_kv_len)
+            n_splits = getattr(batch, "decode_splits", None)
+            if not n_splits:
+                shortest, longest = getattr(batch, "min_kv_len", 0), batch.max_kv_len
+                if window and n_heads == hkv:       # (the rule for heads with keys of their own goes by what is visible)
+                    shortest, longest = min(shortest, window), min(longest, window)
+                n_splits = decode_ranges(q.shape[0], hkv, n_heads // hkv, d, shortest, longest)
             return decode_attention(q, batch.positions, batch.seq_of_token, cache.block_table, cache.k, cache.v, out, n_heads, scale,
                                     window, status, n_splits, max_new_tokens=batch.max_q_len)
         if d in (64, 128) and PREFILL_ATTENTION == "tcgen05" and prefill_tc_supports(q, out):

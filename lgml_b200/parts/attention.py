@@ -73,6 +73,7 @@ class Attention(Part):
         return specs + self.position.tensor_specs(prefix)
 
     def bind(self, prefix, tensors, rt):
+        rt.own_keys = rt.own_keys or self.n_heads == self.n_kv_heads
         self.wqkv = torch.cat([tensors[prefix + f".{n}_proj.weight"] for n in "qkv"], dim=0).contiguous()
         self.wo = tensors[prefix + ".o_proj.weight"]
         if self.bias:

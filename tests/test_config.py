@@ -142,6 +142,31 @@ def test_key_ranges_of_the_decode_attention_stay_within_their_bounds():
     assert decode_splits(37, 8, 4, 4096) == 1 and decode_splits(1, 8, 4, 4096) == 16 and decode_splits(2, 8, 4, 4096) == 9
 
 
+def test_ranges_of_contexts_that_fill_their_last_round_badly():
+    """More than one range for many CTAs only where all measured contexts gain: heads with keys of their own, even contexts over 1,024
+    tokens, a last round of the chip that is nearly empty.  Everything else is ``decode_splits``."""
+    from lgml_b200.engine.runner import context_reach
+    from lgml_b200.ops import decode_ranges, decode_splits, sm_count
+
+    R = 2 * sm_count()                                              # CTAs of head size 128 that the chip holds at once
+    for ctas, want in ((R, 1), (R + 1, 3), (int(1.3 * R), 3), (int(1.32 * R), 1), (2 * R, 1), (2 * R + 1, 2), (int(2.2 * R), 2), (int(2.3 * R), 1),
+                       (3 * R + 1, 1), (8 * R + 1, 1)):
+        assert decode_ranges(1, ctas, 1, 128, 1025, 2048) == want
+        assert decode_ranges(1, 2 * ctas, 1, 64, 3000, 4096) == want
+        for group, dim, shortest, longest in ((1, 128, 1024, 2048), (1, 128, 70, 1024), (1, 128, 2047, 4096), (1, 128, 1, 4096), (1, 96, 4096, 4096),
+                                              (4, 128, 4096, 4096), (1, 256, 4096, 4096), (1, 128, 512, 512)):
+            assert decode_ranges(1, ctas, group, dim, shortest, longest) == decode_splits(1, ctas, group, longest) == 1
+    for n, g, group in ((1, 8, 4), (4, 8, 1), (8, 32, 1), (2, 5, 9)):
+        assert decode_ranges(n, g, group, 128, 3000, 3000) == decode_splits(n, g, group, 3000)
+    # a captured step is told only what its graph is for: the same answer at both ends of what it replays
+    for lengths, reach, even in (([1], 1024, False), ([513, 1024], 1024, True), ([512, 1024], 1024, False), ([1025], 2048, True),
+                                 ([1025, 2048], 2048, True), ([1024, 1025], 2048, False), ([3585] * 16, 4096, True), ([3585, 20], 4096, False)):
+        assert context_reach(lengths) == (reach, even)
+        if even:
+            answers = {decode_ranges(16, 40, 1, 128, reach // 2 + 1, reach), decode_ranges(16, 40, 1, 128, max(lengths), max(lengths))}
+            assert len(answers) == 1
+
+
 def test_end_tokens_of_generation_config_join_those_of_config(tmp_path):
     import json
 
