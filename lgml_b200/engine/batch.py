@@ -87,6 +87,7 @@ class StepBatch:
         self.decode_splits = None       # a fixed split count (set by a captured graph)
         self.shared = {}                # what one layer of this step keeps for later layers (by name)
         self._tiles = {}
+        self.replayed = False           # are its launches recorded, and run again for other contexts?
         self.after_staged_copy = None   # called after a later copy out of the pinned buffer (its owner marks the buffer busy again)
 
         # Everything below is array arithmetic: a prompt portion brings thousands of tokens, and a

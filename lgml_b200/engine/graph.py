@@ -205,6 +205,7 @@ class PromptGraph:
         batch = StepBatch(self.runner.cache, [req], [list(tokens) + [0] * pad], [list(want)], self.runner.rt.device, pinned,
                           table_widths=self.widths, device_buffer=self.dev)
         batch._tiles = self.tiles
+        batch.replayed = True
         batch.after_staged_copy = None
         if self.graph is None:
             import gc

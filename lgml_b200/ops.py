@@ -2702,11 +2702,24 @@ def attention_f32_supports(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Te
             and out.data_ptr() % 16 == 0)
 
 
+def attention_f32_chunks(n_tokens: int, n_heads: int, n_kv_heads: int, dim: int, max_kv_len: int, window: int) -> tuple:
+    """(Chunks of keys side by side, 0: one after the other; tokens whose chunks' results the scratch holds) for tokens taken each by itself.
+
+    One after the other where there is one chunk, or
+    where the CTAs of whole contexts fill the chip three times an SM and the longest is of up to eight: CTAs of chunks that a short
+    context does not have, the merge and its reading then cost more than what a long context among them takes alone."""
+    chunk = csrc.load("attention_f32").lgml_attention_f32_chunk()
+    n_chunks = max(1, -(-max_kv_len // chunk))
+    runs = -(-(n_heads // n_kv_heads) // 8)
+    if n_chunks == 1 or (n_chunks <= 8 and n_tokens * n_kv_heads * runs >= 3 * sm_count()):
+        return 0, 0
+    return n_chunks, n_tokens
+
+
 def paged_attention_f32(q: torch.Tensor, batch, cache, out: torch.Tensor, n_heads: int, scale: float, window: int, status: torch.Tensor,
                         softcap: float = 0.0) -> torch.Tensor:
     """``paged_attention_ref`` for steps described by ``batch``, where ``attention_f32_supports``: prompts and portions in tiles of 64
-    rows, few tokens with their keys in chunks side by side.  A token's result has the same bits either way.  The line between
-    the two is the bfloat16 path's: at up to eight tokens a request a tile's rows would mostly be padding."""
+    rows, few tokens each by itself.  A token's result has the same bits either way."""
     _need(q, "queries", torch.float32, 2)
     _need(out, "attention output", torch.float32, 2)
     ldq, ldo = _rows_contiguous(q, "queries"), _rows_contiguous(out, "attention output")
@@ -2721,21 +2734,22 @@ def paged_attention_f32(q: torch.Tensor, batch, cache, out: torch.Tensor, n_head
         raise KernelError(f"paged_attention: q {tuple(q.shape)} / out {tuple(out.shape)} do not fit {n_heads} heads of {d}")
     if not k_pages.is_contiguous() or not v_pages.is_contiguous() or not block_table.is_contiguous():
         raise KernelError("paged_attention: pages and block table must be contiguous")
-    tiles, n_chunks, part_o, part_ml = None, 1, None, None
+    tiles, few, n_few, few_kv = None, None, n, batch.max_kv_len
     if batch.max_q_len > DECODE_MAX_Q:
-        tiles = batch.attention_tiles(64 // (n_heads // hkv))
-    else:
-        n_chunks = -(-batch.max_kv_len // 128)
-        if n_chunks > 1:
-            part_o = torch.empty(n * n_heads * n_chunks * d, dtype=torch.float32, device=q.device)
-            part_ml = torch.empty(n * n_heads * n_chunks * 2, dtype=torch.float32, device=q.device)
-    fn = _fn("attention_f32", "lgml_attention_f32", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,
-                                                     c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_float, c_int, c_void_p,
-                                                     c_void_p, c_void_p, c_void_p])
+        tiles, n_few = batch.attention_tiles(64 // (n_heads // hkv)), 0
+    n_chunks, slots, part_o, part_ml = 0, 0, None, None
+    if n_few and not getattr(batch, "replayed", False):     # (a recorded portion meets contexts of any length: one chunk after the other)
+        n_chunks, slots = attention_f32_chunks(n_few, n_heads, hkv, d, few_kv, int(window or 0))
+    if n_chunks:
+        part_o = torch.empty(slots * n_heads * n_chunks * d, dtype=torch.float32, device=q.device)
+        part_ml = torch.empty(slots * n_heads * n_chunks * 2, dtype=torch.float32, device=q.device)
+    fn = _fn("attention_f32", "lgml_attention_f32", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p,
+                                                     c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_float, c_int, c_int,
+                                                     c_void_p, c_void_p, c_void_p, c_void_p])
     _check("attention_f32", fn(_ptr(q), ldq, _ptr(batch.positions), _ptr(batch.seq_of_token), _ptr(tiles), 0 if tiles is None else tiles.shape[0],
-                               _ptr(block_table), block_table.shape[1], _ptr(k_pages), _ptr(v_pages), n_pages, page, _ptr(out), ldo, n, n_heads, hkv, d,
-                               float(scale), int(window or 0), float(softcap or 0.0), n_chunks, _ptr(part_o), _ptr(part_ml), _ptr(status), _stream()),
-           "paged_attention_f32")
+                               _ptr(few), n_few, _ptr(block_table), block_table.shape[1], _ptr(k_pages), _ptr(v_pages), n_pages, page, _ptr(out), ldo,
+                               n_heads, hkv, d, float(scale), int(window or 0), float(softcap or 0.0), n_chunks, slots, _ptr(part_o), _ptr(part_ml),
+                               _ptr(status), _stream()), "paged_attention_f32")
     return out
 
 

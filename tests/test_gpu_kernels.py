@@ -232,6 +232,9 @@ def test_gemm_f32_is_exact_and_batch_invariant(M, N, K):
     (17, 33, 20, 0), (33, 4801, 36, 0), (9, 19000, 16, 0), (100, 11000, 60, 4), (450, 3000, 44, 0), (600, 5001, 28, 0),
     # rows that do not start on 16 bytes
     (5, 70, 129, 1), (16, 5000, 63, 0), (17, 65, 33, 0), (129, 3001, 18, 1), (600, 700, 31, 0),
+    (4, 900, 31, 0), (8, 4739, 65, 0), (16, 40, 259, 0), (9, 9001, 257, 0), (12, 9500, 513, 0), (3, 19000, 65, 0), (7, 19000, 65, 0),
+    # up to 16 rows of a short K
+    (5, 130, 36, 0), (16, 4800, 60, 4), (8, 19000, 32, 0), (2, 66, 8, 0),
 ])
 def test_gemm_f32_same_bits_from_every_kernel(M, N, K, pad):
     """Every output is the sum over k = 0, 1, 2, ..., so a row has the same bits alone and among others, whatever kernel
@@ -467,11 +470,10 @@ def test_rope_angles_at_far_positions(lens):
 # attention
 # ---------------------------------------------------------------------------------------------
 
-def make_attention_case(seed, H, G, D, kv_lens, q_lens, dtype, n_pages=40, aim=True):
+def make_attention_case(seed, H, G, D, kv_lens, q_lens, dtype, n_pages=40, aim=True, page=64):
     """Requests with kv_lens cached tokens of which the last q_lens are this step's queries.
     Pages are shuffled; every cell no request owns holds NaN."""
     g = torch.Generator().manual_seed(seed)
-    page = 64
     perm = torch.randperm(n_pages, generator=g).tolist()
     k_pages = torch.full((n_pages, G, page, D), float("nan"))
     v_pages = torch.full((n_pages, G, page, D), float("nan"))
@@ -599,6 +601,37 @@ def test_attention_f32_kernels(H, G, D, window, softcap):
     one = torch.full_like(q[ends], float("nan"))
     ops.paged_attention_f32(q[ends].contiguous(), few, cache, one, H, scale, window, st, softcap=softcap)
     assert int(st.item()) == 0 and torch.equal(one, out[ends])
+
+
+@pytest.mark.parametrize("H,G,D,page", [(2, 2, 128, 64), (4, 2, 64, 64), (3, 1, 128, 48), (4, 1, 20, 64), (5, 1, 64, 128), (8, 1, 128, 64), (9, 1, 128, 64),
+                                        (24, 2, 64, 32), (64, 1, 16, 64)])
+@pytest.mark.parametrize("window", [0, 1, 100, 129, 300])
+def test_attention_f32_ways_of_one_token(H, G, D, page, window):
+    """A token's chunks one after the other, side by side and a tile of rows: the same
+    bits, and float64's result; contexts and windows that begin and end at, before and behind a block's and a chunk's edges."""
+    from types import SimpleNamespace
+
+    from lgml_b200 import ops
+
+    kv = [1, 63, 64, 65, 127, 128, 129, 192, 256, 257, 300, 641]
+    ql = [1, 2, 1, 3, 1, 2, 8, 1, 1, 3, 8, 2]
+    case = make_attention_case(11, H, G, D, kv_lens=kv, q_lens=ql, dtype=torch.float32, n_pages=100, page=page)
+    scale, st, b = D ** -0.5, status(), FakeBatch(case)
+    q, kp, vp, tab = (case[n].to(DEV) for n in ("q", "k_pages", "v_pages", "table"))
+    cache = SimpleNamespace(k=kp, v=vp, block_table=tab)
+    few = lambda **kw: SimpleNamespace(positions=b.positions, seq_of_token=b.seq_of_token, max_q_len=1, max_kv_len=max(kv), **kw)
+
+    def run(batch):
+        out = torch.full_like(q, float("nan"))
+        ops.paged_attention_f32(q, batch, cache, out, H, scale, window, st)
+        return out
+
+    whole = run(few(replayed=True))
+    assert torch.allclose(whole.double().cpu(), ref_attention(case, scale, window), atol=2e-5, rtol=1e-4)
+    side = run(few())
+    b.max_q_len = 9
+    tiles = run(b)
+    assert int(st.item()) == 0 and torch.equal(whole, side) and torch.equal(whole, tiles)
 
 
 @pytest.mark.parametrize("hidden", [[130], list(range(64, 128)), list(range(128, 200)), list(range(0, 200))])

@@ -33,8 +33,8 @@ def gemm(lib, p):
 
 def attention(lib, p):
     f = ctypes.c_float
-    for n_tiles, n_chunks in ((3, 1), (0, 4)):
-        yield lib.lgml_attention_f32(p, 2048, p, p, p, n_tiles, p, 9, p, p, 90, 64, p, 2048, 3, 16, 4, 128, f(0.1), 0, f(0.0), n_chunks, p, p, p, p)
+    for n_tiles, n_chunks in ((3, 0), (0, 4)):
+        yield lib.lgml_attention_f32(p, 2048, p, p, p, n_tiles, p, 9, p, 9, p, p, 90, 64, p, 2048, 16, 4, 128, f(0.1), 0, f(0.0), n_chunks, 9, p, p, p, p)
 
 
 @pytest.mark.parametrize("name,calls", [("gemm_f32", gemm), ("attention_f32", attention)])
