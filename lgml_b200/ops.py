@@ -2702,18 +2702,23 @@ def attention_f32_supports(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Te
             and out.data_ptr() % 16 == 0)
 
 
+ATTENTION_F32_SCRATCH = 64 << 20        # most bytes of chunks' results between the two kernels; more tokens take their turn
+
+
 def attention_f32_chunks(n_tokens: int, n_heads: int, n_kv_heads: int, dim: int, max_kv_len: int, window: int) -> tuple:
     """(Chunks of keys side by side, 0: one after the other; tokens whose chunks' results the scratch holds) for tokens taken each by itself.
 
-    One after the other where there is one chunk, or
+    A window is touched by as many chunks as fit it and one more, wherever it starts.  One after the other where there is one chunk, or
     where the CTAs of whole contexts fill the chip three times an SM and the longest is of up to eight: CTAs of chunks that a short
     context does not have, the merge and its reading then cost more than what a long context among them takes alone."""
     chunk = csrc.load("attention_f32").lgml_attention_f32_chunk()
     n_chunks = max(1, -(-max_kv_len // chunk))
+    if window:
+        n_chunks = min(n_chunks, (window + chunk - 2) // chunk + 1)
     runs = -(-(n_heads // n_kv_heads) // 8)
     if n_chunks == 1 or (n_chunks <= 8 and n_tokens * n_kv_heads * runs >= 3 * sm_count()):
         return 0, 0
-    return n_chunks, n_tokens
+    return n_chunks, max(1, min(n_tokens, ATTENTION_F32_SCRATCH // (4 * n_heads * n_chunks * (dim + 2))))
 
 
 def paged_attention_f32(q: torch.Tensor, batch, cache, out: torch.Tensor, n_heads: int, scale: float, window: int, status: torch.Tensor,

@@ -167,6 +167,22 @@ def test_ranges_of_contexts_that_fill_their_last_round_badly():
             assert len(answers) == 1
 
 
+def test_chunks_and_scratch_of_tokens_taken_by_themselves():
+    """float32 attention: a window is given the chunks it can touch wherever it starts, not its context's, and the scratch has a bound
+    whatever the batch and the context."""
+    from lgml_b200 import ops
+
+    for window in (1, 2, 100, 127, 128, 129, 256, 257, 4096):
+        touched = max((start + window - 1) // 128 - start // 128 + 1 for start in range(256))
+        assert ops.attention_f32_chunks(1, 8, 8, 64, 1 << 20, window)[0] == (0 if touched == 1 else touched)
+    assert ops.attention_f32_chunks(1, 8, 8, 64, 300, 1000)[0] == 3 and ops.attention_f32_chunks(1, 8, 8, 64, 128, 0) == (0, 0)
+    assert ops.attention_f32_chunks(64, 8, 8, 64, 1024, 0) == (0, 0) and ops.attention_f32_chunks(64, 8, 8, 64, 1025, 0)[0] == 9
+    for n, heads, kv, dim, ctx in ((32, 32, 8, 128, 32768), (2048, 40, 40, 128, 131072), (8, 64, 1, 16, 4096)):
+        chunks, tokens = ops.attention_f32_chunks(n, heads, kv, dim, ctx, 0)
+        floats = tokens * heads * chunks * (dim + 2)
+        assert chunks == -(-ctx // 128) and 1 <= tokens <= n and (4 * floats <= ops.ATTENTION_F32_SCRATCH or tokens == 1)
+
+
 def test_end_tokens_of_generation_config_join_those_of_config(tmp_path):
     import json
 

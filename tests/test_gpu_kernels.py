@@ -606,8 +606,8 @@ def test_attention_f32_kernels(H, G, D, window, softcap):
 @pytest.mark.parametrize("H,G,D,page", [(2, 2, 128, 64), (4, 2, 64, 64), (3, 1, 128, 48), (4, 1, 20, 64), (5, 1, 64, 128), (8, 1, 128, 64), (9, 1, 128, 64),
                                         (24, 2, 64, 32), (64, 1, 16, 64)])
 @pytest.mark.parametrize("window", [0, 1, 100, 129, 300])
-def test_attention_f32_ways_of_one_token(H, G, D, page, window):
-    """A token's chunks one after the other, side by side and a tile of rows: the same
+def test_attention_f32_ways_of_one_token(H, G, D, page, window, monkeypatch):
+    """A token's chunks one after the other, side by side (with scratch for all tokens and for two at a time) and a tile of rows: the same
     bits, and float64's result; contexts and windows that begin and end at, before and behind a block's and a chunk's edges."""
     from types import SimpleNamespace
 
@@ -628,10 +628,13 @@ def test_attention_f32_ways_of_one_token(H, G, D, page, window):
 
     whole = run(few(replayed=True))
     assert torch.allclose(whole.double().cpu(), ref_attention(case, scale, window), atol=2e-5, rtol=1e-4)
+    assert ops.attention_f32_chunks(len(q), H, G, D, max(kv), window)[0] == {0: 6, 1: 0, 100: 2, 129: 2, 300: 4}[window]
     side = run(few())
+    monkeypatch.setattr(ops, "ATTENTION_F32_SCRATCH", 2 * 4 * H * 6 * (D + 2))
+    two = run(few())
     b.max_q_len = 9
     tiles = run(b)
-    assert int(st.item()) == 0 and torch.equal(whole, side) and torch.equal(whole, tiles)
+    assert int(st.item()) == 0 and torch.equal(whole, side) and torch.equal(whole, two) and torch.equal(whole, tiles)
 
 
 @pytest.mark.parametrize("hidden", [[130], list(range(64, 128)), list(range(128, 200)), list(range(0, 200))])
