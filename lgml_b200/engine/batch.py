@@ -172,16 +172,20 @@ class StepBatch:
         self.logit_rows = r[: len(rows)]
         self.block_tables = [take(S * w).view(S, w) for w in self.table_width]
 
-    def attention_tiles(self, tile_tokens: int) -> torch.Tensor:
+    def attention_tiles(self, tile_tokens: int, longer_than: int = 0) -> torch.Tensor:
         """The new tokens cut into tiles of at most ``tile_tokens`` consecutive tokens of one
         request, for the prefill attention kernel: int32 [n_tiles, 4] on the device, rows
         (request row, first token row, tokens, 0), the tile with the most keys to visit first:
         the kernel starts its CTAs in this order, and a long tile that starts last would run on
-        alone at the end.  Made once per tile size."""
-        cached = self._tiles.get(tile_tokens)
+        alone at the end.  Only of requests that bring more than ``longer_than`` tokens.  Made once per tile size."""
+        key = (tile_tokens, longer_than) if longer_than else tile_tokens
+        cached = self._tiles.get(key)
         if cached is None:
             pieces, start = [], 0
             for s, n in enumerate(self.seq_lens):
+                if n <= longer_than:
+                    start += n
+                    continue
                 t0 = np.arange(0, n, tile_tokens, dtype=np.int32)
                 part = np.empty((t0.size, 4), dtype=np.int32)
                 part[:, 0] = s
@@ -194,7 +198,25 @@ class StepBatch:
             arr = arr[np.argsort(-arr[:, 3], kind="stable")]
             arr[:, 3] = 0
             cached = self._to_device(arr.reshape(-1)).view(-1, 4)
-            self._tiles[tile_tokens] = cached
+            self._tiles[key] = cached
+        return cached
+
+    def tiles_and_short(self, tile_tokens: int, limit, rule):
+        """The step's requests in two: (tiles as ``attention_tiles`` of those that bring more than ``limit(seq_lens)`` tokens, the rows of the
+        others' tokens, int32 on the device, the longest context among the others).  No tiles: None, and no rows either, they are all.  No
+        others: None.  Made once per tile size and ``rule``, which stands for ``limit``."""
+        key = ("short", tile_tokens, rule)
+        cached = self._tiles.get(key)
+        if cached is None:
+            up_to = limit(self.seq_lens)
+            lens = np.asarray(self.seq_lens, dtype=np.int64)
+            rows = np.nonzero(np.repeat(lens <= up_to, lens))[0]
+            longest = max((k for k, n in zip(self.kv_lens, self.seq_lens) if n <= up_to), default=0)
+            if rows.size == self.n_tokens:
+                cached = (None, None, longest)
+            else:
+                cached = (self.attention_tiles(tile_tokens, up_to if rows.size else 0), self._to_device(rows.astype(np.int32)) if rows.size else None, longest)
+            self._tiles[key] = cached
         return cached
 
     def _to_device(self, arr: np.ndarray) -> torch.Tensor:

@@ -8,6 +8,7 @@ another device is an error.
 """
 from __future__ import annotations
 
+import collections
 import ctypes
 import os
 from ctypes import c_double, c_float, c_int, c_longlong, c_ulonglong, c_void_p
@@ -2705,6 +2706,28 @@ def attention_f32_supports(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Te
 ATTENTION_F32_SCRATCH = 64 << 20        # most bytes of chunks' results between the two kernels; more tokens take their turn
 
 
+def attention_f32_short(seq_lens, n_heads: int, n_kv_heads: int, dim: int) -> int:
+    """Most new tokens of a request that are taken each by itself, in a step whose requests bring ``seq_lens``.
+
+    A tile takes an SM 11.2 us a block of 64 keys (head sizes up to 64: 7.8) however many of its rows are there, a token's CTA 1.3 us of
+    the SM for one head, 1.5, 1.9 and 2.9 for two, four and eight (0.65 to 1.6), three and more side by side.  So a token by itself where its
+    request's CTAs are less work than its tiles (40 heads on 40: 16 requests of 9 tokens 0.9 of the tiles' time, of 12 1.2), and, from the
+    shortest request on, as long as all of those CTAs take less than one tile does, which is what the few tiles wait for (one
+    request, 16 heads on 4: 9 tokens 0.4 of the tiles' time at their own context and 0.06 at 4,090, 96 tokens 0.5; 40 on 40: 32
+    tokens at 4,090 1.0, 64 1.95)."""
+    runs = -(-(n_heads // n_kv_heads) // 8)
+    heads = -(-(n_heads // n_kv_heads) // runs)
+    size = 0 if heads == 1 else 1 if heads == 2 else 2 if heads <= 4 else 3
+    tile, token = (11.2, (1.3, 1.5, 1.9, 2.9)[size] * runs) if dim > 64 else (7.8, (0.65, 0.75, 1.0, 1.6)[size] * runs)
+    short, tokens = max(1, round(tile / token)), 0
+    for length, count in sorted(collections.Counter(seq_lens).items()):
+        tokens += length * count
+        if tokens * n_kv_heads * token > sm_count() * tile:
+            break
+        short = max(short, length)
+    return short
+
+
 def attention_f32_chunks(n_tokens: int, n_heads: int, n_kv_heads: int, dim: int, max_kv_len: int, window: int) -> tuple:
     """(Chunks of keys side by side, 0: one after the other; tokens whose chunks' results the scratch holds) for tokens taken each by itself.
 
@@ -2723,8 +2746,8 @@ def attention_f32_chunks(n_tokens: int, n_heads: int, n_kv_heads: int, dim: int,
 
 def paged_attention_f32(q: torch.Tensor, batch, cache, out: torch.Tensor, n_heads: int, scale: float, window: int, status: torch.Tensor,
                         softcap: float = 0.0) -> torch.Tensor:
-    """``paged_attention_ref`` for steps described by ``batch``, where ``attention_f32_supports``: prompts and portions in tiles of 64
-    rows, few tokens each by itself.  A token's result has the same bits either way."""
+    """``paged_attention_ref`` for steps described by ``batch``, where ``attention_f32_supports``: the tokens of requests that bring many in
+    tiles of 64 rows, the others each by itself.  A token's result has the same bits either way."""
     _need(q, "queries", torch.float32, 2)
     _need(out, "attention output", torch.float32, 2)
     ldq, ldo = _rows_contiguous(q, "queries"), _rows_contiguous(out, "attention output")
@@ -2739,9 +2762,13 @@ def paged_attention_f32(q: torch.Tensor, batch, cache, out: torch.Tensor, n_head
         raise KernelError(f"paged_attention: q {tuple(q.shape)} / out {tuple(out.shape)} do not fit {n_heads} heads of {d}")
     if not k_pages.is_contiguous() or not v_pages.is_contiguous() or not block_table.is_contiguous():
         raise KernelError("paged_attention: pages and block table must be contiguous")
-    tiles, few, n_few, few_kv = None, None, n, batch.max_kv_len
-    if batch.max_q_len > DECODE_MAX_Q:
-        tiles, n_few = batch.attention_tiles(64 // (n_heads // hkv)), 0
+    tile_tokens, tiles, few, n_few, few_kv = 64 // (n_heads // hkv), None, None, n, batch.max_kv_len
+    if batch.max_q_len > 1:
+        if hasattr(batch, "tiles_and_short"):
+            tiles, few, few_kv = batch.tiles_and_short(tile_tokens, lambda lens: attention_f32_short(lens, n_heads, hkv, d), (n_heads, hkv, d))
+            n_few = n if tiles is None else 0 if few is None else few.numel()
+        elif batch.max_q_len > DECODE_MAX_Q:                # (a description of a step that does not tell its requests apart)
+            tiles, n_few = batch.attention_tiles(tile_tokens), 0
     n_chunks, slots, part_o, part_ml = 0, 0, None, None
     if n_few and not getattr(batch, "replayed", False):     # (a recorded portion meets contexts of any length: one chunk after the other)
         n_chunks, slots = attention_f32_chunks(n_few, n_heads, hkv, d, few_kv, int(window or 0))

@@ -183,6 +183,37 @@ def test_chunks_and_scratch_of_tokens_taken_by_themselves():
         assert chunks == -(-ctx // 128) and 1 <= tokens <= n and (4 * floats <= ops.ATTENTION_F32_SCRATCH or tokens == 1)
 
 
+def test_requests_taken_token_by_token_and_as_tiles():
+    """float32 attention: which requests of a step go token by token (those whose tokens are less work than their tiles, and the shortest as
+    long as all of them take less than one tile), and the two lists of a step that holds both kinds."""
+    from types import SimpleNamespace
+
+    import numpy as np
+    import torch
+
+    from lgml_b200 import ops
+    from lgml_b200.engine.batch import StepBatch
+
+    short = lambda lens, *shape: ops.attention_f32_short(lens, *shape)
+    assert short([9], 16, 4, 128) == 9 and short([96], 16, 4, 128) == 96 and short([300], 16, 4, 128) < 300
+    assert short([9] * 16, 40, 40, 128) == 9 and short([12] * 16, 40, 40, 128) == 9 and short([1] * 500 + [40], 40, 40, 128) == 9 and short([1, 1, 30], 8, 8, 64) == 30
+    for shape in ((8, 8, 64), (40, 40, 128), (64, 1, 128), (24, 8, 128)):
+        assert short([1] * 4096, *shape) >= 1 and short([2048], *shape) < 64
+
+    lens, pos0 = [1, 70, 2, 1, 9], [40, 0, 7, 500, 3]
+    reqs = [SimpleNamespace(id=i, slot=i, n_tokens=p, tables=[]) for i, p in enumerate(pos0)]
+    manager = SimpleNamespace(groups=[])
+    batch = StepBatch(manager, reqs, [[0] * n for n in lens], [[] for _ in lens], torch.device("cpu"))
+    tiles, few, longest = batch.tiles_and_short(16, lambda got: 2 if got == lens else None, "a")
+    assert few.tolist() == [0, 71, 72, 73] and longest == 501
+    rows = sorted((t, n, s) for s, t, n, _ in tiles.tolist())
+    assert rows == [(1, 16, 1), (17, 16, 1), (33, 16, 1), (49, 16, 1), (65, 6, 1), (74, 9, 4)]
+    assert batch.tiles_and_short(16, None, "a")[0] is tiles                     # made once
+    assert batch.tiles_and_short(16, lambda _: 70, "b") == (None, None, 501)
+    tiles, few, longest = batch.tiles_and_short(16, lambda _: 0, "c")
+    assert few is None and longest == 0 and np.array_equal(tiles.numpy(), batch.attention_tiles(16).numpy())
+
+
 def test_end_tokens_of_generation_config_join_those_of_config(tmp_path):
     import json
 
