@@ -59,6 +59,7 @@ class ScanChunks:
     requests: torch.Tensor      # int32 [requests]: which requests of the step they are
     longer_than: int
     short: bool                 # whether the step holds other requests too
+    chunk_tokens: int = 0       # most tokens of a chunk (0: not said)
 
 
 class StepBatch:
@@ -273,7 +274,7 @@ class StepBatch:
             rows = np.stack([lo, np.minimum(lo + chunk_tokens, end[of])], axis=1)
             flat = self._to_device(np.concatenate([rows.reshape(-1), first, reqs]).astype(np.int32))
             a, b = rows.size, rows.size + first.size
-            cached = self._tiles[key] = ScanChunks(flat[:a].view(-1, 2), flat[a:b], flat[b:], longer_than, len(reqs) < len(lens))
+            cached = self._tiles[key] = ScanChunks(flat[:a].view(-1, 2), flat[a:b], flat[b:], longer_than, len(reqs) < len(lens), chunk_tokens)
         return cached
 
     @staticmethod

@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import collections
 import ctypes
+import functools
 import os
 from ctypes import c_double, c_float, c_int, c_longlong, c_ulonglong, c_void_p
 from typing import Optional
@@ -2166,8 +2167,20 @@ def delta_prepare(proj: torch.Tensor, a_pre: torch.Tensor, conv_w: torch.Tensor,
     return out_c, gb
 
 
-# tokens of a block of the delta rule with a decay per channel, and the portion length from which its blocks are worth their preparation
-DELTA_BLOCK, DELTA_BLOCK_FROM = 8, 16
+DELTA_BLOCK_FROM = 16       # the portion length from which blocks of the delta rule with a decay per channel are worth their preparation
+
+
+@functools.lru_cache(maxsize=None)
+def delta_block_tokens() -> int:
+    """Tokens of a block of the delta rule with a decay per channel, as its kernels are built."""
+    return csrc.load("delta_block").lgml_delta_block_tokens()
+
+
+def delta_block_record(dim: int) -> int:
+    """Floats that a block's preparation leaves per head for its scan."""
+    fn = csrc.load("delta_block").lgml_delta_block_record_floats
+    fn.argtypes, fn.restype = [c_int], c_longlong
+    return fn(dim)
 
 
 def delta_scan(qkv_c: torch.Tensor, gb: torch.Tensor, state: torch.Tensor, seq_start: torch.Tensor, slots: torch.Tensor,
@@ -2177,7 +2190,7 @@ def delta_scan(qkv_c: torch.Tensor, gb: torch.Tensor, state: torch.Tensor, seq_s
     ``qkv_c`` [tokens, q | k | v] and ``gb`` [tokens, H, D + 4] (per head the decays, then beta) as
     ``delta_prepare`` returns them, or [tokens, H, 4] (one decay per head, beta, its logarithm, zero) as ``delta_head_prepare`` does.
     Returns o float32 [tokens, H Dv].  ``chunks`` (one decay per head) as for ``chunk_scan``: the requests with many tokens take
-    that form (where the sizes allow), the others the sequential one.  ``blocks`` (a decay per channel; chunks of ``DELTA_BLOCK`` tokens):
+    that form (where the sizes allow), the others the sequential one.  ``blocks`` (a decay per channel; chunks of ``delta_block_tokens()`` tokens):
     the same for eight tokens at a time, whose sums come in another order than the sequential form's."""
     n = qkv_c.shape[0]
     head_decay = gb.dim() == 3 and gb.shape[2] == 4
@@ -2202,7 +2215,10 @@ def delta_scan(qkv_c: torch.Tensor, gb: torch.Tensor, state: torch.Tensor, seq_s
     elif blocks is not None and not head_decay and n and dim % 4 == 0 and dim <= 128 and n_heads * vdim % 4 == 0 \
             and qkv_c.data_ptr() % 16 == 0 and gb.data_ptr() % 16 == 0:
         n_blocks = blocks.rows.shape[0]
-        records = torch.empty(n_blocks * n_heads * (25 * dim + 136), dtype=torch.float32, device=qkv_c.device)
+        cut = getattr(blocks, "chunk_tokens", 0) or delta_block_tokens()
+        if cut != delta_block_tokens():
+            raise KernelError(f"delta_scan: the blocks hold {cut} tokens, the kernels take {delta_block_tokens()}")
+        records = torch.empty(n_blocks * n_heads * delta_block_record(dim), dtype=torch.float32, device=qkv_c.device)
         block_fn = _fn("delta_block", "lgml_delta_block_scan", [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p,
                                                                 c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
         _check("delta_block", block_fn(_ptr(qkv_c), _ptr(gb), _ptr(state), state.stride(0), _ptr(blocks.rows), n_blocks, _ptr(blocks.first),
@@ -2728,13 +2744,19 @@ def attention_f32_short(seq_lens, n_heads: int, n_kv_heads: int, dim: int) -> in
     return short
 
 
+@functools.lru_cache(maxsize=None)
+def attention_f32_chunk() -> int:
+    """Keys of a chunk, as the kernels are built."""
+    return csrc.load("attention_f32").lgml_attention_f32_chunk()
+
+
 def attention_f32_chunks(n_tokens: int, n_heads: int, n_kv_heads: int, dim: int, max_kv_len: int, window: int) -> tuple:
     """(Chunks of keys side by side, 0: one after the other; tokens whose chunks' results the scratch holds) for tokens taken each by itself.
 
     A window is touched by as many chunks as fit it and one more, wherever it starts.  One after the other where there is one chunk, or
     where the CTAs of whole contexts fill the chip three times an SM and the longest is of up to eight: CTAs of chunks that a short
     context does not have, the merge and its reading then cost more than what a long context among them takes alone."""
-    chunk = csrc.load("attention_f32").lgml_attention_f32_chunk()
+    chunk = attention_f32_chunk()
     n_chunks = max(1, -(-max_kv_len // chunk))
     if window:
         n_chunks = min(n_chunks, (window + chunk - 2) // chunk + 1)

@@ -80,7 +80,7 @@ class ChannelDelta(Part):
         # (the 32-bit path keeps the token-by-token form: there a portion's results have the same bits however it is cut)
         blocks = None
         if rt.dtype == torch.bfloat16 and batch.max_q_len >= ops.DELTA_BLOCK_FROM:
-            blocks = batch.scan_chunks(ops.DELTA_BLOCK, ops.DELTA_BLOCK_FROM - 1)
+            blocks = batch.scan_chunks(ops.delta_block_tokens(), ops.DELTA_BLOCK_FROM - 1)
         o = ops.delta_scan(qkv_c, gb, cache.state, batch.seq_start, batch.slots, H, G, D, Dv, blocks=blocks)
         y = ops.delta_output(o, self.norm_w, g_pre, self.eps, rt.dtype, H)
         return rt.linear(y, self.wo, partials_ok=True)

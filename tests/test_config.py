@@ -214,6 +214,16 @@ def test_requests_taken_token_by_token_and_as_tiles():
     assert few is None and longest == 0 and np.array_equal(tiles.numpy(), batch.attention_tiles(16).numpy())
 
 
+def test_layouts_that_the_host_sizes_are_the_kernels_own():
+    """Scratch is sized by what the libraries say of themselves: a record holds at least a block's vectors, triangles and steps."""
+    from lgml_b200 import ops
+
+    n = ops.delta_block_tokens()
+    for dim in (4, 12, 64, 128):
+        assert ops.delta_block_record(dim) >= (3 * n + 1) * dim + 2 * n * n + n and ops.delta_block_record(dim) % 4 == 0
+    assert ops.attention_f32_chunk() % 64 == 0
+
+
 def test_end_tokens_of_generation_config_join_those_of_config(tmp_path):
     import json
 

@@ -251,6 +251,20 @@ def test_delta_scan_in_blocks_is_as_exact_as_token_by_token(D, Dv, Hh, G, spread
     assert torch.equal(o_b[int(ends[1]):int(ends[2])], o_t[int(ends[1]):int(ends[2])])      # the short one takes the sequential form
 
 
+def test_delta_scan_refuses_blocks_of_another_size():
+    """The kernels' block is theirs to say: chunks that a step cut otherwise are refused before anything is launched."""
+    from lgml_b200 import ops
+    from lgml_b200.engine.batch import ScanChunks
+
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    size = ops.delta_block_tokens()
+    blocks = lambda cut: ScanChunks(i32([(t, min(t + cut, 32)) for t in range(0, 32, cut)]), i32([0, -(-32 // cut)]), i32([0]), 15, False, cut)
+    args = lambda: (torch.randn(32, 48, device=DEV), torch.rand(32, 1, 20, device=DEV), torch.zeros(1, 256, device=DEV), i32([0, 32]), i32([0]), 1, 1, 16, 16)
+    ops.delta_scan(*args(), blocks=blocks(size))
+    with pytest.raises(ops.KernelError, match="16 tokens"):
+        ops.delta_scan(*args(), blocks=blocks(16))
+
+
 @pytest.mark.parametrize("D,Dv", [(12, 20), (128, 17)])
 def test_delta_scan_in_blocks_keeps_earlier_tokens_clear_of_later_infinities(D, Dv):
     """An infinite value and a key that is no number inside blocks of eight: finite results and states are those of the token-by-token form,
