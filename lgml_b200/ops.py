@@ -2167,7 +2167,10 @@ def delta_prepare(proj: torch.Tensor, a_pre: torch.Tensor, conv_w: torch.Tensor,
     return out_c, gb
 
 
-DELTA_BLOCK_FROM = 16       # the portion length from which blocks of the delta rule with a decay per channel are worth their preparation
+# The portion length from which blocks of the delta rule with a decay per channel are worth their preparation, whatever else the step holds:
+# 32 requests of 16 heads of 128 x 128 take 85 us token by token and 94 in blocks at 16 tokens, 127 and 136 at 25, 137 and 137 at 28,
+# 157 and 159 at 33 (blocks of eight: 25 to 32 tokens are four); eight requests 30 and 33, 45 and 40; one 14.6 and 9.5, 22 and 11.6.
+DELTA_BLOCK_FROM = 28
 
 
 @functools.lru_cache(maxsize=None)
