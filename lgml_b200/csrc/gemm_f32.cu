@@ -14,7 +14,7 @@
 // One B200, weights from HBM, microseconds before (64 x 64 tiles, element by element) and now:
 //   M, N, K:  4, 2048, 2048: 156 -> 13;  4, 11264, 2048: 225 -> 26;  4, 32000, 2048: 435 -> 59;
 //   89, 2048, 5632: 423 -> 158;  512, 11264, 2048: 998 -> 554 (43 TFLOP/s);  1500, 32000, 2048: 7927 -> 4388.
-// From registers alone the FMA units give 65 TFLOP/s, plain or packed (fma.rn.f32x2).
+// From registers alone (16 independent chains a thread) the FMA units give 72 TFLOP/s.
 
 #include "common.cuh"
 
@@ -373,10 +373,22 @@ float tiled_us(const Call &c, int bm, int bn, float alone, float more) {
     return alone + (float)((tiles + 147) / 148 - 1) * more;
 }
 
+// Whether up to 16 rows go to warps of their own.  Not 9 to 16 rows of a vocabulary's size: a warp's reading of its rows of A, 145 to
+// 170 us at N 32000, K 2048, costs more than what 32 x 32 tiles compute for rows that are not there, 149.  Not five rows and more of
+// a short K, most of a stage being empty (N 4700, K 32: 3.3 to 4.5 us, 64 x 64 tiles element by element 3.0 to 3.3; K 64: 4.4 to 5.0, 5.2).
+// Rows that do not start on 16 bytes come element by element here too, which a longer K, or fewer rows, must pay for
+// (rows here, tiles; N 4700: 8 rows, K 31 4.1, 2.9, K 129 7.3, 9.0; 16 rows, K 129 10.2, 9.1, K 257 14.2, 16.3; N 18000: 8 rows,
+// K 257 56.5, 51.9, K 513 79, 101; N 30000: 8 rows, K 257 83, 55, 4 rows, K 31 8.8, 7.3, K 129 27.1, 29.3).
+template <bool VEC> bool rows_pay(const Call &c) {
+    if (c.M > 16 || (c.M > 8 && c.N > 148 * 128)) return false;
+    if (VEC) return c.M <= 4 || c.K >= 64;
+    if (c.N > 148 * 128) return c.M <= 4 && c.K >= 64;
+    return c.M <= 4 || c.K >= (c.N > 148 * 64 ? 512 : c.M <= 8 ? 64 : 256);
+}
+
 template <bool VEC, typename TO> int run(const Call &c) {
-    // (9 to 16 rows of a vocabulary's size: a warp's reading of its rows of A, 145 to 170 us at N 32000,
-    // costs more than what 32 x 32 tiles compute for rows that are not there, 149)
-    if (c.M <= 8 || (c.M <= 16 && c.N <= 148 * 128)) return run_rows<VEC, TO>(c);
+    if (rows_pay<VEC>(c)) return run_rows<VEC, TO>(c);
+    if (VEC && c.M <= 16 && c.N <= 148 * 128) return launch_ragged<TO>(c);
     if constexpr (VEC) {
         const float t1 = tiled_us(c, 32, 32, 40.f, 19.6f), t2 = tiled_us(c, 32, 64, 58.f, 32.f), t3 = tiled_us(c, 64, 64, 90.f, 58.7f),
                     t4 = tiled_us(c, 64, 128, 148.f, 108.f);
