@@ -37,8 +37,8 @@ static inline int lgml_launch_status(const char *what) {
 }
 
 // ---- programmatic dependent launch -------------------------------------------------------------
-// Every kernel of this package is launched with the "programmatic stream serialization"
-// attribute: the next kernel in the stream may start (its blocks become resident, and may do
+// Nearly every kernel of this package is launched with the "programmatic stream serialization"
+// attribute (lgml_launch_alone below is without it): the next kernel in the stream may start (its blocks become resident, and may do
 // work that does not depend on earlier kernels, such as fetching weights) once all blocks of
 // this one have called pdl_trigger().  A kernel calls pdl_wait() before it reads anything an
 // earlier kernel wrote and before it writes anything at all; the wait returns when the
@@ -72,7 +72,7 @@ __device__ __forceinline__ uint4 act_load(const uint4 *p) { return __ldcg(p); }
 // Loads for before pdl_wait(): of weights, and of what the host sent with the step (positions, block tables).  They stay where they
 // are written; the compiler may move an ordinary load of constant data behind the wait, and with it a trip to HBM onto the chain
 // of a decode step.  The host's data is complete by then: its copy ends before the step's first kernel starts, and no kernel of the
-// step starts before that one has.
+// step starts before that one has.  So are weights: what writes them (copies, the seeded fill) lets no kernel behind it start early.
 __device__ __forceinline__ float4 early_weights(const float *p) {
     float4 v;
     asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));

@@ -113,7 +113,7 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 // R lanes share a column, four rows of S each (D <= 4 R), and R / 8 columns a lane: a vector of a block is then read once
 // by R different lanes for R / 8 columns, without a bank asked twice.  (Eight lanes on sixteen rows of one column read
 // the same floats in every column of a warp, which costs shared memory as many cycles as different ones.)
-// 512 tokens of sixteen heads of 128 x 128 on one B200: 74 us, 1,100 cycles a block of eight tokens; a warp a scheduler, stalled
+// 512 tokens of sixteen heads of 128 x 128 on one B200: 74 us, about 2,260 cycles a block of eight tokens; a warp a scheduler, stalled
 // a third of the time on shuffles and on the chain of the substitution.  Token by token 238 us; 2,048 tokens 289 and 937 us.
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     uint64_t r;

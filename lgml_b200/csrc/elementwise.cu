@@ -58,13 +58,15 @@ LGML_API int lgml_embed_rows_as(const void *table, int table_dtype, const int *i
 // group holds the four consecutive elements  slice start + 512 rd + 4 g ...+3  (one 16-byte
 // access when the row allows it), adds their squares in that order, the group adds its threads'
 // sums by warp trees and then the four warps' sums by index, and the slices' sums are added by
-// index.  Four ways of launching share this:
+// index.  Five ways of launching share this:
 //   - few rows (decoding): the slices of a row are the groups of 128 threads of one block (a
 //     slice then has at most 1,024 elements); for wider rows they are the CTAs of a thread-block
 //     cluster, whose sums cross through distributed shared memory;
-//   - many rows (prompts): one block of 128 threads takes all slices of its row one after the
-//     other, with every load of the row issued before any is used;
-//   - rows too wide for the registers of those two: one block per row that walks the row twice.
+//   - many rows (prompts) whose slices are one round each: slices side by side in a block of as many
+//     threads as they have quads (rmsnorm_slices_kernel; most widths up to 4,096);
+//   - many rows otherwise, and whole rounds of width 4,096 with at most one delta: one block of 128 threads
+//     takes all slices of its row one after the other, with every load of the row issued before any is used;
+//   - rows too wide for the registers of those: one block per row that walks the row twice.
 // ---------------------------------------------------------------------------------------
 namespace rms {
 constexpr int PER = 4, GROUP = 128, WARPS = GROUP / 32, MAX_CS = 8;
@@ -224,7 +226,8 @@ __global__ void __launch_bounds__(MODE == 2 ? GROUP * MAX_CS : GROUP) rmsnorm_ke
     auto end = [&](int k) { return FULL ? (1 << 30) : (k < n_slices ? min(width, (rank0 + k + 1) * per_cta) : 0); };
     // One slice a thread, which is how few rows run: the weights come while the kernel ahead ends (in a decode step they come
     // from HBM, a trip on the step's chain: with the position chain of rope_cache.cu 12.58 -> 12.07 ms for 17 steps of 16 requests, width 5,120)
-    // (two rounds in a block of 1,024 threads have no registers to keep them in: there they are only brought into L2)
+    // (two rounds in a block of 1,024 threads have no registers to keep them in: there they are only brought into L2.  16 rows of 5,120 with
+    // nine partial sums 6.3 us without, 6.9 with registers that spill, 5.9 so; with the weights in HBM 7.0 and 6.5)
     constexpr bool AHEAD = GROUPED && ROUNDS > 1, EARLY = SLICES == 1 && !AHEAD;
     float4 we[EARLY ? ROUNDS : 1];
     if (EARLY || AHEAD) {
