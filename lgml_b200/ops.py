@@ -2587,18 +2587,18 @@ def decode_ranges(n_tokens: int, n_kv_heads: int, group: int, dim: int, shortest
     """``decode_splits``, and more than its one range where CTAs of whole contexts fill their last round badly.
 
     ``shortest`` and ``longest`` bound the contexts (or what a window leaves of them).  With a little more CTAs than the chip holds once
-    or twice, whole ranges leave their last round nearly empty; three ranges (two behind a second round) fill it.  Only where every query head
+    or twice, whole ranges leave their last round nearly empty; three ranges fill it.  Only where every query head
     has keys of its own, the contexts are of one size and over 1,024 tokens: there it is never slower.  32 heads of 128 on 32, in microseconds at
     1,025, 2,049 and 4,097 tokens with 1 range and with 3: 10 requests (1.08 rounds) 46, 86, 163 and 40, 67, 121; 12 (1.30) 48, 89, 172 and
-    45, 73, 133; with 1 and 2: 20 (2.16) 71, 130, 251 and 69, 118, 220.  Further on it is not (1.51 rounds: 51, 90, 176 and 52, 86,
-    156; 1.73: 50, 92, 175 and 58, 99, 178; 2.59 with 2: 75, 136, 275 and 80, 141, 278), nor for short contexts (600 tokens, 1.30 rounds:
+    45, 73, 133; 20 (2.16) 71, 130, 251 and 69, 117, 218.  Further on it is not (1.51 rounds: 51, 90, 176 and 52, 86,
+    156; 1.73: 50, 92, 175 and 58, 99, 178; 2.59: 75, 136, 275 and 81, 139, 262), nor for short contexts (600 tokens, 1.30 rounds:
     32.5 and 32.4; 70 tokens: 8.5 and 11.7), nor for uneven ones, whose short requests fill the last round by themselves (12 of up
     to 600: 20 and 22).  Heads that share keys keep whole ranges (64 requests at 1,548, 32 on 8: 73 with 1, 85 with 2)."""
     full = DECODE_CTAS_PER_SM.get(dim, 0) * sm_count()
     if group == 1 and full and shortest > 1024 and longest <= 2 * shortest:
         rounds, rest = divmod(n_tokens * n_kv_heads, full)
         if (rounds == 1 and 0 < rest <= 0.31 * full) or (rounds == 2 and 0 < rest <= 0.2 * full):
-            return 3 if rounds == 1 else 2
+            return 3
     return decode_splits(n_tokens, n_kv_heads, group, longest)
 
 

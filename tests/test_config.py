@@ -149,7 +149,7 @@ def test_ranges_of_contexts_that_fill_their_last_round_badly():
     from lgml_b200.ops import decode_ranges, decode_splits, sm_count
 
     R = 2 * sm_count()                                              # CTAs of head size 128 that the chip holds at once
-    for ctas, want in ((R, 1), (R + 1, 3), (int(1.3 * R), 3), (int(1.32 * R), 1), (2 * R, 1), (2 * R + 1, 2), (int(2.2 * R), 2), (int(2.3 * R), 1),
+    for ctas, want in ((R, 1), (R + 1, 3), (int(1.3 * R), 3), (int(1.32 * R), 1), (2 * R, 1), (2 * R + 1, 3), (int(2.2 * R), 3), (int(2.3 * R), 1),
                        (3 * R + 1, 1), (8 * R + 1, 1)):
         assert decode_ranges(1, ctas, 1, 128, 1025, 2048) == want
         assert decode_ranges(1, 2 * ctas, 1, 64, 3000, 4096) == want
