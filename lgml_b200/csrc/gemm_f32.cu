@@ -1,20 +1,23 @@
-// True 32-bit matrix product: C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]), float32 operands,
-// float32 FMA accumulation, no tensor cores and no reduced-precision mode.  Every output
-// element sums its K products in the order k = 0, 1, 2, ... whatever M, N and the tile it
-// falls in, so a row's result does not depend on what else is in the batch.  It stands
-// where mischief/lgml calls mul_mat with the f32 flag (src/lgml.c:1811-1839).
+// 32-bit matrix product: C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]), float32 operands and results.  The order
+// in which an output's products are added depends on K alone, whatever M, N and the tile it falls in, so a row's
+// result does not depend on what else is in the batch.  It stands where mischief/lgml calls mul_mat with the f32
+// flag (src/lgml.c:1811-1839).
 //
-// That order makes one chain of K dependent FMAs of every output (4 cycles each: 8.5 us at
-// K = 4096), so K is never cut; the kernels differ in what they keep busy beside the chain:
-//   * gemm_f32_rows_kernel, up to 16 rows (decoding): the matrix is what has to be read.  A warp
-//     streams 8 to 32 rows of W through shared memory of its own, a lane owns one feature for a few
-//     rows; the first stages are asked for before the kernel ahead is done.
+// K >= 64: on the tensor cores, both operands in two tf32 halves (below).  A chain of K dependent FMAs takes
+// 4 cycles a step and the FMA units give 72 TFLOP/s at the very best (43 in tiles); three tf32 products of m16n8k8 give
+// 92, and a K that is added up in segments can be shared out among warps.  Off 64 bits by (2-norm, random signs; chain of FMAs, here):
+//   K = 64 1.4e-7, 1.1e-7;  256 2.9e-7, 1.2e-7;  2048 8.1e-7, 1.4e-7;  14336 2.2e-6, 2.3e-7.   (K = 32: 1.03e-7, 1.05e-7; 16: 0.7e-7, 1.0e-7.)
+//   * gemm_f32_few_kernel, up to 32 rows (or more of few features): warps stream W, each its segments of K.
+//   * gemm_f32_many_kernel: tiles of 64 x 64.
+// K < 64: every output sums its products in the order k = 0, 1, 2, ..., one chain of FMAs.
+//   * gemm_f32_rows_kernel, up to 4 rows: a warp streams 8 or 16 rows of W through shared memory of its own.
 //   * gemm_f32_tile_kernel, more rows: tiles of A and W by asynchronous copies, several blocks an SM.
 //   * gemm_f32_ragged_kernel, more rows that do not all start on 16 bytes: tiles element by element.
-// One B200, weights from HBM, microseconds before (64 x 64 tiles, element by element) and now:
-//   M, N, K:  4, 2048, 2048: 156 -> 13;  4, 11264, 2048: 225 -> 26;  4, 32000, 2048: 435 -> 59;
-//   89, 2048, 5632: 423 -> 158;  512, 11264, 2048: 998 -> 554 (43 TFLOP/s);  1500, 32000, 2048: 7927 -> 4388.
-// From registers alone (16 independent chains a thread) the FMA units give 72 TFLOP/s.
+// One B200, weights from HBM, microseconds, one chain of FMAs an output and now:
+//   M, N, K:  4, 2048, 2048: 12.3 -> 5.6;  4, 2048, 5632: 29.6 -> 10.2;  4, 11264, 2048: 28.7 -> 20.4;  4, 32000, 2048: 58.6 -> 47 (5.6 TB/s);
+//   32, 2048, 5632: 109 -> 24;  89, 2048, 5632: 159 -> 66;  812, 11264, 2048: 874 -> 641 (58 TFLOP/s);  2048, 32000, 2048: 5,872 -> 4,274.
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -120,8 +123,8 @@ __global__ void __launch_bounds__(32) gemm_f32_rows_kernel(const float *__restri
 #pragma unroll
             for (int j = 0; j < MT; ++j) acc[j] = fmaf(a[j].w, w.w, acc[j]);
         };
-        if constexpr (MT <= 4) {
-            constexpr int AHEAD = MT <= 2 ? 4 : 2, GROUPS = ROWS_BK / 4 / AHEAD;
+        {
+            constexpr int AHEAD = 4, GROUPS = ROWS_BK / 4 / AHEAD;
             float4 w[2][AHEAD], a[2][AHEAD][MT];
 #pragma unroll
             for (int u = 0; u < AHEAD; ++u) read(u * 4, w[0][u], a[0][u]);
@@ -133,13 +136,6 @@ __global__ void __launch_bounds__(32) gemm_f32_rows_kernel(const float *__restri
                 }
 #pragma unroll
                 for (int u = 0; u < AHEAD; ++u) add(w[g & 1][u], a[g & 1][u]);
-            }
-        } else {
-#pragma unroll 8
-            for (int k = 0; k < ROWS_BK; k += 4) {
-                float4 w, a[MT];
-                read(k, w, a);
-                add(w, a);
             }
         }
         __syncwarp();
@@ -309,6 +305,318 @@ __global__ void __launch_bounds__(256) gemm_f32_ragged_kernel(const float *__res
     }
 }
 
+// ---- products of a long K: three tensor-core products of two halves each --------------------------
+// w = hi + lo, hi being w rounded to the 11 bits of a tf32 number and lo what that lost (exact; its own 11 bits are read by the tensor
+// core).  Of a run of 16 k the products lo hi, hi lo and then hi hi are added up by mma.sync (m16n8k8, 16 features by 8 rows) from
+// zero, the run's sum joins the sum of its segment of 128 k in float32, and the segments' sums join in order.  The tensor core cuts
+// what it adds instead of rounding it, which is why so little is added up there (measured at K = 1024 against 64 bits, random signs:
+// 2.5e-6 in one go); what hi lo and lo hi lose is under 2^-11 of that.  One order for every kernel below, so a row has the same bits
+// in each.  A result that is not finite, or below 2^-96, is formed again as the plain chain of FMAs: infinities, NaNs and overflows
+// come out as they do there, and so do sums of numbers so small that a lo is cut (a tf32 number below the normal ones is a multiple
+// of 2^-136, so an operand under 2^-112 has fewer than 24 bits; that shows beside operands over 2^16 only).
+constexpr int SEGMENT = 128, SPLIT_FROM = 64;
+
+__device__ __forceinline__ void split(float x, uint32_t &hi, uint32_t &lo) {
+    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+    lo = __float_as_uint(x - __uint_as_float(hi));
+}
+__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+__device__ __forceinline__ void mma_tf32_from_zero(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.f));
+}
+
+// sum += the products of one run of 16 k: `w` the float4 of features g and g + 8 of MT tiles of 16 features, `a` that of row g of NT tiles
+// of 8 rows, g = lane / 4; lane % 4 says which four k a float4 holds.
+template <int MT, int NT> __device__ __forceinline__ void add_run(float (&sum)[MT][NT][4], const float4 (&w)[MT][2], const float4 (&a)[NT]) {
+    float acc[MT][NT][4];
+    uint32_t wh[2][MT][4], ah[2][NT][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {           // two of every lane's four k at a time
+        uint32_t wl[MT][4], al[NT][2];
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                split(h ? w[i][r].z : w[i][r].x, wh[h][i][r], wl[i][r]);
+                split(h ? w[i][r].w : w[i][r].y, wh[h][i][2 + r], wl[i][2 + r]);
+            }
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            split(h ? a[j].z : a[j].x, ah[h][j][0], al[j][0]);
+            split(h ? a[j].w : a[j].y, ah[h][j][1], al[j][1]);
+        }
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                if (h == 0) mma_tf32_from_zero(acc[i][j], wl[i], ah[h][j]);
+                else mma_tf32(acc[i][j], wl[i], ah[h][j]);
+            }
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) mma_tf32(acc[i][j], wh[h][i], al[j]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) mma_tf32(acc[i][j], wh[h][i], ah[h][j]);
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum[i][j][e] += acc[i][j][e];
+}
+
+__device__ __noinline__ float chain(const float *a, const float *w, int K) {
+    float v = 0.f;
+    for (int k = 0; k < K; ++k) v = fmaf(act_load(a + k), w[k], v);
+    return v;
+}
+template <typename TO>
+__device__ __forceinline__ void store_split(float v, const float *A, const float *W, const float *bias, TO *C, int m, int n, int M, int N, int K, int lda,
+                                            int ldw, int ldc) {
+    if (m >= M || n >= N) return;
+    if (!(fabsf(v) <= 3.402823466e38f) || (fabsf(v) < 0x1p-96f && v != 0.f)) v = chain(A + (size_t)m * lda, W + (size_t)n * ldw, K);
+    C[(size_t)m * ldc + n] = from_f32<TO>(bias ? v + bias[n] : v);
+}
+
+// 16 bytes of a row's elements k .. k + 3 into shared memory, zeros for those past K.  Rows that do not start on 16 bytes come
+// element by element (through L1: such a kernel is launched without the early start).
+template <bool VEC> __device__ __forceinline__ void copy_4(uint32_t dst, const float *src, int k, int K) {
+    const int n = min(max(K - k, 0), 4);
+    if constexpr (VEC) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(n ? src : src - k), "r"(n * 4) : "memory");
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * i), "l"(i < n ? src + i : src - k), "r"(i < n ? 4 : 0) : "memory");
+    }
+}
+// ROWS rows of 32 floats, k0 on, by THREADS threads of eight a row.  `x` is the first row at this thread's 16 bytes of it; off[] are its rows.
+// The halves of every second row change places in shared memory, so that eight lanes' 16-byte reads of one half of two rows fall
+// into all 32 banks.
+template <bool VEC> using RowOffset = typename std::conditional<VEC, int, long long>::type;
+template <bool VEC, int ROWS, int THREADS>
+__device__ __forceinline__ void copy_rows(uint32_t dst, const float *x, const RowOffset<VEC> (&off)[ROWS * 8 / THREADS], int k0, int c, int K, int rows = ROWS) {
+    constexpr int N = ROWS * 8 / THREADS, BYTES = THREADS / 8 * 128;
+    if (VEC && k0 + 32 <= K) {
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (i * (THREADS / 8) < rows) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * BYTES), "l"(x + k0 + off[i]) : "memory");
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (i * (THREADS / 8) < rows) copy_4<VEC>(dst + i * BYTES, x + k0 + off[i], k0 + c, K);
+    }
+}
+__device__ __forceinline__ int swizzled(int row, int chunk) { return row * 32 + ((chunk ^ ((row & 1) << 2)) << 2); }
+
+// Few rows: a block has 16 features and up to 8 NT rows; its eight warps take a segment of K each, turn by turn, and stream W
+// through shared memory of their own (no barrier but at the end of a turn).  Rows that are not there repeat the last one.
+constexpr int FEW_EACH = 4, SEGMENT_STEPS = SEGMENT / 32;
+template <int NT, int STAGES, int WARPS> struct FewShape {
+    static constexpr int STAGE_FLOATS = (16 + 8 * NT) * 32;
+    static constexpr int OUTS = NT * 128;               // of a block
+    static constexpr size_t SMEM = sizeof(float) * (WARPS * STAGES * STAGE_FLOATS + WARPS * FEW_EACH * OUTS);
+};
+
+template <int NT, int STAGES, int WARPS, bool VEC, typename TO>
+__global__ void __launch_bounds__(WARPS * 32) gemm_f32_few_kernel(const float *__restrict__ A, const float *__restrict__ W,
+                                                                      const float *__restrict__ bias, TO *__restrict__ C, int M, int N, int K, int lda,
+                                                                      int ldw, int ldc) {
+    using S = FewShape<NT, STAGES, WARPS>;
+    constexpr int SEGS = WARPS * FEW_EACH, STEPS = FEW_EACH * SEGMENT_STEPS;        // of a turn: segments of the block, steps of a warp
+    static_assert(STEPS % STAGES == 0, "a step's stage is known when it is compiled");
+    extern __shared__ __align__(16) float smem_f[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    const int n0 = blockIdx.x * 16, m0 = blockIdx.y * 8 * NT;
+    float *mine = smem_f + warp * STAGES * S::STAGE_FLOATS, *parts = smem_f + WARPS * STAGES * S::STAGE_FLOATS;
+    const int n_seg = (K + SEGMENT - 1) / SEGMENT;
+    const int r = lane >> 3, c = (lane & 7) * 4;
+    const float *wp = W + (size_t)n0 * ldw + c, *ap = A + (size_t)m0 * lda + c;
+    RowOffset<VEC> w_off[4], a_off[2 * NT];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w_off[i] = (RowOffset<VEC>)min(i * 4 + r, N - 1 - n0) * ldw;
+#pragma unroll
+    for (int i = 0; i < 2 * NT; ++i) a_off[i] = (RowOffset<VEC>)min(i * 4 + r, M - 1 - m0) * lda;
+    const uint32_t to = smem_addr(mine + swizzled(r, lane & 7));
+    // step s of a turn that starts at segment `first`: 32 k of this warp's segment s / SEGMENT_STEPS; behind STEPS the next turn's
+    auto k_of = [&](int first, int s) { return (first + s / SEGMENT_STEPS * WARPS + warp) * SEGMENT + s % SEGMENT_STEPS * 32; };
+    auto load_w = [&](int k0, int s) {
+        if (k0 < K) copy_rows<VEC, 16, 32>(to + (s % STAGES) * S::STAGE_FLOATS * 4, wp, w_off, k0, c, K);
+    };
+    auto load_a = [&](int k0, int s) {
+        if (k0 < K) copy_rows<VEC, 8 * NT, 32>(to + ((s % STAGES) * S::STAGE_FLOATS + 16 * 32) * 4, ap, a_off, k0, c, K, M - m0);
+    };
+    // the weights of the first stages do not depend on the kernels ahead
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) load_w(k_of(0, s), s);
+    pdl_wait();
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        load_a(k_of(0, s), s);
+        cp_async_commit();
+    }
+    constexpr int OUTS = (S::OUTS + WARPS * 32 - 1) / (WARPS * 32);         // ... of a thread
+    float total[OUTS];
+#pragma unroll
+    for (int o = 0; o < OUTS; ++o) total[o] = 0.f;
+    const int frag = swizzled(g, q), frag_other = frag ^ 16;          // the row's first and second 16 k (rows 8 apart have the same order)
+    for (int first = 0; first < n_seg; first += SEGS) {
+#pragma unroll
+        for (int i = 0; i < FEW_EACH; ++i) {
+            if (first + i * WARPS + warp >= n_seg) break;
+            float sum[1][NT][4];
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sum[0][j][e] = 0.f;
+#pragma unroll
+            for (int ss = 0; ss < SEGMENT_STEPS; ++ss) {
+                const int s = i * SEGMENT_STEPS + ss, k0 = k_of(first, s), ahead = s + STAGES - 1;
+                cp_async_wait<STAGES - 2>();
+                __syncwarp();
+                load_w(k_of(first, ahead), ahead);
+                load_a(k_of(first, ahead), ahead);
+                cp_async_commit();
+                const float *ws = mine + (s % STAGES) * S::STAGE_FLOATS;
+                if (k0 < K) {
+#pragma unroll
+                    for (int run = 0; run < 2; ++run) {
+                        const float *at = ws + (run ? frag_other : frag);
+                        float4 w[1][2], a[NT];
+                        w[0][0] = *reinterpret_cast<const float4 *>(at);
+                        w[0][1] = *reinterpret_cast<const float4 *>(at + 8 * 32);
+#pragma unroll
+                        for (int j = 0; j < NT; ++j) a[j] = *reinterpret_cast<const float4 *>(at + (16 + j * 8) * 32);
+                        add_run<1, NT>(sum, w, a);
+                    }
+                }
+                __syncwarp();
+            }
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) parts[(i * WARPS + warp) * S::OUTS + (j * 4 + e) * 32 + lane] = sum[0][j][e];
+        }
+        // the turn's segments, in order
+        __syncthreads();
+        const int segs = min(SEGS, n_seg - first);
+#pragma unroll
+        for (int o = 0; o < OUTS; ++o) {
+            const int at = o * WARPS * 32 + threadIdx.x;
+            if (at < S::OUTS) {
+#pragma unroll 8
+                for (int s = 0; s < segs; ++s) total[o] += parts[s * S::OUTS + at];
+            }
+        }
+        if (first + SEGS < n_seg) __syncthreads();
+    }
+    pdl_trigger();      // at the end: blocks of the kernels behind that start earlier are placed where there is room, not where there is time
+#pragma unroll
+    for (int o = 0; o < OUTS; ++o) {
+        const int at = o * WARPS * 32 + threadIdx.x, l = at & 31, e = (at >> 5) & 3, j = at >> 7;
+        if (at < S::OUTS) store_split(total[o], A, W, bias, C, m0 + j * 8 + (l & 3) * 2 + (e & 1), n0 + (l >> 2) + (e >> 1) * 8, M, N, K, lda, ldw, ldc);
+    }
+}
+
+// Many rows: tiles of 64 features by 64 rows, 32 x 32 a warp.  The tensor pipe bounds it (m16n8k8: 278 TFLOP/s by itself, three a
+// product).  A segment's sum and the sum of segments stay in registers.
+constexpr int MANY_STAGES = 4, MANY_STAGE_FLOATS = 128 * 32;
+constexpr size_t MANY_SMEM = sizeof(float) * MANY_STAGES * MANY_STAGE_FLOATS;
+
+template <bool VEC, typename TO>
+__global__ void __launch_bounds__(128, 3) gemm_f32_many_kernel(const float *__restrict__ A, const float *__restrict__ W, const float *__restrict__ bias,
+                                                               TO *__restrict__ C, int M, int N, int K, int lda, int ldw, int ldc, int tiles_m) {
+    constexpr int STAGES = MANY_STAGES;
+    extern __shared__ __align__(16) float smem_f[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    const int f0 = (warp & 1) * 32, r0 = (warp >> 1) * 32;
+    // row tiles fastest: the blocks that run at one time share a few tiles of W, and A stays in L2
+    const int m0 = (int)(blockIdx.x % tiles_m) * 64, n0 = (int)(blockIdx.x / tiles_m) * 64;
+    const int n_kt = (K + 31) / 32;
+    const int r = threadIdx.x >> 3, c = (threadIdx.x & 7) * 4;
+    const float *wp = W + (size_t)n0 * ldw + c, *ap = A + (size_t)m0 * lda + c;
+    RowOffset<VEC> w_off[4], a_off[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        w_off[i] = (RowOffset<VEC>)min(i * 16 + r, N - 1 - n0) * ldw;
+        a_off[i] = (RowOffset<VEC>)min(i * 16 + r, M - 1 - m0) * lda;
+    }
+    const uint32_t to = smem_addr(smem_f + swizzled(r, threadIdx.x & 7));
+    auto load_w = [&](int t) { copy_rows<VEC, 64, 128>(to + (t % STAGES) * MANY_STAGE_FLOATS * 4, wp, w_off, t * 32, c, K); };
+    auto load_a = [&](int t) { copy_rows<VEC, 64, 128>(to + ((t % STAGES) * MANY_STAGE_FLOATS + 64 * 32) * 4, ap, a_off, t * 32, c, K); };
+    // the weights of the first stages do not depend on the kernels ahead
+    for (int t = 0; t < STAGES - 1; ++t)
+        if (t < n_kt) load_w(t);
+    pdl_wait();
+    for (int t = 0; t < STAGES - 1; ++t) {
+        if (t < n_kt) load_a(t);
+        cp_async_commit();
+    }
+    float sum[2][4][4], total[2][4][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum[i][j][e] = total[i][j][e] = 0.f;
+    const int frag = swizzled(g, q);
+    for (int t = 0; t < n_kt; ++t) {
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();
+        if (t + STAGES - 1 < n_kt) {
+            load_w(t + STAGES - 1);
+            load_a(t + STAGES - 1);
+        }
+        cp_async_commit();
+        const float *st = smem_f + (t % STAGES) * MANY_STAGE_FLOATS;
+#pragma unroll
+        for (int run = 0; run < 2; ++run) {
+            if (run == 0 || t * 32 + 16 < K) {
+                const float *ws = st + f0 * 32 + (frag ^ (run * 16)), *as = st + (64 + r0) * 32 + (frag ^ (run * 16));
+                float4 w[2][2], a[4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) w[i][h] = *reinterpret_cast<const float4 *>(ws + (i * 16 + h * 8) * 32);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) a[j] = *reinterpret_cast<const float4 *>(as + j * 8 * 32);
+                add_run<2, 4>(sum, w, a);
+            }
+        }
+        if (t % (SEGMENT / 32) == SEGMENT / 32 - 1 || t + 1 == n_kt) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        total[i][j][e] += sum[i][j][e];
+                        sum[i][j][e] = 0.f;
+                    }
+        }
+    }
+    pdl_trigger();      // at the end: the blocks of a product fill their SMs
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                store_split(total[i][j][e], A, W, bias, C, m0 + r0 + j * 8 + q * 2 + (e & 1), n0 + f0 + i * 16 + g + (e >> 1) * 8, M, N, K, lda, ldw, ldc);
+}
+
 // ---- host side -----------------------------------------------------------------------------------
 // (At every launch: the attribute belongs to the kernel on the current device, and a process may use several.)
 template <typename Kernel> int allow_smem(Kernel kernel, size_t smem) {
@@ -357,13 +665,10 @@ template <typename TO> int launch_ragged(const Call &c) {
     return lgml_launch_status("gemm_f32");
 }
 
-// Features a warp for M <= 16 rows.  Eight where that is one warp for each of the chip's 592 schedulers or
-// fewer (N 2048, K 2048: 12.5 us at 4 rows; 15 with sixteen, 21 with thirty-two); more features beside a
-// reading of A as soon as there are warps enough (N 11264, 4 rows: 38, 26 and 29 us; 8 rows: 45, 49 and 36).
+// Features a warp for M <= 4 rows: eight where that is one warp for each of the chip's 592 schedulers or fewer.
 template <bool VEC, typename TO> int run_rows(const Call &c) {
-    if (c.N <= 592 * 8) return c.M <= 4 ? launch_rows<8, 1, VEC, TO>(c) : (c.M <= 8 ? launch_rows<8, 2, VEC, TO>(c) : launch_rows<8, 4, VEC, TO>(c));
-    if (c.M <= 4) return c.M <= 2 ? launch_rows<16, 1, VEC, TO>(c) : launch_rows<16, 2, VEC, TO>(c);
-    return c.M <= 8 ? launch_rows<32, 8, VEC, TO>(c) : launch_rows<32, 16, VEC, TO>(c);
+    if (c.N <= 592 * 8) return launch_rows<8, 1, VEC, TO>(c);
+    return c.M <= 2 ? launch_rows<16, 1, VEC, TO>(c) : launch_rows<16, 2, VEC, TO>(c);
 }
 
 // Time of a product on tiles of bm x bn, in microseconds at K = 2048: an SM's first tile takes `alone`
@@ -373,21 +678,46 @@ float tiled_us(const Call &c, int bm, int bn, float alone, float more) {
     return alone + (float)((tiles + 147) / 148 - 1) * more;
 }
 
-// Whether up to 16 rows go to warps of their own.  Not 9 to 16 rows of a vocabulary's size: a warp's reading of its rows of A, 145 to
-// 170 us at N 32000, K 2048, costs more than what 32 x 32 tiles compute for rows that are not there, 149.  Not five rows and more of
-// a short K, most of a stage being empty (N 4700, K 32: 3.3 to 4.5 us, 64 x 64 tiles element by element 3.0 to 3.3; K 64: 4.4 to 5.0, 5.2).
-// Rows that do not start on 16 bytes come element by element here too, which a longer K, or fewer rows, must pay for
-// (rows here, tiles; N 4700: 8 rows, K 31 4.1, 2.9, K 129 7.3, 9.0; 16 rows, K 129 10.2, 9.1, K 257 14.2, 16.3; N 18000: 8 rows,
-// K 257 56.5, 51.9, K 513 79, 101; N 30000: 8 rows, K 257 83, 55, 4 rows, K 31 8.8, 7.3, K 129 27.1, 29.3).
-template <bool VEC> bool rows_pay(const Call &c) {
-    if (c.M > 16 || (c.M > 8 && c.N > 148 * 128)) return false;
-    if (VEC) return c.M <= 4 || c.K >= 64;
-    if (c.N > 148 * 128) return c.M <= 4 && c.K >= 64;
-    return c.M <= 4 || c.K >= (c.N > 148 * 64 ? 512 : c.M <= 8 ? 64 : 256);
+template <int NT, int STAGES, int WARPS, bool VEC, typename TO> int launch_few(const Call &c) {
+    auto kernel = gemm_f32_few_kernel<NT, STAGES, WARPS, VEC, TO>;
+    constexpr size_t smem = FewShape<NT, STAGES, WARPS>::SMEM;
+    if (allow_smem(kernel, smem)) return -1;
+    const dim3 grid((unsigned)((c.N + 15) / 16), (unsigned)((c.M + 8 * NT - 1) / (8 * NT)));
+    // decoding's products start early: their first weights come while the kernel ahead ends (about 2 us each)
+    if (!VEC || NT > 2) lgml_launch_alone(kernel, grid, WARPS * 32, smem, c.stream, c.A, c.W, c.bias, (TO *)c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc);
+    else lgml_launch(kernel, grid, WARPS * 32, smem, c.stream, c.A, c.W, c.bias, (TO *)c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc);
+    return lgml_launch_status("gemm_f32");
+}
+template <bool VEC, typename TO> int launch_many(const Call &c) {
+    auto kernel = gemm_f32_many_kernel<VEC, TO>;
+    if (allow_smem(kernel, MANY_SMEM)) return -1;
+    const int tiles_m = (c.M + 63) / 64;
+    const long long tiles = (long long)tiles_m * ((c.N + 63) / 64);
+    if (tiles > 0x7fffffffLL) LGML_FAIL("gemm_f32: M=%d N=%d make too many tiles", c.M, c.N);
+    const dim3 grid((unsigned)tiles);
+    if (!VEC || balanced(c)) lgml_launch_alone(kernel, grid, 128, MANY_SMEM, c.stream, c.A, c.W, c.bias, (TO *)c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc, tiles_m);
+    else lgml_launch(kernel, grid, 128, MANY_SMEM, c.stream, c.A, c.W, c.bias, (TO *)c.C, c.M, c.N, c.K, c.lda, c.ldw, c.ldc, tiles_m);
+    return lgml_launch_status("gemm_f32");
+}
+// Time of a product on blocks of 16 features by 32 rows, and on tiles of 64 by 64, in microseconds at K = 2048: a round of blocks
+// takes 9; an SM's first tile takes 58 (one warp a scheduler), every further one 37.
+template <bool VEC, typename TO> int run_split(const Call &c) {
+    // Where there is one block an SM it has sixteen warps, else two blocks share the SM (4 rows, N x K, sixteen warps and eight:
+    // 2048 x 5632 10.2 and 13.2, 2048 x 2048 5.6 and 5.9, 3072 x 2048 9.6 and 7.3, 11264 x 2048 24.6 and 21.2).
+    const bool one = c.N <= 148 * 16;
+    if (c.M <= 8) return one ? launch_few<1, 4, 16, VEC, TO>(c) : launch_few<1, 4, 8, VEC, TO>(c);
+    if (c.M <= 16) return one ? launch_few<2, 2, 16, VEC, TO>(c) : launch_few<2, 2, 8, VEC, TO>(c);
+    const long long blocks = (long long)((c.M + 31) / 32) * ((c.N + 15) / 16), tiles = (long long)((c.M + 63) / 64) * ((c.N + 63) / 64);
+    if ((blocks + 147) / 148 * 9 <= 58 + ((tiles + 147) / 148 - 1) * 37) return launch_few<4, 2, 8, VEC, TO>(c);
+    return launch_many<VEC, TO>(c);
 }
 
+// A short K as chains of FMAs.  Five to sixteen rows: most of a stage of the rows kernel would be empty (N 4700, K 32: 3.3 to
+// 4.5 us, 64 x 64 tiles element by element 3.0 to 3.3), and so it is for rows element by element of a vocabulary's size (4 rows of
+// N 30000, K 31: 8.8 and 7.3).
 template <bool VEC, typename TO> int run(const Call &c) {
-    if (rows_pay<VEC>(c)) return run_rows<VEC, TO>(c);
+    if (c.K >= SPLIT_FROM) return run_split<VEC, TO>(c);
+    if (c.M <= 4 && (VEC || c.N <= 148 * 128)) return run_rows<VEC, TO>(c);
     if (VEC && c.M <= 16 && c.N <= 148 * 128) return launch_ragged<TO>(c);
     if constexpr (VEC) {
         const float t1 = tiled_us(c, 32, 32, 40.f, 19.6f), t2 = tiled_us(c, 32, 64, 58.f, 32.f), t3 = tiled_us(c, 64, 64, 90.f, 58.7f),
@@ -409,8 +739,8 @@ LGML_API int lgml_gemm_f32(const float *A, const float *W, const float *bias, vo
     if (M == 0) return 0;
     LGML_REQUIRE((M + 63) / 64 <= 65535, "gemm_f32: M=%d is over %d rows", M, 65535 * 64);
     const Call c = {A, W, bias, C, M, N, K, lda, ldw, ldc, stream};
-    // 16-byte copies need rows that start on 16 bytes; any other matrix goes element by element
-    const bool vec = lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+    // 16-byte copies need rows that start on 16 bytes, and a tile's rows within 31 bits; any other matrix goes element by element
+    const bool vec = lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 && lda <= 1 << 25 && ldw <= 1 << 25;
     if (out_dtype == LGML_F32) return vec ? run<true, float>(c) : run<false, float>(c);
     if (out_dtype == LGML_BF16) return vec ? run<true, __nv_bfloat16>(c) : run<false, __nv_bfloat16>(c);
     LGML_FAIL("gemm_f32: unknown output type %d", out_dtype);

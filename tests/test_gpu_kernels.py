@@ -257,6 +257,58 @@ def test_gemm_f32_same_bits_from_every_kernel(M, N, K, pad):
         assert torch.equal(one[0], out[m, :N])
 
 
+@pytest.mark.parametrize("M,N,K,pad,scale", [
+    # where chains of FMAs end; segments of 128 k, whole, one short and one over; the eight and the sixteen warps' second turn
+    (3, 40, 63, 1, 1.0), (3, 40, 64, 0, 1.0), (8, 2368, 127, 1, 1.0), (9, 2369, 128, 0, 1.0), (16, 17, 129, 3, 1.0), (2, 2384, 4100, 0, 1.0),
+    (1, 33, 8196, 4, 1.0), (12, 50, 8200, 0, 1.0),
+    # 8, 16, 32 and 64 rows and one over; tiles of 64 x 64 with one row and one column too many
+    (17, 2400, 200, 0, 1.0), (33, 100, 96, 0, 1.0), (300, 5000, 80, 0, 1.0), (65, 9500, 132, 0, 1.0), (513, 2049, 161, 0, 1.0),
+    # halves below the smallest normal number (tf32 keeps multiples of 2^-136 there), operands of very different size
+    (5, 64, 64, 0, 2e-33), (70, 6000, 72, 0, 2e-33), (5, 64, 64, 0, 1e30),
+])
+def test_gemm_f32_in_halves(M, N, K, pad, scale):
+    """Both operands in two tf32 halves: what the halves lose is 3 2^-24 of a product, a run of 16 k cuts six sums (12 2^-24), and
+    the sums of runs and segments round K / 128 + 8 times; a row has the same bits alone and among others."""
+    from lgml_b200 import ops
+
+    torch.manual_seed(M + N + K)
+    a = (torch.randn(M, K + pad) * scale).to(DEV)[:, :K]
+    w = (torch.randn(N, K + pad) / scale ** 0.9).to(DEV)[:, :K]
+    out = torch.empty(M, N, device=DEV)
+    ops.gemm_f32(a, w, out)
+    bound = (24 + K / 128) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t())
+    assert bool(((out.double() - a.double() @ w.double().t()).abs() <= bound).all())
+    for m in {0, M // 2, M - 1}:
+        one = torch.empty(1, N, device=DEV)
+        ops.gemm_f32(a[m:m + 1], w, one)
+        assert torch.equal(one[0], out[m])
+
+
+@pytest.mark.parametrize("M", [1, 20, 200])
+def test_gemm_f32_of_infinite_and_huge_values(M):
+    """What a chain of FMAs gives: an infinity times an exact number is infinite, not lost between the halves; a sum that overflows is infinite
+    and its neighbours are what they are without it; results below the normal numbers are exact to their last bit."""
+    from lgml_b200 import ops
+
+    torch.manual_seed(M)
+    a, w = torch.randn(M, 96), torch.randn(2500, 96)
+    a[0, 5], w[:, 5], w[7, 5] = float("inf"), 1.0, -2.0
+    w[11, 3], w[12, 4] = float("nan"), 3.3e38
+    a[-1, 4] = 2.0
+    w[20] = 0.0
+    w[20, 9], a[:, 9] = 2.0 ** -120, 2.0 ** -20
+    out = torch.empty(M, 2500, device=DEV)
+    ops.gemm_f32(a.to(DEV), w.to(DEV), out)
+    out = out.cpu()
+    want = (a.double() @ w.double().t()).float()
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want))
+    there = torch.isfinite(want)
+    assert torch.equal(out[~there & ~torch.isnan(want)], want[~there & ~torch.isnan(want)])
+    assert torch.allclose(out[there], want[there], rtol=1e-5, atol=1e-4)
+    if M > 1:
+        assert torch.equal(out[1:, 20], want[1:, 20])
+
+
 @pytest.mark.parametrize("M,N,K,bias,f32,splits", [
     (1, 128, 64, False, False, None), (8, 331 * 8, 120, True, True, None), (5, 200, 192, True, False, 3),
     (64, 1000, 1096, True, True, 4), (100, 320, 96, False, False, None), (129, 520, 264, True, False, None),
