@@ -35,6 +35,7 @@ from typing import Dict, Hashable, List, Optional, Sequence, Tuple
 
 import torch
 
+from .. import host
 from .pages import PagePool, PoolFull
 
 PAGE_SIZE = 64  # tokens per page: BLOCK of lua/lgml/transformer.lua:30
@@ -209,8 +210,7 @@ class CacheManager:
             found = self._cached_prefix(tokens)
             for gi, grp in enumerate(self.groups):
                 pages = [p[gi] for p in found]
-                for page in pages:
-                    grp.pool.share(page)
+                grp.pool.share_all(pages)
                 req.tables[gi] += pages
             req.n_tokens += len(found) * self.page_size
         return req
@@ -219,16 +219,22 @@ class CacheManager:
     def _keys(self, tokens: Sequence[int], n_blocks: int):
         """The keys of the first ``n_blocks`` full pages of ``tokens``: each hashes the key
         before it and its own tokens, so a key stands for the whole prefix."""
-        # (eight pages' tokens are packed at a time: a prompt of thousands of tokens costs more in packing than in hashing)
+        # (some pages at a time: a prompt of thousands of tokens costs more in reading the list than in hashing, and most prompts
+        # are not in the cache.  64 prompts of 1,537 cached tokens: 4.1 ms packed and hashed from here, 2.1 in C.)
         key = b"lgml_b200 page %d" % self.page_size
-        page, sha256 = self.page_size, hashlib.sha256
-        size = struct.calcsize("<q") * page
-        for b in range(0, n_blocks, 8):
-            part = tokens[b * page:min(b + 8, n_blocks) * page]
-            raw = struct.pack(f"<{len(part)}q", *part)
-            for at in range(0, len(raw), size):
-                key = sha256(key + raw[at:at + size]).digest()
+        page, b = self.page_size, 0
+        while b < n_blocks and type(tokens) is list:
+            n = min(8 if b == 0 else 64, n_blocks - b)
+            raw = host.page_keys(tokens, b, n, page, key)
+            if raw is None:
+                break
+            for at in range(0, 32 * n, 32):
+                key = raw[at:at + 32]
                 yield key
+            b += n
+        for b in range(b, n_blocks):
+            key = hashlib.sha256(key + struct.pack(f"<{page}q", *tokens[b * page:(b + 1) * page])).digest()
+            yield key
 
     def _cached_prefix(self, tokens: Sequence[int]) -> List[List[int]]:
         """Per leading full page of ``tokens`` that every group still holds under its key: the

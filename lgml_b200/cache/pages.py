@@ -89,6 +89,19 @@ class PagePool:
             raise ValueError(f"page {page} is neither cached nor a held page with a key")
         self.shared_total += 1
 
+    def share_all(self, pages: List[int]) -> None:
+        """``share`` for the pages of a prefix."""
+        cached, refs, keyed = self._cached, self._refs, self._key_of
+        for page in pages:
+            if page in cached:
+                del cached[page]
+                refs[page] = 1
+            elif page in keyed and refs[page] > 0:
+                refs[page] += 1
+            else:
+                raise ValueError(f"page {page} is neither cached nor a held page with a key")
+            self.shared_total += 1
+
     def ref(self, page: int) -> None:
         if not (0 <= page < self.n_pages) or self._refs[page] <= 0:
             raise ValueError(f"page {page} is not held")

@@ -62,10 +62,14 @@ LIBRARIES: Dict[str, tuple] = {
 
 _HEADERS = ["common.cuh", "page_map.cuh"]
 
-# The host library (plain C, the system compiler): the safetensors reader and the sampler.
-HOST_LIBRARY = "host"
-HOST_SOURCE, HOST_HEADERS = "host/lgml_host.c", ["host/lgml_host.h"]
-CC_FLAGS = ["-std=c11", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall"]
+# The host libraries (plain C, the system compiler): the safetensors reader and the sampler; what step descriptions and
+# page keys are made of, which reads Python's lists and so is called with the interpreter's lock held.
+HOST_LIBRARY, STEPS_LIBRARY = "host", "steps"
+HOST_LIBRARIES: Dict[str, tuple] = {
+    HOST_LIBRARY: ("host/lgml_host.c", ["host/lgml_host.h"], ["-O2"]),
+    STEPS_LIBRARY: ("host/lgml_steps.c", [], ["-O3"]),
+}
+CC_FLAGS = ["-std=c11", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall"]
 _loaded: Dict[str, ctypes.CDLL] = {}
 _lock = threading.Lock()
 
@@ -126,8 +130,9 @@ def _find_build_dir() -> Path:
 
 def _digest(name: str) -> str:
     h = hashlib.sha256()
-    if name == HOST_LIBRARY:
-        files, flags = [HOST_SOURCE] + HOST_HEADERS, CC_FLAGS
+    if name in HOST_LIBRARIES:
+        src, headers, extra = HOST_LIBRARIES[name]
+        files, flags = [src] + headers, CC_FLAGS + extra
     else:
         src, extra = LIBRARIES[name]
         files, flags = [src] + _HEADERS + list(LIBRARY_HEADERS.get(name, [])), NVCC_FLAGS + list(extra)
@@ -156,15 +161,15 @@ def _say(msg: str) -> None:
 
 def compile_library(name: str, verbose: bool = True) -> Path:
     """Compile one library if its object is not there yet; returns the object's path."""
-    if name not in LIBRARIES and name != HOST_LIBRARY:
+    if name not in LIBRARIES and name not in HOST_LIBRARIES:
         raise KernelBuildError(f"unknown kernel library '{name}'")
     out = library_path(name)
     if out.exists():
         return out
     tmp = out.with_suffix(f".tmp{os.getpid()}.so")
-    if name == HOST_LIBRARY:
-        src = HOST_SOURCE
-        cmd = [find_cc()] + CC_FLAGS + ["-I", str(HERE / "host"), str(HERE / src), "-o", str(tmp), "-lm"]
+    if name in HOST_LIBRARIES:
+        src, _, extra = HOST_LIBRARIES[name]
+        cmd = [find_cc()] + CC_FLAGS + extra + ["-I", str(HERE / "host"), str(HERE / src), "-o", str(tmp), "-lm"]
         if verbose:
             _say(f"compiling {src} ...")
     else:
@@ -212,7 +217,7 @@ def load(name: str) -> ctypes.CDLL:
         if lib is None:
             path = compile_library(name)
             try:
-                lib = ctypes.CDLL(str(path))
+                lib = (ctypes.PyDLL if name == STEPS_LIBRARY else ctypes.CDLL)(str(path))
             except OSError as e:
                 raise KernelBuildError(f"cannot load {path}: {e}") from None
             _loaded[name] = lib
@@ -221,7 +226,7 @@ def load(name: str) -> ctypes.CDLL:
 
 def build_all(names: Optional[Iterable[str]] = None, jobs: int = 0, verbose: bool = True) -> List[Path]:
     """Compile every library (in parallel); used by the build check and before a first run."""
-    names = list(names or list(LIBRARIES) + [HOST_LIBRARY])
+    names = list(names or list(LIBRARIES) + list(HOST_LIBRARIES))
     jobs = jobs or min(len(names), os.cpu_count() or 1)
     with ThreadPoolExecutor(max_workers=jobs) as ex:
         return list(ex.map(lambda n: compile_library(n, verbose), names))

@@ -16,11 +16,14 @@ built (the reference fills an (n, window) mask on the host each pass,
 """
 from __future__ import annotations
 
+from ctypes import byref, c_int64
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence
 
 import numpy as np
 import torch
+
+from ..host import steps
 
 
 @dataclass
@@ -67,11 +70,16 @@ class StepBatch:
 
     ``table_widths`` forces the width of each group's block table and ``device_buffer``
     makes the views live in a buffer the caller keeps: both are what a captured CUDA graph
-    needs, since its kernels were recorded with fixed addresses and strides."""
+    needs, since its kernels were recorded with fixed addresses and strides.
+
+    ``lists``: which tiles and pieces the layers of this model have asked for in steps so far; this step's then come
+    with its one copy, and what a layer asks for that is not among them is added (a copy of its own this time)."""
+
+    MAX_LISTS = 16
 
     def __init__(self, cache_manager, requests: Sequence, tokens: Sequence[Sequence[int]], want: Sequence[Sequence[int]],
                  device, pinned: Optional[torch.Tensor] = None, table_widths: Optional[Sequence[int]] = None,
-                 device_buffer: Optional[torch.Tensor] = None):
+                 device_buffer: Optional[torch.Tensor] = None, lists: Optional[Dict[tuple, None]] = None):
         cm = cache_manager
         self.cache_manager = cm
         self.requests = list(requests)
@@ -91,12 +99,12 @@ class StepBatch:
         self.replayed = False           # are its launches recorded, and run again for other contexts?
         self.after_staged_copy = None   # called after a later copy out of the pinned buffer (its owner marks the buffer busy again)
 
-        # Everything below is array arithmetic: a prompt portion brings thousands of tokens, and a
-        # Python loop over them would cost as much as the step's first layers.
-        tok_arrays = [np.asarray(t, dtype=np.int64).reshape(-1) for t in tokens]
-        lens_a = np.asarray(lens, dtype=np.int64)
-        starts = np.zeros(S + 1, dtype=np.int64)
-        np.cumsum(lens_a, out=starts[1:])
+        # Rows of tokens are written by C: a prompt portion brings thousands of them, and Python's way with them costs as much as
+        # the step's first layers.
+        self._lens, self._pos0 = (c_int64 * S)(*lens), (c_int64 * S)(*self.pos0)
+        starts = [0]
+        for n in lens:
+            starts.append(starts[-1] + n)
         rows: List[int] = []
         self.rows_of_seq: List[List[int]] = []
         for s, w in enumerate(want):
@@ -105,7 +113,7 @@ class StepBatch:
                 if not 0 <= i < lens[s]:
                     raise IndexError(f"wanted place {i} is outside the {lens[s]} tokens request {self.requests[s].id!r} brings")
                 mine.append(len(rows))
-                rows.append(int(starts[s]) + int(i))
+                rows.append(starts[s] + int(i))
             self.rows_of_seq.append(mine)
         self.n_rows = len(rows)
 
@@ -114,7 +122,12 @@ class StepBatch:
             tables.append(cm.block_table_rows(self.requests, g, table_widths[g] if table_widths else None))
         self.table_width = [len(t[0]) if t else 1 for t in tables]
         n_rows_field = max(len(rows), 1)
-        total = 3 * N + (S + 1) + 3 * S + n_rows_field + S * sum(self.table_width)
+        described = total = 3 * N + (S + 1) + 3 * S + n_rows_field + S * sum(self.table_width)
+        self._lists = lists
+        ahead = [k for k in lists or () if self._wanted(k)]
+        total += sum(self._room(k) + 3 for k in ahead)          # (each from a 16-byte boundary)
+        if pinned is None or pinned.numel() < total or device_buffer is not None:
+            ahead, total = [], described
         if pinned is not None and pinned.numel() >= total:
             host = pinned[:total]
             self._pinned, self._pinned_used = pinned, total
@@ -122,16 +135,12 @@ class StepBatch:
             host = torch.empty(total, dtype=torch.int32)
             self._pinned, self._pinned_used = None, 0
         h = host.numpy()
-        seq_of = np.repeat(np.arange(S, dtype=np.int64), lens_a)
         off = 0
-        h[off:off + N] = np.concatenate(tok_arrays) if S else 0
-        off += N
-        # position of token j of request s: its first position + j
-        h[off:off + N] = np.asarray(self.pos0, dtype=np.int64)[seq_of] + (np.arange(N, dtype=np.int64) - starts[seq_of]) if N else 0
-        off += N
-        h[off:off + N] = seq_of
-        off += N
-        h[off:off + S + 1] = starts
+        for t, n in zip(tokens, lens):
+            h[off:off + n] = t if isinstance(t, np.ndarray) else np.asarray(t, dtype=np.int64).reshape(-1)
+            off += n
+        steps().lgml_steps_rows(host.data_ptr() + 4 * N, S, self._lens, self._pos0)
+        off = 3 * N
         off += S + 1
         h[off:off + S] = self.pos0
         off += S
@@ -145,6 +154,15 @@ class StepBatch:
             if S:
                 h[off:off + S * w] = np.asarray(t, dtype=np.int64).reshape(-1)
             off += S * w
+        written = []
+        for k in ahead:
+            off = -(-off // 4) * 4
+            n, shape = self._write(k, host.data_ptr() + 4 * off)
+            written.append((k, off, n, shape))
+            off += n
+        if ahead:
+            total = self._pinned_used = off
+            host = pinned[:total]
         if device_buffer is not None:
             if device_buffer.numel() < total:
                 raise ValueError("the step's description does not fit the buffer kept for it")
@@ -172,35 +190,52 @@ class StepBatch:
         r = take(max(len(rows), 1))
         self.logit_rows = r[: len(rows)]
         self.block_tables = [take(S * w).view(S, w) for w in self.table_width]
+        for k, at, n, shape in written:
+            self._tiles[k] = self._views(k, dev[at:at + n], shape)
 
-    def attention_tiles(self, tile_tokens: int, longer_than: int = 0) -> torch.Tensor:
+    # ---- tiles and pieces: ("tiles", tokens, longer than), ("pieces", tokens), ("chunks", tokens, longer than) ----
+    def _wanted(self, key) -> bool:
+        return key[0] != "chunks" or self.max_q_len > key[2]
+
+    def _room(self, key) -> int:
+        """Most 32-bit integers that the list takes."""
+        n = sum(-(-x // key[1]) for x in self.seq_lens)
+        return 4 * n if key[0] == "tiles" else 2 * n + 2 * self.n_seqs + 1
+
+    def _write(self, key, at: int):
+        """The list at address ``at``: (integers, what ``_views`` has to know of it)."""
+        if key[0] == "tiles":
+            n = steps().lgml_steps_tiles(at, self.n_seqs, self._lens, self._pos0, key[1], key[2])
+            return 4 * n, n
+        reqs = c_int64()
+        n = steps().lgml_steps_pieces(at, self.n_seqs, self._lens, key[1], key[2] if key[0] == "chunks" else -1, byref(reqs))
+        return 2 * n + reqs.value + 1 + (reqs.value if key[0] == "chunks" else 0), (n, reqs.value)
+
+    def _views(self, key, flat, shape):
+        if key[0] == "tiles":
+            return flat.view(-1, 4)
+        n, reqs = shape
+        rows, first = flat[:2 * n].view(-1, 2), flat[2 * n:2 * n + reqs + 1]
+        return (rows, first) if key[0] == "pieces" else ScanChunks(rows, first, flat[2 * n + reqs + 1:], key[2], reqs < self.n_seqs, key[1])
+
+    def _list(self, key, remember: bool = True):
+        cached = self._tiles.get(key)
+        if cached is None:
+            if remember and self._lists is not None and len(self._lists) < self.MAX_LISTS:
+                self._lists[key] = None
+            arr = np.empty(self._room(key), dtype=np.int32)
+            n, shape = self._write(key, arr.ctypes.data)
+            cached = self._tiles[key] = self._views(key, self._to_device(arr[:n]), shape)
+        return cached
+
+    def attention_tiles(self, tile_tokens: int, longer_than: int = 0, remember: bool = True) -> torch.Tensor:
         """The new tokens cut into tiles of at most ``tile_tokens`` consecutive tokens of one
         request, for the prefill attention kernel: int32 [n_tiles, 4] on the device, rows
         (request row, first token row, tokens, 0), the tile with the most keys to visit first:
         the kernel starts its CTAs in this order, and a long tile that starts last would run on
-        alone at the end.  Only of requests that bring more than ``longer_than`` tokens.  Made once per tile size."""
-        key = (tile_tokens, longer_than) if longer_than else tile_tokens
-        cached = self._tiles.get(key)
-        if cached is None:
-            pieces, start = [], 0
-            for s, n in enumerate(self.seq_lens):
-                if n <= longer_than:
-                    start += n
-                    continue
-                t0 = np.arange(0, n, tile_tokens, dtype=np.int32)
-                part = np.empty((t0.size, 4), dtype=np.int32)
-                part[:, 0] = s
-                part[:, 1] = start + t0
-                part[:, 2] = np.minimum(tile_tokens, n - t0)
-                part[:, 3] = self.pos0[s] + np.minimum(t0 + tile_tokens, n)         # how far it has to look
-                pieces.append(part)
-                start += n
-            arr = np.concatenate(pieces) if pieces else np.zeros((0, 4), dtype=np.int32)
-            arr = arr[np.argsort(-arr[:, 3], kind="stable")]
-            arr[:, 3] = 0
-            cached = self._to_device(arr.reshape(-1)).view(-1, 4)
-            self._tiles[key] = cached
-        return cached
+        alone at the end.  Only of requests that bring more than ``longer_than`` tokens.  Made once per tile size (``remember``: for later
+        steps of the model too).  (What comes fourth in a row has done its part when they are sorted.)"""
+        return self._list(("tiles", tile_tokens, longer_than), remember)
 
     def tiles_and_short(self, tile_tokens: int, limit, rule):
         """The step's requests in two: (tiles as ``attention_tiles`` of those that bring more than ``limit(seq_lens)`` tokens, the rows of the
@@ -216,7 +251,7 @@ class StepBatch:
             if rows.size == self.n_tokens:
                 cached = (None, None, longest)
             else:
-                cached = (self.attention_tiles(tile_tokens, up_to if rows.size else 0), self._to_device(rows.astype(np.int32)) if rows.size else None, longest)
+                cached = (self.attention_tiles(tile_tokens, up_to if rows.size else 0, remember=False), self._to_device(rows.astype(np.int32)) if rows.size else None, longest)
             self._tiles[key] = cached
         return cached
 
@@ -241,41 +276,14 @@ class StepBatch:
         recurrence that runs the pieces side by side: (int32 [n_pieces, 2] rows [first token row, the row past the
         last), a request's pieces in a row; int32 [requests + 1], the first piece of every request).  Made once per
         piece size."""
-        cached = self._tiles.get(("pieces", piece_tokens))
-        if cached is None:
-            lens = np.asarray(self.seq_lens, dtype=np.int64)
-            counts = -(-lens // piece_tokens)
-            first = np.concatenate([[0], np.cumsum(counts)])
-            ends = np.cumsum(lens)
-            of = np.repeat(np.arange(len(lens)), counts)                              # the request of every piece
-            lo = (ends - lens)[of] + (np.arange(first[-1]) - first[of]) * piece_tokens
-            pieces = np.stack([lo, np.minimum(lo + piece_tokens, ends[of])], axis=1)
-            both = self._to_device(np.concatenate([pieces.reshape(-1), first]).astype(np.int32))
-            cached = (both[:2 * len(pieces)].view(-1, 2), both[2 * len(pieces):])
-            self._tiles[("pieces", piece_tokens)] = cached
-        return cached
+        return self._list(("pieces", piece_tokens))
 
     def scan_chunks(self, chunk_tokens: int, longer_than: int) -> Optional[ScanChunks]:
         """The long requests of this step in chunks (None when no request brings more than ``longer_than`` tokens), for a
         recurrence that takes those as matrix products and the others token by token.  Made once per chunk size."""
         if self.max_q_len <= longer_than:
             return None
-        key = ("chunks", chunk_tokens, longer_than)
-        cached = self._tiles.get(key)
-        if cached is None:
-            lens = np.asarray(self.seq_lens, dtype=np.int64)
-            reqs = np.nonzero(lens > longer_than)[0]
-            start = (np.cumsum(lens) - lens)[reqs]
-            end = start + lens[reqs]
-            counts = -(-lens[reqs] // chunk_tokens)
-            first = np.concatenate([[0], np.cumsum(counts)])
-            of = np.repeat(np.arange(len(reqs)), counts)                             # the long request of every chunk
-            lo = start[of] + (np.arange(first[-1]) - first[of]) * chunk_tokens
-            rows = np.stack([lo, np.minimum(lo + chunk_tokens, end[of])], axis=1)
-            flat = self._to_device(np.concatenate([rows.reshape(-1), first, reqs]).astype(np.int32))
-            a, b = rows.size, rows.size + first.size
-            cached = self._tiles[key] = ScanChunks(flat[:a].view(-1, 2), flat[a:b], flat[b:], longer_than, len(reqs) < len(lens), chunk_tokens)
-        return cached
+        return self._list(("chunks", chunk_tokens, longer_than))
 
     @staticmethod
     def buffer_ints(n_tokens: int, n_seqs: int, n_rows: int, table_widths: Sequence[int]) -> int:

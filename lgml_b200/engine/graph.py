@@ -108,7 +108,7 @@ class DecodeBatch:
 class DecodeGraph:
     """One captured decode step of a fixed batch size."""
 
-    RING = 4
+    RING = 8          # steps that the host may be ahead: opening 64 requests takes as long as five of their steps
 
     def __init__(self, runner, S: int, reach: Optional[int] = None, even: bool = False):
         self.runner = runner

@@ -15,7 +15,7 @@ from typing import Hashable, List, Optional, Sequence, Tuple
 import numpy as np
 import torch
 
-from .. import ops
+from .. import host, ops
 from ..cache import CacheManager, PoolFull, Request
 from ..models import build_model
 from ..weights import load_tensors, random_tensors
@@ -56,6 +56,18 @@ def context_reach(lengths: Sequence[int]) -> Tuple[int, bool]:
     return reach, 2 * min(lengths) > reach
 
 
+def token_array(tokens: Sequence[int], vocab: int) -> Tuple[np.ndarray, Optional[int]]:
+    """A portion's token ids as an array, and the first that is outside the vocabulary."""
+    if type(tokens) is list:
+        arr = np.empty(len(tokens), dtype=np.int32)
+        at = host.steps().lgml_steps_ints(tokens, arr.ctypes.data, len(tokens), vocab)
+        if at != host.NOT_INTS:
+            return arr, None if at < 0 else int(tokens[at])
+    arr = np.asarray(tokens, dtype=np.int64)
+    bad = np.nonzero((arr < 0) | (arr >= vocab))[0]
+    return arr, int(arr[bad[0]]) if bad.size else None
+
+
 class StepError(ValueError):
     """A step the runner refuses before anything is launched."""
 
@@ -79,6 +91,7 @@ class ModelRunner:
         max_pos = model.max_position or (n_pages * self.cache.page_size)
         self._graph_widths = [min(g.pool.n_pages, -(-max_pos // self.cache.page_size)) for g in self.cache.groups]
         self.graph_replays = 0
+        self._lists = {}                # what the layers ask of a step's description beside it (StepBatch.lists)
 
     # ---- construction ------------------------------------------------------------------
     @classmethod
@@ -133,8 +146,9 @@ class ModelRunner:
         self.cache.close(req)
 
     # ---- the step ----------------------------------------------------------------------
-    def validate(self, entries: Sequence[Tuple[Request, Sequence[int], Sequence[int]]]) -> None:
-        seen = set()
+    def validate(self, entries: Sequence[Tuple[Request, Sequence[int], Sequence[int]]]) -> List[Sequence[int]]:
+        """Refuses what a step cannot run; returns every entry's tokens, those of portions as arrays."""
+        seen, brought = set(), []
         vocab = self.model.vocab_size
         max_pos = self.model.max_position
         if not entries:
@@ -148,11 +162,12 @@ class ModelRunner:
             if len(tokens) == 0:
                 raise StepError(f"request {req.id!r} brings no tokens")
             if len(tokens) > 16:
-                arr = np.asarray(tokens, dtype=np.int64)
-                bad = np.nonzero((arr < 0) | (arr >= vocab))[0]
-                if bad.size:
-                    raise StepError(f"request {req.id!r}: token id {int(arr[bad[0]])} is outside the vocabulary of {vocab}")
+                arr, bad = token_array(tokens, vocab)
+                if bad is not None:
+                    raise StepError(f"request {req.id!r}: token id {bad} is outside the vocabulary of {vocab}")
+                brought.append(arr)
             else:
+                brought.append(tokens)
                 for t in tokens:
                     if not 0 <= int(t) < vocab:
                         raise StepError(f"request {req.id!r}: token id {t} is outside the vocabulary of {vocab}")
@@ -161,6 +176,7 @@ class ModelRunner:
                     raise StepError(f"request {req.id!r}: wanted place {i} is outside the {len(tokens)} tokens it brings")
             if max_pos is not None and req.n_tokens + len(tokens) > max_pos:
                 raise StepError(f"request {req.id!r}: context full ({req.n_tokens} + {len(tokens)} tokens > {max_pos} positions)")
+        return brought
 
     def _reserve_all(self, wanted: Sequence[Tuple[Request, int]]) -> None:
         """Pages for every entry of a step, or for none: when one entry finds no page, the
@@ -176,7 +192,7 @@ class ModelRunner:
     def step(self, entries: Sequence[Tuple[Request, Sequence[int], Sequence[int]]]) -> torch.Tensor:
         """entries: (request, its next tokens, the places among them whose logits are
         wanted).  Returns float32 [wanted, vocab] in the order of entries and places."""
-        self.validate(entries)
+        brought = self.validate(entries)
         self._reserve_all([(req, len(tokens)) for req, tokens, _ in entries])
         stage = self._pinned[self.steps % len(self._pinned)]
         if stage[1] is not None:
@@ -187,8 +203,8 @@ class ModelRunner:
         elif self._graphs_now() and self._prompt_graph_fits(entries):
             logits = self._prompt_graph_step(entries[0], stage)
         else:
-            batch = StepBatch(self.cache, [e[0] for e in entries], [e[1] for e in entries], [e[2] for e in entries],
-                              self.rt.device, stage[0])
+            batch = StepBatch(self.cache, [e[0] for e in entries], brought, [e[2] for e in entries],
+                              self.rt.device, stage[0], lists=self._lists)
             self._mark_busy(stage)
             batch.after_staged_copy = lambda: self._mark_busy(stage)
             self.last_batch = batch

@@ -1,6 +1,7 @@
-"""ctypes bindings of the host library (``csrc/host/lgml_host.c``): the safetensors reader and
-the sampler, in C as in mischief/lgml (``src/safetensors.c``, ``src/sample.c``).  Built with the
-system's C compiler the first time something needs it; there is no other implementation."""
+"""ctypes bindings of the host libraries: the safetensors reader and the sampler
+(``csrc/host/lgml_host.c``), in C as in mischief/lgml (``src/safetensors.c``, ``src/sample.c``), and what step
+descriptions and page keys are made of (``csrc/host/lgml_steps.c``).  Built with the
+system's C compiler the first time something needs them; there is no other implementation."""
 from __future__ import annotations
 
 import ctypes
@@ -51,6 +52,33 @@ def lib() -> ctypes.CDLL:
         l.lgml_sampler_logprobs.restype, l.lgml_sampler_logprobs.argtypes = c_int, [c_void_p, c_int32, c_int, POINTER(c_double), c_void_p, c_void_p]
         _lib = l
     return _lib
+
+
+_steps: Optional[ctypes.PyDLL] = None
+
+
+def steps() -> ctypes.PyDLL:
+    global _steps
+    if _steps is None:
+        l = csrc.load(csrc.STEPS_LIBRARY)
+        l.lgml_steps_ints.restype, l.lgml_steps_ints.argtypes = c_int64, [ctypes.py_object, c_void_p, c_int64, c_int64]
+        l.lgml_steps_rows.restype, l.lgml_steps_rows.argtypes = None, [c_void_p, c_int64, c_void_p, c_void_p]
+        l.lgml_steps_tiles.restype, l.lgml_steps_tiles.argtypes = c_int64, [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64]
+        l.lgml_steps_pieces.restype, l.lgml_steps_pieces.argtypes = c_int64, [c_void_p, c_int64, c_void_p, c_int64, c_int64, POINTER(c_int64)]
+        l.lgml_steps_page_keys.restype = c_int
+        l.lgml_steps_page_keys.argtypes = [ctypes.py_object, c_int64, c_int64, c_int64, c_char_p, c_int64, c_void_p, c_int]
+        _steps = l
+    return _steps
+
+
+NOT_INTS = -2          # of lgml_steps_ints and lgml_steps_page_keys: not a list of integers, or one beyond 64 bits
+
+
+def page_keys(tokens: list, first: int, n: int, page: int, key: bytes, plain: bool = False) -> Optional[bytes]:
+    """The SHA-256 keys (32 bytes each, one behind the other) of full pages ``first`` .. ``first + n - 1`` of a list of token ids, ``key`` being the one
+    before them: each hashes the key before it and its tokens as 64-bit integers.  None when the list holds something else."""
+    out = ctypes.create_string_buffer(32 * n)
+    return out.raw if steps().lgml_steps_page_keys(tokens, first, n, page, key, len(key), out, plain) == 0 else None
 
 
 def last_error() -> str:

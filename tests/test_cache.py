@@ -263,3 +263,35 @@ def test_a_step_that_finds_no_page_leaves_the_books_as_they_were():
     with pytest.raises(ValueError, match="cannot cut"):
         cm.unreserve(a, [0, 0])                     # never below what holds keys
     cm.check()
+
+
+@pytest.mark.parametrize("page", [1, 7, 64, 100])
+@pytest.mark.parametrize("plain", [False, True])
+def test_page_keys_are_sha256_chains(page, plain):
+    """The keys of pages against hashlib, with and without the processor's SHA instructions, from the middle of a chain too; ids of any 64-bit
+    value; what is no list of such integers is left to the caller."""
+    import hashlib
+    import random
+    import struct
+
+    from lgml_b200 import host
+
+    rng = random.Random(page)
+    tokens = [rng.choice([rng.randrange(32000), -rng.randrange(1, 1 << 62), rng.randrange(1 << 62), True]) for _ in range(12 * page)]
+    key, want = b"start", []
+    for b in range(12):
+        want.append(hashlib.sha256((want[-1] if want else key) + struct.pack(f"<{page}q", *tokens[b * page:(b + 1) * page])).digest())
+    assert host.page_keys(tokens, 0, 12, page, key, plain) == b"".join(want)
+    assert host.page_keys(tokens, 5, 3, page, want[4], plain) == b"".join(want[5:8])
+    assert host.page_keys(tokens, 5, 8, page, want[4], plain) is None and host.page_keys(tokens[:-1] + [1 << 63], 0, 12, page, key, plain) is None
+    assert host.page_keys(tokens[:-1] + [0.5], 0, 12, page, key, plain) is None
+
+
+def test_keys_do_not_depend_on_the_kind_of_sequence():
+    import numpy as np
+
+    cm = _prefix_manager()
+    tokens = list(range(5, 5 + 40 * 64))
+    want = list(cm._keys(tokens, 40))
+    assert len(set(want)) == 40
+    assert list(cm._keys(tuple(tokens), 40)) == want and list(cm._keys([np.int64(t) for t in tokens], 40)) == want and list(cm._keys(np.array(tokens), 40)) == want

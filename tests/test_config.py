@@ -240,3 +240,39 @@ def test_end_tokens_of_generation_config_join_those_of_config(tmp_path):
     (tmp_path / "generation_config.json").write_text(json.dumps({"eos_token_id": "x"}))
     with pytest.raises(ConfigError, match="eos_token_id"):
         load_config(tmp_path)
+
+
+@pytest.mark.parametrize("lens,pos0", [([1], [5]), ([64], [0]), ([65, 1, 300, 2, 300], [0, 900, 12, 63, 40]), ([28, 27, 29], [7, 7, 7])])
+def test_tiles_and_pieces_of_a_step(lens, pos0):
+    """Against the rule in Python, asked for one by one and sent with the step's description; from 16-byte boundaries there."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from lgml_b200.engine.batch import StepBatch
+
+    reqs = [SimpleNamespace(id=i, slot=i, n_tokens=p, tables=[]) for i, p in enumerate(pos0)]
+    ids = [[7 * s + j for j in range(n)] for s, n in enumerate(lens)]
+    lists = {}
+    starts = [sum(lens[:s]) for s in range(len(lens))]
+    for round_ in range(2):
+        pinned = torch.full((4096,), -7, dtype=torch.int32)
+        b = StepBatch(SimpleNamespace(groups=[]), reqs, ids, [[n - 1] for n in lens], torch.device("cpu"), pinned, lists=lists)
+        assert len(b._tiles) == (0 if round_ == 0 else len(lists))
+        assert b.token_ids.tolist() == sum(ids, []) and b.seq_start.tolist() == starts + [sum(lens)] and b.logit_rows.tolist() == [a + n - 1 for a, n in zip(starts, lens)]
+        assert b.positions.tolist() == [p + j for p, n in zip(pos0, lens) for j in range(n)] and b.seq_of_token.tolist() == [s for s, n in enumerate(lens) for _ in range(n)]
+        for tile, longer in ((16, 0), (64, 0), (16, 27)):
+            want = [(s, a + t, min(tile, n - t), p + min(t + tile, n)) for s, (a, n, p) in enumerate(zip(starts, lens, pos0)) if n > longer for t in range(0, n, tile)]
+            got = b.attention_tiles(tile, longer)
+            assert got.tolist() == [[s, a, n, 0] for s, a, n, _ in sorted(want, key=lambda r: -r[3])]
+            assert round_ == 0 or (got.data_ptr() - b._dev.data_ptr()) % 16 == 0
+        pieces, first = b.scan_pieces(16)
+        want = [[[a + t, a + min(t + 16, n)] for t in range(0, n, 16)] for a, n in zip(starts, lens)]
+        assert pieces.tolist() == sum(want, []) and first.tolist() == [sum(map(len, want[:s])) for s in range(len(lens) + 1)]
+        got = b.scan_chunks(32, 27)
+        long = [s for s, n in enumerate(lens) if n > 27]
+        assert (got is None) == (not long)
+        if long:
+            want = [[[starts[s] + t, starts[s] + min(t + 32, lens[s])] for t in range(0, lens[s], 32)] for s in long]
+            assert got.rows.tolist() == sum(want, []) and got.requests.tolist() == long and got.short == (len(long) < len(lens))
+            assert got.first.tolist() == [sum(map(len, want[:s])) for s in range(len(long) + 1)] and (got.longer_than, got.chunk_tokens) == (27, 32)
