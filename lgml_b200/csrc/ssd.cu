@@ -14,6 +14,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "tf32_halves.cuh"
 
 LGML_DEFINE_LAST_ERROR(lgml_ssd)
 
@@ -186,6 +187,257 @@ __global__ void __launch_bounds__(256) ssd_chain_kernel(float *__restrict__ scra
     *st = S;
 }
 
+// ---- a long portion in chunks of 64 tokens, as matrix products ------------------------------------------------
+// With G_i the sum of a chunk's log decays up to token i (in double precision, so that a difference keeps float32's) and S0 the state
+// ahead of the chunk:
+//
+//   left behind  e^(G_last) S0 + sum_j e^(G_last - G_j) dt_j x_j B_j^T
+//   y_i          e^(G_i) S0 C_i + sum_(j <= i) e^(G_i - G_j) dt_j (C_i . B_j) x_j + D x_i
+//
+// The first kernel gives what every chunk leaves from a zero state, ssd_chain_kernel the state each starts from, the second kernel y: the
+// chunks side by side.  The products go through the tensor cores in halves (tf32_halves.cuh).  Bound by what a block waits for between its
+// few products (two blocks an SM); 32 heads of 64 columns by 128 entries, scans of every chunk from zero and from its start, and now: 129 tokens
+// 86 and 27 us, 1,012 tokens in two requests 208 and 65, 2,048 tokens 306 and 105.  Off 64 bits 2.0e-7 and 1.6e-7 (y, 1,012 tokens), with
+// decays of a few per cent a chunk 1.9e-6 and 1.8e-7.
+constexpr int CHUNK = 64, CHUNK_THREADS = 256;
+constexpr int CHUNK_N = 128, CHUNK_P = 64;                  // most state entries a column; columns of a block
+constexpr int LD_T = 8;                                     // rows that are walked along k: row lengths of 8 over a multiple of 32 put k = 0 .. 3 of
+constexpr int LD_B = CHUNK_N + LD_T, LD_X = CHUNK_P + LD_T; // eight neighbouring columns into all banks
+constexpr int LD_C = CHUNK_N + 16;                          // rows read 16 bytes a lane, two rows at a time: 16 over
+constexpr int LD_M = CHUNK + 4;
+
+struct ChunkArgs {
+    const float *xbc;
+    int ldx;
+    const float *dt_raw;
+    int ldd;
+    const float *dt_bias, *a_log, *d_skip;
+    const int *chunks;              // [n_chunks][2]: first token, past the last
+    float *left, *decay;            // [n_chunks][Hs P N], [n_chunks][Hs]
+    float *y;
+    int ldy, Hs, G, P, N;
+};
+
+__device__ __forceinline__ void copy_16(float *dst, const float *src, bool there) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_there() { asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory"); }
+
+// dt and the sums of the log decays of a chunk's tokens (0 behind the last), by one warp
+__device__ __forceinline__ void chunk_decays(const ChunkArgs &p, int h, int t0, int nt, float *dts, double *Gs) {
+    const int lane = threadIdx.x & 31;
+    const float a = expf(__ldg(p.a_log + h)), bias = __ldg(p.dt_bias + h);
+    double l[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int i = 2 * lane + u;
+        const float dt = i < nt ? softplus_(act_load(p.dt_raw + (size_t)(t0 + i) * p.ldd + h) + bias) : 0.f;
+        dts[i] = dt;
+        l[u] = -(double)(a * dt);
+    }
+    double sum = l[0] + l[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double up = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += up;
+    }
+    Gs[2 * lane] = sum - l[1], Gs[2 * lane + 1] = sum;
+}
+
+// A result that is no finite number, formed again by itself: what an infinity loses between its halves, or where a later token's
+// meets the zero of an earlier row.
+__device__ __noinline__ float left_again(const float *b, const float *x, int nt) {
+    float v = 0.f;
+    for (int t = 0; t < nt; ++t) v = fmaf(b[t * LD_B], x[t * LD_X], v);
+    return v;
+}
+__device__ __noinline__ float y_again(const float *c, const float *B, int ldx, const float *s0, const float *x, const double *G, const float *dts, int i, int N) {
+    float old = 0.f, now = 0.f;
+    for (int n = 0; n < N; ++n) old = fmaf(c[n], s0[n], old);
+    for (int t = 0; t <= i; ++t) {
+        float dot = 0.f;
+        for (int n = 0; n < N; ++n) dot = fmaf(c[n], act_load(B + (size_t)t * ldx + n), dot);
+        now = fmaf(dot * (expf((float)(G[i] - G[t])) * dts[t]), x[t * LD_X], now);
+    }
+    return fmaf(expf((float)G[i]), old, now);
+}
+
+// Block: (chunk, head, 64 columns).  A warp has 32 state entries of 32 columns.
+__global__ void __launch_bounds__(CHUNK_THREADS) ssd_chunk_left_kernel(const ChunkArgs p) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm[];
+    float *Bs = sm, *Xs = Bs + CHUNK * LD_B;
+    __shared__ float dts[CHUNK], fs[CHUNK];
+    __shared__ double Gs[CHUNK];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+    const int c = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * CHUNK_P, cols = min(CHUNK_P, p.P - col0);
+    const int t0 = p.chunks[2 * c], nt = min(p.chunks[2 * c + 1] - t0, CHUNK);
+    const float *B = p.xbc + (size_t)t0 * p.ldx + p.Hs * p.P + (h / (p.Hs / p.G)) * p.N, *X = p.xbc + (size_t)t0 * p.ldx + h * p.P + col0;
+    for (int i = tid; i < CHUNK * (CHUNK_N / 4); i += CHUNK_THREADS) {
+        const int r = i / (CHUNK_N / 4), n = i % (CHUNK_N / 4) * 4;
+        const bool there = r < nt && n < p.N;
+        copy_16(Bs + r * LD_B + n, there ? B + (size_t)r * p.ldx + n : B, there);
+    }
+    if (warp == 0) {
+        chunk_decays(p, h, t0, nt, dts, Gs);
+        __syncwarp();
+        for (int i = lane; i < CHUNK; i += 32) fs[i] = expf((float)(Gs[CHUNK - 1] - Gs[i])) * dts[i];
+        if (blockIdx.z == 0 && lane == 0) p.decay[(size_t)c * p.Hs + h] = expf((float)Gs[CHUNK - 1]);
+    }
+    __syncthreads();
+    for (int i = tid; i < CHUNK * (CHUNK_P / 4); i += CHUNK_THREADS) {
+        const int r = i / (CHUNK_P / 4), x = i % (CHUNK_P / 4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < nt && x < cols) v = act_load(reinterpret_cast<const float4 *>(X + (size_t)r * p.ldx + x));
+        const float f = fs[r];
+        *reinterpret_cast<float4 *>(Xs + r * LD_X + x) = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+    }
+    copies_there();
+    __syncthreads();
+    const int n0 = (warp & 3) * 32, x0 = (warp >> 2) * 32;
+    if (n0 >= p.N || x0 >= cols) return;
+    float sum[2][4][4] = {};
+#pragma unroll 1
+    for (int k0 = 0; k0 < nt; k0 += 16) {
+        float w[2][2][4], a[4][4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const float *bk = Bs + (k0 + 4 * s + q) * LD_B + n0 + g, *xk = Xs + (k0 + 4 * s + q) * LD_X + x0 + g;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i >> 1][i & 1][s] = bk[8 * i], a[i][s] = xk[8 * i];
+        }
+        float4 wv[2][2], av[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            wv[i >> 1][i & 1] = make_float4(w[i >> 1][i & 1][0], w[i >> 1][i & 1][1], w[i >> 1][i & 1][2], w[i >> 1][i & 1][3]);
+            av[i] = make_float4(a[i][0], a[i][1], a[i][2], a[i][3]);
+        }
+        add_run<2, 4>(sum, wv, av);
+    }
+    float *out = p.left + ((size_t)c * p.Hs + h) * p.P * p.N + (size_t)col0 * p.N;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int n = n0 + i * 16 + (e >> 1) * 8 + g, x = x0 + j * 8 + q * 2 + (e & 1);
+                if (n < p.N && x < cols) {
+                    float v = sum[i][j][e];
+                    if (!isfinite(v)) v = left_again(Bs + n, Xs + x, nt);
+                    out[(size_t)x * p.N + n] = v;
+                }
+            }
+}
+
+// Block: (chunk, `heads` heads of a group, 64 columns).  A warp has 16 tokens (four runs of them) and half of the columns; C B^T, the same for all
+// heads of a group, stays in its registers.
+constexpr size_t CHUNK_OUT_SMEM = sizeof(float) * (2 * CHUNK * LD_C + CHUNK * LD_X + CHUNK * LD_M);
+constexpr size_t CHUNK_LEFT_SMEM = sizeof(float) * CHUNK * (LD_B + LD_X);
+
+__global__ void __launch_bounds__(CHUNK_THREADS) ssd_chunk_out_kernel(const ChunkArgs p, int heads) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm[];
+    float *Cs = sm, *BS = Cs + CHUNK * LD_C, *Xs = BS + CHUNK * LD_C, *Ms = Xs + CHUNK * LD_X;       // BS: B, then a head's state
+    __shared__ float dts[CHUNK];
+    __shared__ double Gs[CHUNK];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+    const int c = blockIdx.x, h0 = blockIdx.y * heads, col0 = blockIdx.z * CHUNK_P, cols = min(CHUNK_P, p.P - col0);
+    const int t0 = p.chunks[2 * c], nt = min(p.chunks[2 * c + 1] - t0, CHUNK), kn = (p.N + 15) / 16 * 16;
+    const float *B = p.xbc + (size_t)t0 * p.ldx + p.Hs * p.P + (h0 / (p.Hs / p.G)) * p.N, *C = B + p.G * p.N;
+    for (int i = tid; i < CHUNK * (CHUNK_N / 4); i += CHUNK_THREADS) {
+        const int r = i / (CHUNK_N / 4), n = i % (CHUNK_N / 4) * 4;
+        const bool there = r < nt && n < p.N;
+        copy_16(BS + r * LD_C + n, there ? B + (size_t)r * p.ldx + n : B, there);
+        copy_16(Cs + r * LD_C + n, there ? C + (size_t)r * p.ldx + n : C, there);
+    }
+    copies_there();
+    __syncthreads();
+    const int i0 = (warp & 3) * 16, x0 = (warp >> 2) * 32;           // this warp's tokens, and its columns (of C B^T: earlier tokens)
+    float cb[1][4][4] = {};
+    if (x0 <= i0 + 15) {
+        for (int k = 0; k < kn; k += 16) {
+            float4 w[1][2], a[4];
+            w[0][0] = *reinterpret_cast<const float4 *>(Cs + (i0 + g) * LD_C + k + 4 * q);
+            w[0][1] = *reinterpret_cast<const float4 *>(Cs + (i0 + 8 + g) * LD_C + k + 4 * q);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) a[j] = *reinterpret_cast<const float4 *>(BS + (x0 + j * 8 + g) * LD_C + k + 4 * q);
+            add_run<1, 4>(cb, w, a);
+        }
+    }
+    for (int h = h0; h < h0 + heads; ++h) {
+        __syncthreads();                                             // the head before is done with BS, Xs, Ms and its decays
+        const float *S0 = p.left + ((size_t)c * p.Hs + h) * p.P * p.N + (size_t)col0 * p.N, *X = p.xbc + (size_t)t0 * p.ldx + h * p.P + col0;
+        for (int i = tid; i < CHUNK_P * (CHUNK_N / 4); i += CHUNK_THREADS) {
+            const int r = i / (CHUNK_N / 4), n = i % (CHUNK_N / 4) * 4;
+            const bool there = r < cols && n < p.N;
+            copy_16(BS + r * LD_C + n, there ? S0 + (size_t)r * p.N + n : S0, there);
+        }
+        for (int i = tid; i < CHUNK * (CHUNK_P / 4); i += CHUNK_THREADS) {
+            const int r = i / (CHUNK_P / 4), x = i % (CHUNK_P / 4) * 4;
+            const bool there = r < nt && x < cols;
+            copy_16(Xs + r * LD_X + x, there ? X + (size_t)r * p.ldx + x : X, there);
+        }
+        if (warp == 0) chunk_decays(p, h, t0, nt, dts, Gs);
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int i = i0 + (e >> 1) * 8 + g, t = x0 + j * 8 + q * 2 + (e & 1);
+                Ms[i * LD_M + t] = t <= i ? cb[0][j][e] * (expf((float)(Gs[i] - Gs[t])) * dts[t]) : 0.f;
+            }
+        copies_there();
+        __syncthreads();
+        if (x0 < cols && i0 < nt) {
+            float old[1][4][4] = {}, now[1][4][4] = {};
+            for (int k = 0; k < kn; k += 16) {
+                float4 w[1][2], a[4];
+                w[0][0] = *reinterpret_cast<const float4 *>(Cs + (i0 + g) * LD_C + k + 4 * q);
+                w[0][1] = *reinterpret_cast<const float4 *>(Cs + (i0 + 8 + g) * LD_C + k + 4 * q);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) a[j] = *reinterpret_cast<const float4 *>(BS + (x0 + j * 8 + g) * LD_C + k + 4 * q);
+                add_run<1, 4>(old, w, a);
+            }
+            for (int k = 0; k <= i0; k += 16) {                      // tokens behind this warp's last have no part
+                float w[2][4], a[4][4];
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    const int t = k + 4 * s + q;
+                    w[0][s] = Ms[(i0 + g) * LD_M + t], w[1][s] = Ms[(i0 + 8 + g) * LD_M + t];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) a[j][s] = Xs[t * LD_X + x0 + j * 8 + g];
+                }
+                float4 wv[1][2], av[4];
+                wv[0][0] = make_float4(w[0][0], w[0][1], w[0][2], w[0][3]), wv[0][1] = make_float4(w[1][0], w[1][1], w[1][2], w[1][3]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) av[j] = make_float4(a[j][0], a[j][1], a[j][2], a[j][3]);
+                add_run<1, 4>(now, wv, av);
+            }
+            const float skip = __ldg(p.d_skip + h);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int i = i0 + r * 8 + g;
+                const float kept = expf((float)Gs[i]);
+                if (i < nt) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int x = x0 + j * 8 + q * 2;
+                        if (x >= cols) continue;
+                        const float2 xv = *reinterpret_cast<const float2 *>(Xs + i * LD_X + x);
+                        float2 v = make_float2(fmaf(kept, old[0][j][2 * r], now[0][j][2 * r]), fmaf(kept, old[0][j][2 * r + 1], now[0][j][2 * r + 1]));
+                        if (!isfinite(v.x)) v.x = y_again(Cs + i * LD_C, B, p.ldx, BS + x * LD_C, Xs + x, Gs, dts, i, p.N);
+                        if (!isfinite(v.y)) v.y = y_again(Cs + i * LD_C, B, p.ldx, BS + (x + 1) * LD_C, Xs + x + 1, Gs, dts, i, p.N);
+                        *reinterpret_cast<float2 *>(p.y + (size_t)(t0 + i) * p.ldy + (size_t)h * p.P + col0 + x) = make_float2(fmaf(skip, xv.x, v.x), fmaf(skip, xv.y, v.y));
+                    }
+                }
+            }
+        }
+    }
+}
+
 // out[t, c] = (y[t, c] silu(z[t, c])) / rms over c's part * w[c]; block (token, part).  The gated values wait in shared
 // memory between the sum of squares and the division when a part fits there (keep != 0): y and z are then read once.
 template <typename TO, int NT>
@@ -318,4 +570,30 @@ LGML_API int lgml_ssd_chain(float *scratch, long long scratch_ld, const float *d
     dim3 grid((Hs * P * N + 255) / 256, n_seqs);
     lgml_launch(ssd_chain_kernel, grid, 256, 0, stream, scratch, scratch_ld, decay, state, state_ld, first_piece, slots, Hs, P * N);
     return lgml_launch_status("ssd_chain");
+}
+
+// A portion in chunks of 64 tokens: what every chunk leaves from a zero state (y null), or y from the states that ssd_chain made of it.  `left`: [n_chunks, Hs P N],
+// 16-byte aligned; N a multiple of 4 up to 128, P a multiple of 4, rows of xbc on 16 bytes.
+LGML_API int lgml_ssd_chunks(const float *xbc, int ldx, const float *dt_raw, int ldd, const float *dt_bias, const float *a_log, const float *d_skip,
+                             const int *chunks, int n_chunks, float *left, float *decay, float *y, int ldy, int Hs, int G, int P, int N, cudaStream_t stream) {
+    LGML_REQUIRE(n_chunks >= 0 && Hs > 0 && G > 0 && P > 0 && N > 0 && Hs % G == 0 && Hs <= 65535, "ssd_chunks: bad sizes");
+    LGML_REQUIRE(N % 4 == 0 && N <= CHUNK_N && P % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)xbc | (uintptr_t)left) & 15) == 0, "ssd_chunks: sizes or rows it does not take");
+    LGML_REQUIRE(ldx >= Hs * P + 2 * G * N && ldd >= Hs, "ssd_chunks: rows too short");
+    LGML_REQUIRE(y == nullptr || (ldy >= Hs * P && ldy % 2 == 0 && ((uintptr_t)y & 7) == 0), "ssd_chunks: rows too short or not aligned");
+    if (n_chunks == 0) return 0;
+    const ChunkArgs p = {xbc, ldx, dt_raw, ldd, dt_bias, a_log, d_skip, chunks, left, decay, y, ldy, Hs, G, P, N};
+    const int tiles = (P + CHUNK_P - 1) / CHUNK_P;
+    auto kernel_smem = [](const void *kernel, size_t smem) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); };
+    if (y == nullptr) {
+        if (kernel_smem((const void *)ssd_chunk_left_kernel, CHUNK_LEFT_SMEM) != cudaSuccess) return lgml_launch_status("ssd_chunks");
+        lgml_launch(ssd_chunk_left_kernel, dim3(n_chunks, Hs, tiles), CHUNK_THREADS, CHUNK_LEFT_SMEM, stream, p);
+    } else {
+        if (kernel_smem((const void *)ssd_chunk_out_kernel, CHUNK_OUT_SMEM) != cudaSuccess) return lgml_launch_status("ssd_chunks");
+        // As many heads a block as leave nearly two blocks an SM (32 heads, 1, 2 and 4 a block, all three kernels: 129 tokens 27, 34 and 50 us,
+        // 488 tokens 40, 43 and 57, 1,012 tokens 72, 65 and 85, 2,048 tokens 118, 111 and 105).
+        int heads = 4;
+        while (heads > 1 && ((Hs / G) % heads || (long long)n_chunks * tiles * (Hs / heads) < 252)) heads /= 2;
+        lgml_launch(ssd_chunk_out_kernel, dim3(n_chunks, Hs / heads, tiles), CHUNK_THREADS, CHUNK_OUT_SMEM, stream, p, heads);
+    }
+    return lgml_launch_status("ssd_chunks");
 }

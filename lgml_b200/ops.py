@@ -1784,7 +1784,8 @@ SSD_PIECE_TOKENS = 64      # tokens of a piece when a long portion's recurrence 
 
 
 def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor, state: torch.Tensor,
-             seq_start: torch.Tensor, slots: torch.Tensor, n_heads: int, n_groups: int, head_dim: int, n_state: int, pieces=None) -> torch.Tensor:
+             seq_start: torch.Tensor, slots: torch.Tensor, n_heads: int, n_groups: int, head_dim: int, n_state: int, pieces=None,
+             piece_tokens: int = 0) -> torch.Tensor:
     """The state-space recurrence of a step's tokens, request by request (all float32):
 
         dt = softplus(dt_raw + dt_bias_h);  S <- exp(-exp(A_log_h) dt) S + dt B x^T;  y = S^T C + D_h x
@@ -1797,7 +1798,8 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_l
     piece of every request), as ``StepBatch.scan_pieces`` gives them: the pieces run side by side in three launches.
     Every piece is scanned from zero (what it leaves and the product of its decays are kept), a chain over each
     request's pieces turns that into the state every piece starts from (and the slot's new state), and every
-    piece is scanned again from there, which gives y."""
+    piece is scanned again from there, which gives y.  ``piece_tokens``: no piece is longer than this (0: not said); pieces of up to
+    64 tokens are matrix products instead of scans where the sizes allow."""
     _need(xbc, "convolved x, B and C", torch.float32, 2)
     _need(dt_raw, "step sizes", torch.float32, 2)
     ldx, ldd = _rows_contiguous(xbc, "convolved x, B and C"), _rows_contiguous(dt_raw, "step sizes")
@@ -1823,6 +1825,14 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_l
     if pieces is None:
         scan(state, ld_state, seq_start, slots, y, n_seqs, False, False, None)
         return y
+    if 0 < piece_tokens <= SSD_PIECE_TOKENS and n_state % 4 == 0 and n_state <= 128 and head_dim % 4 == 0 and ldx % 4 == 0 and xbc.data_ptr() % 16 == 0:
+        fn_chunks = _fn("ssd", "lgml_ssd_chunks", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                                                   c_int, c_int, c_int, c_int, c_int, c_void_p])
+
+        def scan(left, _, rows, __, out, count, ___, ____, decay):          # noqa: F811
+            _check("ssd", fn_chunks(_ptr(xbc), ldx, _ptr(dt_raw), ldd, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(rows), count, _ptr(left), _ptr(decay),
+                                    _ptr(out), inner, n_heads, n_groups, head_dim, n_state, _stream()), "ssd_chunks")
+
     _scan_in_pieces(scan, pieces, n_seqs, n_heads, head_dim, n_state, state, ld_state, slots, y)
     return y
 

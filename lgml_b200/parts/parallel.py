@@ -185,7 +185,7 @@ class StateSpaceDual(Part):
         # a long portion's recurrence runs in pieces side by side
         pieces = batch.scan_pieces(ops.SSD_PIECE_TOKENS) if batch.max_q_len > SSD_PIECES_FROM else None
         y = ops.ssd_scan(xbc, proj[:, inner + C:inner + C + Hs], self.dt_bias, self.a_log, self.d_skip, cache.state, batch.seq_start, batch.slots,
-                         Hs, self.n_groups, self.head_dim, self.n_state, pieces=pieces)
+                         Hs, self.n_groups, self.head_dim, self.n_state, pieces=pieces, piece_tokens=ops.SSD_PIECE_TOKENS)
         g = ops.ssd_gate_norm(y, proj[:, :inner], self.norm_w, self.norm_groups, self.eps, rt.dtype)
         return rt.linear(g, self.wo, out_dtype=torch.float32)
 

@@ -242,6 +242,49 @@ def test_state_space_scan_whole_in_pieces_and_token_by_token_with_slow_decay(Hs,
             assert np.abs(got_rows - w).max() < 2e-4 * (1 + np.abs(w).max()), f"pieces of {size}"
 
 
+@pytest.mark.parametrize("Hs,G,Pd,N,lens", [
+    # state entries below, at and between the runs of 16 and the warps' 32; columns in part of a warp, of one block and of two
+    (3, 1, 4, 4, (64, 1)), (4, 2, 8, 12, (65, 63)), (6, 3, 32, 20, (130, 16)), (2, 1, 36, 32, (17, 200)), (3, 3, 64, 48, (300, 41)),
+    (2, 2, 68, 100, (129, 15)), (1, 1, 128, 128, (100, 64)),
+    # one, two and four heads a block
+    (32, 1, 64, 128, (129, 2)), (32, 1, 64, 128, (700, 300)), (32, 2, 64, 64, (1024, 1030)),
+])
+def test_state_space_scan_in_chunks(Hs, G, Pd, N, lens):
+    """Pieces of up to 64 tokens as matrix products: no further from the recurrence than its scan, and the scan's state; an
+    infinity stays out of earlier tokens, of other heads and of other columns."""
+    from lgml_b200 import ops
+
+    rng = np.random.default_rng(Hs * 1000 + N)
+    inner, n, C = Hs * Pd, sum(lens), Hs * Pd + 2 * G * N
+    x, dt = f32(rng.normal(size=(n, C + 4))), f32(rng.normal(size=(n, Hs)) * 0.5)
+    vecs = [f32(rng.normal(size=Hs) * 0.3 + m) for m in (-2.5, -2.0, 1.0)]
+    rows, first = [], [0]
+    for r, length in enumerate(lens):
+        rows += [(sum(lens[:r]) + t, sum(lens[:r]) + min(t + 64, length)) for t in range(0, length, 64)]
+        first.append(len(rows))
+    pieces, starts = (torch.tensor(rows, dtype=torch.int32, device=DEV), i32(first)), i32([0, lens[0], n])
+    state0 = torch.randn(4, inner * N + 4, device=DEV)
+
+    def run(how, x):
+        state = state0.clone()
+        y = ops.ssd_scan(x[:, :C], dt, vecs[0], vecs[1], vecs[2], state, starts, i32([3, 1]), Hs, G, Pd, N, **how)
+        return y, state
+
+    y, state = run(dict(pieces=pieces, piece_tokens=64), x)
+    want, want_state = run({}, x)
+    # K products of float32 operands, each sum once more rounded for the decays it went through
+    assert float((y - want).abs().max()) < 1e-5 * (1 + float(want.abs().max())) and float((state - want_state).abs().max()) < 1e-5 * (1 + float(want_state.abs().max()))
+    at = lens[0] // 2
+    x[at, Pd - 1] = float("inf")                                    # an x of the first head's last column
+    x[at, inner] = float("nan") if G > 1 else x[at, inner]          # a B of the first group
+    y, state = run(dict(pieces=pieces, piece_tokens=64), x)
+    want, want_state = run({}, x)
+    assert torch.equal(torch.isfinite(y), torch.isfinite(want)) and torch.equal(torch.isfinite(state), torch.isfinite(want_state))
+    there = torch.isfinite(want)
+    assert bool(there[:at].all()) and not bool(there.all())
+    assert float((y - want)[there].abs().max()) < 1e-5 * (1 + float(want[there].abs().max()))
+
+
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("inner,groups", [(20, 1), (48, 3), (96, 2), (640, 5)])
 def test_gate_then_norm_in_parts(out_dtype, inner, groups):
