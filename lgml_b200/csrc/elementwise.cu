@@ -3,6 +3,8 @@
 // every mode; norms and the activation compute in float32.
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 LGML_DEFINE_LAST_ERROR(lgml_elementwise)
@@ -10,9 +12,20 @@ LGML_DEFINE_LAST_ERROR(lgml_elementwise)
 // ---------------------------------------------------------------------------------------
 // x[t, :] = table[ids[t], :]            (lua/lgml/transformer.lua:2303: get_rows, no scale)
 // ---------------------------------------------------------------------------------------
-template <typename TW, typename TO>
-__global__ void embed_rows_kernel(const TW *__restrict__ table, const int *__restrict__ ids,
-                                  TO *__restrict__ out, int width, int vocab, int *__restrict__ status) {
+template <typename T> using Quad = typename std::conditional<sizeof(T) == 4, float4, uint2>::type;
+__device__ __forceinline__ void put_quad(float4 v, float *to) { *reinterpret_cast<float4 *>(to) = v; }
+__device__ __forceinline__ void put_quad(uint2 v, __nv_bfloat16 *to) { *reinterpret_cast<uint2 *>(to) = v; }
+__device__ __forceinline__ void put_quad(uint2 v, float *to) {
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&v.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&v.y));
+    *reinterpret_cast<float4 *>(to) = make_float4(a.x, a.y, b.x, b.y);
+}
+
+// Four neighbouring elements in one access each way where rows and widths allow it, ROUNDS such quads a thread, all asked for before the first
+// is written: with one, many rows are waves of blocks that wait for an id and then for a row (2,048 rows of 4,096, bfloat16 to
+// float32: 20 us element by element, 18 with one quad a thread, 7.5 with four; 8 rows 2.2 and, one quad, 1.7).
+template <int ROUNDS, typename TW, typename TO>
+__global__ void __launch_bounds__(128) embed_rows_kernel(const TW *__restrict__ table, const int *__restrict__ ids,
+                                  TO *__restrict__ out, int width, int vocab, int *__restrict__ status, int quads) {
     pdl_trigger();
     pdl_wait();
     const int t = blockIdx.x;
@@ -20,10 +33,33 @@ __global__ void embed_rows_kernel(const TW *__restrict__ table, const int *__res
     const bool ok = id >= 0 && id < vocab;           // the host checks ids first; never read out of the table
     if (!ok && threadIdx.x == 0 && blockIdx.y == 0) atomicExch(status, 1);
     const TW *row = table + (size_t)(ok ? id : 0) * width;
-    const int i0 = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    TO *to = out + (size_t)t * width;
+    const int i0 = (blockIdx.y * ROUNDS * 128 + threadIdx.x) * 4;
+    if (quads && ok) {
+        Quad<TW> v[ROUNDS];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-        if (i0 + j < width) out[(size_t)t * width + i0 + j] = from_f32<TO>(ok ? to_f32(row[i0 + j]) : 0.f);
+        for (int r = 0; r < ROUNDS; ++r)
+            if (i0 + r * 512 < width) v[r] = *reinterpret_cast<const Quad<TW> *>(row + i0 + r * 512);
+#pragma unroll
+        for (int r = 0; r < ROUNDS; ++r)
+            if (i0 + r * 512 < width) put_quad(v[r], to + i0 + r * 512);
+        return;
+    }
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int i = i0 + r * 512 + j;
+            if (i < width) to[i] = from_f32<TO>(ok ? to_f32(row[i]) : 0.f);
+        }
+}
+
+template <typename TW, typename TO>
+static int embed_rows(const TW *table, const int *ids, TO *out, int n_tokens, int width, int vocab, int *status, cudaStream_t stream) {
+    const int quads = width % 4 == 0 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0;
+    if (n_tokens <= 64) lgml_launch(embed_rows_kernel<1, TW, TO>, dim3(n_tokens, (width + 511) / 512), 128, 0, stream, table, ids, out, width, vocab, status, quads);
+    else lgml_launch(embed_rows_kernel<4, TW, TO>, dim3(n_tokens, (width + 2047) / 2048), 128, 0, stream, table, ids, out, width, vocab, status, quads);
+    return lgml_launch_status("embed_rows");
 }
 
 // out_dtype: float32, or the table's own type
@@ -31,18 +67,11 @@ LGML_API int lgml_embed_rows_as(const void *table, int table_dtype, const int *i
                                 int width, int vocab, int *status, cudaStream_t stream) {
     LGML_REQUIRE(n_tokens >= 0 && width > 0 && vocab > 0, "embed_rows: bad sizes");
     if (n_tokens == 0) return 0;
-    const int threads = 128;
-    dim3 grid(n_tokens, (width + threads * 4 - 1) / (threads * 4));
-    if (table_dtype == LGML_F32 && out_dtype == LGML_F32)
-        lgml_launch(embed_rows_kernel<float, float>, grid, threads, 0, stream, (const float *)table, ids, (float *)out, width, vocab, status);
-    else if (table_dtype == LGML_BF16 && out_dtype == LGML_BF16)
-        lgml_launch(embed_rows_kernel<__nv_bfloat16, __nv_bfloat16>, grid, threads, 0, stream, (const __nv_bfloat16 *)table, ids, (__nv_bfloat16 *)out, width,
-                    vocab, status);
-    else if (table_dtype == LGML_BF16)
-        lgml_launch(embed_rows_kernel<__nv_bfloat16, float>, grid, threads, 0, stream, (const __nv_bfloat16 *)table, ids, (float *)out, width, vocab, status);
-    else
-        LGML_FAIL("embed_rows: types %d -> %d are not built", table_dtype, out_dtype);
-    return lgml_launch_status("embed_rows");
+    if (table_dtype == LGML_F32 && out_dtype == LGML_F32) return embed_rows((const float *)table, ids, (float *)out, n_tokens, width, vocab, status, stream);
+    if (table_dtype == LGML_BF16 && out_dtype == LGML_BF16)
+        return embed_rows((const __nv_bfloat16 *)table, ids, (__nv_bfloat16 *)out, n_tokens, width, vocab, status, stream);
+    if (table_dtype == LGML_BF16) return embed_rows((const __nv_bfloat16 *)table, ids, (float *)out, n_tokens, width, vocab, status, stream);
+    LGML_FAIL("embed_rows: types %d -> %d are not built", table_dtype, out_dtype);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -99,6 +99,24 @@ def test_embed_rows(dtype):
     assert int(st.item()) == 1 and float(out[1].abs().sum()) == 0.0 and float(out[2].abs().sum()) == 0.0
 
 
+@pytest.mark.parametrize("table_dtype,out_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("n,width,shift", [(1, 4, 0), (64, 2052, 0), (65, 2052, 0), (65, 511, 0), (130, 2048, 2), (200, 6, 0), (70, 4100, 0)])
+def test_embed_rows_of_every_shape(table_dtype, out_dtype, n, width, shift):
+    """Few rows and many, widths of whole quads and not, a table that does not start on 16 bytes; ids outside give zeros."""
+    from lgml_b200 import ops
+
+    torch.manual_seed(n + width)
+    flat = torch.randn(50 * width + shift, device=DEV).to(table_dtype)
+    table = flat[shift:].view(50, width)
+    ids = torch.randint(0, 50, (n,), dtype=torch.int32, device=DEV)
+    ids[n // 2] = 50
+    out, st = torch.full((n, width), 7.0, dtype=out_dtype, device=DEV), status()
+    ops.embed_rows(table, ids, out, st)
+    want = table[ids.clamp(max=49).long()].to(out_dtype)
+    want[n // 2] = 0
+    assert torch.equal(out, want) and int(st.item()) == 1
+
+
 @pytest.mark.parametrize("paired", [False, True])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_silu_mul(paired, dtype):
