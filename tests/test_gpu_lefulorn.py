@@ -422,6 +422,29 @@ def test_delta_prepare_carries_the_filter_inputs_across_portions(taps):
     assert bool((state[[0, 2]] == 0).all()) and bool((state[1, :S_floats] == 0).all())
 
 
+@pytest.mark.parametrize("H,G,D,Dv,taps", [(3, 1, 20, 12, 4), (4, 2, 128, 128, 4), (2, 2, 100, 70, 3), (5, 1, 33, 40, 2), (2, 1, 128, 8, 1), (2, 1, 132, 16, 4), (2, 1, 16, 16, 5)])
+def test_delta_prepare_has_the_same_bits_however_it_is_cut(H, G, D, Dv, taps):
+    """Portions of three requests beside each other, in runs of eight tokens that end in the middle of a request, against token by token."""
+    from lgml_b200 import ops
+
+    torch.manual_seed(D)
+    C, lens = 2 * G * D + H * Dv, [21, 2, 10]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    x, a_pre = (torch.randn(sum(lens), w, device=DEV) for w in (C + H + 4, H * D))
+    conv_w, a_log, dt_bias = torch.randn(C, taps, device=DEV), torch.randn(H, device=DEV), torch.randn(H * D, device=DEV)
+    start = torch.randn(4, H * D * Dv + (taps - 1) * C + 3, device=DEV)
+    slots, first = [2, 0, 3], [0, 21, 23, 33]
+    whole = start.clone()
+    c, gb = ops.delta_prepare(x, a_pre, conv_w, whole, H * D * Dv, i32([s for s, n in enumerate(lens) for _ in range(n)]), i32(first), i32(slots), a_log, dt_bias,
+                              H, G, D, Dv)
+    one = start.clone()
+    for s, n in enumerate(lens):
+        for t in range(first[s], first[s] + n):
+            c1, gb1 = ops.delta_prepare(x[t:t + 1], a_pre[t:t + 1], conv_w, one, H * D * Dv, i32([0]), i32([0, 1]), i32([slots[s]]), a_log, dt_bias, H, G, D, Dv)
+            assert torch.equal(c1[0], c[t]) and torch.equal(gb1[0], gb[t])
+    assert torch.equal(whole, one)
+
+
 def test_delta_output_norm_and_relu_squared():
     from lgml_b200 import ops
 
