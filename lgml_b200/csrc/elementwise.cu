@@ -75,6 +75,37 @@ LGML_API int lgml_embed_rows_as(const void *table, int table_dtype, const int *i
 }
 
 // ---------------------------------------------------------------------------------------
+// dev[at] = value for a few integers that come with the launch itself: what changes of a captured step's description from one step to
+// the next (tokens, positions, a page here and there).  A copy of the whole costs the stream the change to the copy engine and back,
+// 4 to 9 us between two steps, and the host a copy and an event.
+// ---------------------------------------------------------------------------------------
+template <int N> struct Edits {
+    int2 at_value[N];
+};
+template <int N> __global__ void __launch_bounds__(128) edit_ints_kernel(int *__restrict__ dev, int n, const __grid_constant__ Edits<N> e) {
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    if (i < n) dev[e.at_value[i].x] = e.at_value[i].y;
+}
+template <int N> static int edit_ints(int *dev, const int2 *at_value, int n, cudaStream_t stream) {
+    Edits<N> e;
+    for (int i = 0; i < n; ++i) e.at_value[i] = at_value[i];
+    for (int i = n; i < N; ++i) e.at_value[i] = make_int2(0, 0);
+    lgml_launch_alone(edit_ints_kernel<N>, dim3((n + 127) / 128), dim3(128), 0, stream, dev, n, e);
+    return lgml_launch_status("edit_ints");
+}
+
+LGML_API int lgml_edit_ints_most(void) { return 480; }
+
+// at_value: host memory, n pairs (place below n_dev, value)
+LGML_API int lgml_edit_ints(int *dev, int n_dev, const int *at_value, int n, cudaStream_t stream) {
+    LGML_REQUIRE(n >= 0 && n <= 480, "edit_ints: %d edits in one launch", n);
+    for (int i = 0; i < n; ++i) LGML_REQUIRE(at_value[2 * i] >= 0 && at_value[2 * i] < n_dev, "edit_ints: place %d of %d", at_value[2 * i], n_dev);
+    if (n == 0) return 0;
+    const int2 *av = reinterpret_cast<const int2 *>(at_value);
+    return n <= 48 ? edit_ints<48>(dev, av, n, stream) : edit_ints<480>(dev, av, n, stream);
+}
+
+// ---------------------------------------------------------------------------------------
 // RMSNorm: y = x / sqrt(mean(x^2) + eps) * w   (src/lgml.c:1626-1633 + the multiply at
 // lua/lgml/transformer.lua:1760).  Options, all in one pass over the row:
 //   delta != null : x[row] += delta[row] first, and the sum is written back (the residual add)

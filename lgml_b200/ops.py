@@ -15,6 +15,7 @@ import os
 from ctypes import c_double, c_float, c_int, c_longlong, c_ulonglong, c_void_p
 from typing import Optional
 
+import numpy as np
 import torch
 
 from . import csrc
@@ -199,6 +200,18 @@ def embed_rows(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, status
     fn = _fn("elementwise", "lgml_embed_rows_as", [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p], label="embed_rows")
     _check("elementwise", fn(_ptr(table), dtype_code(table.dtype), _ptr(ids), _ptr(out), dtype_code(out.dtype), n, width, table.shape[0], _ptr(status), _stream()), "embed_rows")
     return out
+
+
+EDITS = 480            # most integers of one ``edit_ints``
+
+
+def edit_ints(dev: torch.Tensor, at_value: np.ndarray) -> None:
+    """dev[at] = value for the rows (at, value) of a contiguous int32 array on the host, at most ``EDITS``; they travel with the launch."""
+    _need(dev, "integers to edit", torch.int32, 1)
+    if at_value.dtype != np.int32 or at_value.ndim != 2 or at_value.shape[1] != 2 or not at_value.flags.c_contiguous or not dev.is_contiguous():
+        raise KernelError("edit_ints: contiguous int32 rows of two")
+    fn = _fn("elementwise", "lgml_edit_ints", [c_void_p, c_int, c_void_p, c_int, c_void_p])
+    _check("elementwise", fn(dev.data_ptr(), dev.numel(), at_value.ctypes.data, at_value.shape[0], _stream()), "edit_ints")
 
 
 class Partials:

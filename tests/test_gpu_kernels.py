@@ -117,6 +117,27 @@ def test_embed_rows_of_every_shape(table_dtype, out_dtype, n, width, shift):
     assert torch.equal(out, want) and int(st.item()) == 1
 
 
+@pytest.mark.parametrize("n", [0, 1, 48, 49, 128, 129, 480])
+def test_edit_ints(n):
+    """So many integers of a buffer and no other; places outside it and more edits than a launch holds are refused."""
+    import numpy as np
+
+    from lgml_b200 import ops
+
+    assert ops.EDITS == ops.csrc.load("elementwise").lgml_edit_ints_most()
+    rng = np.random.default_rng(n)
+    dev = torch.arange(1000, dtype=torch.int32, device=DEV)
+    want = np.arange(1000, dtype=np.int32)
+    edits = np.stack([rng.permutation(1000)[:n], rng.integers(-2 ** 31, 2 ** 31, n)], axis=1).astype(np.int32)
+    want[edits[:, 0]] = edits[:, 1]
+    ops.edit_ints(dev, np.ascontiguousarray(edits))
+    assert np.array_equal(dev.cpu().numpy(), want)
+    for bad in (np.array([[1000, 1]]), np.array([[-1, 1]]), np.zeros((481, 2))):
+        with pytest.raises(ops.KernelError):
+            ops.edit_ints(dev, np.ascontiguousarray(bad.astype(np.int32)))
+    assert np.array_equal(dev.cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("paired", [False, True])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_silu_mul(paired, dtype):
