@@ -9,7 +9,7 @@
 // last `taps` inputs, [taps, C], the input of position p in row p mod taps (absent with one tap): what a step of one token
 // writes is then not what anyone reads, and every block of channels may work on its own.
 //
-//   rglru_step    one token a request: convolution, both gates, recurrence and output in one kernel, a block per (8 tokens, 32 channels)
+//   rglru_step    one token a request: convolution, both gates, recurrence and output in one kernel, a block per (8 tokens, 32 or 8 channels)
 //   rglru_conv    the convolution alone for longer portions; also brings the ring up to date
 //   rglru_gates   a_t and the pushed term sqrt(1 - a^2) i u of longer portions as products of 8 rows
 //   rglru_finish  the same from logits that a grouped product on tensor cores has left: a group a part of the channels, u in three
@@ -58,15 +58,15 @@ __device__ __forceinline__ float conv_at(const float *__restrict__ x, int ldx, c
     return v;
 }
 
-// The logits of both gates for the 8 tokens in `us` and the 32 channels from k_out on of part b: zs [2][NT][CH].  A warp takes four
+// The logits of both gates for the 8 tokens in `us` and the CHB channels from k_out on of part b: zs [2][NT][CHB].  A warp takes CHB / 8
 // channels, lane groups of `lanes` a channel at a time.
-template <typename T>
+template <typename T, int CHB>
 __device__ __forceinline__ void gate_logits(const T *__restrict__ ra, const T *__restrict__ ri, const float *us, int ldu, int b, int P, int k_out, int lanes, int vec,
                                             float *zs) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, per = 32 / lanes, sub = lane % lanes;
-    for (int j0 = 0; j0 < 4; j0 += per) {
-        const int q = j0 + lane / lanes, ch = warp * 4 + q, k = k_out + ch;       // this lane group's channel of the part
-        const bool mine = q < 4 && k < P;
+    for (int j0 = 0; j0 < CHB / 8; j0 += per) {
+        const int q = j0 + lane / lanes, ch = warp * (CHB / 8) + q, k = k_out + ch;       // this lane group's channel of the part
+        const bool mine = q < CHB / 8 && k < P;
         float zr[NT], zi[NT];
 #pragma unroll
         for (int j = 0; j < NT; ++j) zr[j] = zi[j] = 0.f;
@@ -78,14 +78,14 @@ __device__ __forceinline__ void gate_logits(const T *__restrict__ ra, const T *_
         few_rows_reduce<NT>(zi, lanes);
         if (mine && sub == 0) {
 #pragma unroll
-            for (int j = 0; j < NT; ++j) zs[j * CH + ch] = zr[j], zs[(NT + j) * CH + ch] = zi[j];
+            for (int j = 0; j < NT; ++j) zs[j * CHB + ch] = zr[j], zs[(NT + j) * CHB + ch] = zi[j];
         }
     }
 }
 
 // ---- one token a request ---------------------------------------------------------------------------
 // TAPS: the taps at compile time (0: any number).
-template <typename T, typename TO, int TAPS>
+template <typename T, typename TO, int TAPS, int CHB>
 __global__ void __launch_bounds__(256) rglru_step_kernel(const float *__restrict__ proj, int ldp, const float *__restrict__ conv_w,
                                                          const float *__restrict__ conv_b, float *__restrict__ state, long long state_ld,
                                                          const int *__restrict__ slots, const int *__restrict__ positions, const T *__restrict__ ra,
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(256) rglru_step_kernel(const float *__restrict
     pdl_trigger();
     // the gates' matrices depend on no earlier kernel: have this block's rows of them in L2 by the time it may go on
     {
-        const size_t first = ((size_t)blockIdx.y * P + blockIdx.x * CH) * P, bytes = (size_t)min(CH, P - (int)blockIdx.x * CH) * P * sizeof(T);
+        const size_t first = ((size_t)blockIdx.y * P + blockIdx.x * CHB) * P, bytes = (size_t)min(CHB, P - (int)blockIdx.x * CHB) * P * sizeof(T);
         for (size_t o = (size_t)threadIdx.x * 128; o < bytes; o += (size_t)blockDim.x * 128) {
             asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(ra + first) + o));
             asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(ri + first) + o));
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(256) rglru_step_kernel(const float *__restrict
     }
     pdl_wait();
     extern __shared__ __align__(16) float us[];        // u of up to 8 tokens, the whole part of the channels
-    __shared__ float zs[2 * NT * CH];
+    __shared__ float zs[2 * NT * CHB];
     const int ldu = (P + 3) & ~3, taps = TAPS > 0 ? TAPS : any_taps;
     const int b = blockIdx.y, t0 = blockIdx.z * NT, nt = min(NT, n - t0);
     if (TAPS > 0) {
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256) rglru_step_kernel(const float *__restrict
         }
     }
     // a thread finishes one channel of one token: what it needs beside the logits is on its way meanwhile
-    const int my_j = threadIdx.x / CH, my_k = blockIdx.x * CH + threadIdx.x % CH;
+    const int my_j = threadIdx.x / CHB, my_k = blockIdx.x * CHB + threadIdx.x % CHB;
     const bool mine = my_j < nt && my_k < P;
     const int t = t0 + my_j, c = b * P + my_k;
     float *row = nullptr;
@@ -160,11 +160,11 @@ __global__ void __launch_bounds__(256) rglru_step_kernel(const float *__restrict
         s_old = act_load(row + c), y = act_load(proj + (size_t)t * ldp + C + c), x_in = act_load(proj + (size_t)t * ldp + c);
     }
     __syncthreads();
-    gate_logits<T>(ra, ri, us, ldu, b, P, blockIdx.x * CH, lanes, vec, zs);
+    gate_logits<T, CHB>(ra, ri, us, ldu, b, P, blockIdx.x * CHB, lanes, vec, zs);
     __syncthreads();
     if (!mine) return;
     float a, push;
-    gate_pair(zs[my_j * CH + threadIdx.x % CH] + ra_b[c], zs[(NT + my_j) * CH + threadIdx.x % CH] + ri_b[c], sp8[c], us[my_j * ldu + my_k], a, push);
+    gate_pair(zs[my_j * CHB + threadIdx.x % CHB] + ra_b[c], zs[(NT + my_j) * CHB + threadIdx.x % CHB] + ri_b[c], sp8[c], us[my_j * ldu + my_k], a, push);
     const float S = fmaf(a, s_old, push);
     row[c] = S;
     out[(size_t)t * C + c] = from_f32<TO>(S * gelu_tanh(y));
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(256) rglru_gates_rows_kernel(const float *__re
         us[e] = j < nt && k < P ? act_load(u + (size_t)(t0 + j) * C + b * P + k) : 0.f;
     }
     __syncthreads();
-    gate_logits<T>(ra, ri, us, ldu, b, P, blockIdx.z * CH, lanes, vec, zs);
+    gate_logits<T, CH>(ra, ri, us, ldu, b, P, blockIdx.z * CH, lanes, vec, zs);
     __syncthreads();
     const int j = threadIdx.x / CH, ch = threadIdx.x % CH, k = blockIdx.z * CH + ch, c = b * P + k;
     if (j >= nt || k >= P) return;
@@ -500,9 +500,15 @@ LGML_API int lgml_rglru_step(const float *proj, int ldp, const float *conv_w, co
     LGML_REQUIRE(smem <= 48 * 1024, "rglru_step: parts of %d channels are too wide", P);
     LGML_REQUIRE((n_tokens + NT - 1) / NT <= 65535, "rglru_step: too many tokens");
     if (n_tokens == 0) return 0;
-    dim3 grid((P + CH - 1) / CH, C / P, (n_tokens + NT - 1) / NT);
+    // Eight channels a block instead of 32 (one a warp instead of four) where that leaves two blocks an SM at most: four channels one behind the other
+    // are most of a block's time, every block convolves its whole part again (behind a product, 32 channels and 8: 2,048 channels in parts
+    // of 256, eight requests 11.9 and 7.9 us, one 11.7 and 8.1, 32 requests 17.3 and 26.2; 1,024 in parts of 128, eight requests 7.5 and 5.7;
+    // 4,096 in parts of 256 12.3 and 14.1; 2,560 in parts of 640 22.0 and 23.8).
+    const bool narrow = P <= 256 && (long long)((P + CH - 1) / CH) * (C / P) * ((n_tokens + NT - 1) / NT) <= 64;
+    const int chb = narrow ? 8 : CH;
+    dim3 grid((P + chb - 1) / chb, C / P, (n_tokens + NT - 1) / NT);
     // Alone where there is about one block an SM: behind the product ahead the blocks come to lie two and three on some (parts of 256:
-    // 2,048 channels, eight requests, 64 blocks: 13.8 us, alone 11.6; 4,096 channels, 128 blocks: 16.5 and 11.6).  Fewer blocks leave SMs
+    // 2,048 channels, eight requests, 64 blocks of 32: 13.8 us, alone 11.6; 4,096 channels, 128 blocks: 16.5 and 11.6).  Fewer blocks leave SMs
     // free whatever is ahead, and more fill all of them anyway; both gain from the early start (1,024 channels in parts of 128, 32
     // blocks: 6.9 us, alone 7.4; 64 requests of those, 256 blocks: 9.9 and 10.6).
     const long long blocks = (long long)grid.x * grid.y * grid.z;
@@ -511,7 +517,7 @@ LGML_API int lgml_rglru_step(const float *proj, int ldp, const float *conv_w, co
         else lgml_launch(kernel, grid, 256, smem, stream, args...);
     };
 #define RGLRU_STEP(T, TAPS)                                                                                                                        \
-    launch(rglru_step_kernel<T, T, TAPS>, proj, ldp, conv_w, conv_b, state, state_ld, slots, positions, (const T *)ra, \
+    launch(narrow ? rglru_step_kernel<T, T, TAPS, 8> : rglru_step_kernel<T, T, TAPS, CH>, proj, ldp, conv_w, conv_b, state, state_ld, slots, positions, (const T *)ra, \
                 ra_b, (const T *)ri, ri_b, sp8, (T *)out, n_tokens, C, P, taps, few_rows_lanes<T>(P), few_rows_vec<T>(ra, P) && few_rows_vec<T>(ri, P) ? 1 : 0)
 #define RGLRU_STEP_TAPS(T)                 \
     switch (taps) {                        \

@@ -456,6 +456,28 @@ def test_gates_are_32_bit_sums_in_every_form(dtype, C, B, taps):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("C,P,taps", [(256, 32, 4), (192, 24, 2), (520, 260, 4)])
+def test_recurrence_step_has_the_same_bits_in_wide_and_narrow_blocks(dtype, C, P, taps):
+    """80 requests at once, in blocks of 32 channels, and eight at a time, in blocks of eight where a part is narrow enough for them."""
+    from lgml_b200 import ops
+
+    torch.manual_seed(C)
+    n, parts = 80, C // P
+    rnd = lambda *s: torch.randn(*s, device=DEV)
+    proj, conv_w, conv_b = rnd(n, 2 * C), rnd(taps, C), rnd(C)
+    ra, ri = (0.2 * rnd(parts, P, P).to(dtype) for _ in range(2))
+    gates = [ra, rnd(C), ri, rnd(C), torch.rand(C, device=DEV)]
+    state = rnd(n, ops.rglru_state_floats(C, taps))
+    slots, pos = torch.randperm(n, device=DEV).int(), torch.randint(0, 9, (n,), device=DEV, dtype=torch.int32)
+    whole, few = state.clone(), state.clone()
+    out = ops.rglru_step(proj, conv_w, conv_b, whole, slots, pos, *gates)
+    for t in range(0, n, 8):
+        got = ops.rglru_step(proj[t:t + 8], conv_w, conv_b, few, slots[t:t + 8].contiguous(), pos[t:t + 8].contiguous(), *gates)
+        assert torch.equal(got, out[t:t + 8])
+    assert torch.equal(whole, few)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("C,B,taps", RECURRENCES)
 def test_recurrence_whole_in_pieces_and_token_by_token(dtype, C, B, taps):
     """Three requests in steps of every kind: one-token steps (one kernel), portions, long portions in pieces side by side, a request that sits a
