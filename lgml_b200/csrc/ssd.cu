@@ -34,8 +34,8 @@ __device__ __forceinline__ float silu_(float v) { return v / (1.0f + expf(-v)); 
 // The step's tokens come through shared memory in groups of TT: B, C (rows of NS = LN RN floats, zeros behind N),
 // the tile's x, dt and the decay.
 // GIVEN: dt_raw holds the write weights themselves and a_given the decays (row stride ldd too); no skip term.  x has Px
-// columns per head; columns Px .. P - 1 of the state are written with x = 1.
-template <int RN, int CQ, bool GIVEN>
+// columns per head; columns Px .. P - 1 of the state are written with x = 1.  QUADS: the state's groups of four lie on 16 bytes.
+template <int RN, int CQ, bool GIVEN, bool QUADS>
 __global__ void __launch_bounds__(SCAN_THREADS) ssd_scan_kernel(const float *__restrict__ xbc, int ldx, const float *__restrict__ dt_raw, int ldd,
                                                                 const float *__restrict__ dt_bias, const float *__restrict__ a_log,
                                                                 const float *__restrict__ d_skip, float *__restrict__ state, long long state_ld,
@@ -63,7 +63,16 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssd_scan_kernel(const float *__r
 #pragma unroll
     for (int q = 0; q < CQ; ++q)
 #pragma unroll
-        for (int i = 0; i < RN; ++i) S[q][i] = (!zero_start && p0 + q < P && n_of(i) < N) ? act_load(st + (size_t)(p0 + q) * N + n_of(i)) : 0.f;
+        for (int i = 0; i < RN; i += 4) {
+            const float *at = st + (size_t)(p0 + q) * N + n_of(i);
+            if (QUADS) {            // N a multiple of 4: a group is there or not as a whole
+                const float4 v = (!zero_start && p0 + q < P && n_of(i) < N) ? act_load(reinterpret_cast<const float4 *>(at)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                S[q][i] = v.x, S[q][i + 1] = v.y, S[q][i + 2] = v.z, S[q][i + 3] = v.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S[q][i + e] = (!zero_start && p0 + q < P && n_of(i) + e < N) ? act_load(at + e) : 0.f;
+            }
+        }
     float decay = 1.f;
     const bool want_y = y != nullptr;
     for (int tb = t0; tb < t1; tb += TT) {
@@ -150,8 +159,16 @@ __global__ void __launch_bounds__(SCAN_THREADS) ssd_scan_kernel(const float *__r
     for (int q = 0; q < CQ; ++q)
         if (p0 + q < P) {
 #pragma unroll
-            for (int i = 0; i < RN; ++i)
-                if (n_of(i) < N) st[(size_t)(p0 + q) * N + n_of(i)] = S[q][i];
+            for (int i = 0; i < RN; i += 4) {
+                float *at = st + (size_t)(p0 + q) * N + n_of(i);
+                if (QUADS) {
+                    if (n_of(i) < N) *reinterpret_cast<float4 *>(at) = make_float4(S[q][i], S[q][i + 1], S[q][i + 2], S[q][i + 3]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (n_of(i) + e < N) at[e] = S[q][i + e];
+                }
+            }
         }
     if (decay_out != nullptr && blockIdx.x == 0 && tid == 0) decay_out[(size_t)s * Hs + h] = decay;
 }
@@ -246,9 +263,9 @@ __device__ __forceinline__ void chunk_decays(const ChunkArgs &p, int h, int t0, 
 
 // A result that is no finite number, formed again by itself: what an infinity loses between its halves, or where a later token's
 // meets the zero of an earlier row.
-__device__ __noinline__ float left_again(const float *b, const float *x, int nt) {
+__device__ __noinline__ float left_again(const float *b, const float *x, const float *f, int nt) {
     float v = 0.f;
-    for (int t = 0; t < nt; ++t) v = fmaf(b[t * LD_B], x[t * LD_X], v);
+    for (int t = 0; t < nt; ++t) v = fmaf(b[t * LD_B], x[t * LD_X] * f[t], v);
     return v;
 }
 __device__ __noinline__ float y_again(const float *c, const float *B, int ldx, const float *s0, const float *x, const double *G, const float *dts, int i, int N) {
@@ -279,19 +296,16 @@ __global__ void __launch_bounds__(CHUNK_THREADS) ssd_chunk_left_kernel(const Chu
         const bool there = r < nt && n < p.N;
         copy_16(Bs + r * LD_B + n, there ? B + (size_t)r * p.ldx + n : B, there);
     }
+    for (int i = tid; i < CHUNK * (CHUNK_P / 4); i += CHUNK_THREADS) {
+        const int r = i / (CHUNK_P / 4), x = i % (CHUNK_P / 4) * 4;
+        const bool there = r < nt && x < cols;
+        copy_16(Xs + r * LD_X + x, there ? X + (size_t)r * p.ldx + x : X, there);
+    }
     if (warp == 0) {
         chunk_decays(p, h, t0, nt, dts, Gs);
         __syncwarp();
         for (int i = lane; i < CHUNK; i += 32) fs[i] = expf((float)(Gs[CHUNK - 1] - Gs[i])) * dts[i];
         if (blockIdx.z == 0 && lane == 0) p.decay[(size_t)c * p.Hs + h] = expf((float)Gs[CHUNK - 1]);
-    }
-    __syncthreads();
-    for (int i = tid; i < CHUNK * (CHUNK_P / 4); i += CHUNK_THREADS) {
-        const int r = i / (CHUNK_P / 4), x = i % (CHUNK_P / 4) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < nt && x < cols) v = act_load(reinterpret_cast<const float4 *>(X + (size_t)r * p.ldx + x));
-        const float f = fs[r];
-        *reinterpret_cast<float4 *>(Xs + r * LD_X + x) = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
     }
     copies_there();
     __syncthreads();
@@ -303,9 +317,9 @@ __global__ void __launch_bounds__(CHUNK_THREADS) ssd_chunk_left_kernel(const Chu
         float w[2][2][4], a[4][4];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            const float *bk = Bs + (k0 + 4 * s + q) * LD_B + n0 + g, *xk = Xs + (k0 + 4 * s + q) * LD_X + x0 + g;
+            const float *bk = Bs + (k0 + 4 * s + q) * LD_B + n0 + g, *xk = Xs + (k0 + 4 * s + q) * LD_X + x0 + g, f = fs[k0 + 4 * s + q];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) w[i >> 1][i & 1][s] = bk[8 * i], a[i][s] = xk[8 * i];
+            for (int i = 0; i < 4; ++i) w[i >> 1][i & 1][s] = bk[8 * i], a[i][s] = xk[8 * i] * f;
         }
         float4 wv[2][2], av[4];
 #pragma unroll
@@ -325,7 +339,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS) ssd_chunk_left_kernel(const Chu
                 const int n = n0 + i * 16 + (e >> 1) * 8 + g, x = x0 + j * 8 + q * 2 + (e & 1);
                 if (n < p.N && x < cols) {
                     float v = sum[i][j][e];
-                    if (!isfinite(v)) v = left_again(Bs + n, Xs + x, nt);
+                    if (!isfinite(v)) v = left_again(Bs + n, Xs + x, fs, nt);
                     out[(size_t)x * p.N + n] = v;
                 }
             }
@@ -480,7 +494,7 @@ int scan_any(const float *xbc, int ldx, const float *dt_raw, int ldd, const floa
     LGML_REQUIRE(slots != nullptr || pieces, "ssd_scan: requests come with their slots");
     if (n_seqs == 0) return 0;
     // RN entries a lane, LN lanes a column (a power of two up to 32): the pair that wastes least, then the smaller RN.
-    // Four columns a thread with up to 16 entries each (states up to 512 numbers a column), else one column with up to 32.
+    // Up to 16 entries a lane for states of up to 512 numbers a column (four columns a thread then have registers), else up to 32.
     const bool quad = N <= 512;
     static const int rns[6] = {4, 8, 12, 16, 24, 32};
     int best_rn = 32, best_ln = 32, best_cover = 1 << 30;
@@ -492,17 +506,24 @@ int scan_any(const float *xbc, int ldx, const float *dt_raw, int ldd, const floa
         // (at equal cover: with four columns a thread the larger RN, fewer lanes to add up; with one the smaller, more threads)
         if (ln * rns[i] < best_cover || (quad && ln * rns[i] == best_cover)) best_cover = ln * rns[i], best_rn = rns[i], best_ln = ln;
     }
-    const int LN = best_ln, CQ = quad ? 4 : 1, CPB = (SCAN_THREADS / LN) * CQ;
+    // One column a thread (the same sums) up to 512 blocks of four columns a thread: more blocks for SMs without one, and shorter chains.  32 heads of
+    // 64 columns by 128 entries, microseconds, four columns with the state element by element; four with 16 bytes at a time; one: 2 requests
+    // of one token 6.5, 4.1, 3.7; 8 9.0, 6.5, 6.8; 32 24.4, 17.1, 18.5; 2 of 100 tokens 76, 82, 51; 16 of 100 195, 198, 179; 32 of 16 62, 59, 65.
+    const long long wide_blocks = (long long)((P + SCAN_THREADS / best_ln * 4 - 1) / (SCAN_THREADS / best_ln * 4)) * Hs * n_seqs;
+    const bool four = quad && wide_blocks > 512;
+    const int LN = best_ln, CQ = four ? 4 : 1, CPB = (SCAN_THREADS / LN) * CQ;
     const int NS = LN * best_rn;
     int TT = 32;
     while (TT > 1 && (size_t)TT * (2 * NS + CPB + 2) * sizeof(float) > 46 * 1024) TT /= 2;
     const size_t smem = (size_t)TT * (2 * NS + CPB + 2) * sizeof(float);
     dim3 grid((P + CPB - 1) / CPB, Hs, n_seqs);
     const int vec = N % 4 == 0 && ldx % 4 == 0 && (Hs * Px) % 4 == 0 && ((uintptr_t)xbc & 15) == 0;
-#define LGML_SCAN_K(RN, CQ, GIVEN) lgml_launch(ssd_scan_kernel<RN, CQ, GIVEN>, grid, SCAN_THREADS, smem, stream, xbc, ldx, dt_raw, ldd, dt_bias, a_log, d_skip, \
+#define LGML_SCAN_Q(RN, CQ, GIVEN, QUADS) lgml_launch(ssd_scan_kernel<RN, CQ, GIVEN, QUADS>, grid, SCAN_THREADS, smem, stream, xbc, ldx, dt_raw, ldd, dt_bias, a_log, d_skip, \
                                                state, state_ld, seq_start, slots, y, ldy, Hs, G, P, N, LN, TT, pieces, zero_start, decay_out, vec, a_given, Px, max_tokens)
+#define LGML_SCAN_K(RN, CQ, GIVEN) do { if (quads) LGML_SCAN_Q(RN, CQ, GIVEN, true); else LGML_SCAN_Q(RN, CQ, GIVEN, false); } while (0)
 #define LGML_SCAN(RN, CQ) do { if (a_given != nullptr) LGML_SCAN_K(RN, CQ, true); else LGML_SCAN_K(RN, CQ, false); } while (0)
-    if (quad) {
+    const bool quads = N % 4 == 0 && state_ld % 4 == 0 && ((uintptr_t)state & 15) == 0;
+    if (four) {
         switch (best_rn) {
             case 4: LGML_SCAN(4, 4); break;
             case 8: LGML_SCAN(8, 4); break;
@@ -511,6 +532,7 @@ int scan_any(const float *xbc, int ldx, const float *dt_raw, int ldd, const floa
         }
     } else {
         switch (best_rn) {
+            case 4: LGML_SCAN(4, 1); break;
             case 8: LGML_SCAN(8, 1); break;
             case 12: LGML_SCAN(12, 1); break;
             case 16: LGML_SCAN(16, 1); break;
@@ -520,6 +542,7 @@ int scan_any(const float *xbc, int ldx, const float *dt_raw, int ldd, const floa
     }
 #undef LGML_SCAN
 #undef LGML_SCAN_K
+#undef LGML_SCAN_Q
     return lgml_launch_status("ssd_scan");
 }
 }  // namespace
