@@ -246,3 +246,116 @@ LGML_API int lgml_steps_page_keys(PyObject *list, long long b0, long long n, lon
     }
     return 0;
 }
+
+/* ---- launchers called from Python -------------------------------------------------------------------------------------------
+ * A callable for a C function of integers, pointers and up to eight floats: ctypes spends 3 us on the arguments of a launch that takes 3 itself.
+ * On x86-64 (System V) integers and pointers go in order to six registers and then the stack, floats in order to eight
+ * registers of their own, wherever they stand between the integers; what a function does not take it does not look at.  So one call fits all: the
+ * integers as 64-bit words in their order, then the floats (of a float the low half of its register counts). */
+#if defined(__x86_64__) && defined(__linux__)
+typedef struct {
+    const char *name;
+    PyObject *(*meth)(PyObject *, PyObject *const *, intptr_t);
+    int flags;
+    const char *doc;
+} MethodDef;
+extern PyObject *PyCFunction_NewEx(MethodDef *def, PyObject *self, PyObject *module);
+extern PyObject *PyLong_FromVoidPtr(void *p);
+extern void *PyLong_AsVoidPtr(PyObject *v);
+extern long long PyLong_AsLongLong(PyObject *v);
+extern PyObject *PyLong_FromLong(long v);
+extern double PyFloat_AsDouble(PyObject *v);
+extern PyObject *PyTuple_New(intptr_t n);
+extern int PyTuple_SetItem(PyObject *t, intptr_t i, PyObject *v);
+extern PyObject *PyObject_CallObject(PyObject *f, PyObject *args);
+extern void *PyEval_SaveThread(void);
+extern void PyEval_RestoreThread(void *state);
+extern void Py_IncRef(PyObject *o);
+extern void Py_DecRef(PyObject *o);
+extern char _Py_NoneStruct[];          /* None */
+extern void *malloc(size_t n);
+
+enum { MOST_WORDS = 40, MOST_FLOATS = 8, FASTCALL = 0x80 };
+typedef long long W;
+typedef int (*Launcher)(W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, W, double, double,
+                        double, double, double, double, double, double);
+typedef struct {
+    MethodDef def;
+    Launcher fn;
+    PyObject *other;        /* takes what is no plain number */
+    int n;
+    char kinds[MOST_WORDS + MOST_FLOATS + 1];
+} Caller;
+
+static PyObject *call(PyObject *self, PyObject *const *args, intptr_t n) {
+    const Caller *c = (const Caller *)PyLong_AsVoidPtr(self);
+    W w[MOST_WORDS] = {0};
+    union {
+        double d;
+        float f;
+    } x[MOST_FLOATS] = {{0.0}};
+    int nw = 0, nx = 0, ok = n == c->n;
+    for (int i = 0; ok && i < n; ++i) {
+        if (c->kinds[i] == 'w') {
+            w[nw] = args[i] == (PyObject *)_Py_NoneStruct ? 0 : PyLong_AsLongLong(args[i]);
+            ok = w[nw++] != -1 || !PyErr_Occurred();
+        } else {
+            const double v = PyFloat_AsDouble(args[i]);
+            ok = v != -1.0 || !PyErr_Occurred();
+            if (c->kinds[i] == 'f') x[nx++].f = (float)v;
+            else x[nx++].d = v;
+        }
+    }
+    if (!ok) {
+        PyErr_Clear();
+        PyObject *t = PyTuple_New(n), *got;
+        if (!t) return 0;
+        for (intptr_t i = 0; i < n; ++i) {
+            Py_IncRef(args[i]);
+            PyTuple_SetItem(t, i, args[i]);
+        }
+        got = PyObject_CallObject(c->other, t);
+        Py_DecRef(t);
+        return got;
+    }
+    void *state = PyEval_SaveThread();      /* a launch may wait for room in the queue */
+    const int rc = c->fn(w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], w[8], w[9], w[10], w[11], w[12], w[13], w[14], w[15], w[16], w[17], w[18], w[19],
+                         w[20], w[21], w[22], w[23], w[24], w[25], w[26], w[27], w[28], w[29], w[30], w[31], w[32], w[33], w[34], w[35], w[36], w[37], w[38],
+                         w[39], x[0].d, x[1].d, x[2].d, x[3].d, x[4].d, x[5].d, x[6].d, x[7].d);
+    PyEval_RestoreThread(state);
+    return PyLong_FromLong(rc);
+}
+
+/* `kinds`: a letter an argument, w (integer or pointer), f (float) or d (double).  The function must return an int.  `other` is called instead with
+ * arguments that are no numbers, or not as many.  A callable lasts as long as the process; NULL: not here, or too many arguments. */
+LGML_API int lgml_steps_caller_fits(const char *kinds) {
+    int nw = 0, nx = 0;
+    for (const char *k = kinds; *k; ++k) *k == 'w' ? ++nw : ++nx;
+    return nw <= MOST_WORDS && nx <= MOST_FLOATS;
+}
+LGML_API PyObject *lgml_steps_caller(void *fn, const char *kinds, PyObject *other) {
+    Caller *c = malloc(sizeof(*c));
+    if (!c || !lgml_steps_caller_fits(kinds)) {
+        Py_IncRef((PyObject *)_Py_NoneStruct);
+        return (PyObject *)_Py_NoneStruct;
+    }
+    memset(c, 0, sizeof(*c));
+    c->def = (MethodDef){"launcher", call, FASTCALL, 0};
+    c->fn = (Launcher)fn, c->other = other, c->n = (int)strlen(kinds);
+    memcpy(c->kinds, kinds, (size_t)c->n);
+    Py_IncRef(other);
+    PyObject *self = PyLong_FromVoidPtr(c);
+    PyObject *f = PyCFunction_NewEx(&c->def, self, 0);
+    Py_DecRef(self);
+    return f;
+}
+#else
+extern char _Py_NoneStruct[];          /* None */
+extern void Py_IncRef(PyObject *o);
+LGML_API int lgml_steps_caller_fits(const char *kinds) { return kinds == 0; }
+LGML_API PyObject *lgml_steps_caller(void *fn, const char *kinds, PyObject *other) {
+    (void)fn, (void)kinds, (void)other;
+    Py_IncRef((PyObject *)_Py_NoneStruct);
+    return (PyObject *)_Py_NoneStruct;
+}
+#endif

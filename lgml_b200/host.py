@@ -67,8 +67,20 @@ def steps() -> ctypes.PyDLL:
         l.lgml_steps_pieces.restype, l.lgml_steps_pieces.argtypes = c_int64, [c_void_p, c_int64, c_void_p, c_int64, c_int64, POINTER(c_int64)]
         l.lgml_steps_page_keys.restype = c_int
         l.lgml_steps_page_keys.argtypes = [ctypes.py_object, c_int64, c_int64, c_int64, c_char_p, c_int64, c_void_p, c_int]
+        l.lgml_steps_caller.restype, l.lgml_steps_caller.argtypes = ctypes.py_object, [c_void_p, c_char_p, ctypes.py_object]
         _steps = l
     return _steps
+
+
+_KINDS = {c_void_p: b"w", c_int: b"w", c_int64: b"w", c_uint64: b"w", c_float: b"f", c_double: b"d"}
+
+
+def caller(fn):
+    """A ctypes function that returns an int, with its argument types set, as a callable that converts plain numbers itself (and leaves all else to
+    ``fn``); ``fn`` itself where there is no such thing."""
+    kinds = [_KINDS.get(t) for t in fn.argtypes]
+    fast = None if None in kinds else steps().lgml_steps_caller(ctypes.cast(fn, c_void_p), b"".join(kinds), fn)
+    return fn if fast is None else fast
 
 
 NOT_INTS = -2          # of lgml_steps_ints and lgml_steps_page_keys: not a list of integers, or one beyond 64 bits

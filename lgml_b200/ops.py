@@ -18,7 +18,7 @@ from typing import Optional
 import numpy as np
 import torch
 
-from . import csrc
+from . import csrc, host
 
 F32, BF16 = 0, 1
 _DT = {torch.float32: F32, torch.bfloat16: BF16}
@@ -123,10 +123,11 @@ class KernelTimes:
 
 
 class _Timed:
-    """A launcher that, while a ``KernelTimes`` is open, brackets its call with two events."""
+    """A launcher that, while a ``KernelTimes`` is open, brackets its call with two events; ``fast`` is the call alone."""
 
     def __init__(self, fn, name: str):
         self.fn, self.name = fn, name
+        self.fast = host.caller(fn)
 
     def __call__(self, *args):
         kt = KernelTimes.active
@@ -149,7 +150,7 @@ def _fn(lib_name: str, fn_name: str, argtypes, label: Optional[str] = None):
     key = (lib_name, fn_name)
     got = _wrapped.get(key)
     if got is not None:
-        return got
+        return got.fast if KernelTimes.active is None else got
     lib = csrc.load(lib_name)
     fn = getattr(lib, fn_name)
     if key not in _prototyped:
