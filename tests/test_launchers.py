@@ -20,7 +20,7 @@ def signatures():
     for n in (3, 7, 8, 15, 22, 31, 44):
         kinds = [c_void_p, c_int, c_longlong, c_ulonglong] * 5 + [c_float, c_double]
         got = [rng.choice(kinds) for _ in range(n)]
-        while sum(t in (c_float, c_double) for t in got) > 8:
+        while not n - 40 <= sum(t in (c_float, c_double) for t in got) <= 8:
             got = [rng.choice(kinds) for _ in range(n)]
         yield got
 
