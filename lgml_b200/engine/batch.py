@@ -24,6 +24,7 @@ import numpy as np
 import torch
 
 from ..host import steps
+from ..ops import sm_count
 
 
 @dataclass
@@ -193,26 +194,32 @@ class StepBatch:
         for k, at, n, shape in written:
             self._tiles[k] = self._views(k, dev[at:at + n], shape)
 
-    # ---- tiles and pieces: ("tiles", tokens, longer than), ("pieces", tokens), ("chunks", tokens, longer than) ----
+    # ---- tiles and pieces: ("tiles", tokens, longer than), ("halves", tokens, CTAs a tile), ("pieces", tokens), ("chunks", tokens, longer than) ----
     def _wanted(self, key) -> bool:
         return key[0] != "chunks" or self.max_q_len > key[2]
 
     def _room(self, key) -> int:
         """Most 32-bit integers that the list takes."""
-        n = sum(-(-x // key[1]) for x in self.seq_lens)
-        return 4 * n if key[0] == "tiles" else 2 * n + 2 * self.n_seqs + 1
+        n = sum(-(-x // (self._half(key) if key[0] == "halves" else key[1])) for x in self.seq_lens)
+        return 4 * n if key[0] in ("tiles", "halves") else 2 * n + 2 * self.n_seqs + 1
+
+    def _half(self, key) -> int:
+        """Tokens of a tile of ("halves", tokens, CTAs a tile): half as many where a CTA for each of those has an SM to itself."""
+        half = key[1] // 2
+        return half if half and sum(-(-x // half) for x in self.seq_lens) * key[2] <= sm_count() else key[1]
 
     def _write(self, key, at: int):
         """The list at address ``at``: (integers, what ``_views`` has to know of it)."""
-        if key[0] == "tiles":
-            n = steps().lgml_steps_tiles(at, self.n_seqs, self._lens, self._pos0, key[1], key[2])
+        if key[0] in ("tiles", "halves"):
+            tokens, longer = (key[1], key[2]) if key[0] == "tiles" else (self._half(key), 0)
+            n = steps().lgml_steps_tiles(at, self.n_seqs, self._lens, self._pos0, tokens, longer)
             return 4 * n, n
         reqs = c_int64()
         n = steps().lgml_steps_pieces(at, self.n_seqs, self._lens, key[1], key[2] if key[0] == "chunks" else -1, byref(reqs))
         return 2 * n + reqs.value + 1 + (reqs.value if key[0] == "chunks" else 0), (n, reqs.value)
 
     def _views(self, key, flat, shape):
-        if key[0] == "tiles":
+        if key[0] in ("tiles", "halves"):
             return flat.view(-1, 4)
         n, reqs = shape
         rows, first = flat[:2 * n].view(-1, 2), flat[2 * n:2 * n + reqs + 1]
@@ -236,6 +243,13 @@ class StepBatch:
         alone at the end.  Only of requests that bring more than ``longer_than`` tokens.  Made once per tile size (``remember``: for later
         steps of the model too).  (What comes fourth in a row has done its part when they are sorted.)"""
         return self._list(("tiles", tile_tokens, longer_than), remember)
+
+    def twin_tiles(self, tile_tokens: int, ctas: int) -> torch.Tensor:
+        """Tiles for the attention kernel that takes two tiles of rows a CTA, ``ctas`` CTAs each: of ``tile_tokens`` tokens, or of half as many, one
+        tile of rows, where each such CTA has an SM to itself (the same bits; 16 heads on 4 of 128: 512 tokens behind 1,024 28.2 us in 32 CTAs
+        and 23.6 in 64, 488 and 512 tokens 26.3 in 64 and 22.7 in 128, 252 CTAs of a quarter 35; 32 on 8: 512 tokens 17.3 and 14.5, 1,024
+        tokens 26.7 in 128 CTAs and 28.0 in 256)."""
+        return self._list(("halves", tile_tokens, ctas))
 
     def tiles_and_short(self, tile_tokens: int, limit, rule):
         """The step's requests in two: (tiles as ``attention_tiles`` of those that bring more than ``limit(seq_lens)`` tokens, the rows of the

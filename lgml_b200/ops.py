@@ -2723,6 +2723,11 @@ def prefill_twin_tile_tokens(n_heads: int, n_kv_heads: int) -> int:
     return 2 * (128 // min(n_heads // n_kv_heads, 8))
 
 
+def prefill_twin_ctas(n_heads: int, n_kv_heads: int) -> int:
+    """CTAs of that kernel a tile: one a KV head and up to eight of its query heads."""
+    return n_kv_heads * -(-(n_heads // n_kv_heads) // 8)
+
+
 def prefill_attention_twin(q: torch.Tensor, positions: torch.Tensor, tiles: torch.Tensor, block_table: torch.Tensor,
                            k_pages: torch.Tensor, v_pages: torch.Tensor, out: torch.Tensor, n_heads: int, scale: float, window: int,
                            status: torch.Tensor) -> torch.Tensor:
@@ -2860,7 +2865,8 @@ def paged_attention(q, batch, cache, out, n_heads: int, scale: float, window: in
             return decode_attention(q, batch.positions, batch.seq_of_token, cache.block_table, cache.k, cache.v, out, n_heads, scale,
                                     window, status, n_splits, max_new_tokens=batch.max_q_len)
         if d in (64, 128) and PREFILL_ATTENTION == "tcgen05" and prefill_tc_supports(q, out):
-            tiles = batch.attention_tiles(prefill_twin_tile_tokens(n_heads, hkv))
+            tokens = prefill_twin_tile_tokens(n_heads, hkv)
+            tiles = batch.twin_tiles(tokens, prefill_twin_ctas(n_heads, hkv)) if hasattr(batch, "twin_tiles") else batch.attention_tiles(tokens)
             return prefill_attention_twin(q, batch.positions, tiles, cache.block_table, cache.k, cache.v, out, n_heads, scale, window, status)
         if d <= 128 and PREFILL_ATTENTION in ("tcgen05", "single") and prefill_tc_supports(q, out):
             tiles = batch.attention_tiles(prefill_tc_tile_tokens(n_heads, hkv))

@@ -266,6 +266,9 @@ def test_tiles_and_pieces_of_a_step(lens, pos0):
             got = b.attention_tiles(tile, longer)
             assert got.tolist() == [[s, a, n, 0] for s, a, n, _ in sorted(want, key=lambda r: -r[3])]
             assert round_ == 0 or (got.data_ptr() - b._dev.data_ptr()) % 16 == 0
+        for ctas in (1, 8, 1000):           # half a tile while each has an SM to itself
+            size = 32 if sum(-(-n // 32) for n in lens) * ctas <= 148 else 64
+            assert b.twin_tiles(64, ctas).tolist() == b.attention_tiles(size).tolist()
         pieces, first = b.scan_pieces(16)
         want = [[[a + t, a + min(t + 16, n)] for t in range(0, n, 16)] for a, n in zip(starts, lens)]
         assert pieces.tolist() == sum(want, []) and first.tolist() == [sum(map(len, want[:s])) for s in range(len(lens) + 1)]
