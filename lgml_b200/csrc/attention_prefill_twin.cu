@@ -254,12 +254,15 @@ __device__ __forceinline__ void write_p(const uint32_t (&r)[PAGE], uint32_t s_ad
 // normalised output is multiplied by sigmoid(gate) (float32 [tokens, H D], row stride ldg).  Each
 // of the three pointers may be null.  With a window, a request's first keep_first keys stay visible beyond it:
 // the pages that hold them are walked after the window's.  Without BIAS none of it is compiled in.
+// n_ranges: the steps of a tile in so many ranges, blockIdx.z the range; each of more than one leaves its output, its
+// maximum and its sum in part_o and part_ml ([row, head, range]) for twin_merge_kernel, which applies the sink and the gate.
 template <int D, bool BIAS>
 __global__ void __launch_bounds__(THREADS, 1) prefill_attention_twin_kernel(
     const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const __nv_bfloat16 *__restrict__ q, int ldq,
     const int *__restrict__ positions, const int *__restrict__ tiles, const int *__restrict__ block_table, int max_blocks, int n_pages,
     __nv_bfloat16 *__restrict__ out, int ldo, int H, int Hkv, int hpc, int tt, float scale, int window, int *__restrict__ status,
-    const float *__restrict__ slopes, const float *__restrict__ sinks, const float *__restrict__ gate, int ldg, float softcap, int keep_first) {
+    const float *__restrict__ slopes, const float *__restrict__ sinks, const float *__restrict__ gate, int ldg, float softcap, int keep_first, int n_ranges,
+    float *__restrict__ part_o, float2 *__restrict__ part_ml) {
     constexpr int KB = D / 64;                              // 64-element blocks along the head dimension
     constexpr uint32_t TILE_BYTES = KB * ROWS * 128;        // the queries of one tile: [KB][128 rows][128 B]
     constexpr uint32_t PAGE_BYTES = KB * PAGE * 128;        // a page of keys [KB][64 keys][128 B] (K-major: row = key), or of values (N-major: 64 dims per row)
@@ -292,19 +295,31 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_attention_twin_kernel(
     const int n_window = pg_hi - pg_lo + 1;
     // pages of kept first tokens that lie before the window's pages
     const int n_kept = BIAS && window > 0 ? min((keep_first + PAGE - 1) / PAGE, pg_lo) : 0;
-    const int n_steps = n_window + n_kept;                        // a page a step
+    const int total_steps = n_window + n_kept;                    // a page a step
+    // this CTA's range of them (most often all)
+    const int per_range = (total_steps + n_ranges - 1) / n_ranges, j_first = (int)blockIdx.z * per_range;
+    const int n_steps = min(total_steps - j_first, per_range);
+    if (n_steps <= 0) {             // more ranges than this tile has pages for: its rows have no keys here
+        pdl_wait();
+        for (int i = tid; i < n_tok * g_count; i += THREADS)
+            part_ml[((size_t)(row0 + i / g_count) * H + kvh * group + g0 + i % g_count) * n_ranges + blockIdx.z] = make_float2(-INFINITY, 0.f);
+        return;
+    }
     // BIAS walks the pages from the newest to the oldest: the bias falls with a key's age (by 64
     // slopes a page), so a row's maximum is as good as settled on its first page; walking up,
     // a head with a steep slope would have to correct its output on every page.
-    auto page_index = [&](int j) -> int { return BIAS ? (j < n_window ? pg_hi - j : n_steps - 1 - j) : pg_lo + j; };
-    const int j_fix = BIAS ? 0 : n_steps - 1;                     // the step of the page that holds the last key
+    auto page_index = [&](int step) -> int {
+        const int j = j_first + step;
+        return BIAS ? (j < n_window ? pg_hi - j : total_steps - 1 - j) : pg_lo + j;
+    };
+    const int j_fix = BIAS ? 0 : n_steps - 1;                     // the step of the page that holds the last key, where it is in this range
     const int n_act = n_tok > tt ? 2 : 1;                         // tiles that hold tokens
     const float scale_log2 = scale * 1.4426950408889634f;
     // The last page's values behind the last key may be anything, NaN included, and 0 x NaN is
     // NaN: they become zeros before the product reads them.  (Keys there give scores that the
     // softmax masks.)
     const int last_rows = pos_last - pg_hi * PAGE + 1;            // rows of the last page that hold keys
-    const bool fix_last = last_rows < PAGE;
+    const bool fix_last = last_rows < PAGE && (BIAS ? j_first == 0 : j_first + n_steps == total_steps);
 
     if (tid == 0) {
         for (int i = 0; i < STAGES; ++i) {
@@ -516,6 +531,24 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_attention_twin_kernel(
         if (t < n_act) {
             if (alive && !warp_wait(&o_last[t], 0, abort_flag, status)) alive = false;
             tcgen05_fence_after();
+            if (n_ranges > 1) {
+                // a range's sums as they are; the merge divides, and adds what is no key's
+                const bool store = row_valid && alive;
+                const size_t at = ((size_t)(row0 + (row_valid ? t * tt + my_tok : 0)) * H + my_head) * n_ranges + blockIdx.z;
+                if (row_valid) part_ml[at] = store ? make_float2(m_ref, l_run) : make_float2(-INFINITY, 0.f);
+#pragma unroll
+                for (int c0 = 0; c0 < D; c0 += 16) {
+                    uint32_t o[16];
+                    tcgen05_ld_16(o_addr + (uint32_t)c0, o);
+                    tcgen05_wait_ld();
+                    if (store) {
+                        float4 *dst = reinterpret_cast<float4 *>(part_o + at * D + c0);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            dst[i] = make_float4(__uint_as_float(o[4 * i]), __uint_as_float(o[4 * i + 1]), __uint_as_float(o[4 * i + 2]), __uint_as_float(o[4 * i + 3]));
+                    }
+                }
+            } else {
             // the sink: a term of the denominator without a key or a value
             if (BIAS && sinks && m_ref != -INFINITY) l_run += ex2(sinks[my_head] * 1.4426950408889634f - m_ref);
             float inv = l_run > 0.f && l_run < INFINITY ? 1.f / l_run : 0.f;
@@ -550,6 +583,7 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_attention_twin_kernel(
                         *reinterpret_cast<uint4 *>(dst + c0 + c8) = make_uint4(h[0], h[1], h[2], h[3]);
                     }
                 }
+            }
             }
         }
     } else if ((warp == ISSUE_WARP || warp == ISSUE_WARP + 1) && lane == 0 && warp - ISSUE_WARP < n_act) {
@@ -659,11 +693,63 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_attention_twin_kernel(
     }
 }
 
+// ---- the ranges of a tile's keys put together: a warp a token and head --------------------------
+// A tile's pages are a serial chain of about 1.05 us each in one CTA.  A few tiles behind a long context (a question in a
+// conversation: 16 CTAs of 33 pages) left 132 of 148 SMs idle for 37.1 us; in 8 ranges the two kernels take 16.5.  The
+// outputs of the ranges stay float32 and unnormalised until here.  Bound by its one trip to L2 for them (a step of 512
+// tokens in 2 ranges reads 8 MB): about 4 us with its launch, most of which the launch takes.
+constexpr int MERGE_WARPS = 8, MOST_RANGES = 32;
+template <int D>
+__global__ void __launch_bounds__(MERGE_WARPS * 32) twin_merge_kernel(const int *__restrict__ tiles, const float *__restrict__ part_o, const float2 *__restrict__ part_ml,
+                                                                      int n_ranges, __nv_bfloat16 *__restrict__ out, int ldo, int H,
+                                                                      const float *__restrict__ sinks, const float *__restrict__ gate, int ldg) {
+    pdl_trigger();
+    pdl_wait();
+    constexpr int V = D / 32;
+    const int lane = threadIdx.x & 31, u = blockIdx.x * MERGE_WARPS + (threadIdx.x >> 5);
+    const int tok = u / H, head = u - tok * H;
+    if (tok >= tiles[blockIdx.y * 4 + 2]) return;
+    const size_t row = (size_t)tiles[blockIdx.y * 4 + 1] + tok, at = (row * H + head) * n_ranges;
+    const float2 ml = lane < n_ranges ? act_load(part_ml + at + lane) : make_float2(-INFINITY, 0.f);
+    const float top = warp_max(ml.x);
+    const float weight = ml.x == -INFINITY ? 0.f : ex2(ml.x - top);
+    float l = warp_sum(ml.y * weight);
+    if (sinks && top != -INFINITY) l += ex2(sinks[head] * 1.4426950408889634f - top);
+    float inv = l > 0.f && l < INFINITY ? 1.f / l : 0.f;
+    if (gate && ldg < 0) inv *= 1.0f / (1.0f + __expf(-act_load(gate + row * (size_t)(-ldg) + head)));
+    float o[V] = {};
+    for (int r = 0; r < n_ranges; ++r) {
+        const float w = __shfl_sync(0xffffffffu, weight, r);
+        if (w == 0.f) continue;             // (nothing was written there)
+        const float *p = part_o + (at + r) * D + lane * V;
+        float v[V];
+        if constexpr (V == 4) {
+            const float4 x = act_load(reinterpret_cast<const float4 *>(p));
+            v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+        } else {
+            const float2 x = act_load(reinterpret_cast<const float2 *>(p));
+            v[0] = x.x, v[1] = x.y;
+        }
+#pragma unroll
+        for (int i = 0; i < V; ++i) o[i] = fmaf(w, v[i], o[i]);
+    }
+    __nv_bfloat16 *to = out + row * ldo + (size_t)head * D + lane * V;
+#pragma unroll
+    for (int i = 0; i < V; i += 2) {
+        float a = o[i] * inv, b = o[i + 1] * inv;
+        if (gate && ldg > 0) {
+            const float2 g = act_load(reinterpret_cast<const float2 *>(gate + row * ldg + (size_t)head * D + lane * V + i));
+            a *= 1.0f / (1.0f + __expf(-g.x)), b *= 1.0f / (1.0f + __expf(-g.y));
+        }
+        *reinterpret_cast<__nv_bfloat162 *>(to + i) = __floats2bfloat162_rn(a, b);
+    }
+}
+
 // ---- host side ----------------------------------------------------------------------------------
 template <int D, bool BIAS>
 int launch(dim3 grid, const __nv_bfloat16 *q, int ldq, const int *positions, const int *tiles, const int *block_table, int max_blocks,
            const __nv_bfloat16 *k_pages, const __nv_bfloat16 *v_pages, int n_pages, __nv_bfloat16 *out, int ldo, int H, int Hkv, int hpc, int tt,
-           float scale, int window, int *status, cudaStream_t stream, const float *slopes = nullptr, const float *sinks = nullptr,
+           float scale, int window, int *status, cudaStream_t stream, int n_ranges, float *part, int part_rows, const float *slopes = nullptr, const float *sinks = nullptr,
            const float *gate = nullptr, int ldg = 0, float softcap = 0.f, int keep_first = 0) {
     constexpr int KB = D / 64;
     const size_t smem = 2 * (size_t)KB * ROWS * 128 + 2 * STAGES * (size_t)KB * PAGE * 128 + 1024;
@@ -677,9 +763,17 @@ int launch(dim3 grid, const __nv_bfloat16 *q, int ldq, const int *positions, con
     int rc;
     if ((rc = lgml_make_page_map(&mk, k_pages, n_pages, Hkv, D, "prefill_attention_twin"))) return rc;
     if ((rc = lgml_make_page_map(&mv, v_pages, n_pages, Hkv, D, "prefill_attention_twin"))) return rc;
+    grid.z = n_ranges;
+    // `part`: the ranges' outputs [part_rows, H, n_ranges, D], then their maxima and sums
+    float *part_o = n_ranges > 1 ? part : nullptr;
+    float2 *part_ml = n_ranges > 1 ? reinterpret_cast<float2 *>(part + (size_t)part_rows * H * n_ranges * D) : nullptr;
     lgml_launch(prefill_attention_twin_kernel<D, BIAS>, grid, THREADS, smem, stream, mk, mv, q, ldq, positions, tiles, block_table, max_blocks, n_pages,
-                out, ldo, H, Hkv, hpc, tt, scale, window, status, slopes, sinks, gate, ldg, softcap, keep_first);
-    return lgml_launch_status("prefill_attention_twin");
+                out, ldo, H, Hkv, hpc, tt, scale, window, status, slopes, sinks, gate, ldg, softcap, keep_first, n_ranges, part_o, part_ml);
+    rc = lgml_launch_status("prefill_attention_twin");
+    if (rc || n_ranges == 1) return rc;
+    lgml_launch(twin_merge_kernel<D>, dim3((2 * tt * H + MERGE_WARPS - 1) / MERGE_WARPS, grid.y), MERGE_WARPS * 32, 0, stream, tiles, part_o, part_ml, n_ranges, out, ldo, H,
+                sinks, gate, ldg);
+    return lgml_launch_status("prefill_attention_twin merge");
 }
 }  // namespace
 
@@ -696,8 +790,10 @@ LGML_API int lgml_prefill_attention_twin_takes(int D) { return D == 64 || D == 1
 
 LGML_API int lgml_prefill_attention_twin(const void *q, int ldq, const int *positions, const int *tiles, int n_tiles, const int *block_table,
                                          int max_blocks, const void *k_pages, const void *v_pages, int n_pages, int page_size, void *out,
-                                         int ldo, int H, int Hkv, int D, float scale, int window, int *status, cudaStream_t stream) {
+                                         int ldo, int H, int Hkv, int D, float scale, int window, int n_ranges, float *part, int part_rows, int *status, cudaStream_t stream) {
     LGML_REQUIRE(n_tiles >= 0 && H > 0 && Hkv > 0 && max_blocks > 0 && n_pages > 0, "prefill_attention_twin: bad sizes");
+    LGML_REQUIRE(n_ranges >= 1 && n_ranges <= MOST_RANGES && (n_ranges == 1 || (part != nullptr && ((uintptr_t)part & 15) == 0 && part_rows > 0)),
+                 "prefill_attention_twin: %d ranges of keys (1 to 32, with scratch for more than one)", n_ranges);
     LGML_REQUIRE(page_size == PAGE, "prefill_attention_twin: pages of %d tokens, this kernel takes %d", page_size, PAGE);
     LGML_REQUIRE(H % Hkv == 0, "prefill_attention_twin: %d heads are no multiple of %d KV heads", H, Hkv);
     LGML_REQUIRE(D == 64 || D == 128, "prefill_attention_twin: head_dim %d (this kernel takes 64 and 128)", D);
@@ -715,18 +811,24 @@ LGML_API int lgml_prefill_attention_twin(const void *q, int ldq, const int *posi
     const __nv_bfloat16 *qq = (const __nv_bfloat16 *)q, *kk = (const __nv_bfloat16 *)k_pages, *vv = (const __nv_bfloat16 *)v_pages;
     __nv_bfloat16 *oo = (__nv_bfloat16 *)out;
     if (D == 64)
-        return launch<64, false>(grid, qq, ldq, positions, tiles, block_table, max_blocks, kk, vv, n_pages, oo, ldo, H, Hkv, hpc, tile_tokens / 2, scale, window, status, stream);
-    return launch<128, false>(grid, qq, ldq, positions, tiles, block_table, max_blocks, kk, vv, n_pages, oo, ldo, H, Hkv, hpc, tile_tokens / 2, scale, window, status, stream);
+        return launch<64, false>(grid, qq, ldq, positions, tiles, block_table, max_blocks, kk, vv, n_pages, oo, ldo, H, Hkv, hpc, tile_tokens / 2, scale, window, status, stream, n_ranges, part, part_rows);
+    return launch<128, false>(grid, qq, ldq, positions, tiles, block_table, max_blocks, kk, vv, n_pages, oo, ldo, H, Hkv, hpc, tile_tokens / 2, scale, window, status, stream, n_ranges, part, part_rows);
 }
 
+// n_ranges > 1: every tile's pages in so many ranges, a CTA each, put together by a second kernel; `part` holds part_rows * H * n_ranges * (D + 2) floats,
+// part_rows being past every row of the tiles.
+//
 // The same kernel with a distance bias (slopes), a sink in the denominator (sinks) and an output
 // gate (float32 [tokens, H D], row stride ldg; or [tokens, H], row stride -ldg: one per head), each optional; keys and values
 // of one head size, 64 or 128.  keep_first: with a window, the first keys that stay visible beyond it.
 LGML_API int lgml_sink_attention_twin_keep(const void *q, int ldq, const int *positions, const int *tiles, int n_tiles, const int *block_table,
                                       int max_blocks, const void *k_pages, const void *v_pages, int n_pages, int page_size,
                                       const float *slopes, const float *sinks, const float *gate, int ldg, void *out, int ldo, int H, int Hkv,
-                                      int D, float scale, float softcap, int window, int keep_first, int *status, cudaStream_t stream) {
+                                      int D, float scale, float softcap, int window, int keep_first, int n_ranges, float *part, int part_rows, int *status,
+                                      cudaStream_t stream) {
     LGML_REQUIRE(n_tiles >= 0 && H > 0 && Hkv > 0 && max_blocks > 0 && n_pages > 0, "sink_attention_twin: bad sizes");
+    LGML_REQUIRE(n_ranges >= 1 && n_ranges <= MOST_RANGES && (n_ranges == 1 || (part != nullptr && ((uintptr_t)part & 15) == 0 && part_rows > 0)),
+                 "sink_attention_twin: %d ranges of keys (1 to 32, with scratch for more than one)", n_ranges);
     LGML_REQUIRE(page_size == PAGE, "sink_attention_twin: pages of %d tokens, this kernel takes %d", page_size, PAGE);
     LGML_REQUIRE(H % Hkv == 0, "sink_attention_twin: %d heads are no multiple of %d KV heads", H, Hkv);
     LGML_REQUIRE(D == 64 || D == 128, "sink_attention_twin: head_dim %d (this kernel takes 64 and 128)", D);
@@ -749,15 +851,7 @@ LGML_API int lgml_sink_attention_twin_keep(const void *q, int ldq, const int *po
     __nv_bfloat16 *oo = (__nv_bfloat16 *)out;
     if (D == 64)
         return launch<64, true>(grid, qq, ldq, positions, tiles, block_table, max_blocks, kk, vv, n_pages, oo, ldo, H, Hkv, hpc, tile_tokens / 2, scale, window,
-                                status, stream, slopes, sinks, gate, ldg, softcap, keep_first);
+                                status, stream, n_ranges, part, part_rows, slopes, sinks, gate, ldg, softcap, keep_first);
     return launch<128, true>(grid, qq, ldq, positions, tiles, block_table, max_blocks, kk, vv, n_pages, oo, ldo, H, Hkv, hpc, tile_tokens / 2, scale, window,
-                             status, stream, slopes, sinks, gate, ldg, softcap, keep_first);
-}
-
-LGML_API int lgml_sink_attention_twin(const void *q, int ldq, const int *positions, const int *tiles, int n_tiles, const int *block_table,
-                                      int max_blocks, const void *k_pages, const void *v_pages, int n_pages, int page_size,
-                                      const float *slopes, const float *sinks, const float *gate, int ldg, void *out, int ldo, int H, int Hkv,
-                                      int D, float scale, float softcap, int window, int *status, cudaStream_t stream) {
-    return lgml_sink_attention_twin_keep(q, ldq, positions, tiles, n_tiles, block_table, max_blocks, k_pages, v_pages, n_pages, page_size, slopes, sinks,
-                                         gate, ldg, out, ldo, H, Hkv, D, scale, softcap, window, 0, status, stream);
+                             status, stream, n_ranges, part, part_rows, slopes, sinks, gate, ldg, softcap, keep_first);
 }

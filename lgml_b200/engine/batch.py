@@ -98,6 +98,7 @@ class StepBatch:
         self.shared = {}                # what one layer of this step keeps for later layers (by name)
         self._tiles = {}
         self.replayed = False           # are its launches recorded, and run again for other contexts?
+        self.replay_reach = 0           # ... of over half of so many tokens and up to all of them (0: any that are short)
         self.after_staged_copy = None   # called after a later copy out of the pinned buffer (its owner marks the buffer busy again)
 
         # Rows of tokens are written by C: a prompt portion brings thousands of them, and Python's way with them costs as much as

@@ -211,8 +211,8 @@ class PromptGraph:
     them.  The step's description lives in one device buffer as ``StepBatch`` lays it out, with
     block tables of a fixed width; a replay refreshes it with one copy from pinned memory."""
 
-    def __init__(self, runner, n_tokens: int, n_rows: int):
-        self.runner, self.n_tokens, self.n_rows = runner, n_tokens, n_rows
+    def __init__(self, runner, n_tokens: int, n_rows: int, reach: int = 0):
+        self.runner, self.n_tokens, self.n_rows, self.reach = runner, n_tokens, n_rows, reach
         self.widths = list(runner._graph_widths)
         total = StepBatch.buffer_ints(n_tokens, 1, n_rows, self.widths)
         self.dev = torch.zeros(total, dtype=torch.int32, device=runner.rt.device)
@@ -227,7 +227,7 @@ class PromptGraph:
         batch = StepBatch(self.runner.cache, [req], [list(tokens) + [0] * pad], [list(want)], self.runner.rt.device, pinned,
                           table_widths=self.widths, device_buffer=self.dev)
         batch._tiles = self.tiles
-        batch.replayed = True
+        batch.replayed, batch.replay_reach = True, self.reach
         batch.after_staged_copy = None
         if self.graph is None:
             import gc

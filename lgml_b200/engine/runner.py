@@ -247,9 +247,12 @@ class ModelRunner:
         req, tokens, want = entry
         page = self.cache.page_size
         key = (prompt_graph_length(len(tokens), page), len(want))
+        end = req.n_tokens + key[0]
+        if end > 512 and self.rt.dtype == torch.bfloat16:       # into how many ranges attention cuts the keys is recorded too
+            key += (1 << (end - 1).bit_length(),)
         g = self._prompt_graphs.get(key)
         if g is None:
-            g = self._prompt_graphs[key] = PromptGraph(self, key[0], key[1])
+            g = self._prompt_graphs[key] = PromptGraph(self, *key)
         else:
             self.graph_replays += 1
         self.last_batch = g.run(req, tokens, want, stage[0])

@@ -674,11 +674,11 @@ def sink_twin_supports(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor
 def sink_attention_twin(q: torch.Tensor, positions: torch.Tensor, tiles: torch.Tensor, block_table: torch.Tensor, k_pages: torch.Tensor,
                         v_pages: torch.Tensor, out: torch.Tensor, n_heads: int, scale: float, window: int, status: torch.Tensor,
                         slopes: Optional[torch.Tensor] = None, sinks: Optional[torch.Tensor] = None,
-                        gate: Optional[torch.Tensor] = None, keep_first: int = 0, softcap: float = 0.0) -> torch.Tensor:
+                        gate: Optional[torch.Tensor] = None, keep_first: int = 0, softcap: float = 0.0, n_ranges: int = 1) -> torch.Tensor:
     """``sink_attention`` for prompts and portions on tcgen05 tensor cores: the two-tile kernel of
     ``prefill_attention_twin`` with the slopes' bias on the scores, the sink in the denominator and
     the gate on the output.  bfloat16, pages of 64, keys and values of one head size (64 or 128).
-    ``tiles`` as for ``prefill_attention_twin`` (``prefill_twin_tile_tokens``)."""
+    ``tiles`` and ``n_ranges`` as for ``prefill_attention_twin``."""
     _need(q, "queries", torch.bfloat16, 2)
     _need(out, "attention output", torch.bfloat16, 2)
     ldq, ldo = _rows_contiguous(q, "queries"), _rows_contiguous(out, "attention output")
@@ -702,10 +702,13 @@ def sink_attention_twin(q: torch.Tensor, positions: torch.Tensor, tiles: torch.T
     ldg = _gate_stride(gate, n, n_heads, d, "sink_attention_twin")
     fn = _fn("attention_prefill_twin", "lgml_sink_attention_twin_keep", [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
                                                                     c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
-                                                                    c_int, c_float, c_float, c_int, c_int, c_void_p, c_void_p], label="sink_attention_twin")
+                                                                    c_int, c_float, c_float, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p],
+             label="sink_attention_twin")
+    part = _range_scratch(n, n_heads, d, n_ranges, q.device)
     _check("attention_prefill_twin", fn(_ptr(q), ldq, _ptr(positions), _ptr(tiles), tiles.shape[0], _ptr(block_table), block_table.shape[1],
                                         _ptr(k_pages), _ptr(v_pages), n_pages, page, _ptr(slopes), _ptr(sinks), _ptr(gate), ldg, _ptr(out), ldo,
-                                        n_heads, hkv, d, float(scale), float(softcap or 0.0), int(window or 0), int(keep_first or 0), _ptr(status), _stream()), "sink_attention_twin")
+                                        n_heads, hkv, d, float(scale), float(softcap or 0.0), int(window or 0), int(keep_first or 0), n_ranges, _ptr(part), n,
+                                        _ptr(status), _stream()), "sink_attention_twin")
     return out
 
 
@@ -2669,8 +2672,8 @@ def prefill_tile_tokens(n_heads: int, n_kv_heads: int) -> int:
 
 
 def _prefill_attention_call(library: str, symbol: str, label: str, q, positions, tiles, block_table, k_pages, v_pages, out, n_heads, scale,
-                            window, status) -> torch.Tensor:
-    """The checks and the call that the three prefill attention kernels share (one signature)."""
+                            window, status, n_ranges: Optional[int] = None) -> torch.Tensor:
+    """The checks and the call that the three prefill attention kernels share (one signature; the one for two tiles a CTA takes ranges of keys too)."""
     _need(q, "queries", torch.bfloat16, 2)
     _need(out, "attention output", torch.bfloat16, 2)
     ldq, ldo = _rows_contiguous(q, "queries"), _rows_contiguous(out, "attention output")
@@ -2685,11 +2688,14 @@ def _prefill_attention_call(library: str, symbol: str, label: str, q, positions,
         raise KernelError(f"{label}: q {tuple(q.shape)} / out {tuple(out.shape)} / tiles {tuple(tiles.shape)} do not fit")
     if not k_pages.is_contiguous() or not v_pages.is_contiguous() or not block_table.is_contiguous() or not tiles.is_contiguous():
         raise KernelError(f"{label}: pages, block table and tiles must be contiguous")
+    ranges_types = [] if n_ranges is None else [c_int, c_void_p, c_int]
     fn = _fn(library, symbol, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
-                               c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p])
+                               c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int] + ranges_types + [c_void_p, c_void_p])
+    part = None if n_ranges is None else _range_scratch(n, n_heads, d, n_ranges, q.device)
+    ranges = () if n_ranges is None else (n_ranges, _ptr(part), n)
     _check(library, fn(_ptr(q), ldq, _ptr(positions), _ptr(tiles), tiles.shape[0], _ptr(block_table), block_table.shape[1],
                        _ptr(k_pages), _ptr(v_pages), n_pages, page, _ptr(out), ldo, n_heads, hkv, d, float(scale),
-                       int(window or 0), _ptr(status), _stream()), label)
+                       int(window or 0), *ranges, _ptr(status), _stream()), label)
     return out
 
 
@@ -2728,14 +2734,43 @@ def prefill_twin_ctas(n_heads: int, n_kv_heads: int) -> int:
     return n_kv_heads * -(-(n_heads // n_kv_heads) // 8)
 
 
+def prefill_twin_ranges(batch, tiles: torch.Tensor, ctas: int, window: int, keep_first: int = 0) -> int:
+    """How many ranges a tile's pages are cut into: three, or the largest power of two up to 16, that gives every CTA an SM to
+    itself and two pages and more; tiles of fewer than eight pages stay whole.
+
+    One CTA works through its pages one after another (1.05 us each, with a bias 1.1 to 2.5), so a few tiles behind a long
+    context leave most SMs idle; the second kernel adds about 4.  16 CTAs of 33 pages (32 heads of 8, 37 tokens behind
+    2,048): 37.1 us in one range, 25.4 in 2, 18.3 in 4, 16.5 in 8.  8 CTAs of 8 pages: 13.2, 12.2, 10.0.  32 CTAs of 10:
+    16.0, 16.2, 14.7.  40 CTAs of 33: 37.0, 24.4, and 20.2 in 3.  64 CTAs of 24 with a bias: 38.3, 25.3.  Where the CTAs
+    no longer fit side by side it loses (128 of 8 pages: 14.9 against 26.9 in 2), and counts from five that are no powers
+    of two are up to 3 us slower than the power below them.
+
+    A captured portion is replayed for contexts of over half its reach, up to all of it."""
+    longest = batch.max_kv_len
+    if batch.replayed:
+        longest = batch.replay_reach // 2
+    if window:
+        longest = min(longest, window + 64) + keep_first
+    pages = longest // 64
+    most = min(sm_count() // max(tiles.shape[0] * ctas, 1), pages // 2, 16)
+    if most < 2 or pages < 8:
+        return 1
+    return most if most == 3 else 1 << (most.bit_length() - 1)
+
+
+def _range_scratch(n: int, n_heads: int, dim: int, n_ranges: int, device) -> Optional[torch.Tensor]:
+    return torch.empty(n * n_heads * n_ranges * (dim + 2), dtype=torch.float32, device=device) if n_ranges > 1 else None
+
+
 def prefill_attention_twin(q: torch.Tensor, positions: torch.Tensor, tiles: torch.Tensor, block_table: torch.Tensor,
                            k_pages: torch.Tensor, v_pages: torch.Tensor, out: torch.Tensor, n_heads: int, scale: float, window: int,
-                           status: torch.Tensor) -> torch.Tensor:
+                           status: torch.Tensor, n_ranges: int = 1) -> torch.Tensor:
     """bfloat16 attention for prompts and portions on tcgen05 tensor cores, two tiles of 128
     rows per CTA (scores, P and the output in tensor memory), for head sizes 64 and 128.
-    ``tiles`` as for ``prefill_attention``, each at most ``prefill_twin_tile_tokens`` long."""
+    ``tiles`` as for ``prefill_attention``, each at most ``prefill_twin_tile_tokens`` long; ``n_ranges`` (up to 32): every
+    tile's pages in so many ranges, a CTA each."""
     return _prefill_attention_call("attention_prefill_twin", "lgml_prefill_attention_twin", "prefill_attention_twin", q, positions, tiles,
-                                   block_table, k_pages, v_pages, out, n_heads, scale, window, status)
+                                   block_table, k_pages, v_pages, out, n_heads, scale, window, status, n_ranges=n_ranges)
 
 
 def prefill_tc_supports(q: torch.Tensor, out: torch.Tensor) -> bool:
@@ -2865,9 +2900,13 @@ def paged_attention(q, batch, cache, out, n_heads: int, scale: float, window: in
             return decode_attention(q, batch.positions, batch.seq_of_token, cache.block_table, cache.k, cache.v, out, n_heads, scale,
                                     window, status, n_splits, max_new_tokens=batch.max_q_len)
         if d in (64, 128) and PREFILL_ATTENTION == "tcgen05" and prefill_tc_supports(q, out):
-            tokens = prefill_twin_tile_tokens(n_heads, hkv)
-            tiles = batch.twin_tiles(tokens, prefill_twin_ctas(n_heads, hkv)) if hasattr(batch, "twin_tiles") else batch.attention_tiles(tokens)
-            return prefill_attention_twin(q, batch.positions, tiles, cache.block_table, cache.k, cache.v, out, n_heads, scale, window, status)
+            tokens, ctas, n_ranges = prefill_twin_tile_tokens(n_heads, hkv), prefill_twin_ctas(n_heads, hkv), 1
+            if hasattr(batch, "twin_tiles"):
+                tiles = batch.twin_tiles(tokens, ctas)
+                n_ranges = prefill_twin_ranges(batch, tiles, ctas, window)
+            else:
+                tiles = batch.attention_tiles(tokens)
+            return prefill_attention_twin(q, batch.positions, tiles, cache.block_table, cache.k, cache.v, out, n_heads, scale, window, status, n_ranges=n_ranges)
         if d <= 128 and PREFILL_ATTENTION in ("tcgen05", "single") and prefill_tc_supports(q, out):
             tiles = batch.attention_tiles(prefill_tc_tile_tokens(n_heads, hkv))
             return prefill_attention_tc(q, batch.positions, tiles, cache.block_table, cache.k, cache.v, out, n_heads, scale, window, status)

@@ -654,6 +654,36 @@ def run_attention(kind, case, window, n_splits=None):
     return out.double().cpu(), ref_attention(case, scale, window)
 
 
+@pytest.mark.parametrize("H,G,D", [(8, 1, 64), (12, 4, 128), (7, 7, 64), (5, 1, 128)])
+@pytest.mark.parametrize("window,keep,cap", [(0, 0, 0.0), (37, 0, 0.0), (130, 70, 0.0), (0, 0, 8.0)])
+@pytest.mark.parametrize("n_ranges", [2, 3, 16, 32])
+def test_prompt_attention_in_ranges_of_keys(H, G, D, window, keep, cap, n_ranges):
+    """A tile's pages in ranges against the same pages in one: ranges without pages, rows a window leaves without keys in a
+    range, partial last pages (NaN behind them), sinks and both gates.  Each form rounds its probabilities to bfloat16 once (2^-9
+    of a weighted mean of values, so of at most the largest of them), and its result (2^-9 of that)."""
+    from lgml_b200 import ops
+
+    case = make_attention_case(3, H, G, D, kv_lens=[200, 1, 65, 530, 448], q_lens=[200, 1, 2, 130, 64], dtype=torch.bfloat16)
+    q, kp, vp, tab = (case[k].to(DEV) for k in ("q", "k_pages", "v_pages", "table"))
+    b, n, st = FakeBatch(case), case["q"].shape[0], status()
+    tiles = b.attention_tiles(ops.prefill_twin_tile_tokens(H, G))
+    g = torch.Generator().manual_seed(4)
+    sinks, values, heads = torch.randn(H, generator=g).to(DEV), torch.randn(n, H * D, generator=g).to(DEV), torch.randn(n, H, generator=g).to(DEV)
+    slopes = torch.linspace(0.5, 0.004, H).to(DEV)
+    largest = vp.float().nan_to_num(0.0).abs().max().item()
+    for kwargs in ([{}] if not (keep or cap) else []) + [dict(sinks=sinks, gate=values, slopes=slopes), dict(sinks=sinks, gate=heads), dict(slopes=slopes)]:
+        outs = []
+        for ranges in (1, n_ranges):
+            out = torch.full_like(q, float("nan"))
+            if kwargs:
+                ops.sink_attention_twin(q, b.positions, tiles, tab, kp, vp, out, H, D ** -0.5, window, st, keep_first=keep, softcap=cap, n_ranges=ranges, **kwargs)
+            else:
+                ops.prefill_attention_twin(q, b.positions, tiles, tab, kp, vp, out, H, D ** -0.5, window, st, n_ranges=ranges)
+            outs.append(out.float())
+        assert int(st.item()) == 0 and torch.isfinite(outs[1]).all()
+        torch.testing.assert_close(outs[1], outs[0], atol=2.0 ** -8 * largest, rtol=2.0 ** -8)
+
+
 @pytest.mark.parametrize("H,G,D", ATT_SHAPES + [(2, 2, 256), (3, 1, 40)])
 @pytest.mark.parametrize("dtype,window", [(torch.float32, 0), (torch.float32, 37), (torch.bfloat16, 0)])
 def test_attention_ref_kernel(H, G, D, dtype, window):
