@@ -204,3 +204,29 @@ def test_short_portions_replayed_from_captured_steps(tiny, dtype):
         want = H.run_trace(plain, steps)
         assert not plain._prompt_graphs
         assert all(torch.equal(got[k], want[k]) for k in want)
+
+
+def test_short_portions_behind_long_contexts(tmp_path):
+    """Captured portions whose keys attention cuts into ranges: portions of 64 tokens that end at 640 and 1,024 and of 16 that end
+    at 1,040 (two reaches), replayed for a second request, against the plain implementation and against a runner without graphs."""
+    from lgml_b200.engine.engine import parse_dtype
+    from lgml_b200.engine.runner import ModelRunner
+
+    cfg = dict(H.TINY["A"][0], hidden_size=128, num_attention_heads=4, num_key_value_heads=2, head_dim=64, max_position_embeddings=2048)
+    folder = H.make_folder(tmp_path / "long", cfg, 3, dtype="bfloat16", sharpen=SHARPEN["bfloat16"])
+    steps, seqs = [], {"x": H.random_ids(1088, cfg["vocab_size"], 21), "y": H.random_ids(1088, cfg["vocab_size"], 22)}
+    for rid, ids in seqs.items():
+        for a, b in ((0, 576), (576, 640), (640, 960), (960, 1024), (1024, 1040)):
+            steps.append({"step": len(steps), "entries": [{"id": rid, "tokens": ids[a:b], "want": [b - a - 1]}], "end": [rid] if b == 1040 else []})
+    runner = make_runner(folder, "bfloat16", n_pages=20)
+    got = H.run_trace(runner, steps)
+    assert sorted(runner._prompt_graphs) == [(16, 1, 2048), (64, 1, 1024)]
+    plain = ModelRunner.from_folder(folder, parse_dtype("bfloat16"), "cuda:0", n_pages=20, max_slots=4, use_graphs=False)
+    want = H.run_trace(plain, steps)
+    for rid, ids in seqs.items():
+        ref = H.oracle_logits(folder, ids)
+        for rows in (got, want):
+            for (r, pos), row in rows.items():
+                if r == rid:
+                    err = (row.double() - ref[pos]).abs()
+                    assert bool((err <= TOL["bfloat16"]["atol"] + TOL["bfloat16"]["rtol"] * ref[pos].abs()).all()), (rid, pos, float(err.max()))
