@@ -132,11 +132,10 @@ class Runtime:
             if plain and ops.sink_twin_supports(q, out, cache.k, cache.v, gate):
                 # prompts and portions, keys and values of one head size (64 or 128): the two-tile tcgen05 kernel
                 hkv = cache.k.shape[1]
-                ctas = ops.prefill_twin_ctas(n_heads, hkv)
-                tiles = batch.twin_tiles(ops.prefill_twin_tile_tokens(n_heads, hkv), ctas)
+                tiles, n_ranges = ops.prefill_twin_plan(batch, n_heads, hkv, window or 0, keep_first)
                 return ops.sink_attention_twin(q, batch.positions, tiles, cache.block_table, cache.k, cache.v, out, n_heads, scale, window,
                                                self.status, slopes=slopes, sinks=sinks, gate=gate, keep_first=keep_first, softcap=softcap,
-                                               n_ranges=ops.prefill_twin_ranges(batch, tiles, ctas, window, keep_first))
+                                               n_ranges=n_ranges)
             # every other head size up to 128: tiles of 64 tokens, mma.sync
             tiles = batch.attention_tiles(ops.SINK_TILE_TOKENS)
             return ops.sink_attention_mma(q, batch.positions, tiles, cache.block_table, cache.k, cache.v, out, n_heads, scale, window,

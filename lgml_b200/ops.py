@@ -2758,6 +2758,15 @@ def prefill_twin_ranges(batch, tiles: torch.Tensor, ctas: int, window: int, keep
     return most if most == 3 else 1 << (most.bit_length() - 1)
 
 
+def prefill_twin_plan(batch, n_heads: int, n_kv_heads: int, window: int, keep_first: int = 0) -> tuple:
+    """(A step's tiles for two tiles a CTA, ranges of pages).  A step that knows whole tiles only has them in one range."""
+    tokens, ctas = prefill_twin_tile_tokens(n_heads, n_kv_heads), prefill_twin_ctas(n_heads, n_kv_heads)
+    if not hasattr(batch, "twin_tiles"):
+        return batch.attention_tiles(tokens), 1
+    tiles = batch.twin_tiles(tokens, ctas)
+    return tiles, prefill_twin_ranges(batch, tiles, ctas, window, keep_first)
+
+
 def _range_scratch(n: int, n_heads: int, dim: int, n_ranges: int, device) -> Optional[torch.Tensor]:
     return torch.empty(n * n_heads * n_ranges * (dim + 2), dtype=torch.float32, device=device) if n_ranges > 1 else None
 
@@ -2900,12 +2909,7 @@ def paged_attention(q, batch, cache, out, n_heads: int, scale: float, window: in
             return decode_attention(q, batch.positions, batch.seq_of_token, cache.block_table, cache.k, cache.v, out, n_heads, scale,
                                     window, status, n_splits, max_new_tokens=batch.max_q_len)
         if d in (64, 128) and PREFILL_ATTENTION == "tcgen05" and prefill_tc_supports(q, out):
-            tokens, ctas, n_ranges = prefill_twin_tile_tokens(n_heads, hkv), prefill_twin_ctas(n_heads, hkv), 1
-            if hasattr(batch, "twin_tiles"):
-                tiles = batch.twin_tiles(tokens, ctas)
-                n_ranges = prefill_twin_ranges(batch, tiles, ctas, window)
-            else:
-                tiles = batch.attention_tiles(tokens)
+            tiles, n_ranges = prefill_twin_plan(batch, n_heads, hkv, window)
             return prefill_attention_twin(q, batch.positions, tiles, cache.block_table, cache.k, cache.v, out, n_heads, scale, window, status, n_ranges=n_ranges)
         if d <= 128 and PREFILL_ATTENTION in ("tcgen05", "single") and prefill_tc_supports(q, out):
             tiles = batch.attention_tiles(prefill_tc_tile_tokens(n_heads, hkv))
