@@ -250,7 +250,10 @@ __device__ __forceinline__ void chunk_decays(const ChunkArgs &p, int h, int t0, 
         const int i = 2 * lane + u;
         const float dt = i < nt ? softplus_(act_load(p.dt_raw + (size_t)(t0 + i) * p.ldd + h) + bias) : 0.f;
         dts[i] = dt;
-        l[u] = -(double)(a * dt);
+        // (a decay below e^-104 is 0 in float32: nothing is kept.  No lower than e^-200 here, or sums of infinite logarithms would have no
+        // differences: heads with a_log of 88 and more, whose a dt is infinite.  A NaN stays one.)
+        const double log_decay = i < nt ? -(double)(a * dt) : 0.0;
+        l[u] = log_decay < -200.0 ? -200.0 : log_decay;
     }
     double sum = l[0] + l[1];
 #pragma unroll

@@ -285,6 +285,34 @@ def test_state_space_scan_in_chunks(Hs, G, Pd, N, lens):
     assert float((y - want)[there].abs().max()) < 1e-5 * (1 + float(want[there].abs().max()))
 
 
+def test_state_space_chunks_of_heads_that_keep_nothing():
+    """Rates whose product with a step size overflows (a decay of 0), beside ordinary heads, one that forgets nothing and steps so wide that an
+    ordinary head keeps nothing either: in chunks what the scan gives."""
+    from lgml_b200 import ops
+
+    Hs, G, Pd, N, lens = 4, 2, 8, 12, (130, 200)
+    inner, n, C = Hs * Pd, sum(lens), Hs * Pd + 2 * G * N
+    rng = np.random.default_rng(12)
+    x, dt = f32(rng.normal(size=(n, C))), f32(rng.normal(size=(n, Hs)) * 0.5)
+    dt[70, 2], dt[150:153, 2] = 300.0, 1e5
+    bias, a_log, skip = f32(rng.normal(size=Hs) * 0.3 - 2.5), f32([95.0, -200.0, -2.0, 87.5]), f32(rng.normal(size=Hs))
+    rows = [(0, 64), (64, 128), (128, 130), (130, 194), (194, 258), (258, 322), (322, 330)]
+    pieces, starts = (torch.tensor(rows, dtype=torch.int32, device=DEV), i32([0, 3, 7])), i32([0, 130, 330])
+    state0 = torch.randn(4, inner * N, device=DEV)
+
+    def run(**how):
+        state = state0.clone()
+        return ops.ssd_scan(x, dt, bias, a_log, skip, state, starts, i32([3, 1]), Hs, G, Pd, N, **how), state
+
+    y, state = run(pieces=pieces, piece_tokens=64)
+    want, want_state = run()
+    assert bool(torch.isfinite(want).all()) and bool(torch.isfinite(want_state).all())
+    assert bool(torch.isfinite(y).all()) and bool(torch.isfinite(state).all())
+    for got, exact in ((y.view(n, Hs, Pd), want.view(n, Hs, Pd)), (state[[1, 3]].view(2, Hs, -1), want_state[[1, 3]].view(2, Hs, -1))):
+        # (a head against its own largest: the wide steps write some 1e5)
+        assert bool(((got - exact).abs().amax(dim=(0, 2)) <= 1e-5 * (1 + exact.abs().amax(dim=(0, 2)))).all())
+
+
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("inner,groups", [(20, 1), (48, 3), (96, 2), (640, 5)])
 def test_gate_then_norm_in_parts(out_dtype, inner, groups):
