@@ -644,7 +644,8 @@ template <bool VEC, typename TO> int run_split(const Call &c) {
     if (c.M <= 8) return one ? launch_few<1, 4, 16, VEC, TO>(c) : launch_few<1, 4, 8, VEC, TO>(c);
     if (c.M <= 16) return one ? launch_few<2, 2, 16, VEC, TO>(c) : launch_few<2, 2, 8, VEC, TO>(c);
     const long long blocks = (long long)((c.M + 31) / 32) * ((c.N + 15) / 16), tiles = (long long)((c.M + 63) / 64) * ((c.N + 63) / 64);
-    if ((blocks + 147) / 148 * 9 <= 58 + ((tiles + 147) / 148 - 1) * 37) return launch_few<4, 2, 8, VEC, TO>(c);
+    // (the blocks' rows are the grid's second dimension: no more than 65,535 of them)
+    if ((blocks + 147) / 148 * 9 <= 58 + ((tiles + 147) / 148 - 1) * 37 && c.M <= 65535 * 32) return launch_few<4, 2, 8, VEC, TO>(c);
     return launch_many<VEC, TO>(c);
 }
 

@@ -323,6 +323,21 @@ def test_gemm_f32_in_halves(M, N, K, pad, scale):
         assert torch.equal(one[0], out[m])
 
 
+@pytest.mark.parametrize("M,N", [(65535 * 32, 8), (65535 * 32 + 1, 8), (65535 * 32 + 1, 17)])
+def test_gemm_f32_of_millions_of_rows(M, N):
+    """Few features by as many rows as blocks of 32 rows have numbers for in a grid's second dimension, and one more."""
+    from lgml_b200 import ops
+
+    torch.manual_seed(N)
+    a, w, out = torch.randn(M, 64, device=DEV), torch.randn(N, 64, device=DEV), torch.empty(M, N, device=DEV)
+    ops.gemm_f32(a, w, out)
+    for m in (0, M // 2, M - 40):
+        few = torch.empty(40, N, device=DEV)
+        ops.gemm_f32(a[m:m + 40], w, few)
+        assert torch.equal(few, out[m:m + 40])
+    assert torch.allclose(out, a @ w.t(), rtol=1e-2, atol=0.2)           # (torch's product may round its operands to 11 bits)
+
+
 @pytest.mark.parametrize("M", [1, 20, 200])
 def test_gemm_f32_of_infinite_and_huge_values(M):
     """What a chain of FMAs gives: an infinity times an exact number is infinite, not lost between the halves; a sum that overflows is infinite
