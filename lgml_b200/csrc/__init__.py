@@ -148,8 +148,8 @@ LIBRARY_HEADERS: Dict[str, List[str]] = {
     "attention_decode_noalloc": ["attention_decode.cu", "attention_decode_noalloc.h"],
     "attention_heads": ["few_rows.cuh"],
     "rglru": ["few_rows.cuh"],
-    "gemm_f32": ["tf32_halves.cuh"],
-    "ssd": ["tf32_halves.cuh"],
+    "gemm_f32": ["bf16_thirds.cuh"],
+    "ssd": ["bf16_thirds.cuh"],
 }
 
 

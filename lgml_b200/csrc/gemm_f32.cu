@@ -3,24 +3,29 @@
 // result does not depend on what else is in the batch.  It stands where mischief/lgml calls mul_mat with the f32
 // flag (src/lgml.c:1811-1839).
 //
-// K >= 64: on the tensor cores, both operands in two tf32 halves (below).  A chain of K dependent FMAs takes
-// 4 cycles a step and the FMA units give 72 TFLOP/s at the very best (43 in tiles); three tf32 products of m16n8k8 give
-// 92, and a K that is added up in segments can be shared out among warps.  Off 64 bits by (2-norm, random signs; chain of FMAs, here):
-//   K = 64 1.4e-7, 1.1e-7;  256 2.9e-7, 1.2e-7;  2048 8.1e-7, 1.4e-7;  14336 2.2e-6, 2.3e-7.   (K = 32: 1.03e-7, 1.05e-7; 16: 0.7e-7, 1.0e-7.)
+// K >= 64: on the tensor cores, both operands in three bfloat16 parts that hold all their bits (below).  A chain of K dependent FMAs takes
+// 4 cycles a step, and a K that is added up in segments can be shared out among warps.  Off 64 bits by (2-norm, chain of FMAs, here; random signs | one
+// sign | one term in 16 | rows of one term):
+//   K = 64    1.4e-7, 0.6e-7 | 1.1e-7, 0.5e-7 | 4.5e-8, 4.2e-8 | 2.5e-8, 2.5e-8
+//   K = 256   2.9e-7, 0.8e-7 | 2.2e-7, 0.5e-7 | 7.5e-8, 6.0e-8 | 2.5e-8, 2.5e-8
+//   K = 2048  8.1e-7, 1.1e-7 | 6.0e-7, 0.6e-7 | 2.1e-7, 0.9e-7 | 2.5e-8, 2.5e-8
+//   K = 14336 2.1e-6, 2.1e-7 | 1.7e-6, 1.5e-7 | 5.4e-7, 2.0e-7 | 2.5e-8, 2.5e-8
 //   * gemm_f32_few_kernel, up to 32 rows (or more of few features): warps stream W, each its segments of K.
 //   * gemm_f32_many_kernel: tiles of 64 x 64.
 // K < 64: every output sums its products in the order k = 0, 1, 2, ..., one chain of FMAs.
 //   * gemm_f32_rows_kernel, up to 4 rows: a warp streams 8 or 16 rows of W through shared memory of its own.
 //   * gemm_f32_tile_kernel, more rows: tiles of A and W by asynchronous copies, several blocks an SM.
 //   * gemm_f32_ragged_kernel, more rows that do not all start on 16 bytes: tiles element by element.
-// One B200, weights from HBM, microseconds, one chain of FMAs an output and now:
-//   M, N, K:  4, 2048, 2048: 12.3 -> 5.6;  4, 2048, 5632: 29.6 -> 10.2;  4, 11264, 2048: 28.7 -> 20.4;  4, 32000, 2048: 58.6 -> 47 (5.6 TB/s);
-//   32, 2048, 5632: 109 -> 24;  89, 2048, 5632: 159 -> 66;  812, 11264, 2048: 874 -> 641 (58 TFLOP/s);  2048, 32000, 2048: 5,872 -> 4,274.
+// One B200, weights from HBM, launched one behind the other, microseconds, one chain of FMAs an output and now:
+//   M, N, K:  4, 2048, 2048: 14.8 -> 10;  4, 2048, 5632: 31.2 -> 13.5;  4, 11264, 2048: 31 -> 22.4;  4, 32000, 2048: 59 -> 54 (4.9 TB/s);
+//   32, 2048, 5632: 111 -> 38;  89, 2048, 5632: 160 -> 105;  89, 11264, 2048: 144 -> 177;  812, 11264, 2048: 883 -> 862;  2048, 32000, 2048: 5,879 -> 5,745.
+// Two tf32 halves instead of the three parts (six tensor products a run for these eight) took 646 for 812 rows, 67 for 89 and 21 for 4 of 11,264, but
+// held 23 bits: rows of one term were 8.6e-8 off, and one that selects a column did not give it exactly.
 
 #include <type_traits>
 
 #include "common.cuh"
-#include "tf32_halves.cuh"
+#include "bf16_thirds.cuh"
 
 LGML_DEFINE_LAST_ERROR(lgml_gemm_f32)
 
@@ -306,11 +311,12 @@ __global__ void __launch_bounds__(256) gemm_f32_ragged_kernel(const float *__res
     }
 }
 
-// ---- products of a long K: three tensor-core products of two halves each --------------------------
-// A run of 16 k is added up by add_run (tf32_halves.cuh; 16 features by 8 rows), the run's sum joins the sum of its segment of 128 k in
-// float32, and the segments' sums join in order.  One order for every kernel below, so a row has the same bits in each.  A result that is not finite, or below 2^-96, is formed again as the plain chain of FMAs: infinities, NaNs and overflows
-// come out as they do there, and so do sums of numbers so small that a lo is cut (a tf32 number below the normal ones is a multiple
-// of 2^-136, so an operand under 2^-112 has fewer than 24 bits; that shows beside operands over 2^16 only).
+// ---- products of a long K: eight tensor-core products of three parts each -------------------------
+// A run of 16 k is added up by add_run (bf16_thirds.cuh; 16 features by 8 rows), the run's sums join the sum of its segment of 128 k in
+// float32, and the segments' sums join in order.  One order for every kernel below, so a row has the same bits in each.  A result that is
+// not finite, or below 2^-96, is formed again as the plain chain of FMAs: infinities, NaNs and overflows come out as they do there, and so
+// do sums of numbers so small that a part is cut (a bfloat16 number below the normal ones is a multiple of 2^-133, so an operand
+// under 2^-110 has fewer than 24 bits; that shows in larger results beside operands over 2^14 only).
 constexpr int SEGMENT = 128, SPLIT_FROM = 64;
 
 __device__ __noinline__ float chain(const float *a, const float *w, int K) {
@@ -371,8 +377,8 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_f32_few_kernel(const float *_
                                                                       const float *__restrict__ bias, TO *__restrict__ C, int M, int N, int K, int lda,
                                                                       int ldw, int ldc) {
     using S = FewShape<NT, STAGES, WARPS>;
-    constexpr int SEGS = WARPS * FEW_EACH, STEPS = FEW_EACH * SEGMENT_STEPS;        // of a turn: segments of the block, steps of a warp
-    static_assert(STEPS % STAGES == 0, "a step's stage is known when it is compiled");
+    constexpr int SEGS = WARPS * FEW_EACH;                                           // segments of the block in a turn
+    static_assert(SEGMENT_STEPS % STAGES == 0, "a step's stage is known when it is compiled");
     extern __shared__ __align__(16) float smem_f[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
     const int n0 = blockIdx.x * 16, m0 = blockIdx.y * 8 * NT;
@@ -386,7 +392,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_f32_few_kernel(const float *_
 #pragma unroll
     for (int i = 0; i < 2 * NT; ++i) a_off[i] = (RowOffset<VEC>)min(i * 4 + r, M - 1 - m0) * lda;
     const uint32_t to = smem_addr(mine + swizzled(r, lane & 7));
-    // step s of a turn that starts at segment `first`: 32 k of this warp's segment s / SEGMENT_STEPS; behind STEPS the next turn's
+    // step s of a turn that starts at segment `first`: 32 k of this warp's segment s / SEGMENT_STEPS; behind its last the next turn's
     auto k_of = [&](int first, int s) { return (first + s / SEGMENT_STEPS * WARPS + warp) * SEGMENT + s % SEGMENT_STEPS * 32; };
     auto load_w = [&](int k0, int s) {
         if (k0 < K) copy_rows<VEC, 16, 32>(to + (s % STAGES) * S::STAGE_FLOATS * 4, wp, w_off, k0, c, K);
@@ -409,7 +415,9 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_f32_few_kernel(const float *_
     for (int o = 0; o < OUTS; ++o) total[o] = 0.f;
     const int frag = swizzled(g, q), frag_other = frag ^ 16;          // the row's first and second 16 k (rows 8 apart have the same order)
     for (int first = 0; first < n_seg; first += SEGS) {
-#pragma unroll
+        // (loops, not 32 copies of a step: a step is up to 500 instructions, and blocks that start would wait for them from memory; 32 x 2,048 x 5,632:
+        // 53 us with all 16 steps of a turn in a row)
+#pragma unroll 1
         for (int i = 0; i < FEW_EACH; ++i) {
             if (first + i * WARPS + warp >= n_seg) break;
             float sum[1][NT][4];
@@ -417,28 +425,31 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_f32_few_kernel(const float *_
             for (int j = 0; j < NT; ++j)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) sum[0][j][e] = 0.f;
+#pragma unroll(NT <= 2 ? SEGMENT_STEPS / STAGES : 1)
+            for (int s0 = i * SEGMENT_STEPS; s0 < (i + 1) * SEGMENT_STEPS; s0 += STAGES) {
 #pragma unroll
-            for (int ss = 0; ss < SEGMENT_STEPS; ++ss) {
-                const int s = i * SEGMENT_STEPS + ss, k0 = k_of(first, s), ahead = s + STAGES - 1;
-                cp_async_wait<STAGES - 2>();
-                __syncwarp();
-                load_w(k_of(first, ahead), ahead);
-                load_a(k_of(first, ahead), ahead);
-                cp_async_commit();
-                const float *ws = mine + (s % STAGES) * S::STAGE_FLOATS;
-                if (k0 < K) {
+                for (int u = 0; u < STAGES; ++u) {          // (the step's stage)
+                    const int s = s0 + u, k0 = k_of(first, s), ahead = s + STAGES - 1;
+                    cp_async_wait<STAGES - 2>();
+                    __syncwarp();
+                    load_w(k_of(first, ahead), u + STAGES - 1);
+                    load_a(k_of(first, ahead), u + STAGES - 1);
+                    cp_async_commit();
+                    const float *ws = mine + u * S::STAGE_FLOATS;
+                    if (k0 < K) {
 #pragma unroll
-                    for (int run = 0; run < 2; ++run) {
-                        const float *at = ws + (run ? frag_other : frag);
-                        float4 w[1][2], a[NT];
-                        w[0][0] = *reinterpret_cast<const float4 *>(at);
-                        w[0][1] = *reinterpret_cast<const float4 *>(at + 8 * 32);
+                        for (int run = 0; run < 2; ++run) {
+                            const float *at = ws + (run ? frag_other : frag);
+                            float4 w[1][2], a[NT];
+                            w[0][0] = *reinterpret_cast<const float4 *>(at);
+                            w[0][1] = *reinterpret_cast<const float4 *>(at + 8 * 32);
 #pragma unroll
-                        for (int j = 0; j < NT; ++j) a[j] = *reinterpret_cast<const float4 *>(at + (16 + j * 8) * 32);
-                        add_run<1, NT>(sum, w, a);
+                            for (int j = 0; j < NT; ++j) a[j] = *reinterpret_cast<const float4 *>(at + (16 + j * 8) * 32);
+                            add_run<1, NT>(sum, w, a);
+                        }
                     }
+                    __syncwarp();
                 }
-                __syncwarp();
             }
 #pragma unroll
             for (int j = 0; j < NT; ++j)
@@ -466,8 +477,9 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_f32_few_kernel(const float *_
     }
 }
 
-// Many rows: tiles of 64 features by 64 rows, 32 x 32 a warp.  The tensor pipe bounds it (m16n8k8: 278 TFLOP/s by itself, three a
-// product).  A segment's sum and the sum of segments stay in registers.
+// Many rows: tiles of 64 features by 64 rows, 32 x 32 a warp.  The tensor pipe and the schedulers bound it: a product of m16n8k16 holds its
+// scheduler for nearly nine cycles (560 TFLOP/s by itself, eight a product: 596 of the 861 us of 812 x 11,264 x 2,048), the parts and sums take
+// the rest.  A segment's sum and the sum of segments stay in registers.
 constexpr int MANY_STAGES = 4, MANY_STAGE_FLOATS = 128 * 32;
 constexpr size_t MANY_SMEM = sizeof(float) * MANY_STAGES * MANY_STAGE_FLOATS;
 
@@ -636,7 +648,7 @@ template <bool VEC, typename TO> int launch_many(const Call &c) {
     return lgml_launch_status("gemm_f32");
 }
 // Time of a product on blocks of 16 features by 32 rows, and on tiles of 64 by 64, in microseconds at K = 2048: a round of blocks
-// takes 9; an SM's first tile takes 58 (one warp a scheduler), every further one 37.
+// takes 12.5; an SM's first tile takes 70 (one warp a scheduler), every further one 53.
 template <bool VEC, typename TO> int run_split(const Call &c) {
     // Where there is one block an SM it has sixteen warps, else two blocks share the SM (4 rows, N x K, sixteen warps and eight:
     // 2048 x 5632 10.2 and 13.2, 2048 x 2048 5.6 and 5.9, 3072 x 2048 9.6 and 7.3, 11264 x 2048 24.6 and 21.2).
@@ -645,7 +657,7 @@ template <bool VEC, typename TO> int run_split(const Call &c) {
     if (c.M <= 16) return one ? launch_few<2, 2, 16, VEC, TO>(c) : launch_few<2, 2, 8, VEC, TO>(c);
     const long long blocks = (long long)((c.M + 31) / 32) * ((c.N + 15) / 16), tiles = (long long)((c.M + 63) / 64) * ((c.N + 63) / 64);
     // (the blocks' rows are the grid's second dimension: no more than 65,535 of them)
-    if ((blocks + 147) / 148 * 9 <= 58 + ((tiles + 147) / 148 - 1) * 37 && c.M <= 65535 * 32) return launch_few<4, 2, 8, VEC, TO>(c);
+    if ((blocks + 147) / 148 * 12.5f <= 70 + ((tiles + 147) / 148 - 1) * 53 && c.M <= 65535 * 32) return launch_few<4, 2, 8, VEC, TO>(c);
     return launch_many<VEC, TO>(c);
 }
 

@@ -14,7 +14,7 @@
 #include <math.h>
 
 #include "common.cuh"
-#include "tf32_halves.cuh"
+#include "bf16_thirds.cuh"
 
 LGML_DEFINE_LAST_ERROR(lgml_ssd)
 
@@ -212,10 +212,12 @@ __global__ void __launch_bounds__(256) ssd_chain_kernel(float *__restrict__ scra
 //   y_i          e^(G_i) S0 C_i + sum_(j <= i) e^(G_i - G_j) dt_j (C_i . B_j) x_j + D x_i
 //
 // The first kernel gives what every chunk leaves from a zero state, ssd_chain_kernel the state each starts from, the second kernel y: the
-// chunks side by side.  The products go through the tensor cores in halves (tf32_halves.cuh).  Bound by what a block waits for between its
-// few products (two blocks an SM); 32 heads of 64 columns by 128 entries, scans of every chunk from zero and from its start, and now: 129 tokens
-// 86 and 27 us, 1,012 tokens in two requests 208 and 65, 2,048 tokens 306 and 105.  Off 64 bits 2.0e-7 and 1.6e-7 (y, 1,012 tokens), with
-// decays of a few per cent a chunk 1.9e-6 and 1.8e-7.
+// chunks side by side.  The products go through the tensor cores with both operands in three parts that hold all their bits
+// (bf16_thirds.cuh).  Bound by what a block waits for between its few products (two blocks an SM); 32 heads of 64 columns by 128 entries, scans of
+// every chunk from zero and from its start, and now: 1,012 tokens in two requests 208 and 73 us, 2,048 tokens 306 and 123 (62 and 102 with
+// two tf32 halves, which held 23 bits).  Off 64 bits, y and state, 1,012 tokens: 3.5e-7 and 3.8e-7 the scans, 1.3e-7 and 1.1e-7 here; with decays
+// of a few per cent a chunk 3.9e-6 and 5.1e-6, 1.5e-7 and 1.3e-7; of one sign 3.3e-7 and 4.2e-7, 7e-8 and 5e-8; one term in 16 3.7e-7 and
+// 6.3e-7, 8e-8 and 1.2e-7.  Numbers below 2^-110 lose what of their parts is below 2^-133.
 constexpr int CHUNK = 64, CHUNK_THREADS = 256;
 constexpr int CHUNK_N = 128, CHUNK_P = 64;                  // most state entries a column; columns of a block
 constexpr int LD_T = 8;                                     // rows that are walked along k: row lengths of 8 over a multiple of 32 put k = 0 .. 3 of
@@ -264,7 +266,7 @@ __device__ __forceinline__ void chunk_decays(const ChunkArgs &p, int h, int t0, 
     Gs[2 * lane] = sum - l[1], Gs[2 * lane + 1] = sum;
 }
 
-// A result that is no finite number, formed again by itself: what an infinity loses between its halves, or where a later token's
+// A result that is no finite number, formed again by itself: what an infinity loses between its parts, or where a later token's
 // meets the zero of an earlier row.
 __device__ __noinline__ float left_again(const float *b, const float *x, const float *f, int nt) {
     float v = 0.f;
@@ -353,7 +355,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS) ssd_chunk_left_kernel(const Chu
 constexpr size_t CHUNK_OUT_SMEM = sizeof(float) * (2 * CHUNK * LD_C + CHUNK * LD_X + CHUNK * LD_M);
 constexpr size_t CHUNK_LEFT_SMEM = sizeof(float) * CHUNK * (LD_B + LD_X);
 
-__global__ void __launch_bounds__(CHUNK_THREADS) ssd_chunk_out_kernel(const ChunkArgs p, int heads) {
+__global__ void __launch_bounds__(CHUNK_THREADS, 2) ssd_chunk_out_kernel(const ChunkArgs p, int heads) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float sm[];

@@ -1,8 +1,8 @@
 """The runtime a model runs on: device, compute type, and the choice of kernel per operation.
 
 Two modes.  ``float32``: every tensor and every sum is 32-bit, matrix products in an
-order fixed by their length alone (chains of FMAs, or on the tensor cores with both operands in two
-halves that keep their 24 bits: closer to 64 bits than the chain), attention by the 32-bit kernels (the general one for head sizes
+order fixed by their length alone (chains of FMAs, or on the tensor cores with both operands in three bfloat16 parts that
+hold all their 24 bits; as close to 64 bits as the chain or closer), attention by the 32-bit kernels (the general one for head sizes
 they do not take); nothing uses a reduced-precision matrix mode.  ``bfloat16``: weights, activations between
 kernels and the cache are bfloat16; the residual stream, norms, softmax, rotation
 angles and logits stay float32.

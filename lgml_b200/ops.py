@@ -392,7 +392,7 @@ def fill_normal(out: torch.Tensor, mean: float, sd: float, seed: int) -> torch.T
 # ----------------------------------------------------------------------------------------
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """out[M,N] = a[M,K] . w[N,K]^T (+ bias), true float32 with a fixed summation order."""
+    """out[M,N] = a[M,K] . w[N,K]^T (+ bias): float32 operands in all their bits, float32 sums in an order that depends on K alone."""
     _need(a, "gemm input", torch.float32, 2)
     _need(w, "gemm weight", torch.float32, 2)
     _need(out, "gemm output", ndim=2)
@@ -1816,7 +1816,7 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_l
     Every piece is scanned from zero (what it leaves and the product of its decays are kept), a chain over each
     request's pieces turns that into the state every piece starts from (and the slot's new state), and every
     piece is scanned again from there, which gives y.  ``piece_tokens``: no piece is longer than this (0: not said); pieces of up to
-    64 tokens are matrix products instead of scans where the sizes allow."""
+    64 tokens are matrix products (float32 operands in all their bits) instead of scans where the sizes allow."""
     _need(xbc, "convolved x, B and C", torch.float32, 2)
     _need(dt_raw, "step sizes", torch.float32, 2)
     ldx, ldd = _rows_contiguous(xbc, "convolved x, B and C"), _rows_contiguous(dt_raw, "step sizes")

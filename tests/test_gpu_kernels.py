@@ -302,12 +302,12 @@ def test_gemm_f32_same_bits_from_every_kernel(M, N, K, pad):
     (1, 33, 8196, 4, 1.0), (12, 50, 8200, 0, 1.0),
     # 8, 16, 32 and 64 rows and one over; tiles of 64 x 64 with one row and one column too many
     (17, 2400, 200, 0, 1.0), (33, 100, 96, 0, 1.0), (300, 5000, 80, 0, 1.0), (65, 9500, 132, 0, 1.0), (513, 2049, 161, 0, 1.0),
-    # halves below the smallest normal number (tf32 keeps multiples of 2^-136 there), operands of very different size
+    # parts below the smallest normal number (bfloat16 keeps multiples of 2^-133 there), operands of very different size
     (5, 64, 64, 0, 2e-33), (70, 6000, 72, 0, 2e-33), (5, 64, 64, 0, 1e30),
 ])
 def test_gemm_f32_in_halves(M, N, K, pad, scale):
-    """Both operands in two tf32 halves: what the halves lose is 3 2^-24 of a product, a run of 16 k cuts six sums (12 2^-24), and
-    the sums of runs and segments round K / 128 + 8 times; a row has the same bits alone and among others."""
+    """Both operands in three bfloat16 parts: they lose nothing that counts, a run of 16 k cuts two sums (of up to 16 numbers, 2 2^-24 each
+    of a number), and the sums of runs and segments round twice in K / 128 + 16; a row has the same bits alone and among others."""
     from lgml_b200 import ops
 
     torch.manual_seed(M + N + K)
@@ -321,6 +321,32 @@ def test_gemm_f32_in_halves(M, N, K, pad, scale):
         one = torch.empty(1, N, device=DEV)
         ops.gemm_f32(a[m:m + 1], w, one)
         assert torch.equal(one[0], out[m])
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 33, 64), (7, 2400, 201), (16, 40, 4100), (40, 64, 128), (300, 5000, 80), (200, 3000, 257)])
+def test_gemm_f32_of_few_terms(M, N, K):
+    """All 24 bits of both operands count, as in an FMA: rows that select a column give it exactly, products that stand alone are
+    rounded once (half a last place is 2^-24; what is left out, and the small products' own sum, are under 2^-30), and rows of a few terms are off by no more than
+    a float32 sum of them may be: two roundings a term."""
+    from lgml_b200 import ops
+
+    g = torch.Generator().manual_seed(M + N + K)
+    w, at, x = torch.randn(N, K, generator=g), torch.randint(0, K, (M,), generator=g), torch.randn(M, generator=g)
+    w[0], x[0] = 1.0 + 2.0 ** -11, 1.0 + 2.0 ** -11          # (whose square is 2^-22 more than 1 + 2^-10)
+    dev, out = w.to(DEV), torch.empty(M, N, device=DEV)
+    a = torch.zeros(M, K)
+    a[torch.arange(M), at] = 1.0
+    ops.gemm_f32(a.to(DEV), dev, out)
+    assert torch.equal(out.cpu(), w[:, at].t())
+    a[torch.arange(M), at] = x
+    ops.gemm_f32(a.to(DEV), dev, out)
+    want = a.double() @ w.double().t()
+    assert bool(((out.cpu().double() - want).abs() <= (2.0 ** -24 + 2.0 ** -29) * want.abs()).all())
+    a = torch.randn(M, K, generator=g)
+    keep = torch.rand(M, K, generator=g).argsort(dim=1) < 4
+    a = torch.where(keep, a, torch.zeros(()))
+    ops.gemm_f32(a.to(DEV), dev, out)
+    assert bool(((out.cpu().double() - a.double() @ w.double().t()).abs() <= 8 * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t())).all())
 
 
 @pytest.mark.parametrize("M,N", [(65535 * 32, 8), (65535 * 32 + 1, 8), (65535 * 32 + 1, 17)])
@@ -340,7 +366,7 @@ def test_gemm_f32_of_millions_of_rows(M, N):
 
 @pytest.mark.parametrize("M", [1, 20, 200])
 def test_gemm_f32_of_infinite_and_huge_values(M):
-    """What a chain of FMAs gives: an infinity times an exact number is infinite, not lost between the halves; a sum that overflows is infinite
+    """What a chain of FMAs gives: an infinity times an exact number is infinite, not lost between the parts; a sum that overflows is infinite
     and its neighbours are what they are without it; results below the normal numbers are exact to their last bit."""
     from lgml_b200 import ops
 
