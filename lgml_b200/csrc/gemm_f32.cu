@@ -319,17 +319,44 @@ __global__ void __launch_bounds__(256) gemm_f32_ragged_kernel(const float *__res
 // under 2^-110 has fewer than 24 bits; that shows in larger results beside operands over 2^14 only).
 constexpr int SEGMENT = 128, SPLIT_FROM = 64;
 
-__device__ __noinline__ float chain(const float *a, const float *w, int K) {
-    float v = 0.f;
-    for (int k = 0; k < K; ++k) v = fmaf(act_load(a + k), w[k], v);
-    return v;
+__device__ __forceinline__ bool by_chain(float v) { return !(fabsf(v) <= 3.402823466e38f) || (fabsf(v) < 0x1p-96f && v != 0.f); }
+
+// The chains of a block that has such a result, of all its outputs side by side: FEATURES rows of W and ROWS of A come through shared memory STEP
+// elements at a time, and add(w, a) has every thread's FMAs of one k (row r's at w[r (STEP + 1)]).  One thread's chain after another, from memory,
+// took up to 40 times as long as a product without (812 x 11,264 x 2,048 with a NaN in every row: 26,000 us, 2,500 here, 860 without one; 4 rows 320,
+// 155 and 40).
+template <int FEATURES, int ROWS, int THREADS, int STEP, typename Add>
+__device__ __forceinline__ void chain_tile(const float *A, const float *W, int m0, int n0, int M, int N, int K, int lda, int ldw, float *ws, Add &&add) {
+    constexpr int LD = STEP + 1, EACH = (FEATURES + ROWS) * STEP / THREADS, NOW = EACH % 8 ? 6 : 8;
+    static_assert((FEATURES + ROWS) * STEP % THREADS == 0 && EACH % NOW == 0, "whole rounds of loads");
+    cp_async_wait<0>();
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += STEP) {
+        const int n = min(STEP, K - k0);
+        __syncthreads();
+#pragma unroll 1
+        for (int i0 = 0; i0 < EACH; i0 += NOW) {
+            float v[NOW];
+#pragma unroll
+            for (int i = 0; i < NOW; ++i) {
+                const int at = (i0 + i) * THREADS + threadIdx.x, r = at / STEP, k = min(at % STEP, n - 1);
+                v[i] = act_load(r < FEATURES ? W + (size_t)min(n0 + r, N - 1) * ldw + k0 + k : A + (size_t)min(m0 + r - FEATURES, M - 1) * lda + k0 + k);
+            }
+#pragma unroll
+            for (int i = 0; i < NOW; ++i) {
+                const int at = (i0 + i) * THREADS + threadIdx.x;
+                ws[at / STEP * LD + at % STEP] = v[i];
+            }
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int i = 0; i < n; ++i) add(ws + i, ws + FEATURES * LD + i);
+    }
 }
+
 template <typename TO>
-__device__ __forceinline__ void store_split(float v, const float *A, const float *W, const float *bias, TO *C, int m, int n, int M, int N, int K, int lda,
-                                            int ldw, int ldc) {
-    if (m >= M || n >= N) return;
-    if (!(fabsf(v) <= 3.402823466e38f) || (fabsf(v) < 0x1p-96f && v != 0.f)) v = chain(A + (size_t)m * lda, W + (size_t)n * ldw, K);
-    C[(size_t)m * ldc + n] = from_f32<TO>(bias ? v + bias[n] : v);
+__device__ __forceinline__ void store_split(float v, const float *bias, TO *C, int m, int n, int M, int N, int ldc) {
+    if (m < M && n < N) C[(size_t)m * ldc + n] = from_f32<TO>(bias ? v + bias[n] : v);
 }
 
 // 16 bytes of a row's elements k .. k + 3 into shared memory, zeros for those past K.  Rows that do not start on 16 bytes come
@@ -470,11 +497,28 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_f32_few_kernel(const float *_
         if (first + SEGS < n_seg) __syncthreads();
     }
     pdl_trigger();      // at the end: blocks of the kernels behind that start earlier are placed where there is room, not where there is time
+    // an output of a thread: its feature and its row in the block
+    auto feature = [&](int o) { return ((o * WARPS * 32 + (int)threadIdx.x) & 31) / 4 + (((o * WARPS * 32 + (int)threadIdx.x) >> 6) & 1) * 8; };
+    auto row = [&](int o) { return (o * WARPS * 32 + (int)threadIdx.x) / 128 * 8 + (threadIdx.x & 3) * 2 + (((o * WARPS * 32 + (int)threadIdx.x) >> 5) & 1); };
+    auto there = [&](int o) { return o * WARPS * 32 + (int)threadIdx.x < S::OUTS && m0 + row(o) < M && n0 + feature(o) < N; };
+    bool again = false;
 #pragma unroll
-    for (int o = 0; o < OUTS; ++o) {
-        const int at = o * WARPS * 32 + threadIdx.x, l = at & 31, e = (at >> 5) & 3, j = at >> 7;
-        if (at < S::OUTS) store_split(total[o], A, W, bias, C, m0 + j * 8 + (l & 3) * 2 + (e & 1), n0 + (l >> 2) + (e >> 1) * 8, M, N, K, lda, ldw, ldc);
+    for (int o = 0; o < OUTS; ++o) again |= there(o) && by_chain(total[o]);
+    if (__syncthreads_or(again)) {
+        float v[OUTS] = {};
+        constexpr int STEP = 128, LD = STEP + 1;
+        chain_tile<16, 8 * NT, WARPS * 32, STEP>(A, W, m0, n0, M, N, K, lda, ldw, smem_f, [&](const float *w, const float *a) {
+#pragma unroll
+            for (int o = 0; o < OUTS; ++o)
+                if (there(o)) v[o] = fmaf(a[row(o) * LD], w[feature(o) * LD], v[o]);
+        });
+#pragma unroll
+        for (int o = 0; o < OUTS; ++o)
+            if (by_chain(total[o])) total[o] = v[o];
     }
+#pragma unroll
+    for (int o = 0; o < OUTS; ++o)
+        if (there(o)) store_split(total[o], bias, C, m0 + row(o), n0 + feature(o), M, N, ldc);
 }
 
 // Many rows: tiles of 64 features by 64 rows, 32 x 32 a warp.  The tensor pipe and the schedulers bound it: a product of m16n8k16 holds its
@@ -556,13 +600,40 @@ __global__ void __launch_bounds__(128, 3) gemm_f32_many_kernel(const float *__re
         }
     }
     pdl_trigger();      // at the end: the blocks of a product fill their SMs
+    const int row = r0 + q * 2, feature = f0 + g;               // of output (i, j, e): row + 8 j + e % 2, feature + 16 i + 8 (e / 2)
+    bool again = false;
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                store_split(total[i][j][e], A, W, bias, C, m0 + r0 + j * 8 + q * 2 + (e & 1), n0 + f0 + i * 16 + g + (e >> 1) * 8, M, N, K, lda, ldw, ldc);
+            for (int e = 0; e < 4; ++e) again |= m0 + row + 8 * j + (e & 1) < M && n0 + feature + 16 * i + 8 * (e >> 1) < N && by_chain(total[i][j][e]);
+    if (__syncthreads_or(again)) {
+        float v[2][4][4] = {};
+        constexpr int STEP = 64, LD = STEP + 1;
+        chain_tile<64, 64, 128, STEP>(A, W, m0, n0, M, N, K, lda, ldw, smem_f, [&](const float *w, const float *a) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        v[i][j][e] = fmaf(a[(row + 8 * j + (e & 1)) * LD], w[(feature + 16 * i + 8 * (e >> 1)) * LD], v[i][j][e]);
+        });
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (by_chain(total[i][j][e])) total[i][j][e] = v[i][j][e];
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) store_split(total[i][j][e], bias, C, m0 + row + 8 * j + (e & 1), n0 + feature + 16 * i + 8 * (e >> 1), M, N, ldc);
 }
 
 // ---- host side -----------------------------------------------------------------------------------

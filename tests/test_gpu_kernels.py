@@ -389,6 +389,48 @@ def test_gemm_f32_of_infinite_and_huge_values(M):
         assert torch.equal(out[1:, 20], want[1:, 20])
 
 
+@pytest.mark.parametrize("M,N,K,pad", [(3, 40, 65, 0), (9, 2400, 96, 0), (20, 130, 4128, 1), (40, 3000, 161, 3), (200, 3000, 100, 0), (300, 5001, 65, 0)])
+def test_gemm_f32_chains_beside_ordinary_results(M, N, K, pad):
+    """Blocks with results that are formed again as chains of FMAs (a row of NaN, one with an infinity, one of numbers whose results are below
+    2^-96): those to the last place of what float32 keeps of them (2^-149), the others with the bits that they have without such rows."""
+    from lgml_b200 import ops
+
+    g = torch.Generator().manual_seed(M + K)
+    a, w = torch.randn(M, K + pad, generator=g)[:, :K], torch.randn(N, K + pad, generator=g)
+    plain, out, w = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV), w.to(DEV)[:, :K]
+    ops.gemm_f32(a.contiguous().to(DEV), w, plain)
+    odd = a.clone()
+    odd[0, K - 1], odd[M // 2, 7], odd[M - 1] = float("nan"), float("inf"), odd[M - 1] * 2.0 ** -112
+    ops.gemm_f32(odd.contiguous().to(DEV), w, out)
+    assert bool(torch.isnan(out[0]).all()) and torch.equal(out[M // 2], w[:, 7].sign() * float("inf"))
+    want, size = odd[M - 1].double().to(DEV) @ w.double().t(), odd[M - 1].double().abs().to(DEV) @ w.double().abs().t()
+    assert bool(((out[M - 1].double() - want).abs() <= K * (2.0 ** -24 * size + 2.0 ** -149)).all())
+    rest = [m for m in range(M) if m not in (0, M // 2, M - 1)]
+    assert torch.equal(out[rest], plain[rest])
+
+
+@pytest.mark.parametrize("M,N,K", [(4, 11264, 2048), (32, 2048, 5632), (300, 4096, 2048)])
+def test_gemm_f32_of_nan_takes_about_as_long(M, N, K):
+    """A NaN in every row of A: the chains that all results then are run side by side (one after another in a thread: 10 to 40 times as long as
+    without the NaN; side by side under five times)."""
+    from lgml_b200 import ops
+
+    a, w, out = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV), torch.empty(M, N, device=DEV)
+    times = []
+    for x in (a, a.index_fill(1, torch.tensor([5], device=DEV), float("nan"))):
+        best = float("inf")
+        for _ in range(6):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            for _ in range(4):
+                ops.gemm_f32(x, w, out)
+            end.record()
+            torch.cuda.synchronize()
+            best = min(best, start.elapsed_time(end))
+        times.append(best)
+    assert bool(torch.isnan(out).all()) and times[1] < 8 * times[0], times
+
+
 @pytest.mark.parametrize("M,N,K,bias,f32,splits", [
     (1, 128, 64, False, False, None), (8, 331 * 8, 120, True, True, None), (5, 200, 192, True, False, 3),
     (64, 1000, 1096, True, True, 4), (100, 320, 96, False, False, None), (129, 520, 264, True, False, None),
