@@ -272,7 +272,9 @@ extern void *PyEval_SaveThread(void);
 extern void PyEval_RestoreThread(void *state);
 extern void Py_IncRef(PyObject *o);
 extern void Py_DecRef(PyObject *o);
+extern PyObject *PyObject_Type(PyObject *o);
 extern char _Py_NoneStruct[];          /* None */
+extern char PyLong_Type[];             /* int */
 extern void *malloc(size_t n);
 
 enum { MOST_WORDS = 40, MOST_FLOATS = 8, FASTCALL = 0x80 };
@@ -287,6 +289,12 @@ typedef struct {
     char kinds[MOST_WORDS + MOST_FLOATS + 1];
 } Caller;
 
+static int is_int(PyObject *o) {
+    PyObject *type = PyObject_Type(o);
+    Py_DecRef(type);            /* (lives on: the object holds it) */
+    return type == (PyObject *)PyLong_Type;
+}
+
 static PyObject *call(PyObject *self, PyObject *const *args, intptr_t n) {
     const Caller *c = (const Caller *)PyLong_AsVoidPtr(self);
     W w[MOST_WORDS] = {0};
@@ -296,8 +304,15 @@ static PyObject *call(PyObject *self, PyObject *const *args, intptr_t n) {
     } x[MOST_FLOATS] = {{0.0}};
     int nw = 0, nx = 0, ok = n == c->n;
     for (int i = 0; ok && i < n; ++i) {
-        if (c->kinds[i] == 'w') {
-            w[nw] = args[i] == (PyObject *)_Py_NoneStruct ? 0 : PyLong_AsLongLong(args[i]);
+        if (c->kinds[i] == 'p') {
+            /* None, or an int itself: ctypes takes nothing else that could be turned into one */
+            if (args[i] == (PyObject *)_Py_NoneStruct) w[nw++] = 0;
+            else {
+                ok = is_int(args[i]);
+                if (ok) w[nw] = PyLong_AsLongLong(args[i]), ok = w[nw++] != -1 || !PyErr_Occurred();
+            }
+        } else if (c->kinds[i] == 'w') {
+            w[nw] = PyLong_AsLongLong(args[i]);
             ok = w[nw++] != -1 || !PyErr_Occurred();
         } else {
             const double v = PyFloat_AsDouble(args[i]);
@@ -326,16 +341,16 @@ static PyObject *call(PyObject *self, PyObject *const *args, intptr_t n) {
     return PyLong_FromLong(rc);
 }
 
-/* `kinds`: a letter an argument, w (integer or pointer), f (float) or d (double).  The function must return an int.  `other` is called instead with
+/* `kinds`: a letter an argument, w (integer), p (pointer), f (float) or d (double).  The function must return an int.  `other` is called instead with
  * arguments that are no numbers, or not as many.  A callable lasts as long as the process; NULL: not here, or too many arguments. */
 LGML_API int lgml_steps_caller_fits(const char *kinds) {
     int nw = 0, nx = 0;
-    for (const char *k = kinds; *k; ++k) *k == 'w' ? ++nw : ++nx;
+    for (const char *k = kinds; *k; ++k) *k == 'w' || *k == 'p' ? ++nw : ++nx;
     return nw <= MOST_WORDS && nx <= MOST_FLOATS;
 }
 LGML_API PyObject *lgml_steps_caller(void *fn, const char *kinds, PyObject *other) {
-    Caller *c = malloc(sizeof(*c));
-    if (!c || !lgml_steps_caller_fits(kinds)) {
+    Caller *c = lgml_steps_caller_fits(kinds) ? malloc(sizeof(*c)) : 0;
+    if (!c) {
         Py_IncRef((PyObject *)_Py_NoneStruct);
         return (PyObject *)_Py_NoneStruct;
     }

@@ -72,7 +72,7 @@ def steps() -> ctypes.PyDLL:
     return _steps
 
 
-_KINDS = {c_void_p: b"w", c_int: b"w", c_int64: b"w", c_uint64: b"w", c_float: b"f", c_double: b"d"}
+_KINDS = {c_void_p: b"p", c_int: b"w", c_int64: b"w", c_uint64: b"w", c_float: b"f", c_double: b"d"}
 
 
 def caller(fn):

@@ -4,7 +4,9 @@ import random
 import subprocess
 from ctypes import c_double, c_float, c_int, c_longlong, c_ulonglong, c_void_p
 
+import numpy as np
 import pytest
+import torch
 
 from lgml_b200 import csrc, host
 
@@ -60,6 +62,38 @@ def test_callers_pass_what_ctypes_passes(tmp_path):
         if sig:
             with pytest.raises(TypeError):                   # too few
                 fast(*args[:-1])
+
+
+class Index:
+    def __index__(self):
+        return 7
+
+
+class Float:
+    def __float__(self):
+        return 7.0
+
+
+@pytest.mark.parametrize("name,kind", [("f", c_int), ("g", c_longlong), ("u", c_ulonglong), ("h", c_float), ("d", c_double), ("p", c_void_p)])
+def test_callers_take_and_refuse_what_ctypes_does(tmp_path, name, kind):
+    """Every sort of value in the place of every kind: the same result, or the same error."""
+    (tmp_path / "f.c").write_text("int f(int a) { return a; } int g(long long a) { return (int)(a ^ a >> 32); } int u(unsigned long long a) { return (int)(a ^ a >> 32); }\n"
+                                  "int h(float a) { return (int)a; } int d(double a) { return (int)a; } int p(void *a) { return (int)(long)a; }\n")
+    subprocess.run([csrc.find_cc(), "-O2", "-shared", "-fPIC", str(tmp_path / "f.c"), "-o", str(tmp_path / "f.so")], check=True)
+    fn = getattr(ctypes.CDLL(str(tmp_path / "f.so")), name)
+    fn.argtypes, fn.restype = [kind], c_int
+    fast = host.caller(fn)
+    assert fast is not fn
+
+    def tried(call, value):
+        try:
+            return call(value)
+        except Exception as e:
+            return type(e)
+
+    for value in (None, 5, True, -1, 2 ** 31, 2 ** 32 + 5, 2 ** 63 - 1, 2 ** 63, 2 ** 64 - 1, -2 ** 63, 2.5, -1.0, "a", Index(), Float(), np.int64(5), np.int32(-1),
+                  np.float32(2.5), np.float64(2.5), np.bool_(True), torch.tensor(5), torch.tensor(2.5), c_int(5), c_void_p(5), c_float(1.5), object()):
+        assert tried(fast, value) == tried(fn, value), (name, value)
 
 
 def test_other_signatures_stay_with_ctypes():
