@@ -275,7 +275,8 @@ class ModelRunner:
         # which are one range, so that no kernel merges ranges (2 us a layer: three layers of 96, 70 and 65 us a step; contexts of up to four pages in
         # one range: 8B layers, one request of 100 to 200 tokens, 235 us a step against 228).
         # Heads with keys of their own are also cut by how even the contexts are (ops.decode_ranges): a graph for each of the two.
-        lengths = [r.n_tokens + 1 for r in reqs]
+        # (Without pages there is nothing to cut: one graph, whatever the lengths.)
+        lengths = [r.n_tokens + 1 for r in reqs] if self.cache.groups else [1]
         reach, even = context_reach(lengths) if max(lengths) > self.cache.page_size else (self.cache.page_size, False)
         key = (size, reach, even and self.rt.own_keys and self.rt.dtype == torch.bfloat16)
         if key not in self._graph_seen:

@@ -617,3 +617,27 @@ def test_command_line_generates_with_the_folders_architecture(model):
     for i, tok in enumerate(got):
         row = L.oracle_logits(cfg, weights, prompt + got[:i])[-1]
         assert float(row.max() - row[tok]) <= 1e-4
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_a_model_without_pages_has_one_captured_step_for_all_lengths(tmp_path, dtype):
+    """Layers of the delta rule alone: from the first token on past a page's 64 and a reach's 1,024, one graph, and the eager runner's logits."""
+    from lgml_b200.engine.engine import parse_dtype
+    from lgml_b200.engine.runner import ModelRunner
+
+    folder = L.write_folder(tmp_path / "m", L.ONLY_DELTA, L.random_weights(L.ONLY_DELTA, L.ONLY_DELTA_RANKS, 7))
+    ids, rows = H.random_ids(1100, 50, 3), {}
+    for use_graphs in (True, False):
+        runner = ModelRunner.from_folder(folder, parse_dtype(dtype), DEV, n_pages=4, max_slots=2, use_graphs=use_graphs)
+        req = runner.open("a", [])
+        rows[use_graphs], n = [], 0
+        while n < 1030:
+            portion = 1 if n < 70 or n > 1015 else min(200, 1016 - n)
+            logits = runner.step([(req, ids[n:n + portion], [portion - 1])])
+            n += portion
+            rows[use_graphs].append(logits[0].clone())
+        if use_graphs:
+            assert len(runner._graphs) == 1 and runner.graph_replays > 80
+        runner.close(req)
+    for a, b in zip(rows[True], rows[False]):
+        assert torch.equal(a, b)
