@@ -266,22 +266,49 @@ __device__ __forceinline__ void chunk_decays(const ChunkArgs &p, int h, int t0, 
     Gs[2 * lane] = sum - l[1], Gs[2 * lane + 1] = sum;
 }
 
-// A result that is no finite number, formed again by itself: what an infinity loses between its parts, or where a later token's
-// meets the zero of an earlier row.
-__device__ __noinline__ float left_again(const float *b, const float *x, const float *f, int nt) {
-    float v = 0.f;
-    for (int t = 0; t < nt; ++t) v = fmaf(b[t * LD_B], x[t * LD_X] * f[t], v);
-    return v;
-}
-__device__ __noinline__ float y_again(const float *c, const float *B, int ldx, const float *s0, const float *x, const double *G, const float *dts, int i, int N) {
-    float old = 0.f, now = 0.f;
-    for (int n = 0; n < N; ++n) old = fmaf(c[n], s0[n], old);
-    for (int t = 0; t <= i; ++t) {
-        float dot = 0.f;
-        for (int n = 0; n < N; ++n) dot = fmaf(c[n], act_load(B + (size_t)t * ldx + n), dot);
-        now = fmaf(dot * (expf((float)(G[i] - G[t])) * dts[t]), x[t * LD_X], now);
+// A block with a result that is no finite number goes through its chunk again token by token, as the scan above does, and such results
+// come from there: an infinity is lost between the parts of a product, or meets the zero of an earlier row.  A thread owns up to 32 entries of a column.
+// OUT: y, from the state S0 (else what is left, from zero).
+template <bool OUT>
+__device__ __noinline__ void scan_again(const ChunkArgs &p, int c, int h, int col0, int cols, int t0, int nt, const float *Xs, const float *dts, const float *Bs,
+                                        const float *Cs, const float *S0) {
+    const int col = threadIdx.x >> 2, part = threadIdx.x & 3;
+    const float a = expf(__ldg(p.a_log + h)), skip = OUT ? __ldg(p.d_skip + h) : 0.f;
+    const float *B = p.xbc + (size_t)t0 * p.ldx + p.Hs * p.P + (h / (p.Hs / p.G)) * p.N;
+    float S[CHUNK_N / 4];
+#pragma unroll
+    for (int i = 0; i < CHUNK_N / 4; ++i) S[i] = OUT ? S0[col * LD_C + (i >> 2) * 16 + part * 4 + (i & 3)] : 0.f;
+#pragma unroll 1
+    for (int t = 0; t < nt; ++t) {
+        const float x = Xs[t * LD_X + col], dA = expf(-a * dts[t]), dx = dts[t] * x;
+        float acc = 0.f;
+#pragma unroll
+        for (int i = 0; i < CHUNK_N / 16; ++i) {
+            const int n = i * 16 + part * 4;
+            if (n >= p.N) continue;
+            const float4 b = OUT ? act_load(reinterpret_cast<const float4 *>(B + (size_t)t * p.ldx + n)) : *reinterpret_cast<const float4 *>(Bs + t * LD_B + n);
+            S[4 * i] = fmaf(dA, S[4 * i], dx * b.x), S[4 * i + 1] = fmaf(dA, S[4 * i + 1], dx * b.y);
+            S[4 * i + 2] = fmaf(dA, S[4 * i + 2], dx * b.z), S[4 * i + 3] = fmaf(dA, S[4 * i + 3], dx * b.w);
+            if (OUT) {
+                const float4 v = *reinterpret_cast<const float4 *>(Cs + t * LD_C + n);
+                acc = fmaf(S[4 * i], v.x, acc), acc = fmaf(S[4 * i + 1], v.y, acc), acc = fmaf(S[4 * i + 2], v.z, acc), acc = fmaf(S[4 * i + 3], v.w, acc);
+            }
+        }
+        if (OUT) {
+            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+            acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+            float *y = p.y + (size_t)(t0 + t) * p.ldy + (size_t)h * p.P + col0 + col;
+            if (part == 0 && col < cols && !isfinite(act_load(y))) *y = fmaf(skip, x, acc);
+        }
     }
-    return fmaf(expf((float)G[i]), old, now);
+    if (!OUT && col < cols) {
+        float *left = p.left + ((size_t)c * p.Hs + h) * p.P * p.N + (size_t)(col0 + col) * p.N;
+#pragma unroll
+        for (int i = 0; i < CHUNK_N / 4; ++i) {
+            const int n = (i >> 2) * 16 + part * 4 + (i & 3);
+            if (n < p.N && !isfinite(act_load(left + n))) left[n] = S[i];
+        }
+    }
 }
 
 // Block: (chunk, head, 64 columns).  A warp has 32 state entries of 32 columns.
@@ -315,39 +342,41 @@ __global__ void __launch_bounds__(CHUNK_THREADS) ssd_chunk_left_kernel(const Chu
     copies_there();
     __syncthreads();
     const int n0 = (warp & 3) * 32, x0 = (warp >> 2) * 32;
-    if (n0 >= p.N || x0 >= cols) return;
-    float sum[2][4][4] = {};
+    bool again = false;
+    if (n0 < p.N && x0 < cols) {
+        float sum[2][4][4] = {};
 #pragma unroll 1
-    for (int k0 = 0; k0 < nt; k0 += 16) {
-        float w[2][2][4], a[4][4];
+        for (int k0 = 0; k0 < nt; k0 += 16) {
+            float w[2][2][4], a[4][4];
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const float *bk = Bs + (k0 + 4 * s + q) * LD_B + n0 + g, *xk = Xs + (k0 + 4 * s + q) * LD_X + x0 + g, f = fs[k0 + 4 * s + q];
+            for (int s = 0; s < 4; ++s) {
+                const float *bk = Bs + (k0 + 4 * s + q) * LD_B + n0 + g, *xk = Xs + (k0 + 4 * s + q) * LD_X + x0 + g, f = fs[k0 + 4 * s + q];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) w[i >> 1][i & 1][s] = bk[8 * i], a[i][s] = xk[8 * i] * f;
-        }
-        float4 wv[2][2], av[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            wv[i >> 1][i & 1] = make_float4(w[i >> 1][i & 1][0], w[i >> 1][i & 1][1], w[i >> 1][i & 1][2], w[i >> 1][i & 1][3]);
-            av[i] = make_float4(a[i][0], a[i][1], a[i][2], a[i][3]);
-        }
-        add_run<2, 4>(sum, wv, av);
-    }
-    float *out = p.left + ((size_t)c * p.Hs + h) * p.P * p.N + (size_t)col0 * p.N;
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int n = n0 + i * 16 + (e >> 1) * 8 + g, x = x0 + j * 8 + q * 2 + (e & 1);
-                if (n < p.N && x < cols) {
-                    float v = sum[i][j][e];
-                    if (!isfinite(v)) v = left_again(Bs + n, Xs + x, fs, nt);
-                    out[(size_t)x * p.N + n] = v;
-                }
+                for (int i = 0; i < 4; ++i) w[i >> 1][i & 1][s] = bk[8 * i], a[i][s] = xk[8 * i] * f;
             }
+            float4 wv[2][2], av[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                wv[i >> 1][i & 1] = make_float4(w[i >> 1][i & 1][0], w[i >> 1][i & 1][1], w[i >> 1][i & 1][2], w[i >> 1][i & 1][3]);
+                av[i] = make_float4(a[i][0], a[i][1], a[i][2], a[i][3]);
+            }
+            add_run<2, 4>(sum, wv, av);
+        }
+        float *out = p.left + ((size_t)c * p.Hs + h) * p.P * p.N + (size_t)col0 * p.N;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int n = n0 + i * 16 + (e >> 1) * 8 + g, x = x0 + j * 8 + q * 2 + (e & 1);
+                    if (n < p.N && x < cols) {
+                        out[(size_t)x * p.N + n] = sum[i][j][e];
+                        again |= !isfinite(sum[i][j][e]);
+                    }
+                }
+    }
+    if (__syncthreads_or(again)) scan_again<false>(p, c, h, col0, cols, t0, nt, Xs, dts, Bs, nullptr, nullptr);
 }
 
 // Block: (chunk, `heads` heads of a group, 64 columns).  A warp has 16 tokens (four runs of them) and half of the columns; C B^T, the same for all
@@ -410,6 +439,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) ssd_chunk_out_kernel(const C
             }
         copies_there();
         __syncthreads();
+        bool again = false;
         if (x0 < cols && i0 < nt) {
             float old[1][4][4] = {}, now[1][4][4] = {};
             for (int k = 0; k < kn; k += 16) {
@@ -447,13 +477,14 @@ __global__ void __launch_bounds__(CHUNK_THREADS, 2) ssd_chunk_out_kernel(const C
                         if (x >= cols) continue;
                         const float2 xv = *reinterpret_cast<const float2 *>(Xs + i * LD_X + x);
                         float2 v = make_float2(fmaf(kept, old[0][j][2 * r], now[0][j][2 * r]), fmaf(kept, old[0][j][2 * r + 1], now[0][j][2 * r + 1]));
-                        if (!isfinite(v.x)) v.x = y_again(Cs + i * LD_C, B, p.ldx, BS + x * LD_C, Xs + x, Gs, dts, i, p.N);
-                        if (!isfinite(v.y)) v.y = y_again(Cs + i * LD_C, B, p.ldx, BS + (x + 1) * LD_C, Xs + x + 1, Gs, dts, i, p.N);
-                        *reinterpret_cast<float2 *>(p.y + (size_t)(t0 + i) * p.ldy + (size_t)h * p.P + col0 + x) = make_float2(fmaf(skip, xv.x, v.x), fmaf(skip, xv.y, v.y));
+                        v = make_float2(fmaf(skip, xv.x, v.x), fmaf(skip, xv.y, v.y));
+                        again |= !isfinite(v.x) || !isfinite(v.y);
+                        *reinterpret_cast<float2 *>(p.y + (size_t)(t0 + i) * p.ldy + (size_t)h * p.P + col0 + x) = v;
                     }
                 }
             }
         }
+        if (__syncthreads_or(again)) scan_again<true>(p, c, h, col0, cols, t0, nt, Xs, dts, nullptr, Cs, BS);
     }
 }
 

@@ -285,6 +285,70 @@ def test_state_space_scan_in_chunks(Hs, G, Pd, N, lens):
     assert float((y - want)[there].abs().max()) < 1e-5 * (1 + float(want[there].abs().max()))
 
 
+@pytest.mark.parametrize("Hs,G,Pd,N,lens", [(3, 1, 4, 4, (64, 70)), (4, 2, 36, 20, (130, 65)), (2, 1, 68, 128, (200, 129))])
+def test_state_space_chunks_with_infinities(Hs, G, Pd, N, lens):
+    """Infinite x, B, C, steps and states: what is infinite, of which sign, and what is no number, as the scan of the same pieces has it; the rest as
+    close to it as without them.  Rates from 0.05 to 5, so that some heads forget within a chunk (an infinity stays for ever)."""
+    from lgml_b200 import ops
+
+    rng = np.random.default_rng(Pd + N)
+    inner, n, C = Hs * Pd, sum(lens), Hs * Pd + 2 * G * N
+    x, dt = f32(rng.normal(size=(n, C + 4))), f32(rng.normal(size=(n, Hs)) * 0.5)
+    vecs = [f32(rng.normal(size=Hs) * 0.3 + 0.5), f32(np.linspace(-3.0, 1.6, Hs)), f32(rng.normal(size=Hs))]
+    rows, first = [], [0]
+    for r, length in enumerate(lens):
+        rows += [(sum(lens[:r]) + t, sum(lens[:r]) + min(t + 64, length)) for t in range(0, length, 64)]
+        first.append(len(rows))
+    pieces, starts = (torch.tensor(rows, dtype=torch.int32, device=DEV), i32(first)), i32([0, lens[0], n])
+    state0 = torch.randn(4, inner * N, device=DEV)
+    inf = float("inf")
+    for case in ("x", "B", "C", "dt", "state"):
+        xi, di, si = x.clone(), dt.clone(), state0.clone()
+        if case == "x":
+            xi[3, 1], xi[40, Pd - 1] = -inf, inf
+        elif case == "B":
+            xi[20, inner + N - 1] = inf
+        elif case == "C":
+            xi[lens[0] + 5, inner + G * N] = -inf
+        elif case == "dt":
+            di[10, Hs - 1] = inf
+        else:
+            si[3, 1] = inf
+        got, want = [], []
+        for out, how in ((got, dict(piece_tokens=64)), (want, {})):
+            state = si.clone()
+            out += [ops.ssd_scan(xi[:, :C], di, vecs[0], vecs[1], vecs[2], state, starts, i32([3, 1]), Hs, G, Pd, N, pieces=pieces, **how), state]
+        for a, b in zip(got, want):
+            assert not bool(torch.isfinite(b).all()) or case == "C"
+            assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a[torch.isinf(b)], b[torch.isinf(b)]), case
+            there = torch.isfinite(b)
+            assert float((a - b)[there].abs().max()) < 1e-5 * (1 + float(b[there].abs().max())), case
+
+
+def test_state_space_chunks_with_nan_take_about_as_long():
+    """A NaN in the first token makes every result of every chunk one: some three times as long as without (each formed by itself: 20 times)."""
+    from lgml_b200 import ops
+
+    Hs, Pd, N, n = 32, 64, 128, 1024
+    rng = np.random.default_rng(1)
+    x, dt, vecs = f32(rng.normal(size=(n, Hs * Pd + 2 * N))), f32(rng.normal(size=(n, Hs))), [f32(rng.normal(size=Hs) * 0.3 + m) for m in (-2.5, -2.0, 1.0)]
+    pieces = torch.tensor([(t, t + 64) for t in range(0, n, 64)], dtype=torch.int32, device=DEV), i32([0, n // 64])
+    bad, times = x.clone(), []
+    bad[0] = float("nan")
+    for xs in (x, bad):
+        state, best = torch.zeros(1, Hs * Pd * N, device=DEV), float("inf")
+        for _ in range(6):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            for _ in range(4):
+                y = ops.ssd_scan(xs, dt, *vecs, state, i32([0, n]), i32([0]), Hs, 1, Pd, N, pieces=pieces, piece_tokens=64)
+            end.record()
+            torch.cuda.synchronize()
+            best = min(best, start.elapsed_time(end))
+        times.append(best)
+    assert bool(torch.isnan(y).all()) and times[1] < 8 * times[0], times
+
+
 def test_state_space_chunks_of_heads_that_keep_nothing():
     """Rates whose product with a step size overflows (a decay of 0), beside ordinary heads, one that forgets nothing and steps so wide that an
     ordinary head keeps nothing either: in chunks what the scan gives."""
