@@ -250,7 +250,8 @@ def test_state_space_scan_whole_in_pieces_and_token_by_token_with_slow_decay(Hs,
     (32, 1, 64, 128, (129, 2)), (32, 1, 64, 128, (700, 300)), (32, 2, 64, 64, (1024, 1030)),
 ])
 def test_state_space_scan_in_chunks(Hs, G, Pd, N, lens):
-    """Pieces of up to 64 tokens as matrix products: no further from the recurrence than its scan, and the scan's state; an
+    """Pieces of up to 64 tokens as matrix products: no further from the recurrence in 64 bits than its scan is, with decays of
+    some per cent a token and of some a chunk (the scan rounds its state at every token: 1e-6 there, 1e-7 here); an
     infinity stays out of earlier tokens, of other heads and of other columns."""
     from lgml_b200 import ops
 
@@ -270,10 +271,25 @@ def test_state_space_scan_in_chunks(Hs, G, Pd, N, lens):
         y = ops.ssd_scan(x[:, :C], dt, vecs[0], vecs[1], vecs[2], state, starts, i32([3, 1]), Hs, G, Pd, N, **how)
         return y, state
 
-    y, state = run(dict(pieces=pieces, piece_tokens=64), x)
-    want, want_state = run({}, x)
-    # K products of float32 operands, each sum once more rounded for the decays it went through
-    assert float((y - want).abs().max()) < 1e-5 * (1 + float(want.abs().max())) and float((state - want_state).abs().max()) < 1e-5 * (1 + float(want_state.abs().max()))
+    def exact():
+        v = [t.double() for t in (x[:, :C], dt, *vecs)]
+        S, rows = state0[[3, 1], :inner * N].double().view(2, Hs, Pd, N), []
+        for r, length in enumerate(lens):
+            for t in range(sum(lens[:r]), sum(lens[:r]) + length):
+                d = torch.nn.functional.softplus(v[1][t] + v[2], threshold=1e9)
+                xt = v[0][t, :inner].view(Hs, Pd)
+                B, Ct = (v[0][t, lo:lo + G * N].view(G, N).repeat_interleave(Hs // G, 0) for lo in (inner, inner + G * N))
+                S[r] = torch.exp(-torch.exp(v[3]) * d)[:, None, None] * S[r] + (d[:, None] * xt)[:, :, None] * B[:, None]
+                rows.append(((S[r] * Ct[:, None]).sum(2) + v[4][:, None] * xt).view(-1))
+        return torch.stack(rows), S.view(2, -1)
+
+    for slower in (0.0, 5.0):
+        vecs[1] = vecs[1] - slower
+        y, state = run(dict(pieces=pieces, piece_tokens=64), x)
+        want, want_state = run({}, x)
+        for got, scanned, true in zip((y, state[[3, 1], :inner * N]), (want, want_state[[3, 1], :inner * N]), exact()):
+            off, scan_off = (float((t.double() - true).norm() / true.norm()) for t in (got, scanned))
+            assert off <= max(scan_off, 3e-7), (slower, off, scan_off)         # (3e-7: five roundings, where short portions hardly show one)
     at = lens[0] // 2
     x[at, Pd - 1] = float("inf")                                    # an x of the first head's last column
     x[at, inner] = float("nan") if G > 1 else x[at, inner]          # a B of the first group
