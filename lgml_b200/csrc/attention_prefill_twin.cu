@@ -470,7 +470,8 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_attention_twin_kernel(
                 }
             }
             // (four chains each: the order of a maximum or of these float32 partial sums is a
-            //  function of the column only, so a row's result does not depend on the batch)
+            //  function of the column only, so with its pages in as many ranges a row's result does not
+            //  depend on the batch; how many ranges there are, the caller's plan decides by the step's tiles)
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
             if (edge) {
 #pragma unroll

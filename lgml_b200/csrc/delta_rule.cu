@@ -17,7 +17,8 @@
 // the chunked form in chunk_scan.cu instead.
 //
 // Four kernels a step:
-//   delta_prepare      one block per token, all tokens at once: convolution (the inputs before a
+//   delta_prepare      all tokens at once, a block per eight tokens of a q or k head or of 128 channels (a block per
+//                      token for more than four taps or heads over 128): convolution (the inputs before a
 //                      portion's first token come from the slot), SiLU, norms, beta, decay (beta
 //                      rides behind each head's decays, so the scan copies both as one row)
 //   delta_conv_state   per request: the slot's last taps - 1 inputs after this step

@@ -2745,6 +2745,10 @@ def prefill_twin_ranges(batch, tiles: torch.Tensor, ctas: int, window: int, keep
     no longer fit side by side it loses (128 of 8 pages: 14.9 against 26.9 in 2), and counts from five that are no powers
     of two are up to 3 us slower than the power below them.
 
+    So a row's probabilities are rounded to bfloat16 against the maximum of as many ranges as the step's other tiles leave SMs for: its
+    result is as close to 64 bits as in one range (within 2 %), but its last bits depend on the batch, as those of decode attention and of products
+    cut along K do.
+
     A captured portion is replayed for contexts of over half its reach, up to all of it."""
     longest = batch.max_kv_len
     if batch.replayed:

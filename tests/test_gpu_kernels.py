@@ -767,6 +767,43 @@ def test_prompt_attention_in_ranges_of_keys(H, G, D, window, keep, cap, n_ranges
         torch.testing.assert_close(outs[1], outs[0], atol=2.0 ** -8 * largest, rtol=2.0 ** -8)
 
 
+class PlannedBatch(FakeBatch):
+    """A step that plans its tiles as the engine's steps do."""
+
+    replayed, replay_reach = False, 0
+
+    def twin_tiles(self, tokens, ctas):
+        from lgml_b200.engine.batch import StepBatch
+
+        self.tile_tokens = StepBatch._half(self, ("halves", tokens, ctas))
+        return self.attention_tiles(self.tile_tokens)
+
+
+@pytest.mark.parametrize("H,G,D,kv_lens,q_lens,half,ranges", [
+    (32, 8, 128, [2085], [37], True, True), (8, 1, 64, [2304, 200], [64, 30], True, True), (16, 4, 128, [700], [60], True, True),
+    (16, 4, 128, [1500, 900], [500, 480], True, False), (8, 8, 64, [700, 300], [448, 300], True, True), (16, 4, 128, [1100] * 2, [1000] * 2, False, False),
+])
+def test_prompt_attention_as_planned(H, G, D, kv_lens, q_lens, half, ranges):
+    """``paged_attention`` with the tiles and ranges that a step's plan gives: as close to 64 bits as the same tokens in whole tiles and one range (each form
+    rounds its probabilities once, against a maximum of its own)."""
+    from lgml_b200 import ops
+    from lgml_b200.engine.batch import CacheView
+
+    case = make_attention_case(5, H, G, D, kv_lens=kv_lens, q_lens=q_lens, dtype=torch.bfloat16)
+    q, kp, vp, tab = (case[k].to(DEV) for k in ("q", "k_pages", "v_pages", "table"))
+    b, st, scale = PlannedBatch(case), status(), D ** -0.5
+    tiles, n_ranges = ops.prefill_twin_plan(b, H, G, 0)
+    assert (b.tile_tokens < ops.prefill_twin_tile_tokens(H, G)) == half and (n_ranges > 1) == ranges, (b.tile_tokens, n_ranges)
+    outs = [torch.full_like(q, float("nan")) for _ in range(3)]
+    ops.paged_attention(q, b, CacheView(k=kp, v=vp, block_table=tab), outs[0], H, scale, 0, st)
+    ops.prefill_attention_twin(q, b.positions, b.attention_tiles(ops.prefill_twin_tile_tokens(H, G)), tab, kp, vp, outs[1], H, scale, 0, st)
+    ops.prefill_attention_twin(q, b.positions, tiles, tab, kp, vp, outs[2], H, scale, 0, st)
+    want = ref_attention(case, scale, 0)
+    planned, whole = (float((o.double().cpu() - want).norm() / want.norm()) for o in outs[:2])
+    assert int(st.item()) == 0 and planned <= 1.02 * whole, (planned, whole)
+    assert torch.equal(outs[1], outs[2])            # (half tiles alone: the same bits)
+
+
 @pytest.mark.parametrize("H,G,D", ATT_SHAPES + [(2, 2, 256), (3, 1, 40)])
 @pytest.mark.parametrize("dtype,window", [(torch.float32, 0), (torch.float32, 37), (torch.bfloat16, 0)])
 def test_attention_ref_kernel(H, G, D, dtype, window):
