@@ -295,3 +295,29 @@ def test_keys_do_not_depend_on_the_kind_of_sequence():
     want = list(cm._keys(tokens, 40))
     assert len(set(want)) == 40
     assert list(cm._keys(tuple(tokens), 40)) == want and list(cm._keys([np.int64(t) for t in tokens], 40)) == want and list(cm._keys(np.array(tokens), 40)) == want
+
+
+def test_page_keys_of_every_sequence_come_from_c(monkeypatch):
+    """Tuples and arrays as lists: the same keys, formed in C; what is no integer is refused as before."""
+    import struct
+    from types import SimpleNamespace
+
+    import numpy as np
+    import torch
+
+    from lgml_b200 import host
+    from lgml_b200.cache import manager
+
+    calls, formed = [], host.page_keys
+    monkeypatch.setattr(manager.host, "page_keys", lambda *a: calls.append(a[2]) or formed(*a))
+    it, tokens = SimpleNamespace(page_size=64), [(7 * i * i) % 32000 for i in range(80 * 64)]
+    keys = lambda t, n=80: list(manager.CacheManager._keys(it, t, n))
+    want = keys(tokens)
+    assert len(want) == 80 and sum(calls) == 80
+    for other in (tuple(tokens), np.array(tokens), np.array(tokens, dtype=np.int32), torch.tensor(tokens)):
+        calls.clear()
+        assert keys(other) == want and sum(calls) == 80
+    for other in ([0.5] * 64, (0.5,) * 64, np.full(64, 0.5)):
+        with pytest.raises(struct.error):
+            keys(other, 1)
+
