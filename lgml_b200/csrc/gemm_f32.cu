@@ -13,7 +13,7 @@
 //   * gemm_f32_few_kernel, up to 32 rows (or more of few features): warps stream W, each its segments of K.
 //   * gemm_f32_many_kernel: tiles of 64 x 64.
 // K < 64: every output sums its products in the order k = 0, 1, 2, ..., one chain of FMAs.
-//   * gemm_f32_rows_kernel, up to 4 rows: a warp streams 8 or 16 rows of W through shared memory of its own.
+//   * gemm_f32_rows_kernel, one to four rows: a warp streams 8 or 16 rows of W through shared memory of its own.
 //   * gemm_f32_tile_kernel, more rows: tiles of A and W by asynchronous copies, several blocks an SM.
 //   * gemm_f32_ragged_kernel, more rows that do not all start on 16 bytes: tiles element by element.
 // One B200, weights from HBM, launched one behind the other, microseconds, one chain of FMAs an output and now:
@@ -690,8 +690,9 @@ template <bool VEC, typename TO> int run_rows(const Call &c) {
     return c.M <= 2 ? launch_rows<16, 1, VEC, TO>(c) : launch_rows<16, 2, VEC, TO>(c);
 }
 
-// Time of a product on tiles of bm x bn, in microseconds at K = 2048: an SM's first tile takes `alone`
-// (one block does not fill the FMA units), every further one `more`.
+// Time of a product on tiles of bm x bn, in microseconds at K = 2048, where the shapes were first compared: an SM's first tile takes `alone`
+// (one block does not fill the FMA units), every further one `more`.  For 5 to 2,000 rows of 512 to 32,000 features and K of 4 to 60 the shape that it says is
+// within 5 % of the best of the four on average, 27 % at worst; one shape for all sizes is 8 % (32 x 64) to 47 % (64 x 128) behind on average.
 float tiled_us(const Call &c, int bm, int bn, float alone, float more) {
     const long long tiles = (long long)((c.M + bm - 1) / bm) * ((c.N + bn - 1) / bn);
     return alone + (float)((tiles + 147) / 148 - 1) * more;
@@ -722,7 +723,8 @@ template <bool VEC, typename TO> int launch_many(const Call &c) {
 // takes 12.5; an SM's first tile takes 70 (one warp a scheduler), every further one 53.
 template <bool VEC, typename TO> int run_split(const Call &c) {
     // Where there is one block an SM it has sixteen warps, else two blocks share the SM (4 rows, N x K, sixteen warps and eight:
-    // 2048 x 5632 10.2 and 13.2, 2048 x 2048 5.6 and 5.9, 3072 x 2048 9.6 and 7.3, 11264 x 2048 24.6 and 21.2).
+    // 2048 x 5632 12.3 and 15.5, 2048 x 2048 6.3 and 6.9, 3072 x 2048 11.2 and 9.3, 11264 x 2048 28.5 and 22.3; 16 rows 16.6 and 21.9, 7.3 and 8.7, 13.8
+    // and 12.7, 34.2 and 30.3).
     const bool one = c.N <= 148 * 16;
     if (c.M <= 8) return one ? launch_few<1, 4, 16, VEC, TO>(c) : launch_few<1, 4, 8, VEC, TO>(c);
     if (c.M <= 16) return one ? launch_few<2, 2, 16, VEC, TO>(c) : launch_few<2, 2, 8, VEC, TO>(c);
@@ -732,13 +734,13 @@ template <bool VEC, typename TO> int run_split(const Call &c) {
     return launch_many<VEC, TO>(c);
 }
 
-// A short K as chains of FMAs.  Five to sixteen rows: most of a stage of the rows kernel would be empty (N 4700, K 32: 3.3 to
-// 4.5 us, 64 x 64 tiles element by element 3.0 to 3.3), and so it is for rows element by element of a vocabulary's size (4 rows of
-// N 30000, K 31: 8.8 and 7.3).
+// A short K as chains of FMAs.  Tiles, but for one and two rows of K > 32 (two rows here and there: K 60, 512 features 1.3 and 2.1 us, 8,192 2.1 and 3.0,
+// 32,000 5.0 and 6.5; K 32, 2,048 features 1.8 and 1.6, 32,000 4.7 and 3.9; four rows, K 48: 2.2 and 1.9, 32,000 6.2 and 5.1).  Element by element the
+// tiles are slower (8 rows of 8,192 features, K 48: 6.8 us, in tiles of 16-byte copies 2.6), so rows that do not start on 16 bytes keep warps of their own up
+// to four, but not of a vocabulary's size (4 rows of N 30000, K 31: 8.8 and 7.3).
 template <bool VEC, typename TO> int run(const Call &c) {
     if (c.K >= SPLIT_FROM) return run_split<VEC, TO>(c);
-    if (c.M <= 4 && (VEC || c.N <= 148 * 128)) return run_rows<VEC, TO>(c);
-    if (VEC && c.M <= 16 && c.N <= 148 * 128) return launch_ragged<TO>(c);
+    if (VEC ? c.M <= 2 && c.K > 32 : c.M <= 4 && c.N <= 148 * 128) return run_rows<VEC, TO>(c);
     if constexpr (VEC) {
         const float t1 = tiled_us(c, 32, 32, 40.f, 19.6f), t2 = tiled_us(c, 32, 64, 58.f, 32.f), t3 = tiled_us(c, 64, 64, 90.f, 58.7f),
                     t4 = tiled_us(c, 64, 128, 148.f, 108.f);
