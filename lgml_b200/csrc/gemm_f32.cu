@@ -734,13 +734,14 @@ template <bool VEC, typename TO> int run_split(const Call &c) {
     return launch_many<VEC, TO>(c);
 }
 
-// A short K as chains of FMAs.  Tiles, but for one and two rows of K > 32 (two rows here and there: K 60, 512 features 1.3 and 2.1 us, 8,192 2.1 and 3.0,
+// A short K as chains of FMAs.  Tiles, but for one and two rows of K > 32, or four of up to 1,024 features (four rows of 512, K 60: 1.5 us, in tiles
+// 2.1; two rows here and there: K 60, 512 features 1.3 and 2.1 us, 8,192 2.1 and 3.0,
 // 32,000 5.0 and 6.5; K 32, 2,048 features 1.8 and 1.6, 32,000 4.7 and 3.9; four rows, K 48: 2.2 and 1.9, 32,000 6.2 and 5.1).  Element by element the
 // tiles are slower (8 rows of 8,192 features, K 48: 6.8 us, in tiles of 16-byte copies 2.6), so rows that do not start on 16 bytes keep warps of their own up
 // to four, but not of a vocabulary's size (4 rows of N 30000, K 31: 8.8 and 7.3).
 template <bool VEC, typename TO> int run(const Call &c) {
     if (c.K >= SPLIT_FROM) return run_split<VEC, TO>(c);
-    if (VEC ? c.M <= 2 && c.K > 32 : c.M <= 4 && c.N <= 148 * 128) return run_rows<VEC, TO>(c);
+    if (VEC ? c.K > 32 && c.M <= (c.N <= 1024 ? 4 : 2) : c.M <= 4 && c.N <= 148 * 128) return run_rows<VEC, TO>(c);
     if constexpr (VEC) {
         const float t1 = tiled_us(c, 32, 32, 40.f, 19.6f), t2 = tiled_us(c, 32, 64, 58.f, 32.f), t3 = tiled_us(c, 64, 64, 90.f, 58.7f),
                     t4 = tiled_us(c, 64, 128, 148.f, 108.f);

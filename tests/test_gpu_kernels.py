@@ -274,8 +274,8 @@ def test_gemm_f32_is_exact_and_batch_invariant(M, N, K):
     (4, 900, 31, 0), (8, 4739, 65, 0), (16, 40, 259, 0), (9, 9001, 257, 0), (12, 9500, 513, 0), (3, 19000, 65, 0), (7, 19000, 65, 0),
     # up to 16 rows of a short K
     (5, 130, 36, 0), (16, 4800, 60, 4), (8, 19000, 32, 0), (2, 66, 8, 0),
-    # where one and two rows have warps of their own: K 32 and one quad more, a third row
-    (2, 66, 32, 0), (2, 66, 36, 0), (3, 4800, 36, 0), (2, 4800, 60, 0), (1, 19000, 40, 0), (6, 19000, 60, 0),
+    # where one and two rows, or four of few features, have warps of their own: K 32 and one quad more, 1,024 features and more, a row more
+    (2, 66, 32, 0), (2, 66, 36, 0), (4, 1024, 36, 0), (4, 1028, 60, 0), (5, 512, 60, 0), (3, 4800, 36, 0), (2, 4800, 60, 0), (1, 19000, 40, 0), (6, 19000, 60, 0),
 ])
 def test_gemm_f32_same_bits_from_every_kernel(M, N, K, pad):
     """Every output is the sum over k = 0, 1, 2, ..., so a row has the same bits alone and among others, whatever kernel
