@@ -248,7 +248,8 @@ class ModelRunner:
         page = self.cache.page_size
         key = (prompt_graph_length(len(tokens), page), len(want))
         end = req.n_tokens + key[0]
-        if end > 512 and self.rt.dtype == torch.bfloat16:       # into how many ranges attention cuts the keys is recorded too
+        # into how many ranges attention cuts the keys is recorded too, where its kernel does (bfloat16, heads of 64 and 128)
+        if end > 512 and self.rt.dtype == torch.bfloat16 and any(g.spec.head_dim in (64, 128) for g in self.cache.groups):
             key += (1 << (end - 1).bit_length(),)
         g = self._prompt_graphs.get(key)
         if g is None:

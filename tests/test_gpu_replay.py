@@ -230,3 +230,21 @@ def test_short_portions_behind_long_contexts(tmp_path):
                 if r == rid:
                     err = (row.double() - ref[pos]).abs()
                     assert bool((err <= TOL["bfloat16"]["atol"] + TOL["bfloat16"]["rtol"] * ref[pos].abs()).all()), (rid, pos, float(err.max()))
+
+
+def test_short_portions_of_heads_that_are_never_cut_into_ranges(tmp_path):
+    """Heads of 32 in bfloat16: portions of one size have one captured step whatever the context, and its logits are the eager runner's."""
+    from lgml_b200.engine.engine import parse_dtype
+    from lgml_b200.engine.runner import ModelRunner
+
+    cfg = dict(H.TINY["A"][0], hidden_size=128, num_attention_heads=4, num_key_value_heads=2, head_dim=32, max_position_embeddings=2048)
+    folder = H.make_folder(tmp_path / "long", cfg, 3, dtype="bfloat16", sharpen=SHARPEN["bfloat16"])
+    ids, steps = H.random_ids(1216, cfg["vocab_size"], 23), []
+    for a, b in ((0, 64), (64, 576), (576, 640), (640, 1088), (1088, 1152), (1152, 1216)):
+        steps.append({"step": len(steps), "entries": [{"id": "x", "tokens": ids[a:b], "want": [b - a - 1]}], "end": []})
+    runner = make_runner(folder, "bfloat16", n_pages=20)
+    got = H.run_trace(runner, steps)
+    assert sorted(runner._prompt_graphs) == [(64, 1)]
+    plain = ModelRunner.from_folder(folder, parse_dtype("bfloat16"), "cuda:0", n_pages=20, max_slots=4, use_graphs=False)
+    want = H.run_trace(plain, steps)
+    assert all(torch.equal(got[k], want[k]) for k in want)
